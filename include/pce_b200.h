@@ -281,13 +281,19 @@ PCE_API size_t pce_csr_from_pairs_workspace_bytes(int32_t n_pairs, int32_t n_row
  * `weights` or `packed_weights` may be NULL when the kernel that needs it is not
  * the one chosen.  The CUDA-core kernel walks mask/rowptr/nbr; the tensor-core
  * kernel needs `tiles` (from pce_build_tile_lists) and runs only when both
- * `tiles` and `packed_weights` are given.  Results do not depend on the kernel's
+ * `tiles` and `packed_weights` are given; fp32 features with 128-row `tiles` and `weights` run on the tiled fp32
+ * kernel.  Results do not depend on the kernel's
  * processing order. */
 PCE_API int pce_conv_fwd(const void* in_feats, int32_t n_in, int32_t c_in, const void* weights,
                          const void* packed_weights, int32_t kv, int32_t c_out, const uint32_t* mask,
                          const int32_t* rowptr, const int32_t* nbr, const pce_tile_lists* tiles, int32_t n_out,
                          void* out_feats, int32_t dtype, const pce_epilogue* ep, int32_t kernel_choice,
                          void* stream);
+
+/* 1 when a layer of these widths is best computed from tile lists (on the tensor cores in fp16, by the tiled
+ * fp32 kernel in fp32), 0 when it had better walk mask / rowptr / nbr: what a caller builds for it.  (An fp32 layer
+ * of any widths runs from 128-row lists with slots = 1 when pce_conv_fwd is given some.) */
+PCE_API int32_t pce_conv_takes_lists(int32_t c_in, int32_t c_out, int32_t kv, int32_t dtype);
 
 /* Processing order for the tensor-core kernel: output rows sorted (stable radix sort) by
  * their indicator bitmask with the bits permuted by rarity, the rarest offset most

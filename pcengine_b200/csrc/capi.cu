@@ -5,6 +5,9 @@
 namespace pce {
 int conv_simt(const void* in, const void* w, const uint32_t* mask, const int* rowptr, const int* nbr, int n_out,
               int cin, int cout, int kv, void* out, int dtype, const pce_epilogue* ep, bool ident, cudaStream_t st);
+bool conv_f32_preferred(int cin, int cout);
+int conv_f32(const void* in, const void* w, const pce_tile_lists* tiles, int n_out, int cin, int cout, int kv, void* out,
+             const pce_epilogue* ep, cudaStream_t st);
 bool conv_umma_supported(int cin, int cout, int dtype);
 size_t umma_packed_bytes(int kv, int cin, int cout);
 int umma_pack_weights(const void* w, int kv, int cin, int cout, void* packed, cudaStream_t st);
@@ -132,6 +135,12 @@ size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in,
   return conv_split_scratch_bytes(n_rows, n_src, c_in, c_out, kv, sm_count);
 }
 
+int32_t pce_conv_takes_lists(int32_t c_in, int32_t c_out, int32_t kv, int32_t dtype) {
+  if (c_in < 1 || c_out < 1 || kv < 1 || kv > 128) return 0;
+  if (dtype == PCE_F32) return conv_f32_preferred(c_in, c_out) ? 1 : 0;
+  return conv_umma_supported(c_in, c_out, dtype) ? 1 : 0;
+}
+
 int pce_debug_timeout(int32_t* where4) {
   if (!where4) return PCE_ERR_INVALID;
   return umma_where_fetch(where4);
@@ -159,6 +168,9 @@ int pce_conv_fwd(const void* in_feats, int32_t n_in, int32_t c_in, const void* w
   if (ep && (ep->extra_feats || ep->push_slot[0] || ep->push_slot[1] || (ep->in_ld > 0 && ep->in_ld != c_in) ||
              (ep->out_ld > 0 && ep->out_ld != c_out)))
     return PCE_ERR_UNSUPPORTED;  // the second operand, the halo push and row pitches need the tensor-core kernel
+  if (dtype == PCE_F32 && weights && tiles && tiles->tile_ptr && tiles->stage_kp && tiles->stage_nbr && tiles->tile_rows == 128 &&
+      tiles->slots <= 1 && n_in > 0 && kernel_choice != PCE_KERNEL_SIMT)
+    return conv_f32(in_feats, weights, tiles, n_out, c_in, c_out, kv, out_feats, ep, st);
   if (!weights || !mask || !rowptr || (n_in > 0 && !nbr)) return PCE_ERR_INVALID;
   return conv_simt(in_feats, weights, mask, rowptr, nbr, n_out, c_in, c_out, kv, out_feats, dtype, ep, false, st);
 }
@@ -176,6 +188,8 @@ int pce_linear_fwd(const void* in_feats, int32_t n, int32_t c_in, const void* we
     return conv_umma(in_feats, n, packed_weights, 1, nullptr, n, c_in, c_out, out_feats, ep, st);
   if (!weights) return PCE_ERR_INVALID;
   if (ep && ((ep->in_ld > 0 && ep->in_ld != c_in) || (ep->out_ld > 0 && ep->out_ld != c_out))) return PCE_ERR_UNSUPPORTED;
+  if (dtype == PCE_F32 && conv_f32_preferred(c_in, c_out))
+    return conv_f32(in_feats, weights, nullptr, n, c_in, c_out, 1, out_feats, ep, st);
   return conv_simt(in_feats, weights, nullptr, nullptr, nullptr, n, c_in, c_out, 1, out_feats, dtype, ep, true, st);
 }
 

@@ -38,6 +38,19 @@ inline int cuda_fail(cudaError_t e) {
 
 inline int div_up(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 
+// Multiprocessors of the current device (looked up once per device), 0 on failure.
+inline int device_sm_count() {
+  static int count[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = __atomic_load_n(&count[dev], __ATOMIC_RELAXED);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    __atomic_store_n(&count[dev], n, __ATOMIC_RELAXED);
+  }
+  return n;
+}
+
 // Carves 256-byte aligned pieces out of the caller's workspace.
 struct Arena {
   char* base;

@@ -16,6 +16,9 @@ int conv_umma(const void* in, int n_in, const void* wpacked, int kv, const pce_t
 int conv_umma_kb64(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out, int cin,
                    int cout, void* out, const pce_epilogue* ep, cudaStream_t st);
 
+int conv_f32(const void* in, const void* w, const pce_tile_lists* tiles, int n_out, int cin, int cout, int kv, void* out,
+             const pce_epilogue* ep, cudaStream_t st);
+
 struct EpiDev {
   const float* scale;
   const float* shift;
@@ -221,17 +224,18 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
     k_d1_gather<T><<<div_up(static_cast<long long>(n_in) * 32, 256), 256, 0, st>>>(in_t, n_in, cin, qkpos, icsr, imap,
                                                                                     bin);
     PCE_LAUNCH_CHECK();
-    // The per-offset GEMM: tensor cores when packed weights are given and the scratch for the
-    // tile lists fits behind the two halves of the buffer, else CUDA cores.
+    // The per-offset GEMM: the tile-list kernels (tensor cores when packed weights are given, the tiled fp32 one)
+    // when the scratch for the lists fits behind the two halves of the buffer, else one thread group per row.
     const int n_tiles = qsum / 128;
     const size_t used = static_cast<size_t>(qsum) * (cin + cout) * sizeof(T);
     const size_t lists_at = (used + 255) & ~size_t(255);
     const size_t lists_bytes = sizeof(int) * (static_cast<size_t>(n_tiles) * 258 + 2);
-    const bool tc = wpacked != nullptr && conv_umma_supported(cin, cout, dtype) && qsum % 128 == 0 &&
-                    lists_at + lists_bytes <= buffer_bytes &&
+    const bool room = qsum % 128 == 0 && lists_at + lists_bytes <= buffer_bytes;
+    const bool f32 = dtype == PCE_F32 && room && w != nullptr && kv <= 256;  // (stage_kp keeps offsets in 8 bits)
+    const bool tc = wpacked != nullptr && conv_umma_supported(cin, cout, dtype) && room &&
                     ((reinterpret_cast<uintptr_t>(buffer) | reinterpret_cast<uintptr_t>(wpacked)) % 16 == 0) &&
                     (static_cast<size_t>(qsum) * cin * sizeof(T)) % 16 == 0;
-    if (tc) {
+    if (tc || f32) {
       int* base = reinterpret_cast<int*>(static_cast<char*>(buffer) + lists_at);
       int* order = base;
       int* stage_nbr = order + static_cast<size_t>(n_tiles) * 128;
@@ -241,7 +245,10 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
                                                                                                tile_ptr, stage_kp, stage_nbr);
       PCE_LAUNCH_CHECK();
       pce_tile_lists tl{order, tile_ptr, stage_kp, stage_nbr, 128, 0, 1, 0};
-      PCE_TRY(conv_umma(bin, qsum, wpacked, kv, &tl, qsum, cin, cout, bout, nullptr, st));
+      if (f32)
+        PCE_TRY(conv_f32(bin, w, &tl, qsum, cin, cout, 1, bout, nullptr, st));
+      else
+        PCE_TRY(conv_umma(bin, qsum, wpacked, kv, &tl, qsum, cin, cout, bout, nullptr, st));
     } else {
       if (w == nullptr) return PCE_ERR_INVALID;
       int need = (cout + 3) / 4, g = 1;
@@ -255,7 +262,7 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
     const T* centre = nullptr;
     if (centre_kp >= 0) {
       // the centre offset is a dense rows x matrix product: on the tensor-core kernel when the packed
-      // weights allow it (written into `out`, which the scatter then reads row by row and overwrites),
+      // weights allow it, on the tiled fp32 kernel in fp32 (written into `out`, which the scatter then reads row by row and overwrites),
       // else formed inside the scatter from W[centre]
       const int kblocks = (cin + 63) / 64;
       const bool tc_centre = wpacked != nullptr && conv_umma_supported(cin, cout, dtype) &&
@@ -264,6 +271,9 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
       if (tc_centre) {
         const __half* wp = static_cast<const __half*>(wpacked) + static_cast<size_t>(centre_kp) * kblocks * cout * 64;
         PCE_TRY(conv_umma_kb64(in, n_in, wp, 1, nullptr, n_out, cin, cout, out, nullptr, st));
+        centre = static_cast<const T*>(out);
+      } else if (dtype == PCE_F32 && w != nullptr) {
+        PCE_TRY(conv_f32(in, w_t + static_cast<size_t>(centre_kp) * cin * cout, nullptr, n_out, cin, cout, 1, out, nullptr, st));
         centre = static_cast<const T*>(out);
       } else {
         if (w == nullptr) return PCE_ERR_INVALID;

@@ -45,13 +45,14 @@ class NeighbourCSR:
     ``fill``: a callable returning (rowptr, nbr) for a CSR that arrives without them (a planned map
     whose tile lists were filled straight from the dense table); they are then built on first use."""
 
-    __slots__ = ("mask", "_rowptr", "_nbr", "n_rows", "n_src", "kv", "_order", "_tiles", "_fill", "_pairs")
+    __slots__ = ("mask", "_rowptr", "_nbr", "n_rows", "n_src", "kv", "_order", "_tiles", "_fp32", "_fill", "_pairs")
 
     def __init__(self, mask, rowptr, nbr, n_rows, n_src, kv=None, fill=None, pairs=None):
         self.mask, self._rowptr, self._nbr, self.n_rows, self.n_src = mask, rowptr, nbr, n_rows, n_src
         self.kv = kv
         self._order = None
         self._tiles = {}
+        self._fp32 = None
         self._fill = fill
         self._pairs = pairs  # callable -> one-element device tensor, for a CSR without rowptr
 
@@ -98,6 +99,14 @@ class NeighbourCSR:
             self._order = out
         return self._order
 
+    def lists_fp32(self):
+        """The lists of the tiled fp32 kernel (sorted rows, 128 per tile, one offset per stage), built on first use.
+        Kept apart from ``tiles``, which feed the tensor cores."""
+        hit = self._fp32
+        if hit is None:
+            hit = self._fp32 = self._build_tiles(True, 128, False, 1)
+        return hit[0]
+
     def tiles(self, sort_rows: bool = True, tile_rows: int | None = None, identity: bool = False, slots: int = 1):
         """The map as tile lists (a ``_lib.TileLists`` struct of device pointers) for the
         tensor-core kernel; built once per CSR, ordering, tile height and ``identity`` (every tile
@@ -115,6 +124,10 @@ class NeighbourCSR:
             if not hit[0].settled and (len(hit) < 6 or hit[5].query()):
                 hit[0].settled = 1
             return hit[0]
+        hit = self._tiles[key] = self._build_tiles(*key)
+        return hit[0]
+
+    def _build_tiles(self, sort_rows: bool, tile_rows: int, identity: bool, slots: int):
         dev = self.mask.device
         n_tiles = (self.n_rows + tile_rows - 1) // tile_rows
         if sort_rows:
@@ -136,8 +149,7 @@ class NeighbourCSR:
                             tile_rows, 1 if identity else 0, int(slots), 0)
         built = torch.cuda.Event()
         built.record(torch.cuda.current_stream(dev))
-        self._tiles[key] = (st, order, tile_ptr, stage_kp, stage_nbr, built)
-        return st
+        return (st, order, tile_ptr, stage_kp, stage_nbr, built)
 
 
 class KernelMap:

@@ -116,7 +116,8 @@ def _pair_counter(knnz, identity_rows: int):
 class PlannedKernelMap(KernelMap):
     """A :class:`KernelMap` whose arrays were produced by the planner."""
 
-    def __init__(self, out: _lib.PlannedMap, spec: dict, in_coords: torch.Tensor, cmin, keep, device):
+    def __init__(self, out: _lib.PlannedMap, spec: dict, in_coords: torch.Tensor, cmin, keep, device,
+                 fp32: bool = False):
         self.device = device
         self.ks, self.stride, self.pad = spec["ks"], spec["stride"], spec["pad"]
         self.subm = spec["subm"]
@@ -161,10 +162,13 @@ class PlannedKernelMap(KernelMap):
                 n_tiles = (csr.n_rows + t.tile_rows - 1) // t.tile_rows
                 csr._order = _DevArray(t.order, (csr.n_rows,), device, keep)
                 entries = n_tiles * ((kv + slots - 1) // slots + int(t.identity_stage)) * slots
-                csr._tiles[(True, int(t.tile_rows), bool(t.identity_stage), slots)] = (
-                    lists, csr._order, _DevArray(t.tile_ptr, (n_tiles + 1,), device, keep),
-                    _DevArray(t.stage_kp, (entries,), device, keep),
-                    _DevArray(t.stage_nbr, (entries * t.tile_rows,), device, keep))
+                hit = (lists, csr._order, _DevArray(t.tile_ptr, (n_tiles + 1,), device, keep),
+                       _DevArray(t.stage_kp, (entries,), device, keep),
+                       _DevArray(t.stage_nbr, (entries * t.tile_rows,), device, keep))
+                if fp32:
+                    csr._fp32 = hit
+                else:
+                    csr._tiles[(True, int(t.tile_rows), bool(t.identity_stage), slots)] = hit
             self._csr[transposed] = csr
 
 
@@ -193,7 +197,8 @@ class PlannedPass:
         if in_coords is None:
             in_coords = _DevArray(out.in_coords, (out.n_in, 4), self.device, self._handle).tensor()
             self.level_coords[spec["in_level"]] = in_coords
-        kmap = PlannedKernelMap(out, spec, in_coords, self.cmin, self._handle, self.device)
+        kmap = PlannedKernelMap(out, spec, in_coords, self.cmin, self._handle, self.device,
+                                self.plan.dtype == torch.float32)
         if not spec["subm"]:
             self.level_coords[spec["out_level"]] = kmap.out_coords
         input.kmaps[key] = kmap
@@ -250,7 +255,8 @@ class MapPlan:
 
     def _c_specs(self):
         arr = (_lib.PlanMapSpec * len(self.specs))()
-        tensor_cores = self.dtype == torch.float16
+        half = self.dtype == torch.float16
+        code = _lib.dtype_code(self.dtype)
         for s, c in zip(self.specs, arr):
             for d in range(3):
                 c.ks[d], c.stride[d], c.pad[d] = s["ks"][d], s["stride"][d], s["pad"][d]
@@ -258,9 +264,12 @@ class MapPlan:
             c.want_fwd, c.want_tr = (1 if s["fwd"] else 0), (1 if s["tr"] else 0)
             for name in ("fwd", "tr"):
                 dst_out, dst_in = (c.c_out_fwd, c.c_in_fwd) if name == "fwd" else (c.c_out_tr, c.c_in_tr)
-                widths = [u for u in s[name] if tensor_cores and u[0] <= 256]
+                # the uses that run on tile lists; in fp32 all of them on 128-row lists with one offset per stage
+                # (c_in = 0), which the map's size does not change
+                kv = s["ks"][0] * s["ks"][1] * s["ks"][2]
+                widths = [u for u in s[name] if lib.pce_conv_takes_lists(u[1], u[0], kv, code)]
                 for i, (w_out, w_in) in enumerate(widths):
-                    dst_out[i], dst_in[i] = w_out, (w_in if PF.PACK_OFFSETS else 0)
+                    dst_out[i], dst_in[i] = w_out, (w_in if PF.PACK_OFFSETS and half else 0)
         return arr
 
     def _handle_for(self, device) -> int:
