@@ -396,6 +396,13 @@ PCE_API int pce_linear_fwd(const void* in_feats, int32_t n, int32_t c_in, const 
 PCE_API int pce_scale_shift_act(const void* x, int64_t n, int32_t c, void* y, int32_t dtype,
                         const pce_epilogue* ep, void* stream);
 
+/* Eval-mode BatchNorm over feature rows in one pass: y = x * s + (beta - mean * s), s = gamma / sqrt(var + eps)
+ * (ref: script/batchnorm.py:7-11).  mean, var, gamma, beta: [c] in param_dtype on the device; gamma and beta may be
+ * NULL (1 and 0).  x and y 16-byte aligned and c <= 4096, else PCE_ERR_UNSUPPORTED (fold the constants and call
+ * pce_scale_shift_act). */
+PCE_API int pce_batchnorm(const void* x, int64_t n, int32_t c, void* y, int32_t dtype, const void* mean, const void* var,
+                          const void* gamma, const void* beta, int32_t param_dtype, float eps, void* stream);
+
 /* Copies rows rows[i] (rows == NULL: row i) of a row-major matrix into consecutive rows of dst, 16 bytes per
  * store.  dst may be a neighbouring GPU's memory mapped into this process (a peer pointer): the halo exchange
  * of a slab-parallel scene outside a convolution's epilogue (pce_epilogue.push_*): a rank stores its boundary

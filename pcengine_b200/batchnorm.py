@@ -1,5 +1,5 @@
 """``BatchNorm`` over the feature rows of an spTensor (script/batchnorm.py:7-11).
-In eval mode the normalisation is one fused scale/shift pass of the engine, and
+In eval mode the normalisation is one pass of the engine, constants included, and
 :func:`bn_scale_shift` exposes the folded constants so a convolution can apply
 them in its epilogue instead."""
 from __future__ import annotations
@@ -28,5 +28,8 @@ class BatchNorm(nn.BatchNorm1d):
     def forward(self, input: spTensor) -> spTensor:
         if self.training or not self.track_running_stats or not input.feats.is_cuda:
             return fapply(input, super().forward)
+        out = PF.batchnorm(input.feats, self)
+        if out is not None:
+            return input._like(out)
         scale, shift = bn_scale_shift(self)
         return fapply(input, PF.scale_shift_act, FusedEpilogue(scale=scale, shift=shift))

@@ -6,6 +6,8 @@
 // epilogue.  Weights are read through the read-only path and stay L1/L2
 // resident.  Role of the reference's CUDA-core fetch-on-demand kernels
 // (ref: backend/spconv.cuh:427-735,832-935,1162-1250) without their atomics.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace pce {
@@ -170,10 +172,100 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Per-channel affine (+ residual, activation) over a dense row-major matrix, taken as one long run of 16-byte pieces:
+// bound by memory alone (it moves each value in once and out once).  A block first puts the channels' scale and shift
+// into shared memory -- as given, or from the statistics and parameters of an eval-mode BatchNorm, which then needs no
+// kernels of its own to fold them -- and every thread takes kPieces pieces a grid apart, all loads in flight before the
+// first use.  The channel of a piece is carried along (one addition per step) instead of divided out.  240 k x 96 fp16:
+// 66 us with one element per thread and step, 17 us so.
+struct NormSrc {
+  const void* mean;
+  const void* var;
+  const void* gamma;  // may be nullptr
+  const void* beta;   // may be nullptr
+  float eps;
+  int half;  // the four are fp16 (else fp32)
+};
+
+__device__ __forceinline__ float param_at(const void* p, int half, int c) {
+  return half ? __half2float(static_cast<const __half*>(p)[c]) : static_cast<const float*>(p)[c];
+}
+
+// SPLIT: a piece may span rows (channel counts that are not a multiple of a piece).
+template <typename T, bool SPLIT>
+__global__ void __launch_bounds__(256) k_scale_shift_act(const T* __restrict__ x, long long total, int c, T* __restrict__ y, EpiDev ep,
+                                                         NormSrc norm, int staged) {
+  constexpr int kVec = 16 / static_cast<int>(sizeof(T));
+  constexpr int kPieces = 4;
+  extern __shared__ float affine[];  // [2][c] when staged
+  const float* scale = ep.scale;
+  const float* shift = ep.shift;
+  if (staged) {
+    for (int ch = threadIdx.x; ch < c; ch += blockDim.x) {
+      float s = 1.f, t = 0.f;
+      if (norm.mean) {
+        s = (norm.gamma ? param_at(norm.gamma, norm.half, ch) : 1.f) / sqrtf(param_at(norm.var, norm.half, ch) + norm.eps);
+        t = (norm.beta ? param_at(norm.beta, norm.half, ch) : 0.f) - param_at(norm.mean, norm.half, ch) * s;
+      } else {
+        if (ep.scale) s = ep.scale[ch];
+        if (ep.shift) t = ep.shift[ch];
+      }
+      affine[ch] = s;
+      affine[c + ch] = t;
+    }
+    __syncthreads();
+    scale = affine;
+    shift = affine + c;
+  }
+  const long long pieces = total / kVec;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long i0 = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  auto one = [&](float v, int ch, float r) {
+    if (scale) v *= scale[ch];
+    if (shift) v += shift[ch];
+    return apply_act(v + r, ep.act, ep.slope);
+  };
+  int ch = static_cast<int>(i0 * kVec % c);
+  const int step = static_cast<int>(stride * kVec % c);
+  for (long long i = i0; i < pieces; i += kPieces * stride) {
+    uint4 v[kPieces], r[kPieces];
+#pragma unroll
+    for (int q = 0; q < kPieces; ++q) {
+      const long long at = i + q * stride;
+      if (at < pieces) {
+        v[q] = *reinterpret_cast<const uint4*>(x + at * kVec);
+        if (ep.residual) r[q] = *reinterpret_cast<const uint4*>(static_cast<const T*>(ep.residual) + at * kVec);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kPieces; ++q) {
+      const long long at = i + q * stride;
+      if (at < pieces) {
+        const T* pv = reinterpret_cast<const T*>(&v[q]);
+        const T* pr = reinterpret_cast<const T*>(&r[q]);
+        alignas(16) T o[kVec];
+        int cc = ch;
+#pragma unroll
+        for (int u = 0; u < kVec; ++u) {
+          o[u] = from_f<T>(one(to_f(pv[u]), cc, ep.residual ? to_f(pr[u]) : 0.f));
+          ++cc;
+          if (SPLIT && cc == c) cc = 0;
+        }
+        *reinterpret_cast<uint4*>(y + at * kVec) = *reinterpret_cast<const uint4*>(o);
+      }
+      ch += step;
+      if (ch >= c) ch -= c;
+    }
+  }
+  const long long e = pieces * kVec + i0;  // the last, incomplete piece
+  if (e < total)
+    y[e] = from_f<T>(one(to_f(x[e]), static_cast<int>(e % c), ep.residual ? to_f(static_cast<const T*>(ep.residual)[e]) : 0.f));
+}
+
+// Matrices that do not start on a 16-byte boundary.
 template <typename T>
-__global__ void k_scale_shift_act(const T* __restrict__ x, long long n, int c, T* __restrict__ y, EpiDev ep) {
+__global__ void k_scale_shift_act_unaligned(const T* __restrict__ x, long long total, int c, T* __restrict__ y, EpiDev ep) {
   long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  long long total = n * c;
   for (; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
     int ch = static_cast<int>(i % c);
     float v = to_f(x[i]);
@@ -182,6 +274,32 @@ __global__ void k_scale_shift_act(const T* __restrict__ x, long long n, int c, T
     if (ep.residual) v += to_f(static_cast<const T*>(ep.residual)[i]);
     y[i] = from_f<T>(apply_act(v, ep.act, ep.slope));
   }
+}
+
+template <typename T>
+static int launch_affine(const void* x, long long total, int c, void* y, const EpiDev& e, const NormSrc& norm, cudaStream_t st) {
+  constexpr int kVec = 16 / static_cast<int>(sizeof(T));
+  const T* x_t = static_cast<const T*>(x);
+  T* y_t = static_cast<T*>(y);
+  const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(e.residual)) & 15) == 0;
+  if (!aligned) {
+    if (norm.mean) return PCE_ERR_UNSUPPORTED;
+    k_scale_shift_act_unaligned<T><<<static_cast<int>(std::min<long long>((total + 255) / 256, 148ll * 16)), 256, 0, st>>>(x_t, total, c, y_t, e);
+    PCE_LAUNCH_CHECK();
+    return PCE_OK;
+  }
+  const size_t smem = sizeof(float) * 2 * c;
+  const int staged = smem <= 32 * 1024 && (norm.mean || e.scale || e.shift) ? 1 : 0;
+  if (norm.mean && !staged) return PCE_ERR_UNSUPPORTED;
+  // enough blocks for every thread to have one round of pieces, at most eight resident per SM
+  const long long want = (total / kVec + 4 * 256 - 1) / (4 * 256);
+  const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(want, 148ll * 8)));
+  if (c % kVec)
+    k_scale_shift_act<T, true><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
+  else
+    k_scale_shift_act<T, false><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
+  PCE_LAUNCH_CHECK();
+  return PCE_OK;
 }
 
 template <typename T>
@@ -271,16 +389,26 @@ int pce_scale_shift_act(const void* x, int64_t n, int32_t c, void* y, int32_t dt
     return PCE_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   EpiDev e = to_dev(ep);
-  long long total = static_cast<long long>(n) * c;
-  int grid = static_cast<int>(std::min<long long>((total + 255) / 256, 148ll * 16));
-  if (dtype == PCE_F32)
-    k_scale_shift_act<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), n, c, static_cast<float*>(y), e);
-  else if (dtype == PCE_F16)
-    k_scale_shift_act<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x), n, c, static_cast<__half*>(y), e);
-  else
-    return PCE_ERR_UNSUPPORTED;
-  PCE_LAUNCH_CHECK();
-  return PCE_OK;
+  const long long total = static_cast<long long>(n) * c;
+  const NormSrc none{nullptr, nullptr, nullptr, nullptr, 0.f, 0};
+  if (dtype == PCE_F32) return launch_affine<float>(x, total, c, y, e, none, st);
+  if (dtype == PCE_F16) return launch_affine<__half>(x, total, c, y, e, none, st);
+  return PCE_ERR_UNSUPPORTED;
+}
+
+int pce_batchnorm(const void* x, int64_t n, int32_t c, void* y, int32_t dtype, const void* mean, const void* var,
+                  const void* gamma, const void* beta, int32_t param_dtype, float eps, void* stream) {
+  if (n < 0 || c < 1 || !mean || !var) return PCE_ERR_INVALID;
+  if (param_dtype != PCE_F32 && param_dtype != PCE_F16) return PCE_ERR_UNSUPPORTED;
+  if (n == 0) return PCE_OK;
+  if (!x || !y) return PCE_ERR_INVALID;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const EpiDev e{nullptr, nullptr, nullptr, PCE_ACT_NONE, 0.f};
+  const NormSrc norm{mean, var, gamma, beta, eps, param_dtype == PCE_F16 ? 1 : 0};
+  const long long total = static_cast<long long>(n) * c;
+  if (dtype == PCE_F32) return launch_affine<float>(x, total, c, y, e, norm, st);
+  if (dtype == PCE_F16) return launch_affine<__half>(x, total, c, y, e, norm, st);
+  return PCE_ERR_UNSUPPORTED;
 }
 
 }  // extern "C"

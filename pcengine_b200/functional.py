@@ -400,3 +400,23 @@ def scale_shift_act(feats: torch.Tensor, epilogue: FusedEpilogue) -> torch.Tenso
                                        _pack(epilogue, c, n, feats.dtype), _lib.stream_ptr(feats.device)),
                "pce_scale_shift_act")
     return out
+
+
+def batchnorm(feats: torch.Tensor, bn: torch.nn.BatchNorm1d) -> torch.Tensor:
+    """Eval-mode BatchNorm over feature rows, its constants folded inside the one kernel; None when the module's
+    tensors do not fit that kernel (mixed types, not on the device, more than 4096 channels)."""
+    params = (bn.running_mean, bn.running_var, bn.weight, bn.bias)
+    dtype = params[0].dtype
+    for p in params:
+        if p is not None and (p.dtype != dtype or not p.is_cuda or not p.is_contiguous()):
+            return None
+    if dtype not in (torch.float32, torch.float16) or feats.size(1) != params[0].numel() or params[0].numel() > 4096:
+        return None
+    feats = feats.contiguous()
+    if feats.data_ptr() % 16:
+        return None
+    out = torch.empty_like(feats)
+    _lib.check(lib.pce_batchnorm(feats.data_ptr(), feats.size(0), feats.size(1), out.data_ptr(), _lib.dtype_code(feats.dtype),
+                                 params[0].data_ptr(), params[1].data_ptr(), _lib.ptr(params[2]), _lib.ptr(params[3]),
+                                 _lib.dtype_code(dtype), float(bn.eps), _lib.stream_ptr(feats.device)), "pce_batchnorm")
+    return out
