@@ -174,6 +174,17 @@ PCE_API int pce_quantize_unique(const float* points, int32_t n, const float* vox
                                 void* workspace, size_t workspace_bytes, int32_t* out_coords,
                                 int32_t* out_index, int32_t* out_inverse, int32_t* n_unique_host,
                                 void* stream);
+/* The same in the types a host in PyTorch hands on: voxels int32 [<= n, 3], index and inverse int64 (optional). */
+PCE_API int pce_voxelise(const float* points, int32_t n, const float* voxel_host, void* workspace, size_t workspace_bytes,
+                         int32_t* out_voxels, int64_t* out_index, int64_t* out_inverse, int32_t* n_unique_host,
+                         void* stream);
+
+/* Coordinates of a batch (ref: script/utils.py:167-196 sparse_collate): the last three of the `width` int32 columns
+ * of every sample's rows, the sample's number in front; out_coords [sum of rows, 4].  coords and rows are host arrays
+ * of n_samples device pointers and counts, scratch 3 device ints.  SYNCHRONISES `stream` once to return the maximum
+ * of x, y, z in cmax_host[3]. */
+PCE_API int pce_collate_coords(const int32_t* const* coords, const int32_t* rows, int32_t n_samples, int32_t width,
+                               int32_t* out_coords, int32_t* scratch, int32_t* cmax_host, void* stream);
 
 /* ------------------------------------------------------------------ maps -- */
 

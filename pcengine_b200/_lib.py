@@ -26,7 +26,7 @@ EXPORTS = [
     "pce_map_build_d2", "pce_map_build_d2_noalloc", "pce_map_pairs", "pce_map_build_d1", "pce_csr_from_dense", "pce_csr_from_pairs",
     "pce_csr_from_pairs_workspace_bytes", "pce_csr_sort_rows", "pce_build_tile_lists", "pce_conv_kernel_choice", "pce_conv_takes_lists", "pce_conv_split_parts", "pce_conv_split_scratch_bytes", "pce_conv_fwd", "pce_packed_weights_bytes",
     "pce_pack_weights", "pce_device_status", "pce_debug_timeout", "pce_tune", "pce_conv_fwd_d1", "pce_linear_fwd", "pce_scale_shift_act", "pce_batchnorm", "pce_push_rows",
-    "pce_quantize_workspace_bytes", "pce_quantize_unique", "pce_tile_rows_for", "pce_plan_create", "pce_plan_destroy", "pce_plan_begin", "pce_pass_map", "pce_pass_release", "pce_net_run",
+    "pce_quantize_workspace_bytes", "pce_quantize_unique", "pce_voxelise", "pce_collate_coords", "pce_tile_rows_for", "pce_plan_create", "pce_plan_destroy", "pce_plan_begin", "pce_pass_map", "pce_pass_release", "pce_net_run",
 ]
 
 
@@ -135,6 +135,8 @@ def _load() -> C.CDLL:
     lib.pce_quantize_workspace_bytes.restype = sz
     lib.pce_quantize_workspace_bytes.argtypes = [i32]
     lib.pce_quantize_unique.argtypes = [vp, i32, C.POINTER(C.c_float), i32, vp, sz, vp, vp, vp, C.POINTER(i32), vp]
+    lib.pce_voxelise.argtypes = [vp, i32, C.POINTER(C.c_float), vp, sz, vp, vp, vp, C.POINTER(i32), vp]
+    lib.pce_collate_coords.argtypes = [C.POINTER(vp), C.POINTER(i32), i32, i32, vp, vp, C.POINTER(i32), vp]
     lib.pce_tile_rows_for.restype = i32
     lib.pce_tile_rows_for.argtypes = [i32, i32, i32, i32]
     lib.pce_plan_create.argtypes = [C.POINTER(PlanMapSpec), i32, C.POINTER(vp)]
