@@ -176,8 +176,7 @@ __global__ void __launch_bounds__(256)
 // bound by memory alone (it moves each value in once and out once).  A block first puts the channels' scale and shift
 // into shared memory -- as given, or from the statistics and parameters of an eval-mode BatchNorm, which then needs no
 // kernels of its own to fold them -- and every thread takes kPieces pieces a grid apart, all loads in flight before the
-// first use.  The channel of a piece is carried along (one addition per step) instead of divided out.  240 k x 96 fp16:
-// 66 us with one element per thread and step, 17 us so.
+// first use.  The channel of a piece is carried along (one addition per step) instead of divided out.
 struct NormSrc {
   const void* mean;
   const void* var;
@@ -191,13 +190,15 @@ __device__ __forceinline__ float param_at(const void* p, int half, int c) {
   return half ? __half2float(static_cast<const __half*>(p)[c]) : static_cast<const float*>(p)[c];
 }
 
-// SPLIT: a piece may span rows (channel counts that are not a multiple of a piece).
-template <typename T, bool SPLIT>
+// MODE 0: the grid's stride is a whole number of rows, so a thread meets the same channels in every piece and keeps
+// their constants in registers (read per piece, they are 32-byte-strided shared-memory reads that take as long as the
+// memory traffic); 1: pieces lie within a row; 2: a piece may span rows (widths that are no multiple of a piece).
+template <typename T, int MODE>
 __global__ void __launch_bounds__(256) k_scale_shift_act(const T* __restrict__ x, long long total, int c, T* __restrict__ y, EpiDev ep,
                                                          NormSrc norm, int staged) {
   constexpr int kVec = 16 / static_cast<int>(sizeof(T));
   constexpr int kPieces = 4;
-  extern __shared__ float affine[];  // [2][c] when staged
+  extern __shared__ __align__(16) float affine[];  // [2][c] when staged
   const float* scale = ep.scale;
   const float* shift = ep.shift;
   if (staged) {
@@ -226,6 +227,14 @@ __global__ void __launch_bounds__(256) k_scale_shift_act(const T* __restrict__ x
     return apply_act(v + r, ep.act, ep.slope);
   };
   int ch = static_cast<int>(i0 * kVec % c);
+  float s_mine[kVec], t_mine[kVec];
+  if (MODE == 0) {
+#pragma unroll
+    for (int u = 0; u < kVec; ++u) {
+      s_mine[u] = scale[ch + u];
+      t_mine[u] = shift[ch + u];
+    }
+  }
   const int step = static_cast<int>(stride * kVec % c);
   for (long long i = i0; i < pieces; i += kPieces * stride) {
     uint4 v[kPieces], r[kPieces];
@@ -244,17 +253,25 @@ __global__ void __launch_bounds__(256) k_scale_shift_act(const T* __restrict__ x
         const T* pv = reinterpret_cast<const T*>(&v[q]);
         const T* pr = reinterpret_cast<const T*>(&r[q]);
         alignas(16) T o[kVec];
-        int cc = ch;
+        if (MODE == 0) {
 #pragma unroll
-        for (int u = 0; u < kVec; ++u) {
-          o[u] = from_f<T>(one(to_f(pv[u]), cc, ep.residual ? to_f(pr[u]) : 0.f));
-          ++cc;
-          if (SPLIT && cc == c) cc = 0;
+          for (int u = 0; u < kVec; ++u)
+            o[u] = from_f<T>(apply_act(to_f(pv[u]) * s_mine[u] + t_mine[u] + (ep.residual ? to_f(pr[u]) : 0.f), ep.act, ep.slope));
+        } else {
+          int cc = ch;
+#pragma unroll
+          for (int u = 0; u < kVec; ++u) {
+            o[u] = from_f<T>(one(to_f(pv[u]), cc, ep.residual ? to_f(pr[u]) : 0.f));
+            ++cc;
+            if (MODE == 2 && cc == c) cc = 0;
+          }
         }
         *reinterpret_cast<uint4*>(y + at * kVec) = *reinterpret_cast<const uint4*>(o);
       }
-      ch += step;
-      if (ch >= c) ch -= c;
+      if (MODE != 0) {
+        ch += step;
+        if (ch >= c) ch -= c;
+      }
     }
   }
   const long long e = pieces * kVec + i0;  // the last, incomplete piece
@@ -293,11 +310,16 @@ static int launch_affine(const void* x, long long total, int c, void* y, const E
   if (norm.mean && !staged) return PCE_ERR_UNSUPPORTED;
   // enough blocks for every thread to have one round of pieces, at most eight resident per SM
   const long long want = (total / kVec + 4 * 256 - 1) / (4 * 256);
-  const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(want, 148ll * 8)));
+  int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(want, 148ll * 8)));
+  const int row_pieces = c / kVec;
+  int unit = row_pieces;  // blocks whose pieces make whole rows: row_pieces / gcd(row_pieces, 256)
+  while (unit > 0 && unit % 2 == 0 && row_pieces / unit < 256) unit /= 2;
   if (c % kVec)
-    k_scale_shift_act<T, true><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
+    k_scale_shift_act<T, 2><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
+  else if (staged && grid >= unit)
+    k_scale_shift_act<T, 0><<<grid / unit * unit, 256, smem, st>>>(x_t, total, c, y_t, e, norm, staged);
   else
-    k_scale_shift_act<T, false><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
+    k_scale_shift_act<T, 1><<<grid, 256, staged ? smem : 0, st>>>(x_t, total, c, y_t, e, norm, staged);
   PCE_LAUNCH_CHECK();
   return PCE_OK;
 }

@@ -90,10 +90,16 @@ __device__ __forceinline__ void sort_pass(cg::grid_group& grid, SortShared& sh, 
     const int d = tid & (kBins - 1), half = tid / kBins;
     const int g = static_cast<int>(gridDim.x), mid = (g + 1) / 2;
     int pre = 0, all = 0;
-    for (int b = half ? mid : 0; b < (half ? g : mid); ++b) {
-      const int c = __ldcg(hist + b * kBins + d);
-      all += c;
-      pre += b < static_cast<int>(blockIdx.x) ? c : 0;
+    // (batches of loads in flight: one after the other they were half of the pass)
+    for (int b0 = half ? mid : 0, end = half ? g : mid; b0 < end; b0 += 16) {
+      int c[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) c[u] = b0 + u < end ? __ldcg(hist + (b0 + u) * kBins + d) : 0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        all += c[u];
+        pre += b0 + u < static_cast<int>(blockIdx.x) ? c[u] : 0;
+      }
     }
     __shared__ int s_pre[kBins], s_all[kBins];
     if (half) {

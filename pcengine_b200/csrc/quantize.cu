@@ -6,6 +6,7 @@
 // float32 points against the Python-float voxel size), the voxels come out in ascending (x,y,z)
 // order (the order of the ravel hash), `index` names the FIRST point of every voxel (stable sort)
 // and `inverse` maps every point to its voxel.
+#include <algorithm>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -373,10 +374,17 @@ __global__ void __launch_bounds__(256) k_collate(const __grid_constant__ Collate
     m[1] = max(m[1], y);
     m[2] = max(m[2], z);
   }
+  __shared__ int s_max[8][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int v = __reduce_max_sync(0xFFFFFFFFu, m[d]);
-    if ((threadIdx.x & 31) == 0 && v > *reinterpret_cast<volatile int*>(cmax + d)) atomicMax(cmax + d, v);
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5][d] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {  // one update per block and axis
+    int v = s_max[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) v = max(v, s_max[w][threadIdx.x]);
+    atomicMax(cmax + threadIdx.x, v);
   }
 }
 }  // namespace pce
@@ -401,7 +409,7 @@ extern "C" int pce_collate_coords(const int32_t* const* coords, const int32_t* r
     }
     const int total = a.first[a.n_samples];
     if (total > 0) {
-      const int grid = div_up(total, 256) < 148 * 8 ? div_up(total, 256) : 148 * 8;
+      const int grid = std::min(div_up(total, 256), 148 * 4);
       k_collate<<<grid, 256, 0, st>>>(a, reinterpret_cast<int4*>(out_coords) + done, scratch);
       PCE_LAUNCH_CHECK();
     }
