@@ -237,6 +237,27 @@ PCE_API int pce_map_build_d2_noalloc(const int32_t* in_coords, int32_t n_in, con
                                      int32_t n_out, const pce_geom* g, int32_t* map, int32_t* knnz, int32_t* kpos,
                                      int32_t* qkpos, int32_t* map_out, int32_t* status, void* stream);
 
+/* A submanifold map with odd kernel sizes up to 5 in the form the convolutions read, without the dense table:
+ * mask[n * ceil(kv/32)] the offsets every row has (the centre included), nbr[starts[row] ..] the rows it finds there
+ * in ascending offset order, rows of a thread block together in no particular order of blocks (starts + nbr serve
+ * wherever rowptr + nbr do, except that rowptr[row + 1] is not the next start).  nbr needs room for kv * n entries.
+ * state [160] outlives the scratch: [0] PCE_ERR_RANGE / TABLE_FULL or 0, [32 + kp] the rows that have offset kp. */
+PCE_API size_t pce_subm_workspace_bytes(int32_t n);
+PCE_API int pce_subm_neighbours(const int32_t* coords, int32_t n, const pce_geom* g, void* workspace,
+                                size_t workspace_bytes, uint32_t* mask, int32_t* starts, int32_t* nbr, int32_t* state,
+                                void* stream);
+
+/* A down-sampling layer with kernel size == stride and no padding (every input has at most one output, its parent), at
+ * most 32 offsets: out_coords (room for n_in rows) as pce_downsample_coords gives them, up_mask[n_in] (the bit of the
+ * one offset that reaches the parent), up_nbr[n_in] (the parent's row or -1), child[kp * n_out + out] = in or -1 (room
+ * for kv * n_in entries; the map_out of pce_map_build_d2) and counts[32] pairs per offset.  SYNCHRONISES `stream` once
+ * to return *n_out_host.  PCE_ERR_TABLE_FULL: the cloud is too sparse for the block tables, use
+ * pce_downsample_coords. */
+PCE_API size_t pce_parents_workspace_bytes(int32_t n);
+PCE_API int pce_parents(const int32_t* in_coords, int32_t n_in, const pce_geom* g, void* workspace,
+                        size_t workspace_bytes, int32_t* out_coords, uint32_t* up_mask, int32_t* up_nbr,
+                        int32_t* child, int32_t* counts, int32_t* n_out_host, void* stream);
+
 /* Indicator -> pair lists ordered by (kp, in): the device form of
  * `nonzero(map != -1)`, `omap = map[idx]`, `imap = idx % n_in`
  * (ref: script/spconv.py:370-372).  Lists have room for pair_cap entries; the
@@ -326,6 +347,16 @@ PCE_API int pce_build_tile_lists(const uint32_t* mask, const int32_t* rowptr, co
                                  int32_t identity_stage, int32_t slots, void* workspace,
                                  size_t workspace_bytes, int32_t* tile_ptr, int32_t* stage_kp,
                                  int32_t* stage_nbr, int32_t stage_cap, void* stream);
+
+/* pce_csr_sort_rows and pce_build_tile_lists of up to four lists in ONE cooperative launch, for maps of at most 32
+ * offsets; same order and lists.  The neighbours come from nbr (row r's from starts[r] on, starts NULL: entry r) or
+ * from a dense table[kp * n + row], which then also gives the mask.  counts[kv] (may be NULL): rows that have each
+ * offset.  lists[v] names the arrays to fill (its `order` is ignored), stage_caps[v] their room in stages. */
+PCE_API size_t pce_order_workspace_bytes(int32_t n);
+PCE_API int pce_order_lists(uint32_t* mask, const int32_t* starts, const int32_t* nbr, const int32_t* table,
+                            const int32_t* counts, int32_t n, int32_t kv, int32_t* order,
+                            const pce_tile_lists* lists, const int32_t* stage_caps, int32_t n_lists,
+                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* Weight re-layout for the tensor-core kernel: per (offset, 64-channel K block) a
  * c_out x 128-byte K-major image with 16-byte chunks XOR-swizzled by the row index

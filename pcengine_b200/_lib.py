@@ -16,6 +16,8 @@ LIB_PATH = os.environ.get("PCE_B200_LIB") or os.path.join(_HERE, "libpce_b200.so
 
 PCE_OK = 0
 PCE_ERR_INVALID = 1
+PCE_ERR_TABLE_FULL = 5
+PCE_ERR_UNSUPPORTED = 6
 PCE_ERR_CAPACITY = 8
 PCE_F32, PCE_F16 = 0, 1
 ACT_NONE, ACT_RELU, ACT_LEAKY = 0, 1, 2
@@ -23,7 +25,8 @@ KERNEL_AUTO, KERNEL_SIMT, KERNEL_UMMA = 0, 1, 2
 
 EXPORTS = [
     "pce_strerror", "pce_version", "pce_last_cuda_error", "pce_kernel_launches", "pce_map_workspace_bytes", "pce_downsample_coords",
-    "pce_map_build_d2", "pce_map_build_d2_noalloc", "pce_map_pairs", "pce_map_build_d1", "pce_csr_from_dense", "pce_csr_from_pairs",
+    "pce_map_build_d2", "pce_map_build_d2_noalloc", "pce_map_pairs", "pce_subm_workspace_bytes", "pce_subm_neighbours", "pce_order_workspace_bytes", "pce_order_lists",
+    "pce_parents_workspace_bytes", "pce_parents", "pce_map_build_d1", "pce_csr_from_dense", "pce_csr_from_pairs",
     "pce_csr_from_pairs_workspace_bytes", "pce_csr_sort_rows", "pce_build_tile_lists", "pce_conv_kernel_choice", "pce_conv_takes_lists", "pce_conv_split_parts", "pce_conv_split_scratch_bytes", "pce_conv_fwd", "pce_packed_weights_bytes",
     "pce_pack_weights", "pce_device_status", "pce_debug_timeout", "pce_tune", "pce_conv_fwd_d1", "pce_linear_fwd", "pce_scale_shift_act", "pce_batchnorm", "pce_push_rows",
     "pce_quantize_workspace_bytes", "pce_quantize_unique", "pce_voxelise", "pce_collate_coords", "pce_tile_rows_for", "pce_plan_create", "pce_plan_destroy", "pce_plan_begin", "pce_pass_map", "pce_pass_release", "pce_net_run",
@@ -103,6 +106,12 @@ def _load() -> C.CDLL:
     lib.pce_downsample_coords.argtypes = [vp, i32, C.POINTER(Geom), vp, sz, vp, i32, C.POINTER(i32), vp]
     lib.pce_map_build_d2.argtypes = [vp, i32, vp, i32, C.POINTER(Geom), vp, sz, vp, vp, vp, vp, vp, vp, vp]
     lib.pce_map_build_d2_noalloc.argtypes = [vp, i32, vp, i32, C.POINTER(Geom), vp, vp, vp, vp, vp, vp, vp]
+    for name in ("pce_subm_workspace_bytes", "pce_order_workspace_bytes", "pce_parents_workspace_bytes"):
+        getattr(lib, name).restype = sz
+        getattr(lib, name).argtypes = [i32]
+    lib.pce_subm_neighbours.argtypes = [vp, i32, C.POINTER(Geom), vp, sz, vp, vp, vp, vp, vp]
+    lib.pce_order_lists.argtypes = [vp, vp, vp, vp, vp, i32, i32, vp, C.POINTER(TileLists), C.POINTER(i32), i32, vp, sz, vp]
+    lib.pce_parents.argtypes = [vp, i32, C.POINTER(Geom), vp, sz, vp, vp, vp, vp, vp, C.POINTER(i32), vp]
     lib.pce_map_pairs.argtypes = [vp, i32, i32, vp, sz, vp, vp, i32, vp]
     lib.pce_map_build_d1.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, sz, vp, vp, vp, vp, vp]
     lib.pce_csr_from_dense.argtypes = [vp, i32, i32, i32, i32, vp, sz, vp, vp, vp, i32, vp]

@@ -49,6 +49,37 @@ __device__ __forceinline__ int block_exclusive(int v, int* warp_sum, int& total)
   return before + incl - v;
 }
 
+// sh.base[d] = entries of lower digits + entries of digit d in earlier blocks, from hist [grid][kBins] (two threads per
+// digit, half the blocks each).
+__device__ __forceinline__ void block_offsets(SortShared& sh, const int* hist) {
+  __shared__ int s_pre[kBins], s_all[kBins];
+  const int tid = threadIdx.x;
+  const int d = tid & (kBins - 1), half = tid / kBins;
+  const int g = static_cast<int>(gridDim.x), mid = (g + 1) / 2;
+  int pre = 0, all = 0;
+  // (batches of loads in flight: one after the other they were half of the pass)
+  for (int b0 = half ? mid : 0, end = half ? g : mid; b0 < end; b0 += 16) {
+    int c[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) c[u] = b0 + u < end ? __ldcg(hist + (b0 + u) * kBins + d) : 0;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      all += c[u];
+      pre += b0 + u < static_cast<int>(blockIdx.x) ? c[u] : 0;
+    }
+  }
+  if (half) {
+    s_pre[d] = pre;
+    s_all[d] = all;
+  }
+  __syncthreads();
+  int total;
+  const int mine = half ? 0 : all + s_all[d];
+  const int lower = block_exclusive(mine, sh.warp_sum, total);
+  if (!half) sh.base[d] = lower + pre + s_pre[d];
+  __syncthreads();
+}
+
 // One pass over the chunk of this block: entry j of a thread is element (warp's first + 32 j + lane), so that warps and
 // then items and then lanes are in array order (stability).  `hist` is [grid][kBins].
 template <int ITEMS>
@@ -84,35 +115,7 @@ __device__ __forceinline__ void sort_pass(cg::grid_group& grid, SortShared& sh, 
     hist[blockIdx.x * kBins + tid] = run;
   }
   grid.sync();
-  // per digit: entries of lower digits + this digit's entries in earlier blocks (two threads per digit, half the
-  // blocks each)
-  {
-    const int d = tid & (kBins - 1), half = tid / kBins;
-    const int g = static_cast<int>(gridDim.x), mid = (g + 1) / 2;
-    int pre = 0, all = 0;
-    // (batches of loads in flight: one after the other they were half of the pass)
-    for (int b0 = half ? mid : 0, end = half ? g : mid; b0 < end; b0 += 16) {
-      int c[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) c[u] = b0 + u < end ? __ldcg(hist + (b0 + u) * kBins + d) : 0;
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        all += c[u];
-        pre += b0 + u < static_cast<int>(blockIdx.x) ? c[u] : 0;
-      }
-    }
-    __shared__ int s_pre[kBins], s_all[kBins];
-    if (half) {
-      s_pre[d] = pre;
-      s_all[d] = all;
-    }
-    __syncthreads();
-    int total;
-    const int mine = half ? 0 : all + s_all[d];
-    const int lower = block_exclusive(mine, sh.warp_sum, total);
-    if (!half) sh.base[d] = lower + pre + s_pre[d];
-    __syncthreads();
-  }
+  block_offsets(sh, hist);
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     if (first + 32 * j < n) {
@@ -136,6 +139,80 @@ __device__ __forceinline__ void load_chunk(int n, const unsigned long long* key_
     key[j] = i < n ? __ldcg(key_in + i) : 0ull;
     val[j] = i < n ? __ldcg(val_in + i) : 0;
   }
+}
+
+// The same pass for any number of entries: nothing stays in registers, a warp walks its stretch of the array twice
+// (count, scatter), four keys in flight.  load(i, key, value) gives entry i.
+template <typename K, typename Load>
+__device__ __forceinline__ void sort_pass_any(cg::grid_group& grid, SortShared& sh, int* hist, int n, int shift, Load load, K* key_out,
+                                              int* val_out) {
+  constexpr int kBatch = 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = static_cast<int>(gridDim.x);
+  const int per_warp = ((n + g * kWarps - 1) / (g * kWarps) + 31) & ~31;
+  const long long lo64 = static_cast<long long>(blockIdx.x * kWarps + warp) * per_warp;
+  const int lo = static_cast<int>(lo64 < n ? lo64 : n), hi = static_cast<int>(lo64 + per_warp < n ? lo64 + per_warp : n);
+  for (int i = tid; i < kWarps * kBins; i += kThreads) (&sh.count[0][0])[i] = 0;
+  __syncthreads();
+  for (int b = lo; b < hi; b += 32 * kBatch) {
+    K key[kBatch];
+    int val;
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      key[u] = 0;
+      if (b + 32 * u + lane < hi) load(b + 32 * u + lane, key[u], val);
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (b + 32 * u >= hi) break;
+      const bool live = b + 32 * u + lane < hi;
+      const int d = live ? static_cast<int>((key[u] >> shift) & (kBins - 1)) : kBins + lane;
+      const unsigned same = __match_any_sync(0xFFFFFFFFu, d);
+      if (live && (same & ((1u << lane) - 1u)) == 0) sh.count[warp][d] += __popc(same);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  if (tid < kBins) {
+    int run = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const int c = sh.count[w][tid];
+      sh.count[w][tid] = run;
+      run += c;
+    }
+    hist[blockIdx.x * kBins + tid] = run;
+  }
+  grid.sync();
+  block_offsets(sh, hist);
+  for (int b = lo; b < hi; b += 32 * kBatch) {
+    K key[kBatch];
+    int val[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      key[u] = 0;
+      val[u] = 0;
+      if (b + 32 * u + lane < hi) load(b + 32 * u + lane, key[u], val[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (b + 32 * u >= hi) break;
+      const bool live = b + 32 * u + lane < hi;
+      const int d = live ? static_cast<int>((key[u] >> shift) & (kBins - 1)) : kBins + lane;
+      const unsigned same = __match_any_sync(0xFFFFFFFFu, d);
+      const unsigned before = same & ((1u << lane) - 1u);
+      const int old = live ? sh.count[warp][d] : 0;
+      __syncwarp();
+      if (live && before == 0) sh.count[warp][d] = old + __popc(same);
+      __syncwarp();
+      if (live) {
+        const int at = sh.base[d] + old + __popc(before);
+        key_out[at] = key[u];
+        val_out[at] = val[u];
+      }
+    }
+  }
+  grid.sync();
 }
 
 // Items per thread for n entries on a grid of at most one block per SM; 0: too many entries.

@@ -312,10 +312,11 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
         if rows == 128 and not pushes:
             split = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
     elif (kernel_choice == "auto" and feats.dtype == torch.float32
-          and (csr._fp32 is not None or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
+          and (csr._fp32 is not None or csr.wants_tiles()
+               or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
         tiles = C.byref(csr.lists_fp32())  # the tiled fp32 kernel (any widths, where a wider layer has left lists)
     # the tensor-core kernel reads the tile lists only: a planned map's rowptr / nbr are not built for its sake
-    rowptr, nbr = (csr._rowptr, csr._nbr) if tiles is not None else (csr.rowptr, csr.nbr)
+    rowptr, nbr = (csr._rowptr, csr._nbr) if tiles is not None else csr.row_lists()
     _lib.check(lib.pce_conv_fwd(feats.data_ptr(), feats.size(0), c_in, kernel.data_ptr(), _lib.ptr(packed), kv, c_out,
                                 csr.mask.data_ptr(), _lib.ptr(rowptr), _lib.ptr(nbr), tiles, csr.n_rows,
                                 out.data_ptr(), _lib.dtype_code(feats.dtype),

@@ -42,19 +42,30 @@ TILE_ROWS = 128
 class NeighbourCSR:
     """mask [rows, ceil(kv/32)] uint32 (as int32 storage), rowptr [rows+1], nbr [cap].
 
-    ``fill``: a callable returning (rowptr, nbr) for a CSR that arrives without them (a planned map
-    whose tile lists were filled straight from the dense table); they are then built on first use."""
+    What the convolutions read may be another form than rowptr / nbr, which are then built on first use by ``fill``, a
+    callable returning (rowptr, nbr):
 
-    __slots__ = ("mask", "_rowptr", "_nbr", "n_rows", "n_src", "kv", "_order", "_tiles", "_fp32", "_fill", "_pairs")
+    * ``lists`` (starts, nbr): a row's neighbours from nbr[starts[row]] on (starts None: entry ``row``), as
+      pce_subm_neighbours leaves them;
+    * ``table``: the dense [kv, rows] table of this direction (a map of at most 32 offsets); the mask then appears with
+      the row order, or with rowptr / nbr (``mask_ready`` False until then);
+    * neither: a planned map whose tile lists were filled by the planner.
 
-    def __init__(self, mask, rowptr, nbr, n_rows, n_src, kv=None, fill=None, pairs=None):
-        self.mask, self._rowptr, self._nbr, self.n_rows, self.n_src = mask, rowptr, nbr, n_rows, n_src
+    ``counts``: device int32 [kv], rows that have each offset."""
+
+    __slots__ = ("_mask", "_rowptr", "_nbr", "n_rows", "n_src", "kv", "_order", "_tiles", "_fp32", "_fill", "_pairs", "_lists",
+                 "_table", "_counts", "_mask_ready")
+
+    def __init__(self, mask, rowptr, nbr, n_rows, n_src, kv=None, fill=None, pairs=None, lists=None, table=None, counts=None,
+                 mask_ready=True):
+        self._mask, self._rowptr, self._nbr, self.n_rows, self.n_src = mask, rowptr, nbr, n_rows, n_src
         self.kv = kv
         self._order = None
         self._tiles = {}
         self._fp32 = None
         self._fill = fill
         self._pairs = pairs  # callable -> one-element device tensor, for a CSR without rowptr
+        self._lists, self._table, self._counts, self._mask_ready = lists, table, counts, mask_ready
 
     def pair_count(self) -> torch.Tensor:
         """Number of (row, offset) pairs as a NEW one-element device tensor (no read-back, and nothing that
@@ -66,7 +77,14 @@ class NeighbourCSR:
     def _materialise(self):
         if self._rowptr is None and self._fill is not None:
             self._rowptr, self._nbr = self._fill()
+            self._mask_ready = True  # (a fill that is given an empty mask writes it)
             self._fill = None
+
+    @property
+    def mask(self):
+        if not self._mask_ready:
+            self._materialise()
+        return self._mask
 
     @property
     def rowptr(self):
@@ -78,20 +96,35 @@ class NeighbourCSR:
         self._materialise()
         return self._nbr
 
+    def wants_tiles(self) -> bool:
+        """Whether tile lists are cheaper than rowptr / nbr here (a map between voxels and their parents)."""
+        return self._rowptr is None and (self._table is not None or (self._lists is not None and self._lists[0] is None))
+
+    def row_lists(self):
+        """(starts, nbr): every row's first neighbour and the neighbours, in whatever form is at hand."""
+        if self._rowptr is None and self._lists is not None and self._lists[0] is not None:
+            return self._lists
+        return self.rowptr, self.nbr
+
     def restrict(self, n_rows: int) -> "NeighbourCSR":
         """The CSR of the first ``n_rows`` output rows only (same inputs, shared storage): what a
         slab of a scene uses to compute its owned rows and not the halo's."""
         if not 0 <= n_rows <= self.n_rows:
             raise ValueError("restrict: n_rows out of range")
+        if self._rowptr is None and self._lists is not None and self._lists[0] is not None:
+            starts, nbr = self._lists
+            return NeighbourCSR(self.mask[:max(n_rows, 1)], None, None, n_rows, self.n_src, self.kv, lists=(starts[: max(n_rows, 1)], nbr),
+                                fill=lambda: (self.rowptr[: n_rows + 1], self.nbr),
+                                pairs=lambda: self.rowptr[n_rows: n_rows + 1].clone())
         return NeighbourCSR(self.mask[:max(n_rows, 1)], self.rowptr[: n_rows + 1], self.nbr, n_rows, self.n_src, self.kv)
 
     def order(self):
         """Output rows sorted by indicator bitmask (int32 [n_rows], built once): the order in which
         the tensor-core kernel forms its 128-row tiles."""
         if self._order is None and self.n_rows == 0:
-            self._order = torch.empty((0,), dtype=torch.int32, device=self.mask.device)
+            self._order = torch.empty((0,), dtype=torch.int32, device=self._mask.device)
         if self._order is None and self.kv is not None:
-            dev = self.mask.device
+            dev = self._mask.device
             out = torch.empty((self.n_rows,), dtype=torch.int32, device=dev)
             ws = _lib.workspace(64 * self.n_rows + (16 << 20), dev)
             _lib.check(lib.pce_csr_sort_rows(self.mask.data_ptr(), self.n_rows, self.kv, ws.data_ptr(), ws.numel(),
@@ -128,28 +161,114 @@ class NeighbourCSR:
         return hit[0]
 
     def _build_tiles(self, sort_rows: bool, tile_rows: int, identity: bool, slots: int):
-        dev = self.mask.device
+        dev = self._mask.device
         n_tiles = (self.n_rows + tile_rows - 1) // tile_rows
-        if sort_rows:
-            order = self.order()
-        else:
-            order = torch.arange(self.n_rows, dtype=torch.int32, device=dev)
         cap = max(1, n_tiles * ((self.kv + slots - 1) // slots + (1 if identity else 0)))
         tile_ptr = torch.empty((n_tiles + 1,), dtype=torch.int32, device=dev)
         stage_kp = torch.empty((cap * slots,), dtype=torch.int32, device=dev)
         stage_nbr = torch.empty((cap * slots * tile_rows,), dtype=torch.int32, device=dev)
-        ws = _lib.workspace(8 * (n_tiles + 1) + (1 << 20), dev)
-        _lib.check(lib.pce_build_tile_lists(self.mask.data_ptr(), self.rowptr.data_ptr(), self.nbr.data_ptr(),
-                                            order.data_ptr(), self.n_rows, self.kv, tile_rows, 1 if identity else 0, int(slots),
-                                            ws.data_ptr(),
-                                            ws.numel(),
-                                            tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(), cap,
-                                            _lib.stream_ptr(dev)), "pce_build_tile_lists")
+        if sort_rows and self._order is None and self.kv <= 32 and self.n_rows > 0:
+            order = self._order_and_lists(tile_rows, identity, slots, tile_ptr, stage_kp, stage_nbr, cap)
+        else:
+            order = self.order() if sort_rows else torch.arange(self.n_rows, dtype=torch.int32, device=dev)
+            starts, nbr = self.row_lists()
+            ws = _lib.workspace(8 * (n_tiles + 1) + (1 << 20), dev)
+            _lib.check(lib.pce_build_tile_lists(self.mask.data_ptr(), starts.data_ptr(), nbr.data_ptr(), order.data_ptr(),
+                                                self.n_rows, self.kv, tile_rows, 1 if identity else 0, int(slots), ws.data_ptr(),
+                                                ws.numel(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(), cap,
+                                                _lib.stream_ptr(dev)), "pce_build_tile_lists")
         st = _lib.TileLists(order.data_ptr(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(),
                             tile_rows, 1 if identity else 0, int(slots), 0)
         built = torch.cuda.Event()
         built.record(torch.cuda.current_stream(dev))
         return (st, order, tile_ptr, stage_kp, stage_nbr, built)
+
+    def _order_and_lists(self, tile_rows, identity, slots, tile_ptr, stage_kp, stage_nbr, cap):
+        """The row order (kept) and one set of lists in one launch, from the form at hand."""
+        dev = self._mask.device
+        order = torch.empty((self.n_rows,), dtype=torch.int32, device=dev)
+        starts = nbr = table = None
+        if self._rowptr is None and self._lists is not None:
+            starts, nbr = self._lists
+        elif self._rowptr is None and self._table is not None:
+            table = self._table
+        else:
+            starts, nbr = self.rowptr, self.nbr
+        want = _lib.TileLists(order.data_ptr(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(), tile_rows,
+                              1 if identity else 0, int(slots), 0)
+        caps = (C.c_int32 * 1)(cap)
+        ws = _lib.workspace(lib.pce_order_workspace_bytes(self.n_rows), dev)
+        _lib.check(lib.pce_order_lists(self._mask.data_ptr(), _lib.ptr(starts), _lib.ptr(nbr), _lib.ptr(table),
+                                       _lib.ptr(self._counts), self.n_rows, self.kv, order.data_ptr(), C.byref(want), caps, 1,
+                                       ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev)), "pce_order_lists")
+        self._order = order
+        if table is not None:
+            self._mask_ready = True
+        return order
+
+
+class _DenseTables:
+    """The dense map of a layer, map[kv][n_in] and (unless the map is its own transpose) map_out[kv][n_out], with its
+    per-offset counts: built on first use.  An object of its own, so that what derives from it later (a CSR's rowptr and
+    nbr) does not have to hold the KernelMap that holds the CSR."""
+
+    NAMES = ("map", "map_out", "knnz", "kpos", "qkpos", "status")
+
+    def __init__(self, in_coords, out_coords, geom, kv, mid, subm, symmetric):
+        self.in_coords, self.out_coords, self.geom, self.kv, self.mid = in_coords, out_coords, geom, kv, mid
+        self.subm, self.symmetric = subm, symmetric
+        self.n_in, self.n_out = int(in_coords.size(0)), int(out_coords.size(0))
+        self.built = False
+
+    def build(self) -> "_DenseTables":
+        """Hash the output coordinates, query every (input, offset) and scan the per-offset counts
+        (idempotent), on PyTorch's current stream."""
+        if self.built:
+            return self
+        dev, kv, in_coords = self.in_coords.device, self.kv, self.in_coords
+        st = _lib.stream_ptr(dev)
+        ws = _lib.workspace(lib.pce_map_workspace_bytes(self.n_in, kv, self.n_out), dev)
+        self.map = torch.empty((kv * self.n_in,), dtype=torch.int32, device=dev)
+        # A submanifold map with odd kernel sizes is its own transpose under kp -> kv-1-kp, so
+        # the output-major table is read out of `map`; otherwise it is written separately.
+        self.map_out = None if self.symmetric else torch.empty((kv * max(self.n_out, 1),), dtype=torch.int32, device=dev)
+        self.knnz = torch.empty((kv,), dtype=torch.int32, device=dev)
+        self.kpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
+        self.qkpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
+        self.status = torch.zeros((1,), dtype=torch.int32, device=dev)
+        _lib.check(lib.pce_map_build_d2(in_coords.data_ptr(), self.n_in, self.out_coords.data_ptr(), self.n_out,
+                                        C.byref(self.geom), ws.data_ptr(), ws.numel(), _lib.ptr(self.map),
+                                        self.knnz.data_ptr(), self.kpos.data_ptr(), self.qkpos.data_ptr(),
+                                        _lib.ptr(self.map_out), self.status.data_ptr(), st), "pce_map_build_d2")
+        self.built = True
+        return self
+
+    def csr(self, transposed: bool, pairs: Optional[int] = None):
+        """(mask, rowptr, nbr) of one direction; ``pairs``: their number, when known."""
+        self.build()
+        dev, kv = self.in_coords.device, self.kv
+        st = _lib.stream_ptr(dev)
+        ident = self.mid if self.subm else -1
+        if self.symmetric:
+            # the table read with kp reversed is the output-major one; under `transposed`
+            # (roles swapped) the table itself is.
+            table, n_rows, reverse = self.map, self.n_out, (0 if transposed else 1)
+        elif transposed:
+            table, n_rows, reverse = self.map, self.n_in, 0
+        else:
+            table, n_rows, reverse = self.map_out, self.n_out, 0
+        words = (kv + 31) // 32
+        cap = max(1, kv * min(self.n_in, self.n_out) if not self.subm else kv * self.n_in)
+        if pairs is not None:
+            cap = max(1, pairs + (self.n_in if self.subm else 0))
+        mask = torch.empty((max(n_rows, 1), words), dtype=torch.int32, device=dev)
+        rowptr = torch.empty((n_rows + 1,), dtype=torch.int32, device=dev)
+        nbr = torch.empty((cap,), dtype=torch.int32, device=dev)
+        ws = _lib.workspace(8 * (n_rows + 1) + (8 << 20), dev)
+        _lib.check(lib.pce_csr_from_dense(_lib.ptr(table), kv, n_rows, reverse, ident, ws.data_ptr(), ws.numel(),
+                                          mask.data_ptr(), rowptr.data_ptr(), nbr.data_ptr(), cap, st),
+                   "pce_csr_from_dense")
+        return mask, rowptr, nbr
 
 
 class KernelMap:
@@ -169,10 +288,14 @@ class KernelMap:
         self.geom = make_geom(ks, stride, pad, cmin, cmax_out, subm)
         st = _lib.stream_ptr(dev)
         kv = self.kv
+        # The block form (kmap_blocks.cu): submanifold maps with odd sizes up to 5, and layers whose outputs are the
+        # parents of their inputs; it leaves what the convolutions read, and the dense table is built when asked for.
+        self._blocks = bool(subm) and all(k % 2 == 1 and k <= 5 for k in ks) and 1 < kv <= 128
+        self._parents = None
         if subm:
             self.out_coords = in_coords
             self.n_out = self.n_in
-        else:
+        elif not self._build_parents(st):
             cap = max(1, self.n_in * candidates_per_input(ks, stride))
             ws = _lib.workspace(lib.pce_map_workspace_bytes(self.n_in, kv, cap), dev)
             oc = torch.empty((cap, 4), dtype=torch.int32, device=dev)
@@ -182,44 +305,62 @@ class KernelMap:
                        "pce_downsample_coords")
             self.n_out = int(n_out.value)
             self.out_coords = oc[: self.n_out]
-        self._built = False
         self._csr: dict = {}
         self._pairs = None
         self._d1 = None
         self._sizes = None
+        self._state = None
         self.dataflow = "D2"
         # A submanifold map with odd kernel sizes is its own transpose under kp -> kv-1-kp, so
         # the output-major table is read out of `map`; otherwise it is written separately.
         self.symmetric = self.subm and all(k % 2 == 1 for k in ks)
-        self.build()
+        self._dense = _DenseTables(in_coords, self.out_coords, self.geom, kv, self.mid, self.subm, self.symmetric)
+        if not self._blocks and self._parents is None:
+            self.build()
+
+    def __getattr__(self, name):
+        if name in _DenseTables.NAMES and "_dense" in self.__dict__:
+            return getattr(self._dense.build(), name)
+        raise AttributeError(name)
+
+    def _build_parents(self, st) -> bool:
+        """The map between the inputs and their parents (kernel size == stride, no padding): output coordinates and
+        both directions at once.  False when the layer, or a very sparse cloud, needs the general form."""
+        ks, dev, kv, n = self.ks, self.device, self.kv, self.n_in
+        if ks != self.stride or any(self.pad) or kv > 32 or n == 0:
+            return False
+        ws = _lib.workspace(lib.pce_parents_workspace_bytes(n), dev)
+        oc = torch.empty((n, 4), dtype=torch.int32, device=dev)
+        up_mask = torch.empty((n, 1), dtype=torch.int32, device=dev)
+        rows = torch.empty(((kv + 1) * n,), dtype=torch.int32, device=dev)
+        up_nbr, child = rows[:n], rows[n:]
+        counts = torch.empty((32,), dtype=torch.int32, device=dev)
+        n_out = C.c_int32(0)
+        status = lib.pce_parents(self.in_coords.data_ptr(), n, C.byref(self.geom), ws.data_ptr(), ws.numel(), oc.data_ptr(),
+                                 up_mask.data_ptr(), up_nbr.data_ptr(), child.data_ptr(), counts.data_ptr(), C.byref(n_out), st)
+        if status in (_lib.PCE_ERR_TABLE_FULL, _lib.PCE_ERR_UNSUPPORTED):
+            return False
+        _lib.check(status, "pce_parents")
+        self.n_out = int(n_out.value)
+        self.out_coords = oc[: self.n_out]
+        self._parents = (up_mask, up_nbr, child, counts)
+        return True
 
     def build(self) -> "KernelMap":
-        """Hash the output coordinates, query every (input, offset) and scan the per-offset counts
-        (idempotent), on PyTorch's current stream."""
-        if self._built:
-            return self
-        dev, kv, in_coords = self.device, self.kv, self.in_coords
-        st = _lib.stream_ptr(dev)
-        ws = _lib.workspace(lib.pce_map_workspace_bytes(self.n_in, kv, self.n_out), dev)
-        self.map = torch.empty((kv * self.n_in,), dtype=torch.int32, device=dev)
-        # A submanifold map with odd kernel sizes is its own transpose under kp -> kv-1-kp, so
-        # the output-major table is read out of `map`; otherwise it is written separately.
-        self.map_out = None if self.symmetric else torch.empty((kv * max(self.n_out, 1),), dtype=torch.int32, device=dev)
-        self.knnz = torch.empty((kv,), dtype=torch.int32, device=dev)
-        self.kpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
-        self.qkpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
-        self.status = torch.zeros((1,), dtype=torch.int32, device=dev)
-        _lib.check(lib.pce_map_build_d2(in_coords.data_ptr(), self.n_in, self.out_coords.data_ptr(), self.n_out,
-                                        C.byref(self.geom), ws.data_ptr(), ws.numel(), _lib.ptr(self.map),
-                                        self.knnz.data_ptr(), self.kpos.data_ptr(), self.qkpos.data_ptr(),
-                                        _lib.ptr(self.map_out), self.status.data_ptr(), st), "pce_map_build_d2")
-        self._built = True
+        """The dense tables (idempotent), on PyTorch's current stream."""
+        self._dense.build()
         return self
 
     # -- sizes that live on the device -------------------------------------
     def sizes(self):
         """(pairs, qsum) read back once (one synchronisation), also validates the status word.
         The reference reads qkpos[-1] the same way (script/spconv.py:376,421)."""
+        if self._sizes is None and self._state is not None and not self._dense.built:
+            state = self._state.cpu().tolist()  # rows per offset: a pair per row, the centre apart
+            if state[0] != 0:
+                _lib.check(state[0], "kernel map build")
+            pairs = [v for kp, v in enumerate(state[32: 32 + self.kv]) if kp != self.mid]
+            self._sizes = (sum(pairs), sum((v + 127) // 128 * 128 for v in pairs))
         if self._sizes is None:
             self.build()
             host = torch.stack([self.kpos[-1], self.qkpos[-1], self.status[0]]).cpu()
@@ -233,32 +374,49 @@ class KernelMap:
         key = bool(transposed)
         if key in self._csr:
             return self._csr[key]
-        self.build()
-        dev, kv = self.device, self.kv
-        st = _lib.stream_ptr(dev)
-        ident = self.mid if self.subm else -1
-        if self.symmetric:
-            # the table read with kp reversed is the output-major one; under `transposed`
-            # (roles swapped) the table itself is.
-            table, n_rows, n_src, reverse = self.map, self.n_out, self.n_in, (0 if transposed else 1)
-        elif transposed:
-            table, n_rows, n_src, reverse = self.map, self.n_in, self.n_out, 0
-        else:
-            table, n_rows, n_src, reverse = self.map_out, self.n_out, self.n_in, 0
-        words = (kv + 31) // 32
-        cap = max(1, kv * min(self.n_in, self.n_out) if not self.subm else kv * self.n_in)
-        if self._sizes is not None:
-            cap = max(1, self._sizes[0] + (self.n_in if self.subm else 0))
-        mask = torch.empty((max(n_rows, 1), words), dtype=torch.int32, device=dev)
-        rowptr = torch.empty((n_rows + 1,), dtype=torch.int32, device=dev)
-        nbr = torch.empty((cap,), dtype=torch.int32, device=dev)
-        ws = _lib.workspace(8 * (n_rows + 1) + (8 << 20), dev)
-        _lib.check(lib.pce_csr_from_dense(_lib.ptr(table), kv, n_rows, reverse, ident, ws.data_ptr(), ws.numel(),
-                                          mask.data_ptr(), rowptr.data_ptr(), nbr.data_ptr(), cap, st),
-                   "pce_csr_from_dense")
-        out = NeighbourCSR(mask, rowptr, nbr, n_rows, n_src, kv)
-        self._csr[key] = out
+        if self._blocks and not key and not self._dense.built:
+            self._csr[key] = self._csr_from_blocks()
+            return self._csr[key]
+        if self._parents is not None and not self._dense.built:
+            self._csr[key] = self._csr_of_parents(key)
+            return self._csr[key]
+        mask, rowptr, nbr = self._dense.csr(key, self._sizes[0] if self._sizes is not None else None)
+        n_rows, n_src = (self.n_in, self.n_out) if key else (self.n_out, self.n_in)
+        out = self._csr[key] = NeighbourCSR(mask, rowptr, nbr, n_rows, n_src, self.kv)
         return out
+
+    def _csr_from_blocks(self) -> NeighbourCSR:
+        dev, kv, n = self.device, self.kv, self.n_in
+        words = (kv + 31) // 32
+        mask = torch.empty((max(n, 1), words), dtype=torch.int32, device=dev)
+        starts = torch.empty((max(n, 1),), dtype=torch.int32, device=dev)
+        nbr = torch.empty((max(kv * n, 1),), dtype=torch.int32, device=dev)
+        state = torch.empty((160,), dtype=torch.int32, device=dev)
+        ws = _lib.workspace(lib.pce_subm_workspace_bytes(n), dev)
+        _lib.check(lib.pce_subm_neighbours(self.in_coords.data_ptr(), n, C.byref(self.geom), ws.data_ptr(), ws.numel(),
+                                           mask.data_ptr(), starts.data_ptr(), nbr.data_ptr(), state.data_ptr(),
+                                           _lib.stream_ptr(dev)), "pce_subm_neighbours")
+        self._state = state
+        counts, dense = state[32: 32 + kv], self._dense
+        return NeighbourCSR(mask, None, None, n, n, kv, fill=lambda: dense.csr(False)[1:], lists=(starts, nbr), counts=counts,
+                            pairs=lambda: counts.sum(0, keepdim=True, dtype=torch.int32))
+
+    def _csr_of_parents(self, transposed: bool) -> NeighbourCSR:
+        up_mask, up_nbr, child, counts = self._parents
+        pairs = lambda: counts.sum(0, keepdim=True, dtype=torch.int32)
+        dense = self._dense
+        if transposed:
+            return NeighbourCSR(up_mask, None, None, self.n_in, self.n_out, self.kv, fill=lambda: dense.csr(True)[1:],
+                                pairs=pairs, lists=(None, up_nbr),
+                                counts=counts)
+        mask = torch.empty((max(self.n_out, 1), 1), dtype=torch.int32, device=self.device)
+
+        def fill():
+            full, rowptr, nbr = dense.csr(False)
+            mask.copy_(full)
+            return rowptr, nbr
+        return NeighbourCSR(mask, None, None, self.n_out, self.n_in, self.kv, fill=fill, pairs=pairs, table=child, counts=counts,
+                            mask_ready=False)
 
     # -- reference forms -----------------------------------------------------
     def pairs(self):

@@ -22,7 +22,7 @@ import torch
 from . import _lib
 from . import functional as PF
 from ._lib import lib
-from .kmap import KernelMap, NeighbourCSR, make_geom
+from .kmap import KernelMap, NeighbourCSR, _DenseTables, make_geom
 from .spconv import _ONES, _triple
 from .utils import conv_info_decoder, conv_info_encoder, output_stride_compute
 
@@ -129,16 +129,18 @@ class PlannedKernelMap(KernelMap):
         self.geom = make_geom(ks, self.stride, self.pad, cmin, list(out.cmax_out), self.subm)
         self.out_coords = in_coords if self.subm else _DevArray(out.out_coords, (self.n_out, 4), device, keep).tensor()
         kv = self.kv
-        self.map = _DevArray(out.map, (kv * self.n_in,), device, keep)
         self.symmetric = bool(out.symmetric)
-        self.map_out = None if self.symmetric else _DevArray(out.map_out, (kv * max(self.n_out, 1),), device, keep)
-        self.knnz = _DevArray(out.knnz, (kv,), device, keep)
-        self.kpos = _DevArray(out.kpos, (kv + 1,), device, keep)
-        self.qkpos = _DevArray(out.qkpos, (kv + 1,), device, keep)
-        self.status = _DevArray(out.status, (1,), device, keep)
-        self._built = True
+        d = self._dense = _DenseTables(in_coords, self.out_coords, self.geom, kv, self.mid, self.subm, self.symmetric)
+        d.map = _DevArray(out.map, (kv * self.n_in,), device, keep)
+        d.map_out = None if self.symmetric else _DevArray(out.map_out, (kv * max(self.n_out, 1),), device, keep)
+        d.knnz = _DevArray(out.knnz, (kv,), device, keep)
+        d.kpos = _DevArray(out.kpos, (kv + 1,), device, keep)
+        d.qkpos = _DevArray(out.qkpos, (kv + 1,), device, keep)
+        d.status = _DevArray(out.status, (1,), device, keep)
+        d.built = True
         self._csr = {}
-        self._pairs = self._d1 = self._sizes = None
+        self._pairs = self._d1 = self._sizes = self._state = self._parents = None
+        self._blocks = False
         self.dataflow = "D2"
         for transposed, has, c in ((False, out.has_fwd, out.fwd), (True, out.has_tr, out.tr)):
             if not has:
