@@ -494,6 +494,12 @@ typedef struct pce_planned_csr {
   int32_t n_lists;
   const int32_t* table;  /* the dense table this direction reads (the map's `map` or `map_out`) */
   int32_t reverse_kp, identity_kp;
+  /* Maps made in block form (pce_planned_map.map == NULL): the row's neighbours as pce_subm_neighbours leaves them
+   * (starts NULL: one entry per row; row_nbr NULL: in `table`, the direction's own dense table) and counts[kv], the
+   * rows that have each offset; table is NULL where there is none. */
+  const int32_t* starts;
+  const int32_t* row_nbr;
+  const int32_t* counts;
   pce_tile_lists lists[PCE_PLAN_MAX_USES]; /* distinct (tile_rows, slots) among the uses; the
                                             * forward lists of a submanifold map carry the
                                             * identity stage */
@@ -504,6 +510,7 @@ typedef struct pce_planned_map {
   int32_t cmax_out[3];
   const int32_t* in_coords;  /* [n_in,4] */
   const int32_t* out_coords; /* [n_out,4]; == in_coords for a submanifold map */
+  /* NULL, with the five below, for a map made in block form: pce_map_build_d2 gives them on demand */
   const int32_t* map;        /* [kv*n_in] as pce_map_build_d2 */
   const int32_t* map_out;    /* [kv*n_out] or NULL when symmetric */
   const int32_t *knnz, *kpos, *qkpos, *status;

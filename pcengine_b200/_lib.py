@@ -58,6 +58,7 @@ class PlannedCSR(C.Structure):
     _fields_ = [("mask", C.c_void_p), ("rowptr", C.c_void_p), ("nbr", C.c_void_p), ("n_rows", C.c_int32),
                 ("n_src", C.c_int32), ("nbr_cap", C.c_int32), ("n_lists", C.c_int32),
                 ("table", C.c_void_p), ("reverse_kp", C.c_int32), ("identity_kp", C.c_int32),
+                ("starts", C.c_void_p), ("row_nbr", C.c_void_p), ("counts", C.c_void_p),
                 ("lists", TileLists * PLAN_MAX_USES)]
 
 

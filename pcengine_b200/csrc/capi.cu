@@ -48,7 +48,7 @@ const char* pce_strerror(int status) {
   }
 }
 
-int pce_version(void) { return 102; }  // 102: pce_planned_csr.table / reverse_kp / identity_kp, rowptr may be NULL
+int pce_version(void) { return 103; }  // 103: pce_planned_csr.starts / row_nbr / counts, pce_planned_map.map may be NULL
 
 int pce_last_cuda_error(void) { return g_last_cuda_error; }
 

@@ -18,11 +18,13 @@ namespace cg = cooperative_groups;
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kBins = 256;
 
+template <int BITS>
 struct SortShared {
+  static constexpr int kBins = 1 << BITS;  // 256 or 512
   int count[kWarps][kBins];  // per warp and digit: first the count, then the offset of the warp's first entry
   int base[kBins];           // where the block's entries of a digit go
+  int part[2][kThreads - kBins > 0 ? kBins : 1];
   int warp_sum[kWarps];
 };
 
@@ -49,13 +51,15 @@ __device__ __forceinline__ int block_exclusive(int v, int* warp_sum, int& total)
   return before + incl - v;
 }
 
-// sh.base[d] = entries of lower digits + entries of digit d in earlier blocks, from hist [grid][kBins] (two threads per
-// digit, half the blocks each).
-__device__ __forceinline__ void block_offsets(SortShared& sh, const int* hist) {
-  __shared__ int s_pre[kBins], s_all[kBins];
+// sh.base[d] = entries of lower digits + entries of digit d in earlier blocks, from hist [grid][bins] (256 bins: two
+// threads per digit, half the blocks each).
+template <int BITS>
+__device__ __forceinline__ void block_offsets(SortShared<BITS>& sh, const int* hist) {
+  constexpr int kBins = 1 << BITS, kHalves = kThreads / kBins;
+  static_assert(kHalves == 1 || kHalves == 2, "256 or 512 bins");
   const int tid = threadIdx.x;
   const int d = tid & (kBins - 1), half = tid / kBins;
-  const int g = static_cast<int>(gridDim.x), mid = (g + 1) / 2;
+  const int g = static_cast<int>(gridDim.x), mid = kHalves == 2 ? (g + 1) / 2 : g;
   int pre = 0, all = 0;
   // (batches of loads in flight: one after the other they were half of the pass)
   for (int b0 = half ? mid : 0, end = half ? g : mid; b0 < end; b0 += 16) {
@@ -68,24 +72,30 @@ __device__ __forceinline__ void block_offsets(SortShared& sh, const int* hist) {
       pre += b0 + u < static_cast<int>(blockIdx.x) ? c[u] : 0;
     }
   }
-  if (half) {
-    s_pre[d] = pre;
-    s_all[d] = all;
+  if (kHalves == 2) {
+    if (half) {
+      sh.part[0][d] = pre;
+      sh.part[1][d] = all;
+    }
+    __syncthreads();
+    if (!half) {
+      pre += sh.part[0][d];
+      all += sh.part[1][d];
+    }
   }
-  __syncthreads();
   int total;
-  const int mine = half ? 0 : all + s_all[d];
-  const int lower = block_exclusive(mine, sh.warp_sum, total);
-  if (!half) sh.base[d] = lower + pre + s_pre[d];
+  const int lower = block_exclusive(half ? 0 : all, sh.warp_sum, total);
+  if (!half) sh.base[d] = lower + pre;
   __syncthreads();
 }
 
 // One pass over the chunk of this block: entry j of a thread is element (warp's first + 32 j + lane), so that warps and
-// then items and then lanes are in array order (stability).  `hist` is [grid][kBins].
+// then items and then lanes are in array order (stability).  `hist` is [grid][256].
 template <int ITEMS>
-__device__ __forceinline__ void sort_pass(cg::grid_group& grid, SortShared& sh, int* hist, int n, int shift,
+__device__ __forceinline__ void sort_pass(cg::grid_group& grid, SortShared<8>& sh, int* hist, int n, int shift,
                                           const unsigned long long (&key)[ITEMS], const int (&val)[ITEMS],
                                           unsigned long long* key_out, int* val_out) {
+  constexpr int kBins = 256;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < kWarps * kBins; i += kThreads) (&sh.count[0][0])[i] = 0;
   __syncthreads();
@@ -143,10 +153,10 @@ __device__ __forceinline__ void load_chunk(int n, const unsigned long long* key_
 
 // The same pass for any number of entries: nothing stays in registers, a warp walks its stretch of the array twice
 // (count, scatter), four keys in flight.  load(i, key, value) gives entry i.
-template <typename K, typename Load>
-__device__ __forceinline__ void sort_pass_any(cg::grid_group& grid, SortShared& sh, int* hist, int n, int shift, Load load, K* key_out,
+template <int BITS, typename K, typename Load>
+__device__ __forceinline__ void sort_pass_any(cg::grid_group& grid, SortShared<BITS>& sh, int* hist, int n, int shift, Load load, K* key_out,
                                               int* val_out) {
-  constexpr int kBatch = 4;
+  constexpr int kBatch = 4, kBins = 1 << BITS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = static_cast<int>(gridDim.x);
   const int per_warp = ((n + g * kWarps - 1) / (g * kWarps) + 31) & ~31;

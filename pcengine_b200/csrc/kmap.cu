@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(512)
     return;
   }
   const int base = __ldg(tile_ptr + t);
-  int cursor = (!DENSE && row >= 0) ? __ldg(rowptr + row) : 0;
+  int cursor = (!DENSE && row >= 0) ? (rowptr ? __ldg(rowptr + row) : row) : 0;  // (no rowptr: one neighbour per row)
   int s = 0;
   for (int w = 0; w < words; ++w) {
     uint32_t m = tm[w];
@@ -914,6 +914,22 @@ static int tile_lists_impl(const uint32_t* mask, const int32_t* rowptr, const in
   else
     k_tile_lists<true><<<n_tiles, tile_rows, 0, st>>>(mask, rowptr, nbr, order, n_rows, words, identity_stage ? 1 : 0, slots,
                                                       nullptr, tile_ptr, stage_kp, stage_nbr, stage_cap);
+  PCE_LAUNCH_CHECK();
+  return PCE_OK;
+}
+
+// The stages of lists whose tile_ptr is known (kmap_blocks.cu), from neighbour lists or a dense table.
+int fill_tile_lists(const uint32_t* mask, const int32_t* starts, const int32_t* nbr, const int32_t* table, const int32_t* order,
+                    int32_t n_rows, int32_t kv, int32_t tile_rows, int32_t identity_stage, int32_t slots, const int32_t* tile_ptr,
+                    int32_t* stage_kp, int32_t* stage_nbr, int32_t stage_cap, cudaStream_t st) {
+  const int n_tiles = div_up(n_rows, tile_rows), words = (kv + 31) / 32;
+  const RowArgs dense{table, kv, n_rows, 0, -1, nullptr, nullptr, n_rows};
+  if (table)
+    k_tile_lists<true, true><<<n_tiles, tile_rows, 0, st>>>(mask, nullptr, nullptr, order, n_rows, words, identity_stage, slots, nullptr,
+                                                            tile_ptr, stage_kp, stage_nbr, stage_cap, dense);
+  else
+    k_tile_lists<true><<<n_tiles, tile_rows, 0, st>>>(mask, starts, nbr, order, n_rows, words, identity_stage, slots, nullptr, tile_ptr,
+                                                      stage_kp, stage_nbr, stage_cap);
   PCE_LAUNCH_CHECK();
   return PCE_OK;
 }
@@ -1174,7 +1190,8 @@ int pce_parents(const int32_t* in_coords, int32_t n_in, const pce_geom* g, void*
   PCE_TRY(blk::chain_place(c, n_in, &g, 1, false, workspace, workspace_bytes));
   c.coords_up = reinterpret_cast<int4*>(out_coords);
   host[0] = PCE_ERR_CUDA;
-  PCE_TRY(blk::chain_build(c, in_coords, n_in, host_dev, st));
+  PCE_TRY(blk::chain_tables(c, in_coords, n_in, st));
+  PCE_TRY(blk::chain_levels(c, host_dev, st));
   PCE_TRY(wait_for_stream(st));
   if (host[0] != PCE_OK) return host[0];
   const int n_out = host[3];

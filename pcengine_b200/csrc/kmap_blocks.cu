@@ -24,6 +24,11 @@
 #include "kmap_blocks.cuh"
 
 namespace pce {
+
+int fill_tile_lists(const uint32_t* mask, const int32_t* starts, const int32_t* nbr, const int32_t* table, const int32_t* order,
+                    int32_t n_rows, int32_t kv, int32_t tile_rows, int32_t identity_stage, int32_t slots, const int32_t* tile_ptr,
+                    int32_t* stage_kp, int32_t* stage_nbr, int32_t stage_cap, cudaStream_t st);
+
 namespace blk {
 
 // ---- the table --------------------------------------------------------------------------------------------
@@ -425,7 +430,7 @@ __global__ void __launch_bounds__(coop::kThreads)
                  int* hist, const __grid_constant__ Levels lv, const __grid_constant__ KeyFields kf, int key_cap, int4* coords,
                  int* perm, int* ctl, int* host) {
   using namespace coop;
-  __shared__ SortShared sh;
+  __shared__ SortShared<8> sh;
   cg::grid_group grid = cg::this_grid();
   const int status = __ldcg(ctl + kCtlStatus);
   const int n = __ldcg(ctl + kCtlRowsUp), top = __ldcg(ctl + kCtlMaxBatch);
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(coop::kThreads)
   for (int p = 0; p < passes; ++p) {
     const unsigned long long* kin = p & 1 ? key0 : key1;
     const int* vin = p & 1 ? val0 : val1;
-    sort_pass_any<unsigned long long>(
+    sort_pass_any<8, unsigned long long>(
         grid, sh, hist, n, 8 * p,
         [&](int i, unsigned long long& k, int& v) {
           if (p == 0) {
@@ -537,36 +542,258 @@ __global__ void __launch_bounds__(256) k_parents(const int4* __restrict__ coords
   if (threadIdx.x < kv && s_count[threadIdx.x]) atomicAdd(counts + threadIdx.x, s_count[threadIdx.x]);
 }
 
-// ---- row order and tile lists -----------------------------------------------------------------------------------
+// ---- row order and stages per tile ------------------------------------------------------------------------------
 
-struct Shared {
-  coop::SortShared sort;
-  int pos[32];                      // bit of offset k in the sort key
-  unsigned warp_mask[coop::kWarps];
+// The row order (rows sorted by bitmask, its bits permuted so that the rarest offset is the most significant one; stable)
+// and tile_ptr of up to four (tile height, identity stage, offsets per stage) of ONE direction of a map with at most 32
+// offsets; the stages themselves are then filled by k_tile_lists (kmap.cu) over the whole GPU.  Two kernels: maps of up
+// to 64 k rows are sorted by ONE cluster of eight blocks (keys in registers, digit counts and the scatter itself through
+// distributed shared memory: nothing waits for L2 or for a grid barrier), larger ones by a cooperative grid.  The
+// library's sort is four passes of 9-11 us, a histogram, a scan and a dozen memsets for the same order.
+constexpr int kOrderBits = 9;  // 27 offsets in three passes
+
+// Bit position in the sort key of every offset, from the number of rows that have it (lane = offset, warp-wide).
+__device__ __forceinline__ int key_bit(int mine, int lane, int kv) {
+  int rank = 0;  // rarer offsets (ties: lower ones) come first
+  for (int j = 0; j < kv; ++j) {
+    const int cj = __shfl_sync(0xFFFFFFFFu, mine, j);
+    rank += (cj < mine || (cj == mine && j < lane)) ? 1 : 0;
+  }
+  return lane < kv ? kv - 1 - rank : 0;
+}
+
+__device__ __forceinline__ unsigned mask_of_row(const Order& o, int i) {
+  if (!o.table) return __ldg(o.mask + i);
+  unsigned m = 0;
+  for (int k = 0; k < o.kv; ++k)
+    if (__ldg(o.table + static_cast<size_t>(k) * o.n + i) >= 0) m |= 1u << k;
+  return m;
+}
+
+__device__ __forceinline__ unsigned key_of_mask(unsigned m, const int* pos) {
+  unsigned key = 0;
+  for (; m; m &= m - 1u) key |= 1u << pos[__ffs(m) - 1];
+  return key;
+}
+
+// ---- up to 64 k rows: one cluster ----
+constexpr int kClusterBlocks = 8, kClusterThreads = 1024, kClusterWarps = 32, kClusterItems = 8;
+constexpr int kClusterRows = kClusterBlocks * kClusterThreads * kClusterItems;
+constexpr int kClusterBins = 1 << kOrderBits;
+
+struct ClusterShared {
+  unsigned key[kClusterThreads * kClusterItems];
+  int val[kClusterThreads * kClusterItems];
+  unsigned short count[kClusterWarps][kClusterBins];  // (a block has at most 8192 rows)
+  int total[kClusterBins];                             // read by the other blocks
+  int base[kClusterBins];
+  int half[2][kClusterBins];
+  unsigned group_mask[kClusterThreads * kClusterItems / 32];
+  int warp_sum[kClusterWarps];
+  int rows_with[32];                                   // read by the other blocks
+  int pos[32];
+  int stages[kMaxVariants];                            // read by the other blocks
+};
+
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClusterThreads) k_order_cluster(const __grid_constant__ Order o) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ClusterShared& sh = *reinterpret_cast<ClusterShared*>(smem_raw);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int me = static_cast<int>(cluster.block_rank());
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = o.n, kv = o.kv;
+  // rows per warp: a multiple of 32 as small as covers n, so that all blocks take part
+  const int items = (n + kClusterBlocks * kClusterThreads - 1) / (kClusterBlocks * kClusterThreads);
+  const int chunk = items * kClusterThreads;          // rows per block, a multiple of every tile height
+  const int local0 = warp * (32 * items) + lane;      // this thread's first row inside the block
+  const int row0 = me * chunk;
+  unsigned key[kClusterItems];
+  int val[kClusterItems];
+#pragma unroll
+  for (int j = 0; j < kClusterItems; ++j) {
+    const int i = row0 + local0 + 32 * j;
+    key[j] = 0u;
+    val[j] = i;
+    if (j < items && i < n) {
+      key[j] = mask_of_row(o, i);
+      if (o.table) o.mask[i] = key[j];
+    }
+  }
+  int mine = 0;
+  if (o.counts) {
+    if (warp == 0) mine = lane < kv ? __ldg(o.counts + lane) : 0;
+  } else {
+    if (tid < 32) sh.rows_with[tid] = 0;
+    __syncthreads();
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < kClusterItems; ++j) {
+      unsigned any = __reduce_or_sync(0xFFFFFFFFu, key[j]);
+      for (; any; any &= any - 1u) {
+        const int bit = __ffs(any) - 1;
+        const int rows = __popc(__ballot_sync(0xFFFFFFFFu, (key[j] >> bit) & 1u));
+        if (lane == bit) c += rows;
+      }
+    }
+    if (c) atomicAdd(&sh.rows_with[lane], c);
+    cluster.sync();
+    if (warp == 0)
+      for (int r = 0; r < kClusterBlocks; ++r) mine += cluster.map_shared_rank(sh.rows_with, r)[lane];
+  }
+  if (warp == 0) sh.pos[lane] = key_bit(mine, lane, kv);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kClusterItems; ++j) key[j] = key_of_mask(key[j], sh.pos);
+  const int passes = (kv + kOrderBits - 1) / kOrderBits;
+  for (int p = 0; p < passes; ++p) {
+    const int shift = p * kOrderBits;
+    for (int i = tid; i < kClusterWarps * kClusterBins / 2; i += kClusterThreads) reinterpret_cast<unsigned*>(&sh.count[0][0])[i] = 0u;
+    __syncthreads();
+    int rank[kClusterItems];
+#pragma unroll
+    for (int j = 0; j < kClusterItems; ++j) {
+      rank[j] = 0;
+      if (j < items) {
+        const bool live = row0 + local0 + 32 * j < n;
+        const int d = live ? static_cast<int>((key[j] >> shift) & (kClusterBins - 1)) : kClusterBins + lane;
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, d);
+        const unsigned before = same & ((1u << lane) - 1u);
+        const int old = live ? sh.count[warp][d] : 0;
+        __syncwarp();
+        if (live && before == 0) sh.count[warp][d] = static_cast<unsigned short>(old + __popc(same));
+        __syncwarp();
+        rank[j] = old + __popc(before);
+      }
+    }
+    __syncthreads();
+    {  // per digit: offsets of the warps (two threads per digit, half the warps each) and the block's total
+      const int d = tid & (kClusterBins - 1), h = tid / kClusterBins;
+      int sum = 0;
+#pragma unroll
+      for (int w = 0; w < kClusterWarps / 2; ++w) sum += sh.count[h * (kClusterWarps / 2) + w][d];
+      sh.half[h][d] = sum;
+      __syncthreads();
+      int run = h ? sh.half[0][d] : 0;
+#pragma unroll
+      for (int w = 0; w < kClusterWarps / 2; ++w) {
+        const int c = sh.count[h * (kClusterWarps / 2) + w][d];
+        sh.count[h * (kClusterWarps / 2) + w][d] = static_cast<unsigned short>(run);
+        run += c;
+      }
+      if (h) sh.total[d] = run;
+    }
+    cluster.sync();
+    {
+      int pre = 0, all = 0;
+      if (tid < kClusterBins) {
+#pragma unroll
+        for (int r = 0; r < kClusterBlocks; ++r) {
+          const int c = cluster.map_shared_rank(sh.total, r)[tid];
+          all += c;
+          pre += r < me ? c : 0;
+        }
+      }
+      int incl = all;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += u;
+      }
+      if (lane == 31) sh.warp_sum[warp] = incl;
+      __syncthreads();
+      int lower = incl - all;
+      for (int w = 0; w < warp; ++w) lower += sh.warp_sum[w];
+      if (tid < kClusterBins) sh.base[tid] = lower + pre;
+      __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < kClusterItems; ++j) {
+      if (j < items && row0 + local0 + 32 * j < n) {
+        const int d = static_cast<int>((key[j] >> shift) & (kClusterBins - 1));
+        const int at = sh.base[d] + sh.count[warp][d] + rank[j];
+        const int to = at / chunk, in = at - to * chunk;
+        cluster.map_shared_rank(sh.key, to)[in] = key[j];
+        cluster.map_shared_rank(sh.val, to)[in] = val[j];
+      }
+    }
+    cluster.sync();
+#pragma unroll
+    for (int j = 0; j < kClusterItems; ++j) {
+      const int i = local0 + 32 * j;
+      if (j < items && row0 + i < n) {
+        key[j] = sh.key[i];
+        val[j] = sh.val[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kClusterItems; ++j) {
+    const int i = local0 + 32 * j;
+    const bool live = j < items && row0 + i < n;
+    if (live) o.order[row0 + i] = val[j];
+    const unsigned m = __reduce_or_sync(0xFFFFFFFFu, live ? key[j] : 0u);
+    if (j < items && lane == 0) sh.group_mask[i / 32] = m;
+  }
+  __syncthreads();
+  // stages of the block's tiles: warp v counts variant v, two 128-row tiles per lane at most
+  int count[2] = {0, 0}, before = 0;
+  if (warp < o.n_variants) {
+    const Variant& V = o.variant[warp];
+    const int tiles = chunk / V.tile_rows, groups = V.tile_rows / 32;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = 2 * lane + u;
+      if (t < tiles && row0 + t * V.tile_rows < n) {
+        unsigned m = 0u;
+        for (int q = 0; q < groups; ++q) m |= sh.group_mask[t * groups + q];
+        count[u] = (__popc(m) + V.slots - 1) / V.slots + V.identity;
+      }
+    }
+    int incl = count[0] + count[1];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    before = incl - count[0] - count[1];
+    if (lane == 31) sh.stages[warp] = incl;
+  }
+  cluster.sync();
+  if (warp < o.n_variants) {
+    const Variant& V = o.variant[warp];
+    const int tiles = chunk / V.tile_rows;
+    int all = 0;
+    for (int r = 0; r < kClusterBlocks; ++r) {
+      const int c = cluster.map_shared_rank(sh.stages, r)[warp];
+      all += c;
+      before += r < me ? c : 0;
+    }
+    const int t0 = row0 / V.tile_rows + 2 * lane;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (2 * lane + u < tiles && row0 + (2 * lane + u) * V.tile_rows < n) V.tile_ptr[t0 + u] = before;
+      before += count[u];
+    }
+    if (me == 0 && lane == 0) V.tile_ptr[(n + V.tile_rows - 1) / V.tile_rows] = all;
+  }
+  cluster.sync();  // no block leaves while another reads its shared memory
+}
+
+// ---- more rows: a cooperative grid ----
+struct GridShared {
+  coop::SortShared<kOrderBits> sort;
+  int pos[32];
   int sums[kMaxVariants];
 };
 
-// Row order (rows sorted by bitmask, its bits permuted so that the rarest offset is the most significant one; stable)
-// and the tile lists of up to four (tile height, identity stage, offsets per stage) of ONE direction of a map with at
-// most 32 offsets, in one cooperative launch: the counterpart of k_row_mask_key32 / k_mask_keys32, the library's radix
-// sort, k_tile_lists<count>, the scan and k_tile_lists<fill> of kmap.cu, which are 8 to 20 launches of 2-10 us each.
-// The neighbours come from lists (starts + nbr; starts == nullptr: one per row) or from a dense table [kv][n].
-__global__ void __launch_bounds__(coop::kThreads) k_order_lists(const __grid_constant__ Order o) {
+__global__ void __launch_bounds__(coop::kThreads) k_order_grid(const __grid_constant__ Order o) {
   using namespace coop;
-  __shared__ Shared sh;
+  __shared__ GridShared sh;
   cg::grid_group grid = cg::this_grid();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = o.n, kv = o.kv;
   const int g = static_cast<int>(gridDim.x);
-  // how many rows have each offset: given, or counted here
-  if (o.table) {  // the bitmask of a direction that only has its dense table
-    for (int i = blockIdx.x * kThreads + tid; i < n; i += g * kThreads) {
-      unsigned m = 0;
-      for (int k = 0; k < kv; ++k)
-        if (__ldg(o.table + static_cast<size_t>(k) * n + i) >= 0) m |= 1u << k;
-      o.mask[i] = m;
-    }
-  }
-  if (o.table && !o.counts) __syncthreads();
+  if (o.table)
+    for (int i = blockIdx.x * kThreads + tid; i < n; i += g * kThreads) o.mask[i] = mask_of_row(o, i);
   if (!o.counts) {
     int mine = 0;
     for (int i0 = (blockIdx.x * kThreads + tid) & ~31; i0 < n; i0 += g * kThreads) {
@@ -594,65 +821,40 @@ __global__ void __launch_bounds__(coop::kThreads) k_order_lists(const __grid_con
         for (int b = 0; b < g; ++b) mine += __ldcg(o.block_counts + b * 32 + lane);
       }
     }
-    int rank = 0;  // rarer offsets (ties: lower ones) come first
-    for (int j = 0; j < kv; ++j) {
-      const int cj = __shfl_sync(0xFFFFFFFFu, mine, j);
-      rank += (cj < mine || (cj == mine && j < lane)) ? 1 : 0;
-    }
-    sh.pos[lane] = lane < kv ? kv - 1 - rank : 0;
+    sh.pos[lane] = key_bit(mine, lane, kv);
   }
+  if (tid < kMaxVariants) sh.sums[tid] = 0;
   __syncthreads();
-  const int passes = (kv + 7) / 8;
+  const int passes = (kv + kOrderBits - 1) / kOrderBits;
   for (int p = 0; p < passes; ++p) {
     const unsigned* kin = p & 1 ? o.key0 : o.key1;
     const int* vin = p & 1 ? o.val0 : o.val1;
-    unsigned* kout = p & 1 ? o.key1 : o.key0;
-    int* vout = p == passes - 1 ? o.order : (p & 1 ? o.val1 : o.val0);
-    sort_pass_any<unsigned>(
-        grid, sh.sort, o.hist, n, 8 * p,
+    sort_pass_any<kOrderBits, unsigned>(
+        grid, sh.sort, o.hist, n, kOrderBits * p,
         [&](int i, unsigned& k, int& v) {
           if (p == 0) {
-            unsigned key = 0;
-            for (unsigned m = __ldcg(o.mask + i); m; m &= m - 1u) key |= 1u << sh.pos[__ffs(m) - 1];
-            k = key;
+            k = key_of_mask(__ldcg(o.mask + i), sh.pos);
             v = i;
           } else {
             k = __ldcg(kin + i);
             v = __ldcg(vin + i);
           }
         },
-        kout, vout);
+        p & 1 ? o.key1 : o.key0, p == passes - 1 ? o.order : (p & 1 ? o.val1 : o.val0));
   }
-  // ---- stages per tile ----
-  auto tile_mask = [&](int t, int rows, int& row, unsigned& my) -> unsigned {  // for the thread group of tile t
-    const int r = tid % rows, slot = t * rows + r;
-    row = -1;
-    my = 0u;
-    if (slot < n) {
-      row = __ldcg(o.order + slot);
-      my = __ldcg(o.mask + row);
-    }
-    const unsigned m = __reduce_or_sync(0xFFFFFFFFu, my);
-    __syncthreads();
-    if (lane == 0) sh.warp_mask[warp] = m;
-    __syncthreads();
-    unsigned tm = 0u;
-    const int w0 = (tid / rows) * (rows / 32);
-    for (int w = 0; w < rows / 32; ++w) tm |= sh.warp_mask[w0 + w];
-    return tm;
-  };
-  if (tid < kMaxVariants) sh.sums[tid] = 0;
+  // stages per tile from the sorted keys (their bits are the masks' bits in another order)
+  const unsigned* sorted = passes & 1 ? o.key0 : o.key1;
   for (int v = 0; v < o.n_variants; ++v) {
     const Variant& V = o.variant[v];
-    const int rows = V.tile_rows, groups = kThreads / rows, n_tiles = (n + rows - 1) / rows;
+    const int rows = V.tile_rows, n_tiles = (n + rows - 1) / rows;
     const int per = (n_tiles + g - 1) / g, ta = min(n_tiles, static_cast<int>(blockIdx.x) * per), tb = min(n_tiles, ta + per);
-    for (int t0 = ta; t0 < tb; t0 += groups) {
-      const int t = t0 + tid / rows;
-      int row;
-      unsigned my;
-      const unsigned tm = tile_mask(t < tb ? t : n_tiles, rows, row, my);
-      if (t < tb && tid % rows == 0) {
-        const int stages = (__popc(tm) + V.slots - 1) / V.slots + V.identity;
+    for (int t = ta + warp; t < tb; t += kWarps) {  // a warp per tile
+      unsigned m = 0u;
+      for (int r = lane; r < rows; r += 32)
+        if (t * rows + r < n) m |= __ldcg(sorted + t * rows + r);
+      m = __reduce_or_sync(0xFFFFFFFFu, m);
+      if (lane == 0) {
+        const int stages = (__popc(m) + V.slots - 1) / V.slots + V.identity;
         V.tile_ptr[t] = stages;
         atomicAdd(&sh.sums[v], stages);
       }
@@ -661,77 +863,31 @@ __global__ void __launch_bounds__(coop::kThreads) k_order_lists(const __grid_con
   __syncthreads();
   if (tid < kMaxVariants) o.block_counts[blockIdx.x * 32 + tid] = sh.sums[tid];
   grid.sync();
-  // ---- lists ----
-  for (int v = 0; v < o.n_variants; ++v) {
-    const Variant& V = o.variant[v];
-    const int rows = V.tile_rows, groups = kThreads / rows, n_tiles = (n + rows - 1) / rows;
+  // first stage of every tile (this block's entries of tile_ptr still hold counts): warp v, variant v
+  if (warp < o.n_variants) {
+    const Variant& V = o.variant[warp];
+    const int n_tiles = (n + V.tile_rows - 1) / V.tile_rows;
     const int per = (n_tiles + g - 1) / g, ta = min(n_tiles, static_cast<int>(blockIdx.x) * per), tb = min(n_tiles, ta + per);
-    // first stage of the block's tiles, then of each of them (this block's entries of tile_ptr still hold counts)
-    if (warp == 0) {
-      int before = 0, all = 0;
-      for (int b = lane; b < g; b += 32) {
-        const int c = __ldcg(o.block_counts + b * 32 + v);
-        all += c;
-        before += b < static_cast<int>(blockIdx.x) ? c : 0;
-      }
-      before = __reduce_add_sync(0xFFFFFFFFu, before);
-      all = __reduce_add_sync(0xFFFFFFFFu, all);
-      for (int t0 = ta; t0 < tb; t0 += 32) {
-        const int c = t0 + lane < tb ? V.tile_ptr[t0 + lane] : 0;
-        int incl = c;
+    int before = 0, all = 0;
+    for (int b = lane; b < g; b += 32) {
+      const int c = __ldcg(o.block_counts + b * 32 + warp);
+      all += c;
+      before += b < static_cast<int>(blockIdx.x) ? c : 0;
+    }
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    all = __reduce_add_sync(0xFFFFFFFFu, all);
+    for (int t0 = ta; t0 < tb; t0 += 32) {
+      const int c = t0 + lane < tb ? V.tile_ptr[t0 + lane] : 0;
+      int incl = c;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-          if (lane >= d) incl += u;
-        }
-        if (t0 + lane < tb) V.tile_ptr[t0 + lane] = before + incl - c;
-        before += __shfl_sync(0xFFFFFFFFu, incl, 31);
+      for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += u;
       }
-      if (lane == 0 && blockIdx.x == 0) V.tile_ptr[n_tiles] = all;
+      if (t0 + lane < tb) V.tile_ptr[t0 + lane] = before + incl - c;
+      before += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
-    __syncthreads();
-    for (int t0 = ta; t0 < tb; t0 += groups) {
-      const int t = t0 + tid / rows;
-      int row;
-      unsigned my;
-      unsigned tm = tile_mask(t < tb ? t : n_tiles, rows, row, my);
-      if (t >= tb) continue;
-      const int r = tid % rows;
-      const int base = V.tile_ptr[t];
-      const int* next = o.nbr;  // this row's next neighbour in its list
-      if (!o.table && row >= 0) next += o.starts ? __ldg(o.starts + row) : row;
-      int s = 0;
-      auto put = [&](int code, int value) {
-        const int stage = base + s / V.slots;
-        if (stage < V.stage_cap) {
-          const size_t e = static_cast<size_t>(stage) * V.slots + s % V.slots;
-          V.stage_nbr[e * rows + r] = value;
-          if (r == 0) V.stage_kp[e] = code;
-        }
-        ++s;
-      };
-      for (; tm; tm &= tm - 1u) {
-        const int kp = __ffs(tm) - 1;
-        int value = -1;
-        if ((my >> kp) & 1u) value = o.table ? __ldg(o.table + static_cast<size_t>(kp) * n + row) : __ldg(next++);
-        int code = kp;
-        if (V.slots == 1 && r == 0) {  // which 128-row parts of the tile have the offset
-          const int w0 = (tid / rows) * (rows / 32);
-          for (int part = 0; part < rows / 128; ++part) {
-            const unsigned m4 = sh.warp_mask[w0 + 4 * part] | sh.warp_mask[w0 + 4 * part + 1] | sh.warp_mask[w0 + 4 * part + 2] |
-                                sh.warp_mask[w0 + 4 * part + 3];
-            if ((m4 >> kp) & 1u) code |= 1 << (8 + part);
-          }
-        }
-        put(code, value);
-      }
-      while (s % V.slots) put(-2, -1);
-      if (V.identity) {
-        put(-1, row);
-        while (s % V.slots) put(-2, -1);
-      }
-    }
-    __syncthreads();
+    if (lane == 0 && blockIdx.x == 0) V.tile_ptr[n_tiles] = all;
   }
 }
 
@@ -820,14 +976,16 @@ int subm_dense(const int* coords, int n, const pce_geom* g, void* ws, size_t ws_
 
 // ---- order and lists ----
 
+// Blocks of the cooperative sort: 4096 rows each.  Its blocks hold their SMs while they wait for one another, beside the
+// convolutions of the pass that runs at the time; fewer rows per block end sooner alone and cost the pass more.
 static int order_grid(int n) {
   const int sms = device_sm_count();
-  return std::max(1, std::min(div_up(n, 2 * coop::kThreads), sms > 0 ? sms : 1));
+  return std::max(1, std::min(div_up(n, 8 * coop::kThreads), sms > 0 ? sms : 1));
 }
 
 size_t order_workspace_bytes(int n) {
   const size_t m = n > 0 ? n : 1;
-  return 4 * pad256(4 * m) + 1024 * (coop::kBins + 32) * sizeof(int) + 4096;
+  return 4 * pad256(4 * m) + 1024 * ((1 << kOrderBits) + 32) * sizeof(int) + 4096;
 }
 
 int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st) {
@@ -840,18 +998,36 @@ int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st) {
     if (o.n == 0) PCE_CUDA(cudaMemsetAsync(V.tile_ptr, 0, sizeof(int), st));
   }
   if (o.n == 0) return PCE_OK;
-  Arena ar(ws, ws_bytes);
-  int g = order_grid(o.n);
-  o.key0 = ar.take<unsigned>(o.n);
-  o.key1 = ar.take<unsigned>(o.n);
-  o.val0 = ar.take<int>(o.n);
-  o.val1 = ar.take<int>(o.n);
-  o.hist = ar.take<int>(static_cast<size_t>(g) * coop::kBins);
-  o.block_counts = ar.take<int>(static_cast<size_t>(g) * 32);
-  if (!ar.ok) return PCE_ERR_WORKSPACE;
-  void* args[] = {&o};
-  PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_order_lists), dim3(g), dim3(coop::kThreads), args, 0, st));
-  PCE_LAUNCH_CHECK();
+  if (o.n <= kClusterRows) {
+    static bool attr_set[64] = {};
+    int dev = 0;
+    PCE_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return PCE_ERR_UNSUPPORTED;
+    if (!attr_set[dev]) {
+      PCE_CUDA(cudaFuncSetAttribute(k_order_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ClusterShared))));
+      attr_set[dev] = true;
+    }
+    k_order_cluster<<<kClusterBlocks, kClusterThreads, sizeof(ClusterShared), st>>>(o);
+    PCE_LAUNCH_CHECK();
+  } else {
+    Arena ar(ws, ws_bytes);
+    int g = order_grid(o.n);
+    o.key0 = ar.take<unsigned>(o.n);
+    o.key1 = ar.take<unsigned>(o.n);
+    o.val0 = ar.take<int>(o.n);
+    o.val1 = ar.take<int>(o.n);
+    o.hist = ar.take<int>(static_cast<size_t>(g) << kOrderBits);
+    o.block_counts = ar.take<int>(static_cast<size_t>(g) * 32);
+    if (!ar.ok) return PCE_ERR_WORKSPACE;
+    void* args[] = {&o};
+    PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_order_grid), dim3(g), dim3(coop::kThreads), args, 0, st));
+    PCE_LAUNCH_CHECK();
+  }
+  for (int v = 0; v < o.n_variants; ++v) {
+    const Variant& V = o.variant[v];
+    PCE_TRY(fill_tile_lists(o.mask, o.starts, o.nbr, o.table, o.order, o.n, o.kv, V.tile_rows, V.identity, V.slots, V.tile_ptr, V.stage_kp,
+                            V.stage_nbr, V.stage_cap, st));
+  }
   return PCE_OK;
 }
 
@@ -874,7 +1050,7 @@ size_t chain_bytes(int n, int n_geoms, bool keep0) {
   size_t b = pad256(sizeof(int) * kCtlWords) + static_cast<size_t>(n_geoms) * pad256(sizeof(Block) * coarse_slots(n));
   if (keep0) b += pad256(sizeof(Block) * table_slots(m)) + 2 * pad256(4 * m);
   b += pad256(4 * up) + pad256(16 * up) + 3 * pad256(8 * up) + 2 * pad256(4 * up);
-  return b + pad256(sizeof(int) * 1024 * coop::kBins) + 4096;
+  return b + pad256(sizeof(int) * 1024 * 256) + 4096;
 }
 
 int chain_place(Chain& c, int n, const pce_geom* const* geoms, int n_geoms, bool keep0, void* mem, size_t bytes) {
@@ -925,13 +1101,13 @@ int chain_place(Chain& c, int n, const pce_geom* const* geoms, int n_geoms, bool
   c.val0 = ar.take<int>(c.up_cap);
   c.val1 = ar.take<int>(c.up_cap);
   c.grid = std::max(1, std::min(div_up(n, 2 * coop::kThreads), device_sm_count()));
-  c.hist = ar.take<int>(static_cast<size_t>(c.grid) * coop::kBins);
+  c.hist = ar.take<int>(static_cast<size_t>(c.grid) * 256);
   if (!ar.ok) return PCE_ERR_WORKSPACE;
   c.cleared = cleared;
   return PCE_OK;
 }
 
-int chain_build(Chain& c, const int* coords, int n, int* host_dev, cudaStream_t st) {
+int chain_tables(Chain& c, const int* coords, int n, cudaStream_t st) {
   const int4* c4 = reinterpret_cast<const int4*>(coords);
   PCE_CUDA(cudaMemsetAsync(c.ctl, 0, c.cleared, st));
   k_block_insert<<<div_up(n, 256), 256, 0, st>>>(c4, n, c.lv, c.slot0, c.ctl);
@@ -941,13 +1117,17 @@ int chain_build(Chain& c, const int* coords, int n, int* host_dev, cudaStream_t 
     if (c.lv.level[l].table) widest = std::max(widest, c.lv.level[l].tmask + 1);
   k_block_places<<<dim3(std::min<unsigned>(widest / 256, 148 * 4), c.lv.n), 256, 0, st>>>(c.lv, c.kf, c.keys, c.up_cap, c.ctl);
   PCE_LAUNCH_CHECK();
-  void* args[] = {&c.keys, &c.key0, &c.key1, &c.val0, &c.val1, &c.hist, &c.lv, &c.kf, &c.up_cap, &c.coords_up, &c.perm_up, &c.ctl, &host_dev};
-  PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_level_sort), dim3(c.grid), dim3(coop::kThreads), args, 0, st));
-  PCE_LAUNCH_CHECK();
   if (c.perm0) {
     k_block_rows<<<div_up(n, 256), 256, 0, st>>>(c4, n, c.lv.level[0].table, c.slot0, c.perm0);
     PCE_LAUNCH_CHECK();
   }
+  return PCE_OK;
+}
+
+int chain_levels(Chain& c, int* host_dev, cudaStream_t st) {
+  void* args[] = {&c.keys, &c.key0, &c.key1, &c.val0, &c.val1, &c.hist, &c.lv, &c.kf, &c.up_cap, &c.coords_up, &c.perm_up, &c.ctl, &host_dev};
+  PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_level_sort), dim3(c.grid), dim3(coop::kThreads), args, 0, st));
+  PCE_LAUNCH_CHECK();
   return PCE_OK;
 }
 

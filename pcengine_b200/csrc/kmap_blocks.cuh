@@ -126,8 +126,10 @@ struct Chain {
 };
 size_t chain_bytes(int n, int n_geoms, bool keep0);
 int chain_place(Chain& c, int n, const pce_geom* const* geoms, int n_geoms, bool keep0, void* mem, size_t bytes);
-// Queues the whole construction; `host` (mapped, device address) receives status, largest batch, rows per level.
-int chain_build(Chain& c, const int* coords, int n, int* host_dev, cudaStream_t st);
+// Queues the tables of all levels (and the input level's row table), then the coarser levels' coordinates and row tables;
+// `host_dev` (mapped, device address) receives status, largest batch, rows per level.
+int chain_tables(Chain& c, const int* coords, int n, cudaStream_t st);
+int chain_levels(Chain& c, int* host_dev, cudaStream_t st);
 int parent_maps(const int* coords, int n, const Level& L, const int* perm, int kv, int n_parents, unsigned* up_mask, int* up_nbr,
                 int* child, int* counts, cudaStream_t st);
 

@@ -26,6 +26,11 @@
 // waits for it; pce_pass_release records an event on the stream that read the maps and the
 // lanes of the pass that recycles the arena wait for that one.  Nothing else ties the planner
 // to the feature stream, so the maps of pass i+1 are built while pass i still computes.
+#include <sched.h>
+#include <sys/prctl.h>
+#include <time.h>
+
+#include <algorithm>
 #include <condition_variable>
 #include <chrono>
 #include <deque>
@@ -34,9 +39,11 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kmap_blocks.cuh"
 
 namespace pce {
 
+int wait_for_stream(cudaStream_t st);
 bool conv_umma_supported(int cin, int cout, int dtype);
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 int conv_umma(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out, int cin,
@@ -98,7 +105,8 @@ struct LevelState {
   const int32_t* coords = nullptr;
   int32_t n = 0;
   int32_t cmax[3] = {0, 0, 0};
-  cudaEvent_t ev = nullptr;  // recorded once the coordinates are written (levels >= 1)
+  cudaEvent_t ev = nullptr;  // recorded once the coordinates (and in block form the level's tables) are written
+  const int* perm = nullptr; // block form: row table of the level (its block table is chain.lv.level[l])
   int ready = 0;             // host side: n is known, ev is recorded (guarded by plan->m)
 };
 
@@ -122,6 +130,8 @@ struct pce_pass {
   std::vector<pce_planned_map> maps;
   // guarded by plan->m
   std::vector<int> queued;
+  blk::Chain chain;                        // block form: tables of all levels, valid once a level is ready
+  int* sizes = nullptr;                    // mapped host words that lane 0's kernels report to
   int next_map = 0;
   int lanes_done = 0;
   int error = PCE_OK;
@@ -149,6 +159,8 @@ struct pce_plan {
   std::vector<pce_plan_map_spec> specs;
   std::vector<int> out_level;  // per spec: the level its outputs live on
   int n_levels = 1;
+  std::vector<char> in_blocks; // per spec: a map the block form covers
+  bool chain = false;          // the strided specs lead from level to level, parents each: block form (kmap_blocks.cu)
   int device = 0;
   int sm_count = 148;
   PlanLane lanes[kLanes];
@@ -282,10 +294,97 @@ static int build_csr(pce_plan* p, PlanLane* l, pce_pass* ps, const int32_t* tabl
   return PCE_OK;
 }
 
+// Waits for an event that may be milliseconds away with short naps between queries: a blocking wait wakes up 50 us and
+// more after the event, which the maps of the pass would start later, and spinning takes the core from the threads that
+// queue the work waited for.  After 20 ms of naps the wait blocks.
+static int doze_on(cudaEvent_t ev) {
+  const auto t0 = std::chrono::steady_clock::now();
+  for (;;) {
+    const cudaError_t q = cudaEventQuery(ev);
+    if (q == cudaSuccess) return PCE_OK;
+    if (q != cudaErrorNotReady) return cuda_fail(q);
+    (void)cudaGetLastError();  // "not ready" is an answer, not a failure
+    if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
+    const timespec nap{0, 10000};
+    nanosleep(&nap, nullptr);
+  }
+  PCE_CUDA(cudaEventSynchronize(ev));
+  return PCE_OK;
+}
+
+// Lane 0 in block form: the tables of all levels and the coordinates of the coarser ones, with one wait for all their
+// sizes.  The input level's maps may be queued as soon as its table is (before the wait).  PCE_ERR_TABLE_FULL /
+// UNSUPPORTED: the cloud does not fit the form, the levels are found one by one instead.
+static int run_chain(pce_plan* p, PlanLane* l, pce_pass* ps) {
+  const int n_geoms = p->n_levels - 1;
+  pce_geom geoms[blk::kMaxLevels];
+  const pce_geom* gp[blk::kMaxLevels];
+  int32_t cmax[blk::kMaxLevels][3];
+  LevelState& in = ps->levels[0];
+  const int32_t* before = in.cmax;
+  int at = 0;
+  for (size_t i = 0; i < p->specs.size(); ++i) {
+    const pce_plan_map_spec& sp = p->specs[i];
+    if (sp.submanifold) continue;
+    for (int d = 0; d < 3; ++d) cmax[at][d] = (before[d] - (sp.ks[d] - 1)) / sp.stride[d];
+    fill_geom(sp, ps->cmin, cmax[at], &geoms[at]);
+    gp[at] = &geoms[at];
+    before = cmax[at];
+    ++at;
+  }
+  const size_t bytes = blk::chain_bytes(in.n, n_geoms, true);
+  void* mem = ps->take(bytes);
+  if (!mem) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+  PCE_TRY(blk::chain_place(ps->chain, in.n, gp, n_geoms, true, mem, bytes));
+  if (!ps->sizes) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ps->sizes), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+  int* sizes_dev = nullptr;
+  PCE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&sizes_dev), ps->sizes, 0));
+  ps->sizes[0] = PCE_ERR_CUDA;
+  PCE_TRY(blk::chain_tables(ps->chain, in.coords, in.n, l->stream));
+  PCE_CUDA(cudaEventRecord(in.ev, l->stream));
+  PCE_TRY(blk::chain_levels(ps->chain, sizes_dev, l->stream));
+  for (int k = 1; k < p->n_levels; ++k) PCE_CUDA(cudaEventRecord(ps->levels[k].ev, l->stream));
+  {
+    std::lock_guard<std::mutex> lk(p->m);
+    in.perm = ps->chain.perm0;
+    in.ready = 1;
+  }
+  p->cv.notify_all();
+  // what is queued in front (the pass before this one) may take milliseconds; the chain itself then takes 100 us
+  PCE_TRY(doze_on(ps->start));
+  PCE_TRY(wait_for_stream(l->stream));
+  if (ps->sizes[0] != PCE_OK) return ps->sizes[0];
+  {
+    std::lock_guard<std::mutex> lk(p->m);
+    int first = 0;
+    for (int k = 1; k < p->n_levels; ++k) {
+      LevelState& lv = ps->levels[k];
+      lv.coords = reinterpret_cast<const int32_t*>(ps->chain.coords_up + first);
+      lv.n = ps->sizes[2 + k];
+      lv.perm = ps->chain.perm_up;
+      for (int d = 0; d < 3; ++d) lv.cmax[d] = cmax[k - 1][d];
+      lv.ready = 1;
+      first += lv.n;
+    }
+  }
+  p->cv.notify_all();
+  return PCE_OK;
+}
+
 // Lane 0: the output coordinates of every strided spec, in order.
 static int run_coords_lane(pce_plan* p, PlanLane* l, pce_pass* ps) {
   PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->start, 0));
   if (ps->has_released) PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->released, 0));
+  if (p->chain && plan_short_route) {
+    const int status = run_chain(p, l, ps);
+    if (status != PCE_ERR_TABLE_FULL && status != PCE_ERR_UNSUPPORTED) return status;
+  }
+  if (!ps->levels[0].ready) {
+    PCE_CUDA(cudaEventRecord(ps->levels[0].ev, l->stream));
+    std::lock_guard<std::mutex> lk(p->m);
+    ps->levels[0].ready = 1;
+  }
+  p->cv.notify_all();
   for (size_t i = 0; i < p->specs.size(); ++i) {
     const pce_plan_map_spec& sp = p->specs[i];
     if (sp.submanifold) continue;
@@ -328,6 +427,122 @@ static bool wait_level(pce_plan* p, pce_pass* ps, int level, LevelState* out) {
   return true;
 }
 
+// One direction of a map in block form: row order and the lists of its uses in one launch.
+static int build_direction(pce_plan* p, PlanLane* l, pce_pass* ps, blk::Order o, int n_src, const int32_t* c_outs, const int32_t* c_ins,
+                           int identity_stage, pce_planned_csr* out) {
+  out->mask = o.mask;
+  out->rowptr = nullptr;
+  out->nbr = nullptr;
+  out->n_rows = o.n;
+  out->n_src = n_src;
+  out->nbr_cap = 0;
+  out->n_lists = 0;
+  out->table = o.table;
+  out->reverse_kp = 0;
+  out->identity_kp = -1;
+  out->starts = o.starts;
+  out->row_nbr = o.nbr;
+  out->counts = o.counts;
+  o.n_variants = 0;
+  for (int u = 0; u < PCE_PLAN_MAX_USES && c_outs[u] > 0; ++u) {
+    const int rows = tile_rows_policy(o.n, c_ins[u], c_outs[u], p->sm_count);
+    const int slots = c_ins[u] == 32 ? 2 : (c_ins[u] == 16 ? 4 : 1);
+    bool seen = false;
+    for (int v = 0; v < o.n_variants; ++v) seen = seen || (o.variant[v].tile_rows == rows && o.variant[v].slots == slots);
+    if (seen) continue;
+    if (o.n_variants == blk::kMaxVariants) return PCE_ERR_UNSUPPORTED;
+    const int n_tiles = div_up(o.n, rows);
+    const size_t cap = static_cast<size_t>(n_tiles) * ((o.kv + slots - 1) / slots + (identity_stage ? 1 : 0));
+    blk::Variant& V = o.variant[o.n_variants++];
+    V = blk::Variant{rows, identity_stage, slots, ps->take_n<int32_t>(static_cast<size_t>(n_tiles) + 1), ps->take_n<int32_t>(cap * slots),
+                     ps->take_n<int32_t>(cap * slots * rows), static_cast<int>(cap)};
+    if (!V.tile_ptr || !V.stage_kp || !V.stage_nbr) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+  }
+  if (o.n_variants == 0 || o.n == 0) return PCE_OK;
+  o.order = ps->take_n<int32_t>(o.n);
+  if (!o.order) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+  void* ws = nullptr;
+  PCE_TRY(scratch_for(l, blk::order_workspace_bytes(o.n), &ws));
+  PCE_TRY(blk::order_lists(o, ws, l->scratch_cap, l->stream));
+  for (int v = 0; v < o.n_variants; ++v) {
+    const blk::Variant& V = o.variant[v];
+    out->lists[out->n_lists++] = pce_tile_lists{o.order, V.tile_ptr, V.stage_kp, V.stage_nbr, V.tile_rows, identity_stage, V.slots, 1};
+  }
+  return PCE_OK;
+}
+
+// A map in block form (kmap_blocks.cu): the dense tables are left to whoever asks for them.
+static int build_map_blocks(pce_plan* p, PlanLane* l, pce_pass* ps, int i, const LevelState& in, const LevelState& outl) {
+  const pce_plan_map_spec& sp = p->specs[i];
+  cudaStream_t st = l->stream;
+  pce_planned_map& out = ps->maps[i];
+  const int kv = sp.ks[0] * sp.ks[1] * sp.ks[2], n_in = in.n, n_out = outl.n;
+  for (int d = 0; d < 3; ++d) out.cmax_out[d] = outl.cmax[d];
+  out.n_in = n_in;
+  out.n_out = n_out;
+  out.kv = kv;
+  out.symmetric = sp.submanifold ? 1 : 0;
+  out.in_coords = in.coords;
+  out.out_coords = outl.coords;
+  out.map = out.map_out = out.knnz = out.kpos = out.qkpos = out.status = nullptr;
+  out.has_fwd = sp.want_fwd ? 1 : 0;
+  out.has_tr = sp.want_tr ? 1 : 0;
+  blk::Order o = {};
+  o.kv = kv;
+  if (sp.submanifold) {
+    const blk::Level& L = ps->chain.lv.level[sp.in_level];
+    int32_t* state = ps->take_n<int32_t>(blk::kStateWords);
+    int32_t* rows = ps->take_n<int32_t>(2 * static_cast<size_t>(n_in > 0 ? n_in : 1));
+    int32_t* nbr = ps->take_n<int32_t>(static_cast<size_t>(kv) * (n_in > 0 ? n_in : 1));
+    if (!state || !rows || !nbr) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+    PCE_CUDA(cudaMemsetAsync(state, 0, sizeof(int32_t) * blk::kStateWords, st));
+    // (the row table of a coarser level holds rows of its level: places are numbered over all coarser levels)
+    const blk::Query q{L.table, L.tmask, in.perm, {sp.ks[0], sp.ks[1], sp.ks[2]}, state + 32, reinterpret_cast<unsigned*>(rows),
+                       rows + n_in, nbr, state + 16, nullptr};
+    PCE_TRY(blk::query_lists(in.coords, n_in, q, st));
+    o.mask = reinterpret_cast<unsigned*>(rows);
+    o.starts = rows + n_in;
+    o.nbr = nbr;
+    o.counts = state + 32;
+    o.n = n_in;
+    if (sp.want_fwd) PCE_TRY(build_direction(p, l, ps, o, n_in, sp.c_out_fwd, sp.c_in_fwd, 1, &out.fwd));
+    return PCE_OK;
+  }
+  int32_t* counts = ps->take_n<int32_t>(32);
+  int32_t* up = ps->take_n<int32_t>(2 * static_cast<size_t>(n_in > 0 ? n_in : 1));
+  int32_t* down = ps->take_n<int32_t>((static_cast<size_t>(kv) + 1) * (n_out > 0 ? n_out : 1));
+  if (!counts || !up || !down) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+  int32_t* child = down + n_out;
+  PCE_TRY(blk::parent_maps(in.coords, n_in, ps->chain.lv.level[p->out_level[i]], outl.perm, kv, n_out, reinterpret_cast<unsigned*>(up),
+                           up + n_in, child, counts, st));
+  o.counts = counts;
+  if (sp.want_fwd) {
+    o.mask = reinterpret_cast<unsigned*>(down);
+    o.table = child;
+    o.n = n_out;
+    PCE_TRY(build_direction(p, l, ps, o, n_in, sp.c_out_fwd, sp.c_in_fwd, 0, &out.fwd));
+    out.fwd.nbr_cap = static_cast<int32_t>(std::min<long long>(static_cast<long long>(kv) * n_out, 0x7FFFFFFF));
+  }
+  if (sp.want_tr) {
+    o.mask = reinterpret_cast<unsigned*>(up);
+    o.table = nullptr;
+    o.nbr = up + n_in;
+    o.n = n_in;
+    PCE_TRY(build_direction(p, l, ps, o, n_out, sp.c_out_tr, sp.c_in_tr, 0, &out.tr));
+  }
+  return PCE_OK;
+}
+
+static int map_queued(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
+  PCE_CUDA(cudaEventRecord(ps->ready[i], l->stream));
+  {
+    std::lock_guard<std::mutex> lk(p->m);
+    ps->queued[i] = 1;
+  }
+  p->cv.notify_all();
+  return PCE_OK;
+}
+
 static int build_map(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
   const pce_plan_map_spec& sp = p->specs[i];
   cudaStream_t st = l->stream;
@@ -336,6 +551,10 @@ static int build_map(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
   if (!wait_level(p, ps, p->out_level[i], &outl)) return PCE_OK;
   if (in.ev) PCE_CUDA(cudaStreamWaitEvent(st, in.ev, 0));
   if (outl.ev && outl.ev != in.ev) PCE_CUDA(cudaStreamWaitEvent(st, outl.ev, 0));
+  if (p->in_blocks[i] && outl.perm) {
+    PCE_TRY(build_map_blocks(p, l, ps, i, in, outl));
+    return map_queued(p, l, ps, i);
+  }
   pce_planned_map& out = ps->maps[i];
   pce_geom g;
   fill_geom(sp, ps->cmin, outl.cmax, &g);
@@ -388,13 +607,7 @@ static int build_map(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
     PCE_TRY(build_csr(p, l, ps, map, kv, n_in, n_out, 0, ident, cap_nbr, sp.c_out_tr, sp.c_in_tr, 0, knnz, &out.tr));
     out.has_tr = 1;
   }
-  PCE_CUDA(cudaEventRecord(ps->ready[i], st));
-  {
-    std::lock_guard<std::mutex> lk(p->m);
-    ps->queued[i] = 1;
-  }
-  p->cv.notify_all();
-  return PCE_OK;
+  return map_queued(p, l, ps, i);
 }
 
 // Map lanes: take the next map in first-use order until none is left.
@@ -415,6 +628,7 @@ static int run_map_lane(pce_plan* p, PlanLane* l, pce_pass* ps) {
 
 static void lane_main(pce_plan* p, int lane) {
   cudaSetDevice(p->device);
+  prctl(PR_SET_TIMERSLACK, 1000, 0, 0, 0);  // (the naps of doze_on: 50 us late by default)
   PlanLane* l = &p->lanes[lane];
   for (;;) {
     pce_pass* ps = nullptr;
@@ -445,6 +659,7 @@ int32_t pce_tile_rows_for(int32_t n_rows, int32_t c_in, int32_t c_out, int32_t s
 
 static void free_pass(pce_pass* ps) {
   ps->arena.release();
+  if (ps->sizes) cudaFreeHost(ps->sizes);
   if (ps->start) cudaEventDestroy(ps->start);
   if (ps->released) cudaEventDestroy(ps->released);
   for (cudaEvent_t ev : ps->ready)
@@ -470,6 +685,17 @@ int pce_plan_create(const pce_plan_map_spec* specs, int32_t n_specs, pce_plan** 
   p->specs.assign(specs, specs + n_specs);
   p->out_level = out_level;
   p->n_levels = levels;
+  p->chain = levels >= 2 && levels <= blk::kMaxLevels;
+  for (int i = 0; i < n_specs; ++i) {
+    const pce_plan_map_spec& s = specs[i];
+    pce_geom g;
+    const int32_t zero[3] = {0, 0, 0};
+    fill_geom(s, zero, zero, &g);
+    const bool ok = s.submanifold ? (blk::covers(&g) && s.ks[0] * s.ks[1] * s.ks[2] <= 32 && !s.want_tr) : blk::parents(&g);
+    p->in_blocks.push_back(ok ? 1 : 0);
+    // the chain: every strided layer leads from one level to the next
+    if (!s.submanifold && (!ok || s.in_level != out_level[i] - 1)) p->chain = false;
+  }
   cudaError_t e = cudaGetDevice(&p->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device);
   for (int l = 0; l < kLanes && e == cudaSuccess; ++l)
@@ -545,13 +771,13 @@ int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t*
   if (!ps) {
     ps = new pce_pass();
     ps->plan = p;
-    cudaError_t e = cudaEventCreateWithFlags(&ps->start, cudaEventDisableTiming);
+    cudaError_t e = cudaEventCreateWithFlags(&ps->start, cudaEventDisableTiming | cudaEventBlockingSync);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ps->released, cudaEventDisableTiming);
     ps->ready.assign(p->specs.size(), nullptr);
     ps->levels.assign(p->n_levels, LevelState{});
     for (size_t i = 0; i < p->specs.size() && e == cudaSuccess; ++i)
       e = cudaEventCreateWithFlags(&ps->ready[i], cudaEventDisableTiming);
-    for (int k = 1; k < p->n_levels && e == cudaSuccess; ++k)
+    for (int k = 0; k < p->n_levels && e == cudaSuccess; ++k)
       e = cudaEventCreateWithFlags(&ps->levels[k].ev, cudaEventDisableTiming);
     if (e != cudaSuccess) {
       free_pass(ps);
@@ -563,10 +789,12 @@ int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t*
     ps->levels[k].coords = nullptr;
     ps->levels[k].n = 0;
     ps->levels[k].ready = 0;
+    ps->levels[k].perm = nullptr;
   }
   ps->levels[0].coords = coords;
   ps->levels[0].n = n;
-  ps->levels[0].ready = 1;  // its producer precedes `start`, which every lane's stream waits for
+  // its producer precedes `start`, which every lane's stream waits for (in block form lane 0 adds its table first)
+  ps->levels[0].ready = p->chain && plan_short_route ? 0 : 1;
   for (int d = 0; d < 3; ++d) {
     ps->cmin[d] = cmin[d];
     ps->levels[0].cmax[d] = cmax[d];
@@ -597,6 +825,14 @@ int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t*
 int pce_pass_map(pce_pass* ps, int32_t index, void* stream, pce_planned_map* out) {
   if (!ps || !out || index < 0 || index >= static_cast<int32_t>(ps->maps.size())) return PCE_ERR_INVALID;
   pce_plan* p = ps->plan;
+  // the lane is usually microseconds away: a short poll before the sleep, whose wake-up alone takes 20 to 50 us
+  for (const auto t0 = std::chrono::steady_clock::now(); std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(100);) {
+    {
+      std::lock_guard<std::mutex> lk(p->m);
+      if (ps->queued[index] != 0 || ps->error != PCE_OK || ps->finished) break;
+    }
+    sched_yield();
+  }
   {
     std::unique_lock<std::mutex> lk(p->m);
     const bool done = p->cv.wait_for(lk, std::chrono::seconds(30),

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(coop::kThreads)
     k_voxelise(const float* __restrict__ pts, int n, double vx, double vy, double vz, int batch, unsigned long long* key0,
                unsigned long long* key1, int* val0, int* val1, int* bounds, int* hist, int* counts, VoxelOut out) {
   using namespace coop;
-  __shared__ SortShared sh;
+  __shared__ SortShared<8> sh;
   __shared__ int red[kWarps][7];
   __shared__ int s_b[7];
   cg::grid_group grid = cg::this_grid();
@@ -224,7 +224,7 @@ static int launch_voxelise(const float* points, int n, const float* v, int batch
   int* val0 = ar.take<int>(n);
   int* val1 = ar.take<int>(n);
   int* bounds = ar.take<int>(static_cast<size_t>(g) * 8);
-  int* hist = ar.take<int>(static_cast<size_t>(g) * coop::kBins);
+  int* hist = ar.take<int>(static_cast<size_t>(g) * 256);
   int* counts = ar.take<int>(g);
   if (!ar.ok) return PCE_ERR_WORKSPACE;
   double vx = v[0], vy = v[1], vz = v[2];

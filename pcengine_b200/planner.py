@@ -113,6 +113,21 @@ def _pair_counter(knnz, identity_rows: int):
     return count
 
 
+class _PlannedDense(_DenseTables):
+    """The dense tables of a map that the planner made in block form, as the planner's other arrays look."""
+
+    def build(self) -> "_DenseTables":
+        if not self.built:
+            super().build()
+            for name in self.NAMES:
+                t = getattr(self, name)
+                if t is not None:
+                    a = _DevArray(t.data_ptr(), t.shape, t.device, t)
+                    a._tensor = t
+                    setattr(self, name, a)
+        return self
+
+
 class PlannedKernelMap(KernelMap):
     """A :class:`KernelMap` whose arrays were produced by the planner."""
 
@@ -130,14 +145,15 @@ class PlannedKernelMap(KernelMap):
         self.out_coords = in_coords if self.subm else _DevArray(out.out_coords, (self.n_out, 4), device, keep).tensor()
         kv = self.kv
         self.symmetric = bool(out.symmetric)
-        d = self._dense = _DenseTables(in_coords, self.out_coords, self.geom, kv, self.mid, self.subm, self.symmetric)
-        d.map = _DevArray(out.map, (kv * self.n_in,), device, keep)
-        d.map_out = None if self.symmetric else _DevArray(out.map_out, (kv * max(self.n_out, 1),), device, keep)
-        d.knnz = _DevArray(out.knnz, (kv,), device, keep)
-        d.kpos = _DevArray(out.kpos, (kv + 1,), device, keep)
-        d.qkpos = _DevArray(out.qkpos, (kv + 1,), device, keep)
-        d.status = _DevArray(out.status, (1,), device, keep)
-        d.built = True
+        d = self._dense = _PlannedDense(in_coords, self.out_coords, self.geom, kv, self.mid, self.subm, self.symmetric)
+        if out.map:
+            d.map = _DevArray(out.map, (kv * self.n_in,), device, keep)
+            d.map_out = None if self.symmetric else _DevArray(out.map_out, (kv * max(self.n_out, 1),), device, keep)
+            d.knnz = _DevArray(out.knnz, (kv,), device, keep)
+            d.kpos = _DevArray(out.kpos, (kv + 1,), device, keep)
+            d.qkpos = _DevArray(out.qkpos, (kv + 1,), device, keep)
+            d.status = _DevArray(out.status, (1,), device, keep)
+            d.built = True
         self._csr = {}
         self._pairs = self._d1 = self._sizes = self._state = self._parents = None
         self._blocks = False
@@ -150,12 +166,14 @@ class PlannedKernelMap(KernelMap):
             if c.rowptr:
                 csr = NeighbourCSR(mask, _DevArray(c.rowptr, (c.n_rows + 1,), device, keep),
                                    _DevArray(c.nbr, (c.nbr_cap,), device, keep), int(c.n_rows), int(c.n_src), kv)
+            elif not out.map:
+                csr = self._csr_in_block_form(c, mask, transposed, d, device, keep)
             else:
                 # planned without its neighbour CSR (only tile lists were needed): built on first use
                 csr = NeighbourCSR(mask, None, None, int(c.n_rows), int(c.n_src), kv,
                                    fill=_csr_filler(int(c.table), kv, int(c.n_rows), int(c.reverse_kp), int(c.identity_kp),
                                                     int(c.nbr_cap), device, keep),
-                                   pairs=_pair_counter(self.knnz, int(c.n_rows) if c.identity_kp >= 0 else 0))
+                                   pairs=_pair_counter(d.knnz, int(c.n_rows) if c.identity_kp >= 0 else 0))
             for i in range(c.n_lists):
                 t = c.lists[i]
                 slots = max(int(t.slots), 1)
@@ -172,6 +190,26 @@ class PlannedKernelMap(KernelMap):
                 else:
                     csr._tiles[(True, int(t.tile_rows), bool(t.identity_stage), slots)] = hit
             self._csr[transposed] = csr
+
+    def _csr_in_block_form(self, c, mask, transposed, dense, device, keep) -> NeighbourCSR:
+        n, kv = int(c.n_rows), self.kv
+        counts = _DevArray(c.counts, (kv,), device, keep)
+        lists = table = None
+        if c.row_nbr:
+            starts = _DevArray(c.starts, (n,), device, keep) if c.starts else None
+            lists = (starts, _DevArray(c.row_nbr, (kv * n if c.starts else n,), device, keep))
+        else:
+            table = _DevArray(c.table, (kv * n,), device, keep)
+
+        written = table is None or c.n_lists > 0  # a table's mask appears with the row order
+
+        def fill():
+            full, rowptr, nbr = dense.csr(transposed)
+            if not written:
+                mask.tensor().copy_(full)
+            return rowptr, nbr
+        return NeighbourCSR(mask, None, None, n, int(c.n_src), kv, fill=fill, pairs=_pair_counter(counts, 0), lists=lists, table=table, counts=counts,
+                            mask_ready=written)
 
 
 class PlannedPass:
