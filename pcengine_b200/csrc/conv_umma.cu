@@ -161,6 +161,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, Ctl* ct
   return true;
 }
 
+// One lane of a fully active warp.  Tensor-core, commit and bulk-copy instructions want uniform operands and a single
+// issuing thread, which the compiler can prove behind `elect.sync` but not behind `if (lane == 0)`: there a 64-channel
+// stage's four products and commit took about 1000 cycles to ISSUE (their execution 130 to 200), more than anything
+// else in the kernel; elected, and with the four steps unrolled, about 500.  Whole layers: 96->96 on 240 k rows
+// 50 -> 46 us, 128->128 on 137 k rows 50 -> 44 us, 256->256 on 58 k rows 83 -> 74 us.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
@@ -530,7 +541,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         ok = __all_sync(0xFFFFFFFFu, ok);  // keep the warp convergent
         if (!ok) return;
         const uint32_t a_addr = tiles_addr + s * stage_bytes;
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
           const uint32_t bbar = smem_u32(&ctl->bfull[s]);
           mbar_arrive_expect_tx(bbar, b_bytes);
           const __half* wsrc = second ? sec.w2 + static_cast<size_t>(kb) * cout * KB
@@ -597,7 +608,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         const uint32_t a_addr = tiles_addr + s * stage_bytes;
         const uint32_t b_addr = a_addr + kAStage;
         if (second) {
-          if (tid == 0) {
+          if (warp == 0 && elect_one()) {
             const uint32_t bbar = smem_u32(&ctl->bfull[s]);
             mbar_arrive_expect_tx(bbar, b_bytes);
             bulk_copy_g2s(b_addr, sec.w2 + static_cast<size_t>(kb) * cout * 64, b_bytes, bbar);
@@ -671,7 +682,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
   } else if (warp == kMmaWarp) {
     // =========================== MMA issuer ===========================
     if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (lane == 0) {
+    {
       const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(cout >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
       int j = 0;
       bool ok = true;
@@ -682,39 +693,52 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         const int nst = nst_main + (tile_ident(t) ? kblocks2 : 0);
         // the accumulator must have been drained by the epilogue (two tiles ago)
         if (it >= nacc) ok = mbar_wait(smem_u32(&ctl->accempty[buf]), ((it / nacc) - 1) & 1, ctl);
+        ok = __all_sync(0xFFFFFFFFu, ok);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(buf * SUB * cout);
         uint32_t accumulate = 0;
-        for (int st = 0; st < nst && ok; ++st, ++j) {
+        int kb = 0;  // K block inside the offset
+        for (int st = 0; st < nst; ++st, ++j) {
           const int s = j % kStages;
           const uint32_t par = (j / kStages) & 1;
           ok = mbar_wait(smem_u32(&ctl->afull[s]), par, ctl) && mbar_wait(smem_u32(&ctl->bfull[s]), par, ctl);
+          ok = __all_sync(0xFFFFFFFFu, ok);
           if (!ok) break;
-          fence_proxy_async();  // the gathered rows were written through the generic proxy
-          tc_fence_after();
-          const uint32_t a_addr = tiles_addr + s * stage_bytes;
-          const uint64_t db = make_desc_kb<KB>(a_addr + kAStage);
           const bool second = st >= nst_main;
-          const int kb = second ? st - nst_main : st % kblocks;
-          // with several offsets per stage the whole 64-channel block is always filled (unused slots with zeros)
-          const int ksteps = (SLOTS > 1 && !second) ? 4 : min(KB / 16, ((second ? sec.cin2 : cin) - kb * KB) >> 4);
-          for (int k = 0; k < ksteps; ++k) {
+          if (st == nst_main) kb = 0;
+          if (elect_one()) {
+            fence_proxy_async();  // the gathered rows were written through the generic proxy
+            tc_fence_after();
+            const uint32_t a_addr = tiles_addr + s * stage_bytes;
+            const uint64_t db = make_desc_kb<KB>(a_addr + kAStage);
+            // with several offsets per stage the whole 64-channel block is always filled (unused slots with zeros)
+            const int ksteps = (SLOTS > 1 && !second) ? 4 : min(KB / 16, ((second ? sec.cin2 : cin) - kb * KB) >> 4);
 #pragma unroll
-            for (int sub = 0; sub < SUB; ++sub) {  // the same weight block feeds every sub-tile
-              const uint64_t da = make_desc_kb<KB>(a_addr + sub * (kTileM * kRowBytes));
-              tc_mma_f16(tmem_acc + static_cast<uint32_t>(sub * cout), da + static_cast<uint64_t>(k * 2),
-                         db + static_cast<uint64_t>(k * 2), idesc, accumulate);
+            for (int k = 0; k < KB / 16; ++k) {
+              if (k < ksteps) {
+#pragma unroll
+                for (int sub = 0; sub < SUB; ++sub) {  // the same weight block feeds every sub-tile
+                  const uint64_t da = make_desc_kb<KB>(a_addr + sub * (kTileM * kRowBytes));
+                  tc_mma_f16(tmem_acc + static_cast<uint32_t>(sub * cout), da + static_cast<uint64_t>(k * 2),
+                             db + static_cast<uint64_t>(k * 2), idesc, k > 0 ? 1u : accumulate);
+                }
+              }
             }
-            accumulate = 1;
+            tc_commit(smem_u32(&ctl->empty[s]));
           }
-          tc_commit(smem_u32(&ctl->empty[s]));
+          __syncwarp();
+          accumulate = 1;
+          if (++kb == kblocks && !second) kb = 0;
         }
         if (!ok) break;
-        if (nst > 0)
-          tc_commit(smem_u32(&ctl->accfull[buf]));  // arrives when every MMA of the tile has finished
-        else
-          mbar_arrive(smem_u32(&ctl->accfull[buf]));  // no MMA was issued: the epilogue writes zeros
+        if (elect_one()) {
+          if (nst > 0)
+            tc_commit(smem_u32(&ctl->accfull[buf]));  // arrives when every MMA of the tile has finished
+          else
+            mbar_arrive(smem_u32(&ctl->accfull[buf]));  // no MMA was issued: the epilogue writes zeros
+        }
+        __syncwarp();
       }
     }
     __syncwarp();
