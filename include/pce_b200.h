@@ -405,6 +405,9 @@ PCE_API int32_t pce_conv_split_parts(int32_t n_rows, int32_t n_src, int32_t c_in
  * outputs gathered from n_src input rows; 0 = the layer runs whole. */
 PCE_API size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
+/* The same, but 0 where such a split was measured slower than the whole layer. */
+PCE_API size_t pce_conv_split_scratch_wanted(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
+                                            int32_t kv, int32_t sm_count);
 
 /* Which kernel family pce_conv_fwd runs for these channel counts: PCE_KERNEL_SIMT,
  * PCE_KERNEL_UMMA, or -1 when the forced choice is unsupported. */

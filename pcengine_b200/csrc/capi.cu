@@ -24,6 +24,7 @@ extern int umma_kb32_enabled;
 extern int plan_short_route;
 int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
+size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 extern int kmap_sort_top_bits;
 int conv_umma(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out, int cin,
               int cout, void* out, const pce_epilogue* ep, cudaStream_t st);
@@ -133,6 +134,12 @@ size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in,
                                     int32_t sm_count) {
   if (!conv_umma_supported(c_in, c_out, PCE_F16) || kv > 128) return 0;
   return conv_split_scratch_bytes(n_rows, n_src, c_in, c_out, kv, sm_count);
+}
+
+size_t pce_conv_split_scratch_wanted(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out, int32_t kv,
+                                    int32_t sm_count) {
+  if (!conv_umma_supported(c_in, c_out, PCE_F16) || kv > 128) return 0;
+  return conv_split_scratch_wanted(n_rows, n_src, c_in, c_out, kv, sm_count);
 }
 
 int32_t pce_conv_takes_lists(int32_t c_in, int32_t c_out, int32_t kv, int32_t dtype) {

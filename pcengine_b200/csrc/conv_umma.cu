@@ -309,27 +309,34 @@ __global__ void k_pack_weight_slots(const __half* __restrict__ w, int kv, int ci
   }
 }
 
-// Work of tiles [0, t): their stages plus one unit per tile for its fixed cost (epilogue).
-__device__ __forceinline__ long long cost_before(const int* tile_ptr, int t) {
-  return (tile_ptr ? static_cast<long long>(__ldg(tile_ptr + t)) : static_cast<long long>(t)) + t;
+// Work of tiles [0, t): `unit` per stage, and one per tile for its fixed cost (the epilogue).  A listed offset of up to 64
+// channels costs about what the tile itself does, a wider one twice that (64->64 on 1.5 M rows 118 us with 1:1, 123 with
+// 2:1; 128->128 on 200 k rows 53 with 1:1, 51 with 2:1).
+__device__ __forceinline__ long long cost_before(const int* tile_ptr, int t, int unit) {
+  return static_cast<long long>(unit) * (tile_ptr ? static_cast<long long>(__ldg(tile_ptr + t)) : static_cast<long long>(t)) + t;
 }
 
-// First tile whose preceding work reaches `target` (cost_before is strictly increasing), found by a
-// whole warp: 32 probes per round, so a list of n tiles takes log32(n) dependent loads instead of the
+// The tile that begins nearest to the point where the work reaches `target`: a share then misses its due by at most half
+// a tile at each end.  (Cut at the first tile behind that point it was a whole tile at one end, and tiles hold 1 to 27
+// stages where a share holds about 15.)  cost_before is strictly increasing.  Found by a whole warp: 32 probes per round, so a list of n tiles takes log32(n) dependent loads instead of the
 // log2(n) of a binary search (about 20 L2 round trips per CTA for both ends of its range, a fixed
 // 15 us that was a tenth of the large layers and a third of the small ones).
-__device__ __forceinline__ int warp_tile_at_cost(const int* tile_ptr, int n_tiles, long long target, int lane) {
+__device__ __forceinline__ int warp_tile_at_cost(const int* tile_ptr, int n_tiles, long long target, int unit, int lane) {
   int lo = 0, hi = n_tiles;  // the answer lies in [lo, hi]
   while (lo < hi) {
     const int step = (hi - lo + 31) / 32;
     const int p = min(lo + (lane + 1) * step - 1, hi - 1);
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, cost_before(tile_ptr, p) >= target);
-    if (m == 0) return hi;  // no tile in [lo, hi) reaches the target
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, cost_before(tile_ptr, p, unit) >= target);
+    if (m == 0) {  // no tile in [lo, hi) reaches the target
+      lo = hi;
+      break;
+    }
     const int f = __ffs(m) - 1;
     const int hit = min(lo + (f + 1) * step - 1, hi - 1);
     lo = f == 0 ? lo : min(lo + f * step - 1, hi - 1) + 1;
     hi = hit;
   }
+  if (lo > 0 && target - cost_before(tile_ptr, lo - 1, unit) < cost_before(tile_ptr, lo, unit) - target) --lo;
   return lo;
 }
 
@@ -447,9 +454,10 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
   } else if (warp < 2) {
     // this CTA's contiguous share of the tiles, balanced by work: warp 0 finds its first tile,
     // warp 1 the next CTA's first tile
-    const long long total = cost_before(ls.tile_ptr, n_tiles);
+    const int unit = kblocks > 1 ? 2 : 1;
+    const long long total = cost_before(ls.tile_ptr, n_tiles, unit);
     const unsigned b = blockIdx.x + warp;
-    const int t = b >= gridDim.x ? n_tiles : warp_tile_at_cost(ls.tile_ptr, n_tiles, total * b / gridDim.x, lane);
+    const int t = b >= gridDim.x ? n_tiles : warp_tile_at_cost(ls.tile_ptr, n_tiles, total * b / gridDim.x, unit, lane);
     if (lane == 0) ctl->range[warp] = t;
   }
   tc_fence_before();
@@ -1002,9 +1010,10 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 2 + 4 * EPIW), SUB == 1 ? 2 : 
   }
   if (!ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (warp < 2) {
-    const long long total = cost_before(ls.tile_ptr, n_tiles);
+    const int unit = kblocks > 1 ? 2 : 1;
+    const long long total = cost_before(ls.tile_ptr, n_tiles, unit);
     const unsigned b = blockIdx.x + warp;
-    const int t = b >= gridDim.x ? n_tiles : warp_tile_at_cost(ls.tile_ptr, n_tiles, total * b / gridDim.x, lane);
+    const int t = b >= gridDim.x ? n_tiles : warp_tile_at_cost(ls.tile_ptr, n_tiles, total * b / gridDim.x, unit, lane);
     if (lane == 0) ctl->range[warp] = t;
   }
   tc_fence_before();
@@ -1610,7 +1619,20 @@ int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_co
   const long long slots = static_cast<long long>(sm_count > 0 ? sm_count : 148) * (cout <= 128 ? 3 : 2);
   int p = 8;
   while (p > 1 && (n_tiles * p > slots || chain < 8 * p)) p >>= 1;
-  return p;
+  // Of those, what the estimate says is worth most, in us: a stage of the chain is 0.75, and the partial sums are written
+  // and read at about 6 TB/s by a second kernel (5 to set up).  Chains of one K block never repay it (64->64 on 3 k to
+  // 25 k rows: 20 us whole, 22 in parts); 128->256 on 15 k rows 36 whole, 40 in two, but on 7.5 k rows 35 and 32 in four.
+  if (chain <= 16) return 1;
+  int best = 1;
+  double most = 0.0;
+  for (; p > 1; p >>= 1) {
+    const double gain = 0.75 * chain * (p - 1) / p - 5.0 - 8.0 * p * n_rows * cout / 6e6;
+    if (gain > most) {
+      most = gain;
+      best = p;
+    }
+  }
+  return best;
 }
 
 // Maps of half a wave to one wave of tiles (tiles / CTA slots in (0.5, 1]) that conv_split_parts leaves
@@ -1641,6 +1663,14 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
   if (parts > 1) return static_cast<size_t>(parts) * n_rows * cout * sizeof(float);
   const int grid = conv_streamk_grid(n_rows, n_src, cin, cout, kv, sm_count);
   return grid > 0 ? static_cast<size_t>(grid) * 2 * umma::kTileM * cout * sizeof(float) : 0;
+}
+
+// The same where a split was measured faster; the framework's own callers ask this one.  Equal shares of stages repay
+// their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
+// 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
+size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
+  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) == 1 && chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
+  return conv_split_scratch_bytes(n_rows, n_src, cin, cout, kv, sm_count);
 }
 
 // tiles == nullptr: the dense rows x matrix product (every row fetches itself, one offset).

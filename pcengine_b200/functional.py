@@ -122,7 +122,7 @@ def _split_scratch(n_rows: int, n_src: int, c_in: int, c_out: int, kv: int, devi
     sms = _SM_COUNT.get(idx)
     if sms is None:
         sms = _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    nbytes = int(lib.pce_conv_split_scratch_bytes(n_rows, n_src, c_in, c_out, kv, sms))
+    nbytes = int(lib.pce_conv_split_scratch_wanted(n_rows, n_src, c_in, c_out, kv, sms))
     if nbytes <= 0:
         return None
     return torch.empty((nbytes // 4,), dtype=torch.float32, device=device)
