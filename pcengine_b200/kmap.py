@@ -232,10 +232,9 @@ class _DenseTables:
         # A submanifold map with odd kernel sizes is its own transpose under kp -> kv-1-kp, so
         # the output-major table is read out of `map`; otherwise it is written separately.
         self.map_out = None if self.symmetric else torch.empty((kv * max(self.n_out, 1),), dtype=torch.int32, device=dev)
-        self.knnz = torch.empty((kv,), dtype=torch.int32, device=dev)
-        self.kpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
-        self.qkpos = torch.empty((kv + 1,), dtype=torch.int32, device=dev)
-        self.status = torch.zeros((1,), dtype=torch.int32, device=dev)
+        # one array, so that one copy reads the totals back: [knnz | kpos | qkpos | status]
+        self.words = torch.zeros((3 * kv + 3,), dtype=torch.int32, device=dev)
+        self.knnz, self.kpos, self.qkpos, self.status = self.words.split_with_sizes((kv, kv + 1, kv + 1, 1))
         _lib.check(lib.pce_map_build_d2(in_coords.data_ptr(), self.n_in, self.out_coords.data_ptr(), self.n_out,
                                         C.byref(self.geom), ws.data_ptr(), ws.numel(), _lib.ptr(self.map),
                                         self.knnz.data_ptr(), self.kpos.data_ptr(), self.qkpos.data_ptr(),
@@ -362,11 +361,10 @@ class KernelMap:
             pairs = [v for kp, v in enumerate(state[32: 32 + self.kv]) if kp != self.mid]
             self._sizes = (sum(pairs), sum((v + 127) // 128 * 128 for v in pairs))
         if self._sizes is None:
-            self.build()
-            host = torch.stack([self.kpos[-1], self.qkpos[-1], self.status[0]]).cpu()
-            if int(host[2]) != 0:
-                _lib.check(int(host[2]), "kernel map build")
-            self._sizes = (int(host[0]), int(host[1]))
+            host = self._dense.build().words.tolist()
+            if host[-1] != 0:
+                _lib.check(host[-1], "kernel map build")
+            self._sizes = (host[2 * self.kv], host[-2])
         return self._sizes
 
     # -- neighbour CSR + bitmask (what pce_conv_fwd consumes) ---------------
@@ -436,15 +434,16 @@ class KernelMap:
         """(imap_coded [P], icsr [n_in+1], omap_coded [P], ocsr [n_out+1]): the CSR-coded
         gather/scatter map of backend/hash.cu:20-255 with canonical positions."""
         if self._d1 is None:
+            d = self._dense.build()
             p, _ = self.sizes()
             dev = self.device
             imap_c = torch.empty((max(p, 1),), dtype=torch.int32, device=dev)
             omap_c = torch.empty((max(p, 1),), dtype=torch.int32, device=dev)
             icsr = torch.empty((self.n_in + 1,), dtype=torch.int32, device=dev)
             ocsr = torch.empty((self.n_out + 1,), dtype=torch.int32, device=dev)
-            ws = _lib.workspace(8 * self.kv * max(self.n_in, 1) + 8 * (max(self.n_in, self.n_out) + 1) + (16 << 20), dev)
-            _lib.check(lib.pce_map_build_d1(_lib.ptr(self.map), _lib.ptr(self.map_out), self.kv, self.n_in, self.n_out,
-                                            1 if self.symmetric else 0, self.kpos.data_ptr(), ws.data_ptr(), ws.numel(),
+            ws = _lib.workspace(4 * self.kv * self.n_in + 4 * (self.n_in + self.n_out) + (1 << 20), dev)
+            _lib.check(lib.pce_map_build_d1(_lib.ptr(d.map), _lib.ptr(d.map_out), self.kv, self.n_in, self.n_out,
+                                            1 if d.symmetric else 0, d.kpos.data_ptr(), ws.data_ptr(), ws.numel(),
                                             imap_c.data_ptr(), icsr.data_ptr(), omap_c.data_ptr(), ocsr.data_ptr(),
                                             _lib.stream_ptr(dev)), "pce_map_build_d1")
             self._d1 = (imap_c[:p], icsr, omap_c[:p], ocsr)
