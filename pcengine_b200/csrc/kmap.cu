@@ -1267,7 +1267,7 @@ int pce_order_lists(uint32_t* mask, const int32_t* starts, const int32_t* nbr, c
                                 const_cast<int*>(t.stage_kp), const_cast<int*>(t.stage_nbr), stage_caps[v]};
     if (!t.tile_ptr || (n > 0 && (!t.stage_kp || !t.stage_nbr))) return PCE_ERR_INVALID;
   }
-  return blk::order_lists(o, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  return blk::order_lists(o, workspace, workspace_bytes, true, static_cast<cudaStream_t>(stream));
 }
 
 size_t pce_parents_workspace_bytes(int32_t n) { return blk::chain_bytes(n, 1, false); }

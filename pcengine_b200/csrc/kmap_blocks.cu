@@ -579,6 +579,7 @@ __device__ __forceinline__ unsigned key_of_mask(unsigned m, const int* pos) {
 // ---- up to 64 k rows: one cluster ----
 constexpr int kClusterBlocks = 8, kClusterThreads = 1024, kClusterWarps = 32, kClusterItems = 8;
 constexpr int kClusterRows = kClusterBlocks * kClusterThreads * kClusterItems;
+constexpr int kClusterRowsAlone = 24576;  // with the GPU to itself, more blocks end sooner from there on (60 k rows: 51 us, 31)
 constexpr int kClusterBins = 1 << kOrderBits;
 
 struct ClusterShared {
@@ -976,11 +977,13 @@ int subm_dense(const int* coords, int n, const pce_geom* g, void* ws, size_t ws_
 
 // ---- order and lists ----
 
-// Blocks of the cooperative sort: 4096 rows each.  Its blocks hold their SMs while they wait for one another, beside the
-// convolutions of the pass that runs at the time; fewer rows per block end sooner alone and cost the pass more.
-static int order_grid(int n) {
+// Blocks of the cooperative sort.  They hold their SMs while they wait for one another: beside the convolutions of a
+// pass that runs at the time, 4096 rows each; alone fewer rows each end sooner (60 k rows: 37 us with 4096, 31 with 1024;
+// 120 k: 41, and 37 with 2048; from 256 k on nothing is gained).
+static int order_grid(int n, bool alone) {
   const int sms = device_sm_count();
-  return std::max(1, std::min(div_up(n, 8 * coop::kThreads), sms > 0 ? sms : 1));
+  const int rows = (!alone || n > (1 << 18)) ? 8 : (n > (1 << 16) ? 4 : 2);
+  return std::max(1, std::min(div_up(n, rows * coop::kThreads), sms > 0 ? sms : 1));
 }
 
 size_t order_workspace_bytes(int n) {
@@ -988,7 +991,7 @@ size_t order_workspace_bytes(int n) {
   return 4 * pad256(4 * m) + 1024 * ((1 << kOrderBits) + 32) * sizeof(int) + 4096;
 }
 
-int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st) {
+int order_lists(Order o, void* ws, size_t ws_bytes, bool alone, cudaStream_t st) {
   if (o.n < 0 || o.kv < 1 || o.kv > 32 || o.n_variants < 0 || o.n_variants > kMaxVariants) return PCE_ERR_INVALID;
   for (int v = 0; v < o.n_variants; ++v) {
     const Variant& V = o.variant[v];
@@ -998,7 +1001,7 @@ int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st) {
     if (o.n == 0) PCE_CUDA(cudaMemsetAsync(V.tile_ptr, 0, sizeof(int), st));
   }
   if (o.n == 0) return PCE_OK;
-  if (o.n <= kClusterRows) {
+  if (o.n <= (alone ? kClusterRowsAlone : kClusterRows)) {
     static bool attr_set[64] = {};
     int dev = 0;
     PCE_CUDA(cudaGetDevice(&dev));
@@ -1011,7 +1014,7 @@ int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st) {
     PCE_LAUNCH_CHECK();
   } else {
     Arena ar(ws, ws_bytes);
-    int g = order_grid(o.n);
+    int g = order_grid(o.n, alone);
     o.key0 = ar.take<unsigned>(o.n);
     o.key1 = ar.take<unsigned>(o.n);
     o.val0 = ar.take<int>(o.n);

@@ -106,7 +106,7 @@ int query_lists(const int* coords, int n, const Query& q, cudaStream_t st);
 
 size_t order_workspace_bytes(int n);
 // Row order and lists; o's scratch members are placed in `ws`.
-int order_lists(Order o, void* ws, size_t ws_bytes, cudaStream_t st);
+int order_lists(Order o, void* ws, size_t ws_bytes, bool alone, cudaStream_t st);  // alone: no pass computes meanwhile
 
 // The voxels of the levels >= 1 of a chain of parent layers.  `geoms[l]` leads to level l + 1 (cmin / cmax: its output
 // bounds).  keep0: also build the table and row table of the input level.

@@ -463,7 +463,7 @@ static int build_direction(pce_plan* p, PlanLane* l, pce_pass* ps, blk::Order o,
   if (!o.order) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
   void* ws = nullptr;
   PCE_TRY(scratch_for(l, blk::order_workspace_bytes(o.n), &ws));
-  PCE_TRY(blk::order_lists(o, ws, l->scratch_cap, l->stream));
+  PCE_TRY(blk::order_lists(o, ws, l->scratch_cap, false, l->stream));
   for (int v = 0; v < o.n_variants; ++v) {
     const blk::Variant& V = o.variant[v];
     out->lists[out->n_lists++] = pce_tile_lists{o.order, V.tile_ptr, V.stage_kp, V.stage_nbr, V.tile_rows, identity_stage, V.slots, 1};
