@@ -329,12 +329,15 @@ PCE_API int32_t pce_conv_takes_lists(int32_t c_in, int32_t c_out, int32_t kv, in
 
 /* Processing order for the tensor-core kernel: output rows sorted (stable radix sort) by
  * their indicator bitmask with the bits permuted by rarity, the rarest offset most
- * significant, so rows with the same neighbourhood pattern land in the same tile, rows
+ * significant (kv > 64: by their five rarest offsets, then bitmask by bitmask), so rows with the same neighbourhood pattern land in the same tile, rows
  * with a rare offset land next to each other, and a tile skips every offset none of its
  * rows has.  Purely a scheduling aid with no reference counterpart.  order[n_rows]
  * receives the permutation; kv <= 128; workspace >= 64*n_rows + 16 MiB bytes. */
 PCE_API int pce_csr_sort_rows(const uint32_t* mask, int32_t n_rows, int32_t kv, void* workspace,
                               size_t workspace_bytes, int32_t* order, void* stream);
+/* The same for a caller that knows offset_counts[kv], the rows that have each offset. */
+PCE_API int pce_csr_sort_rows_counted(const uint32_t* mask, const int32_t* offset_counts, int32_t n_rows, int32_t kv,
+                                      void* workspace, size_t workspace_bytes, int32_t* order, void* stream);
 
 /* Fills the arrays of a pce_tile_lists from the neighbour CSR and a row order (NULL =
  * natural order) for tiles of tile_rows = 128, 256 or 512 rows.  tile_ptr needs

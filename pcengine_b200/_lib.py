@@ -27,7 +27,7 @@ EXPORTS = [
     "pce_strerror", "pce_version", "pce_last_cuda_error", "pce_kernel_launches", "pce_map_workspace_bytes", "pce_downsample_coords",
     "pce_map_build_d2", "pce_map_build_d2_noalloc", "pce_map_pairs", "pce_subm_workspace_bytes", "pce_subm_neighbours", "pce_order_workspace_bytes", "pce_order_lists",
     "pce_parents_workspace_bytes", "pce_parents", "pce_map_build_d1", "pce_csr_from_dense", "pce_csr_from_pairs",
-    "pce_csr_from_pairs_workspace_bytes", "pce_csr_sort_rows", "pce_build_tile_lists", "pce_conv_kernel_choice", "pce_conv_takes_lists", "pce_conv_split_parts", "pce_conv_split_scratch_bytes", "pce_conv_split_scratch_wanted", "pce_conv_fwd", "pce_packed_weights_bytes",
+    "pce_csr_from_pairs_workspace_bytes", "pce_csr_sort_rows", "pce_csr_sort_rows_counted", "pce_build_tile_lists", "pce_conv_kernel_choice", "pce_conv_takes_lists", "pce_conv_split_parts", "pce_conv_split_scratch_bytes", "pce_conv_split_scratch_wanted", "pce_conv_fwd", "pce_packed_weights_bytes",
     "pce_pack_weights", "pce_device_status", "pce_debug_timeout", "pce_tune", "pce_conv_fwd_d1", "pce_linear_fwd", "pce_scale_shift_act", "pce_batchnorm", "pce_push_rows",
     "pce_quantize_workspace_bytes", "pce_quantize_unique", "pce_voxelise", "pce_collate_coords", "pce_tile_rows_for", "pce_plan_create", "pce_plan_destroy", "pce_plan_begin", "pce_pass_map", "pce_pass_release", "pce_net_run",
 ]
@@ -123,6 +123,7 @@ def _load() -> C.CDLL:
                                  C.POINTER(Epilogue), i32, vp]
     lib.pce_build_tile_lists.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, sz, vp, vp, vp, i32, vp]
     lib.pce_csr_sort_rows.argtypes = [vp, i32, i32, vp, sz, vp, vp]
+    lib.pce_csr_sort_rows_counted.argtypes = [vp, vp, i32, i32, vp, sz, vp, vp]
     lib.pce_packed_weights_bytes.restype = sz
     lib.pce_packed_weights_bytes.argtypes = [i32, i32, i32]
     lib.pce_pack_weights.argtypes = [vp, i32, i32, i32, i32, vp, vp]

@@ -127,8 +127,9 @@ class NeighbourCSR:
             dev = self._mask.device
             out = torch.empty((self.n_rows,), dtype=torch.int32, device=dev)
             ws = _lib.workspace(64 * self.n_rows + (16 << 20), dev)
-            _lib.check(lib.pce_csr_sort_rows(self.mask.data_ptr(), self.n_rows, self.kv, ws.data_ptr(), ws.numel(),
-                                             out.data_ptr(), _lib.stream_ptr(dev)), "pce_csr_sort_rows")
+            _lib.check(lib.pce_csr_sort_rows_counted(self.mask.data_ptr(), _lib.ptr(self._counts), self.n_rows, self.kv,
+                                                     ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.stream_ptr(dev)),
+                       "pce_csr_sort_rows_counted")
             self._order = out
         return self._order
 
