@@ -466,10 +466,8 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
   const uint32_t tmem_base = ctl->tmem_base;
 
   const int t0 = ctl->range[0], t1 = ctl->range[1];
-  // stage range of tile t that this CTA works on: the whole tile, or its part
-  auto stage_range = [&](int t, int& sa, int& sb) {
-    sa = first_stage(ls.tile_ptr, t);
-    sb = first_stage(ls.tile_ptr, t + 1);
+  // stage range of a tile (its stages [sa, sb)) that this CTA works on: the whole tile, or its part
+  auto stage_range = [&](int& sa, int& sb) {
     if (streamk) {
       sa = max(sa, sk_begin);
       sb = min(sb, sk_end);
@@ -480,27 +478,35 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
       sa = a;
     }
   };
-  // streamk: does this CTA hold only a piece of tile t?
-  auto tile_cut = [&](int t) {
-    return streamk && (sk_begin > first_stage(ls.tile_ptr, t) || sk_end < first_stage(ls.tile_ptr, t + 1));
+  // The tiles' bounds, read a tile ahead: between two tiles the accumulator's hand-over is all there is to wait for.
+  // main: ring stages of the listed offsets (of this CTA's part); ident: with the identity stage, which is the tile's
+  // last and counts with the second operand's K blocks (none without one); cut: stream-K, only a piece of the tile.
+  struct Work {
+    int main, ident;
+    bool cut;
   };
-  // ring stages of tile t (this CTA's part of it): its listed offsets times the K blocks; the identity
-  // stage, which is the tile's last, counts with the second operand's K blocks (none without one)
-  auto tile_ident = [&](int t) {
-    int sa, sb;
-    stage_range(t, sa, sb);
-    return (ls.identity && sb > sa && sb == first_stage(ls.tile_ptr, t + 1)) ? 1 : 0;
+  int bound0 = 0, bound1 = 0, bound2 = 0;
+  auto first_bounds = [&]() {
+    bound1 = first_stage(ls.tile_ptr, t0);
+    bound2 = t0 < t1 ? first_stage(ls.tile_ptr, t0 + 1) : bound1;
   };
-  auto tile_main_stages = [&](int t) {
-    int sa, sb;
-    stage_range(t, sa, sb);
-    return (sb - sa - tile_ident(t)) * kblocks;
+  auto next_work = [&](int t) {
+    bound0 = bound1;
+    bound1 = bound2;
+    if (t + 1 < t1) bound2 = first_stage(ls.tile_ptr, t + 2);
+    int sa = bound0, sb = bound1;
+    stage_range(sa, sb);
+    Work w;
+    w.ident = (ls.identity && sb > sa && sb == bound1) ? 1 : 0;
+    w.main = (sb - sa - w.ident) * kblocks;
+    w.cut = streamk && (sa > bound0 || sb < bound1);
+    return w;
   };
 
   if (warp < kMmaWarp) {
     // =========================== producers ===========================
     int g0 = first_stage(ls.tile_ptr, t0), g1 = first_stage(ls.tile_ptr, t1);
-    if (parts > 1) stage_range(t0, g0, g1);
+    if (parts > 1) stage_range(g0, g1);
     if (streamk) {
       g0 = sk_begin;
       g1 = sk_end;
@@ -694,11 +700,13 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
       const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(cout >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
       int j = 0;
       bool ok = true;
+      first_bounds();
       for (int t = t0; t < t1 && ok; ++t) {
         const int it = t - t0;
         const int buf = it % nacc;
-        const int nst_main = tile_main_stages(t);
-        const int nst = nst_main + (tile_ident(t) ? kblocks2 : 0);
+        const Work work = next_work(t);
+        const int nst_main = work.main;
+        const int nst = nst_main + (work.ident ? kblocks2 : 0);
         // the accumulator must have been drained by the epilogue (two tiles ago)
         if (it >= nacc) ok = mbar_wait(smem_u32(&ctl->accempty[buf]), ((it / nacc) - 1) & 1, ctl);
         ok = __all_sync(0xFFFFFFFFu, ok);
@@ -759,8 +767,10 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
     const bool wide_out = (ep.ld_out & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0;
     const bool wide_res = (reinterpret_cast<uintptr_t>(ep.residual) & 31) == 0;  // (rows of C_out = 16k channels)
     if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
+    first_bounds();
     for (int t = t0; t < t1; ++t) {
       const int it = t - t0;
+      const Work work = next_work(t);
       const int buf = it % nacc;
       int rows_of[SUB];
 #pragma unroll
@@ -769,8 +779,8 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         rows_of[sub] = n_out;
         if (slot < n_out) rows_of[sub] = ls.order ? __ldg(ls.order + slot) : slot;
       }
-      const bool any = tile_main_stages(t) + (tile_ident(t) ? kblocks2 : 0) > 0;
-      const bool cut = tile_cut(t);
+      const bool any = work.main + (work.ident ? kblocks2 : 0) > 0;
+      const bool cut = work.cut;
       if (ep.residual) {
         // the rows are known before the accumulator is: pull the residual rows into L2 while waiting
 #pragma unroll
