@@ -42,6 +42,7 @@ class TileLists(C.Structure):
     _fields_ = [("order", C.c_void_p), ("tile_ptr", C.c_void_p), ("stage_kp", C.c_void_p), ("stage_nbr", C.c_void_p),
                 ("tile_rows", C.c_int32), ("identity_stage", C.c_int32), ("slots", C.c_int32),
                 ("settled", C.c_int32)]
+    stream = None  # the stream of the last launch that used the lists (Python side only)
 
 
 PLAN_MAX_USES = 8

@@ -304,11 +304,19 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
                    start=torch.cuda.Event(enable_timing=True), end=torch.cuda.Event(enable_timing=True))
         rec["start"].record()
     tiles = split = None
+    stream = _lib.stream_ptr(feats.device)
     if packed is not None:
         # (the halo push lives in the one-accumulator kernel: 128-row tiles)
         pushes = epilogue is not None and epilogue.push_slots is not None
         rows = TILE_ROWS or (128 if pushes else _auto_tile_rows(csr.n_rows, c_in, c_out, feats.device))
-        tiles = C.byref(csr.tiles(SORT_ROWS, rows, second, stage_slots(c_in)))
+        lists = csr.tiles(SORT_ROWS, rows, second, stage_slots(c_in))
+        # The first launch that uses the lists waits for the kernels before it.  Behind it on the same stream they are
+        # complete before the kernel that precedes a launch, which may then read them during its set-up, while that
+        # kernel is still finishing.
+        if not lists.settled:
+            lists.settled = 1 if lists.stream == stream else 0
+            lists.stream = stream
+        tiles = C.byref(lists)
         if rows == 128 and not pushes:
             split = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
     elif (kernel_choice == "auto" and feats.dtype == torch.float32
@@ -321,7 +329,7 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
                                 csr.mask.data_ptr(), _lib.ptr(rowptr), _lib.ptr(nbr), tiles, csr.n_rows,
                                 out.data_ptr(), _lib.dtype_code(feats.dtype),
                                 _pack(epilogue, c_out, csr.n_rows, feats.dtype, in_ld, out_ld, split),
-                                _KERNEL[kernel_choice], _lib.stream_ptr(feats.device)), "pce_conv_fwd")
+                                _KERNEL[kernel_choice], stream), "pce_conv_fwd")
     if rec is not None:
         rec["end"].record()
         rec["pairs"] = csr.pair_count()  # (a new tensor: the record must not keep the map's storage alive)

@@ -152,22 +152,16 @@ class NeighbourCSR:
         hit = self._tiles.get(key)
         if hit is None and not identity:
             hit = self._tiles.get((bool(sort_rows), tile_rows, True, int(slots)))
-        if hit is not None:
-            # kept from an earlier call: once the kernels that built the lists have finished, a launch
-            # may read the lists during its set-up (while the kernel before it is still finishing)
-            if not hit[0].settled and (len(hit) < 6 or hit[5].query()):
-                hit[0].settled = 1
-            return hit[0]
-        hit = self._tiles[key] = self._build_tiles(*key)
+        if hit is None:
+            hit = self._tiles[key] = self._build_tiles(*key)
         return hit[0]
 
     def _build_tiles(self, sort_rows: bool, tile_rows: int, identity: bool, slots: int):
         dev = self._mask.device
         n_tiles = (self.n_rows + tile_rows - 1) // tile_rows
         cap = max(1, n_tiles * ((self.kv + slots - 1) // slots + (1 if identity else 0)))
-        tile_ptr = torch.empty((n_tiles + 1,), dtype=torch.int32, device=dev)
-        stage_kp = torch.empty((cap * slots,), dtype=torch.int32, device=dev)
-        stage_nbr = torch.empty((cap * slots * tile_rows,), dtype=torch.int32, device=dev)
+        hit = _TileSet(cap * slots, tile_rows, n_tiles, dev)
+        tile_ptr, stage_kp, stage_nbr = hit.pointers()
         if sort_rows and self._order is None and self.kv <= 32 and self.n_rows > 0:
             order = self._order_and_lists(tile_rows, identity, slots, tile_ptr, stage_kp, stage_nbr, cap)
         else:
@@ -176,13 +170,11 @@ class NeighbourCSR:
             ws = _lib.workspace(8 * (n_tiles + 1) + (1 << 20), dev)
             _lib.check(lib.pce_build_tile_lists(self.mask.data_ptr(), starts.data_ptr(), nbr.data_ptr(), order.data_ptr(),
                                                 self.n_rows, self.kv, tile_rows, 1 if identity else 0, int(slots), ws.data_ptr(),
-                                                ws.numel(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(), cap,
+                                                ws.numel(), tile_ptr, stage_kp, stage_nbr, cap,
                                                 _lib.stream_ptr(dev)), "pce_build_tile_lists")
-        st = _lib.TileLists(order.data_ptr(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(),
-                            tile_rows, 1 if identity else 0, int(slots), 0)
-        built = torch.cuda.Event()
-        built.record(torch.cuda.current_stream(dev))
-        return (st, order, tile_ptr, stage_kp, stage_nbr, built)
+        hit.order = order
+        hit.struct = _lib.TileLists(order.data_ptr(), tile_ptr, stage_kp, stage_nbr, tile_rows, 1 if identity else 0, int(slots), 0)
+        return hit
 
     def _order_and_lists(self, tile_rows, identity, slots, tile_ptr, stage_kp, stage_nbr, cap):
         """The row order (kept) and one set of lists in one launch, from the form at hand."""
@@ -195,8 +187,7 @@ class NeighbourCSR:
             table = self._table
         else:
             starts, nbr = self.rowptr, self.nbr
-        want = _lib.TileLists(order.data_ptr(), tile_ptr.data_ptr(), stage_kp.data_ptr(), stage_nbr.data_ptr(), tile_rows,
-                              1 if identity else 0, int(slots), 0)
+        want = _lib.TileLists(order.data_ptr(), tile_ptr, stage_kp, stage_nbr, tile_rows, 1 if identity else 0, int(slots), 0)
         caps = (C.c_int32 * 1)(cap)
         ws = _lib.workspace(lib.pce_order_workspace_bytes(self.n_rows), dev)
         _lib.check(lib.pce_order_lists(self._mask.data_ptr(), _lib.ptr(starts), _lib.ptr(nbr), _lib.ptr(table),
@@ -206,6 +197,25 @@ class NeighbourCSR:
         if table is not None:
             self._mask_ready = True
         return order
+
+
+class _TileSet:
+    """One set of tile lists: (struct, order, tile_ptr, stage_kp, stage_nbr), the lists in one allocation, whose parts
+    become tensors when somebody asks."""
+
+    __slots__ = ("struct", "order", "store", "parts")
+
+    def __init__(self, entries: int, tile_rows: int, n_tiles: int, device):
+        self.parts = (entries * tile_rows, entries, n_tiles + 1)
+        self.store = torch.empty((sum(self.parts),), dtype=torch.int32, device=device)
+
+    def pointers(self):
+        at = self.store.data_ptr()
+        return at + 4 * (self.parts[0] + self.parts[1]), at + 4 * self.parts[0], at
+
+    def __getitem__(self, i):
+        nbr, kp, ptr = self.store.split_with_sizes(self.parts) if i != 0 else (None, None, None)
+        return (self.struct, self.order, ptr, kp, nbr)[i]
 
 
 class _DenseTables:
