@@ -72,10 +72,10 @@ struct Epi {
   // may read and write a column range of a wider row-major matrix
   int ld_in;
   int ld_out;
-  // parts > 1: `parts` CTAs share every tile (CTA b: tile b / parts, part b % parts of its stage list) and
-  // store raw fp32 sums to partial[(part * n_out + row) * cout + c]; k_sum_parts finishes the layer
-  float* partial;
+  // parts > 1: a cluster of `parts` CTAs shares every tile (CTA b: tile b / parts, part b % parts of its stage list).
+  // Each leaves its fp32 sums in its own shared memory, and finishes its part of the tile's rows from all of them.
   int parts;
+  float* partial;
   // streamk: every CTA takes an equal share of the layer's STAGES (CTA b: stages S*b/G .. S*(b+1)/G of the
   // concatenated tile lists), whatever tiles they fall in.  A tile that lies in one CTA's share is finished by
   // it; a tile cut between CTAs leaves raw fp32 sums in partial[((cta*2 + slot)*128 + row-in-tile)*cout + c]
@@ -364,6 +364,42 @@ __host__ __device__ __forceinline__ int share_begin(long long total, int b, int 
   return static_cast<int>(total * b / g);
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// 16 bytes at this address of the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ float4 cluster_ld4(uint32_t addr, int rank) {
+  uint32_t there;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(there)
+               : "memory");
+  return v;
+}
+
+// The last steps for eight channels of a row whose sums (scaled and shifted) are complete: residual, activation, store.
+__device__ __forceinline__ void finish8(float (&v)[8], int row, int c0, int cout, __half* out, const Epi& ep) {
+  if (ep.residual) {
+    const uint4 r = *reinterpret_cast<const uint4*>(ep.residual + static_cast<size_t>(row) * cout + c0);
+    const __half2* h = reinterpret_cast<const __half2*>(&r);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 f = __half22float2(h[q]);
+      v[2 * q] += f.x;
+      v[2 * q + 1] += f.y;
+    }
+  }
+  uint4 o;
+  __half2* po = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    po[q] = __floats2half2_rn(act_apply(v[2 * q], ep.act, ep.slope), act_apply(v[2 * q + 1], ep.act, ep.slope));
+  *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * ep.ld_out + c0) = o;
+}
+
 // kStages = depth of the smem stage ring.  SUB = 128-row sub-tiles per tile (1 or 2): a tile of 128*SUB output rows
 // has SUB accumulators and every staged weight block feeds SUB MMAs, which halves the weight
 // traffic per row for SUB = 2.  Threads: 4*SUB producer warps, the MMA warp, 4 epilogue warps.
@@ -503,6 +539,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
     return w;
   };
 
+  bool part_any = false;  // epilogue warps of a split tile: this CTA's part has products
   if (warp < kMmaWarp) {
     // =========================== producers ===========================
     int g0 = first_stage(ls.tile_ptr, t0), g1 = first_stage(ls.tile_ptr, t1);
@@ -798,6 +835,10 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
       // last tile of this CTA: once every CTA is here (or gone), the next kernel of the stream may be
       // set up on the SMs; it waits for this grid's completion before it touches memory
       if (t == t1 - 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      if (parts > 1) {  // (one tile per CTA; its sums stay in tensor memory until the cluster adds them up below)
+        part_any = any;
+        break;
+      }
 #pragma unroll
       for (int sub = 0; sub < SUB; ++sub) {
       const int my_row = rows_of[sub];
@@ -835,15 +876,6 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         float v[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
-        if (parts > 1) {  // a part of a split tile: the raw sums go to the scratch, k_sum_parts finishes the row
-          if (store_row) {
-            float4* dst = reinterpret_cast<float4*>(
-                ep.partial + (static_cast<size_t>(blockIdx.x % parts) * n_out + my_row) * cout + c0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-          }
-          continue;
-        }
         if (cut) {  // a piece of a tile cut between CTAs: k_sum_cut_tiles adds the pieces
           float4* dst = reinterpret_cast<float4*>(
               ep.partial + ((static_cast<size_t>(blockIdx.x) * 2 + (t == t0 ? 0 : 1)) * kTileM + slot_in_tile) * cout + c0);
@@ -905,6 +937,61 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
       mbar_arrive(smem_u32(&ctl->accempty[buf]));  // 128 arrivals hand the accumulator back
     }
     tc_fence_before();
+  }
+  if constexpr (SUB == 1 && SLOTS == 1 && !PUSH) {
+    if (parts > 1) {
+      // The parts' sums, added up through the cluster's shared memory.  The ring is idle by now (the accumulator is
+      // complete, so every stage has been consumed): as many columns as fit it at a time, column groups of four
+      // outermost, so that lanes (rows) touch consecutive 16 bytes.  Part p finishes rows p * 128 / parts on.  Against
+      // sums through global memory and a second kernel: 256->256 on 7.5 k rows, four parts, 40 -> 33 us.
+      const int part = static_cast<int>(blockIdx.x) % parts;
+      const int fit = (kStages * stage_bytes / (kTileM * 4)) & ~15;
+      const int rows_each = kTileM / parts;
+      const bool scaled = ep.scale || ep.shift;
+      for (int base = 0; base < cout; base += fit) {
+        const int cols = min(fit, cout - base);
+        __syncthreads();
+        if (warp > kMmaWarp) {
+          const int r = (warp & 3) * 32 + lane;
+          const uint32_t taddr = tmem_base + static_cast<uint32_t>(base) + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+          for (int c0 = 0; c0 < cols; c0 += 16) {
+            uint32_t v[16];
+            if (part_any) {
+              tmem_ld16(taddr + c0, v);
+              tmem_ld_wait();
+            } else {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) v[q] = 0u;
+            }
+            uint4* dst = reinterpret_cast<uint4*>(tiles) + (c0 / 4) * kTileM + r;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dst[q * kTileM] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          }
+        }
+        tc_fence_before();
+        cluster_sync();
+        for (int i = tid; i < rows_each * (cols / 8); i += 32 * (4 * SUB + 5)) {
+          const int r = part * rows_each + i % rows_each, c0 = i / rows_each * 8;
+          const int slot = t0 * kTileM + r;
+          if (slot >= n_out) continue;
+          const int row = ls.order ? __ldg(ls.order + slot) : slot;
+          const uint32_t src = tiles_addr + static_cast<uint32_t>((c0 / 4) * kTileM + r) * 16u;
+          float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          for (int p = 0; p < parts; ++p) {
+            const float4 x = cluster_ld4(src, p), y = cluster_ld4(src + kTileM * 16u, p);
+            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+          }
+          const int c = base + c0;
+          if (scaled) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = fmaf(v[q], affine[c + q], affine[cout + c + q]);
+          }
+          finish8(v, row, c, cout, out, ep);
+        }
+        cluster_sync();  // (the other parts have read this CTA's sums)
+      }
+    }
   }
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -1324,47 +1411,6 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 2 + 4 * EPIW), SUB == 1 ? 2 : 
   }
 }
 
-// Second kernel of a split layer: out[row] = act((sum over parts of partial[part][row]) * scale + shift +
-// residual), parts added in ascending order in fp32; one thread per 8 output channels.
-__global__ void __launch_bounds__(256)
-    k_sum_parts(const float* __restrict__ partial, int parts, int n_out, int cout, __half* __restrict__ out, Epi ep) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the convolution kernel drains
-  const int chunks = cout >> 3;
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= static_cast<long long>(n_out) * chunks) return;
-  const int row = static_cast<int>(i / chunks), c0 = static_cast<int>(i % chunks) * 8;
-  float v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) v[q] = 0.f;
-  for (int p = 0; p < parts; ++p) {
-    const float4* src = reinterpret_cast<const float4*>(partial + (static_cast<size_t>(p) * n_out + row) * cout + c0);
-    const float4 a = __ldg(src), b = __ldg(src + 1);
-    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-    v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-  }
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    if (ep.scale || ep.shift)
-      v[q] = fmaf(v[q], ep.scale ? __ldg(ep.scale + c0 + q) : 1.f, ep.shift ? __ldg(ep.shift + c0 + q) : 0.f);
-  }
-  if (ep.residual) {
-    const uint4 r = *reinterpret_cast<const uint4*>(ep.residual + static_cast<size_t>(row) * cout + c0);
-    const __half2* h = reinterpret_cast<const __half2*>(&r);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float2 f = __half22float2(h[q]);
-      v[2 * q] += f.x;
-      v[2 * q + 1] += f.y;
-    }
-  }
-  uint4 o;
-  __half2* po = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    po[q] = __floats2half2_rn(act_apply(v[2 * q], ep.act, ep.slope), act_apply(v[2 * q + 1], ep.act, ep.slope));
-  *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * ep.ld_out + c0) = o;
-}
-
 // Second kernel of a stream-K layer: for every tile that was cut between CTAs, adds the pieces in CTA order
 // (fp32) and applies the epilogue; tiles that one CTA finished are left alone.  Block (x, t) handles 256 of the
 // tile's (row, 8 output channels) items: its first warp works out which CTAs hold pieces of tile t (consecutive
@@ -1431,22 +1477,7 @@ __global__ void __launch_bounds__(256)
     if (ep.scale || ep.shift)
       v[q] = fmaf(v[q], ep.scale ? __ldg(ep.scale + c0 + q) : 1.f, ep.shift ? __ldg(ep.shift + c0 + q) : 0.f);
   }
-  if (ep.residual) {
-    const uint4 rr = *reinterpret_cast<const uint4*>(ep.residual + static_cast<size_t>(row) * cout + c0);
-    const __half2* h = reinterpret_cast<const __half2*>(&rr);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float2 f = __half22float2(h[q]);
-      v[2 * q] += f.x;
-      v[2 * q + 1] += f.y;
-    }
-  }
-  uint4 o;
-  __half2* po = reinterpret_cast<__half2*>(&o);
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    po[q] = __floats2half2_rn(act_apply(v[2 * q], ep.act, ep.slope), act_apply(v[2 * q + 1], ep.act, ep.slope));
-  *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * ep.ld_out + c0) = o;
+  finish8(v, row, c0, cout, out, ep);
 }
 
 }  // namespace umma
@@ -1583,11 +1614,18 @@ static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in
   cfg.blockDim = dim3(32 * (4 * SUB + 5));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = umma_overlap_launches ? 1 : 0;
+  if (umma_overlap_launches) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (e.parts > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(e.parts);
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   cudaLaunchKernelEx(&cfg, umma::k_conv_umma<NS, SUB, PUSH, SLOTS, KB>, in, w, ls, sec, n_out, cin, cout, out, e, tmem_cols,
                      nacc);
 }
@@ -1600,14 +1638,8 @@ int umma_kb32_enabled = 1;
 // when the caller gives scratch (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
 int umma_split_enabled = 1;
 
-// Parts per tile for a layer of n_rows outputs: 8, 4 or 2 CTAs per tile where all of them are resident at
-// once (tiles x parts <= the SMs' CTA slots) and every part keeps a chain of at least 8 stages.  The chain of
-// a tile is estimated as min(kv, 16) offsets x K blocks: deep levels of a network, where maps are small, are
-// also where tiles have many offsets.  Measured on B200 (LiDAR scans, kernel-only): 256 -> 256 on 27 tiles
-// 104 -> 42 us with 8 parts, on 68 tiles 100 -> 54 us with 4, on 132 tiles 102 -> 77 us with 2; 384 -> 256 on
-// 132 tiles 144 -> 99 us; more parts than slots do not pay for the second kernel and the fp32 round trip
-// (189 tiles, 128 -> 256, two parts on 296 slots: 63 -> 74 us), so such maps stay unsplit.  Layers with 16 or
-// 32 input channels (shallow levels) are never split.
+// Parts per tile for a layer of n_rows outputs (8, 4, 2 or 1; see the rule below).  Layers with 16 or 32 input channels
+// (shallow levels) are never split.
 // Estimated ring stages per tile: min(kv, 16) offsets x K blocks, fewer where the map has fewer source rows than
 // output rows (a transposed 2x2x2 layer has ONE pair per output row: its tiles list up to 8 offsets, each nearly
 // empty, and splitting them only adds the partial sums; measured 16 -> 30 us on 159 tiles of 128 -> 128).
@@ -1626,23 +1658,21 @@ int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_co
   if (cin_p == 16 || cin_p == 32) return 1;
   const int chain = chain_estimate(n_rows, n_src, cin, kv);
   const long long n_tiles = (static_cast<long long>(n_rows) + umma::kTileM - 1) / umma::kTileM;
-  const long long slots = static_cast<long long>(sm_count > 0 ? sm_count : 148) * (cout <= 128 ? 3 : 2);
-  int p = 8;
-  while (p > 1 && (n_tiles * p > slots || chain < 8 * p)) p >>= 1;
-  // Of those, what the estimate says is worth most, in us: a stage of the chain is 0.75, and the partial sums are written
-  // and read at about 6 TB/s by a second kernel (5 to set up).  Chains of one K block never repay it (64->64 on 3 k to
-  // 25 k rows: 20 us whole, 22 in parts); 128->256 on 15 k rows 36 whole, 40 in two, but on 7.5 k rows 35 and 32 in four.
-  if (chain <= 16) return 1;
-  int best = 1;
-  double most = 0.0;
-  for (; p > 1; p >>= 1) {
-    const double gain = 0.75 * chain * (p - 1) / p - 5.0 - 8.0 * p * n_rows * cout / 6e6;
-    if (gain > most) {
-      most = gain;
-      best = p;
-    }
-  }
-  return best;
+  const long long sms = sm_count > 0 ? sm_count : 148;
+  const long long slots = sms * (cout <= 128 ? 3 : 2);
+  // Parts pay while their CTAs are resident at once and each keeps a few stages of a chain that costs 0.6 us a stage; eight
+  // only where they still have about an SM each.  Whole -> split, us (3x3x3, kernel only): 64->64 on 7.5 k rows 18.8 -> 9.6
+  // (4 parts; 2: 12.2), on 25 k rows 18.9 -> 14.3 (2; 4 exceed the slots: 19.6); 128->128 on 2.9 k rows 30.9 -> 12.6 (4; 8:
+  // 12.8), on 12 k rows 23.3 -> 13.7 (4); 256->256 on 7.5 k rows 60.6 -> 27.9 (4; 2: 39.6); 128->256 on 12 k rows 27 -> 22.5
+  // (2), on 23 k rows 38 -> 44 beyond the slots.  Widths that run in 32-channel blocks have half the work per stage and
+  // gain up to a wave of tiles (96->96 on 37 k rows 37.4 -> 32.8, on 54 k rows 38.5 -> 36.5, two parts).  The rows of a
+  // kernel of at most 8 offsets (down and up a level) have fewer of them than the estimate: twice the chain is asked for.
+  const int each = kv <= 8 ? 8 : 4;
+  const bool half_blocks = cin_p % 64 == 32;
+  if (3 * n_tiles * 8 <= 4 * sms && chain >= each * 8) return 8;
+  if (n_tiles * 4 <= slots && chain >= each * 4) return 4;
+  if (n_tiles * 2 <= (half_blocks ? 2 * slots : slots) && chain >= each * 2) return 2;
+  return 1;
 }
 
 // Maps of half a wave to one wave of tiles (tiles / CTA slots in (0.5, 1]) that conv_split_parts leaves
@@ -1679,7 +1709,8 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
 // their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
 // 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
-  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) == 1 && chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
+  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 16;  // (parts add up in shared memory)
+  if (chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
   return conv_split_scratch_bytes(n_rows, n_src, cin, cout, kv, sm_count);
 }
 
@@ -1846,10 +1877,8 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   if (tiles && sub == 1 && slots == 1 && !push && ep && ep->split_scratch &&
       (reinterpret_cast<uintptr_t>(ep->split_scratch) & 15) == 0) {
     parts = conv_split_parts(n_out, n_in, cin, cout, kv, sm_count[dev]);
-    while (parts > 1 && static_cast<size_t>(parts) * n_out * cout * sizeof(float) > ep->split_scratch_bytes) parts >>= 1;
     if (parts > 1) {
       grid = n_tiles * parts;
-      e.partial = static_cast<float*>(ep->split_scratch);
       e.parts = parts;
     } else {
       const int g = conv_streamk_grid(n_out, n_in, cin, cout, kv, sm_count[dev]);
@@ -1895,8 +1924,8 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
 #undef PCE_GO
   }
   PCE_LAUNCH_CHECK();
-  if (parts > 1 || streamk) {
-    // the second kernel of a split layer is set up on the SMs while the convolution's last CTAs drain
+  if (streamk) {
+    // the second kernel of a stream-K layer is set up on the SMs while the convolution's last CTAs drain
     // (programmatic dependent launch; it waits for that grid before it reads a partial sum)
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -1906,16 +1935,11 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = umma_overlap_launches ? 1 : 0;
+    cfg.gridDim = dim3(div_up(umma::kTileM * (cout >> 3), 256), n_tiles);
     const float* partial = e.partial;
-    if (parts > 1) {
-      cfg.gridDim = dim3(div_up(static_cast<long long>(n_out) * (cout >> 3), 256));
-      cudaLaunchKernelEx(&cfg, umma::k_sum_parts, partial, parts, n_out, cout, out_h, e);
-    } else {
-      cfg.gridDim = dim3(div_up(umma::kTileM * (cout >> 3), 256), n_tiles);
-      const int* tile_ptr = ls.tile_ptr;
-      const int* order = ls.order;
-      cudaLaunchKernelEx(&cfg, umma::k_sum_cut_tiles, partial, tile_ptr, order, n_tiles, grid, n_out, cout, out_h, e);
-    }
+    const int* tile_ptr = ls.tile_ptr;
+    const int* order = ls.order;
+    cudaLaunchKernelEx(&cfg, umma::k_sum_cut_tiles, partial, tile_ptr, order, n_tiles, grid, n_out, cout, out_h, e);
     PCE_LAUNCH_CHECK();
   }
   return PCE_OK;

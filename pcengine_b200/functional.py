@@ -115,7 +115,7 @@ SPLIT_TILES = True
 
 
 def _split_scratch(n_rows: int, n_src: int, c_in: int, c_out: int, kv: int, device):
-    """fp32 scratch for the partial sums of a layer that the library will split, or None."""
+    """Scratch of a layer that the library will split between CTAs, or None."""
     if not SPLIT_TILES:
         return None
     idx = device.index if device.index is not None else torch.cuda.current_device()
