@@ -107,11 +107,12 @@ typedef struct pce_epilogue {
    * (offset, K block) stages on one CTA; a map with fewer tiles than the GPU has CTA slots leaves
    * SMs idle while those chains run, and one with a few times as many ends in a half-empty wave.
    * With split_scratch of at least pce_conv_split_scratch_bytes(...) bytes (16-byte aligned) the
-   * tiles are split between CTAs -- 2, 4 or 8 CTAs per tile on small maps, equal shares of the
-   * stages whatever tiles they fall in on mid-size ones --, the CTAs leave fp32 partial sums here
-   * and a second kernel adds them in a fixed order and applies the epilogue (deterministic; the
-   * fp32 sum is associated differently than in the one-CTA chain).  Without scratch the layer runs
-   * whole. */
+   * tiles are split between CTAs -- a cluster of 2, 4 or 8 CTAs per tile on small maps, which add
+   * their fp32 sums through shared memory (any non-empty scratch will do), equal shares of the
+   * stages whatever tiles they fall in on mid-size ones, where the CTAs leave fp32 partial sums
+   * here and a second kernel adds them in a fixed order and applies the epilogue (deterministic;
+   * the fp32 sum is associated differently than in the one-CTA chain).  Without scratch the layer
+   * runs whole. */
   void* split_scratch;
   size_t split_scratch_bytes;
 } pce_epilogue;
@@ -408,7 +409,8 @@ PCE_API int32_t pce_conv_split_parts(int32_t n_rows, int32_t n_src, int32_t c_in
  * outputs gathered from n_src input rows; 0 = the layer runs whole. */
 PCE_API size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
-/* The same, but 0 where such a split was measured slower than the whole layer. */
+/* What the engine gives: 0 where such a split was measured slower than the whole layer, and a
+ * token size where the parts need no scratch of their own. */
 PCE_API size_t pce_conv_split_scratch_wanted(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
 

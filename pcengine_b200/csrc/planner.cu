@@ -101,6 +101,46 @@ struct DeviceArena {
   }
 };
 
+// The 64 pinned bytes in which a pass reads its levels' sizes back, out of one page for all passes of the process (pinning
+// memory takes a millisecond with work in flight).  The page is given back with its last piece; passes beyond its 64 pieces
+// pin their own.
+class SizeWords {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lk(m_);
+    if (!page_ && cudaHostAlloc(reinterpret_cast<void**>(&page_), kPieces * kPiece, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+      page_ = nullptr;
+    for (int i = 0; page_ && i < kPieces; ++i)
+      if (!(used_ >> i & 1ull)) {
+        used_ |= 1ull << i;
+        return reinterpret_cast<int*>(page_ + i * kPiece);
+      }
+    int* own = nullptr;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&own), kPiece, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    return own;
+  }
+  void give(int* p) {
+    std::lock_guard<std::mutex> lk(m_);
+    const char* c = reinterpret_cast<const char*>(p);
+    if (!page_ || c < page_ || c >= page_ + kPieces * kPiece) {
+      cudaFreeHost(p);
+      return;
+    }
+    used_ &= ~(1ull << ((c - page_) / kPiece));
+    if (used_ == 0) {
+      cudaFreeHost(page_);
+      page_ = nullptr;
+    }
+  }
+
+ private:
+  static constexpr int kPieces = 64, kPiece = 64;
+  std::mutex m_;
+  char* page_ = nullptr;
+  unsigned long long used_ = 0;
+};
+static SizeWords size_words;
+
 struct LevelState {
   const int32_t* coords = nullptr;
   int32_t n = 0;
@@ -336,7 +376,8 @@ static int run_chain(pce_plan* p, PlanLane* l, pce_pass* ps) {
   void* mem = ps->take(bytes);
   if (!mem) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
   PCE_TRY(blk::chain_place(ps->chain, in.n, gp, n_geoms, true, mem, bytes));
-  if (!ps->sizes) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ps->sizes), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+  if (!ps->sizes) ps->sizes = size_words.take();
+  if (!ps->sizes) return PCE_ERR_CUDA;
   int* sizes_dev = nullptr;
   PCE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&sizes_dev), ps->sizes, 0));
   ps->sizes[0] = PCE_ERR_CUDA;
@@ -659,7 +700,7 @@ int32_t pce_tile_rows_for(int32_t n_rows, int32_t c_in, int32_t c_out, int32_t s
 
 static void free_pass(pce_pass* ps) {
   ps->arena.release();
-  if (ps->sizes) cudaFreeHost(ps->sizes);
+  if (ps->sizes) size_words.give(ps->sizes);
   if (ps->start) cudaEventDestroy(ps->start);
   if (ps->released) cudaEventDestroy(ps->released);
   for (cudaEvent_t ev : ps->ready)
