@@ -1167,8 +1167,8 @@ int pce_map_build_d2(const int32_t* in_coords, int32_t n_in, const int32_t* out_
   if (!ar.ok) return PCE_ERR_WORKSPACE;
   PCE_CUDA(cudaMemsetAsync(knnz, 0, sizeof(int) * gd.kv, st));
   if (!status) PCE_CUDA(cudaMemsetAsync(st_word, 0, sizeof(int), st));
-  // The dense table from block probes: 5x5x5 always (1.5 M voxels: 1.24 -> 0.4 ms), 3x3x3 on maps whose probes, not
-  // launches, are the time (three launches more: 40 k sparse voxels 17 -> 40 us, 480 k LiDAR voxels 66 -> 45).
+  // The dense table from block probes: 5x5x5 always (1.5 M voxels: 1.29 -> 0.62 ms), 3x3x3 on maps whose probes, not
+  // launches, are the time (three launches more; 480 k LiDAR voxels 126 -> 87 us, 1.5 M indoor 332 -> 318).
   if (n_in > 0 && n_in == n_out && in_coords == out_coords && !map_out && blk::covers(g) && !kmap_query_lanes4 &&
       (gd.kv > 27 || n_in >= (1 << 17))) {
     PCE_TRY(blk::subm_dense(in_coords, n_in, g, workspace, workspace_bytes, map, knnz, status, st));
