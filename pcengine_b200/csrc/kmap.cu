@@ -693,8 +693,7 @@ __global__ void k_offset_counts(const uint32_t* __restrict__ mask, int n_rows, i
   if (threadIdx.x < 128 && local[threadIdx.x]) atomicAdd(&counts[threadIdx.x], local[threadIdx.x]);
 }
 
-// keys = the bitmask with offset k moved to bit kv-1-rank(k), rank 0 = rarest (ties by index);
-// lo holds positions 0..63, hi positions 64..127 (kv > 64 only).
+// The permuted bitmask has offset k at bit kv-1-rank(k), rank 0 = rarest (ties by index).
 // 32 < kv <= 64: keys = the permuted bitmask.  kv > 64: the places of the row's five rarest offsets (7 bits each, 127 less
 // the rank, the rarest first, 0 where there are no more), then 29 bits of a hash of the bitmask, which keep the rows of one
 // bitmask together.  A lexicographic order of sparse bitmasks is one of their rarest offsets: against sorting on all 125
