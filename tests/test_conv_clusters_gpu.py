@@ -1,0 +1,33 @@
+"""Tiles shared by a cluster of CTAs at the edges of their rule, against the oracle (GPU)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import conv_oracle as co
+from oracle import kmap_oracle as ko
+from tests.helpers import cmax_of, surface_cloud
+
+pytestmark = [pytest.mark.gpu, pytest.mark.split_tiles]
+
+
+@pytest.mark.parametrize("n,cin,cout,parts", [(1, 64, 64, 4), (127, 96, 96, 8), (129, 128, 160, 8), (3072, 256, 256, 8), (3073, 256, 256, 4),
+                                              (9400, 64, 256, 4), (9500, 64, 256, 2), (14208, 128, 128, 4), (14209, 128, 128, 2),
+                                              (28416, 64, 64, 2), (28417, 64, 64, 1), (56832, 96, 96, 2), (56833, 96, 96, 1)])
+def test_parts_of_a_tile(n, cin, cout, parts):
+    import pcengine_b200 as pce
+    from pcengine_b200 import _lib
+    from pcengine_b200 import functional as PF
+    coords = np.ascontiguousarray(surface_cloud(8, int(n ** 0.5 * 1.2) + 2)[:n])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        assert _lib.lib.pce_conv_split_parts(n, n, cin, cout, 27, sms) == parts
+    d2 = ko.build_d2(coords, (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
+    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
+    g = torch.Generator().manual_seed(n + cin)
+    x, w = torch.randn(n, cin, generator=g).half(), (torch.randn(27, cin, cout, generator=g) / (27 * cin) ** 0.5).half()
+    shift, res = torch.randn(cout, generator=g), torch.randn(n, cout, generator=g).half()
+    want = torch.relu(co.conv_forward(x, w, d2) + shift + res.float())
+    ep = PF.FusedEpilogue(shift=shift.cuda(), residual=res.cuda(), act="relu")
+    outs = [PF.conv_forward(x.cuda(), w.cuda(), km.csr(), ep) for _ in range(2)]
+    assert torch.equal(*outs) and co.rel_l2(outs[0].float().cpu(), want) <= 1e-3
+    assert PF.device_status() == 0
