@@ -383,8 +383,8 @@ PCE_API int pce_pack_weights(const void* weights, int32_t kv, int32_t c_in, int3
  * what = 6: sort the rows on the most significant `value` bits of their key only (0 = all, default);
  * what = 7: 0 never splits tiles between CTAs; 1 (default) as pce_conv_split_scratch_bytes says;
  *           2 only the split of small maps into parts, no shares of stages on mid-size maps.
- * what = 8: 0 runs layers whose width is an odd multiple of 32 channels with 64-channel K blocks
- *           like every other layer (1, default: with 32-channel blocks, every ring stage full).
+ * what = 8: 0 stages the last K block of a width that is an odd multiple of 32 channels padded to 64
+ *           (1, default: its weights as 32 channels, no padding; same results).
  * what = 9: 0 makes the planner build the neighbour CSR of every map and the tile lists from it; 1 (default)
  *           lets it skip the CSR where only tile lists are used (pce_planned_csr.rowptr == NULL). */
 PCE_API int pce_tune(int32_t what, int32_t value);

@@ -20,7 +20,7 @@ extern int umma_overlap_launches;
 extern int umma_multi_tile;
 extern int kmap_query_lanes4;
 extern int umma_split_enabled;
-extern int umma_kb32_enabled;
+extern int umma_half_blocks;
 extern int plan_short_route;
 int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
@@ -107,7 +107,7 @@ int pce_tune(int32_t what, int32_t value) {
     return PCE_OK;
   }
   if (what == 8) {
-    umma_kb32_enabled = value ? 1 : 0;
+    umma_half_blocks = value ? 1 : 0;
     return PCE_OK;
   }
   if (what == 9) {

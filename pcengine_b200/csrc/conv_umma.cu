@@ -54,7 +54,7 @@ __device__ int g_umma_where[4] = {0, 0, 0, 0};
 namespace umma {
 
 constexpr int kTileM = 128;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 4;
 constexpr int kABytes = kTileM * 128;  // one A stage: 128 rows x 64 fp16
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at 2 GHz
 
@@ -89,6 +89,7 @@ struct Lists {
   const int* stage_kp;   // [stages] offset of every stage
   const int* stage_nbr;  // [stages][tile rows] input row per tile row, -1 absent
   int identity;          // every tile's last stage is the identity stage (stage_kp = -1)
+  const __half* wtail;   // the weights' 32-channel image, for the last K block of a width that is an odd multiple of 32
   const __half* wslots;  // SLOTS > 1: weights as [kv][cout][cin] (one 16-byte chunk row per output channel)
   int settled;           // the lists were complete before the previous kernel of the stream was launched
 };
@@ -98,6 +99,7 @@ struct Lists {
 struct Second {
   const __half* in2;  // [n_out][cin2], nullptr: none
   const __half* w2;   // packed like the weights of one offset: kblocks2 images of cout x 128 B
+  const __half* wtail;  // as Lists::wtail
   int cin2;
 };
 
@@ -407,9 +409,12 @@ __device__ __forceinline__ void finish8(float (&v)[8], int row, int c0, int cout
 // of the 64-channel K block, so SLOTS offsets of a tile share one ring stage: every row gathers one
 // neighbour per slot into its part of the 128-byte row, and the producers assemble the stage's weight
 // block from the per-offset images with cp.async (covered by the same barrier as the rows).
-// KB = channels per K block (64, or 32 for layers whose width is an odd multiple of 32: every stage is then
-// full, where 64-channel blocks would spend half of every second stage's rows and weights on padding).
-template <int kStages, int SUB, bool PUSH, int SLOTS, int KB = 64>
+// K blocks are 64 channels.  HALF: the last one of a width that is an odd multiple of 32 is half: its rows are gathered into the
+// first half of the 128-byte operand rows and its weights come from the second image of the packed weights, 32 channels
+// (64 bytes, 64-byte swizzle) per output channel, so that no padding is staged.  Against three 32-channel stages for 96
+// channels it is two stages per offset: 96->96 on 240 k rows 45.8 -> 43.1 us, on 37 k rows 34.6 -> 32.4.  A variant of its
+// own, since the choice between two images per stage costs every width (64->64 on 200 k rows 30.4 -> 32.1 us).
+template <int kStages, int SUB, bool PUSH, int SLOTS, bool HALF = false>
 __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
     k_conv_umma(const __half* __restrict__ in, const __half* __restrict__ wpacked, Lists ls, Second sec, int n_out, int cin,
                 int cout, __half* __restrict__ out, Epi ep, int tmem_cols, int nacc) {
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
   uint8_t* tiles = smem_raw + pad;  // 1024-byte aligned
   const uint32_t tiles_addr = raw_addr + pad;
-  static_assert(KB == 64 || (KB == 32 && SUB == 1 && SLOTS == 1), "32-channel K blocks: plain variant only");
+  constexpr int KB = 64;                       // channels per K block
   constexpr int kRowBytes = KB * 2;            // one operand row of a stage
   const int b_bytes = cout * kRowBytes;
   constexpr int kRows = kTileM * SUB;          // output rows per tile
@@ -556,8 +561,8 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
     bool ok = true;
     // destination of this thread's copy q inside a stage: row q * kRowsPerInstr + rsub of the warp's 32, chunk
     // swizzled with the row; the swizzle term takes two values (q even / odd), everything else is q * constant
-    const int sw_even = KB == 64 ? (chunk ^ rsub) : (chunk ^ ((rsub >> 1) & 3));
-    const int sw_odd = KB == 64 ? (chunk ^ (rsub + 4)) : sw_even;
+    const int sw_even = chunk ^ rsub;
+    const int sw_odd = chunk ^ (rsub + 4);
     const uint32_t dst_even = (warp * 32 + rsub) * kRowBytes + (sw_even << 4);
     const uint32_t dst_odd = (warp * 32 + rsub) * kRowBytes + (sw_odd << 4);
     if constexpr (SLOTS == 1) {
@@ -594,10 +599,14 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         const uint32_t a_addr = tiles_addr + s * stage_bytes;
         if (warp == 0 && elect_one()) {
           const uint32_t bbar = smem_u32(&ctl->bfull[s]);
-          mbar_arrive_expect_tx(bbar, b_bytes);
+          const __half* wtail = second ? sec.wtail : ls.wtail;
+          const bool tail = HALF && wtail && kb == nkb - 1;
+          const uint32_t bytes = tail ? static_cast<uint32_t>(cout) * 64u : static_cast<uint32_t>(b_bytes);
+          mbar_arrive_expect_tx(bbar, bytes);
           const __half* wsrc = second ? sec.w2 + static_cast<size_t>(kb) * cout * KB
                                       : wpacked + (static_cast<size_t>(kb) + static_cast<size_t>(kp) * kblocks) * cout * KB;
-          bulk_copy_g2s(a_addr + kAStage, wsrc, b_bytes, bbar);
+          if (tail) wsrc = wtail + (static_cast<size_t>(second ? 0 : kp) * (2 * nkb - 1) + 2 * kb) * cout * 32;
+          bulk_copy_g2s(a_addr + kAStage, wsrc, bytes, bbar);
         }
         if (chunk < min(kCpr, (width - kb * KB) >> 3)) {
           const char* src_kb = src_base + kb * (KB * 2);
@@ -764,7 +773,8 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
             fence_proxy_async();  // the gathered rows were written through the generic proxy
             tc_fence_after();
             const uint32_t a_addr = tiles_addr + s * stage_bytes;
-            const uint64_t db = make_desc_kb<KB>(a_addr + kAStage);
+            const bool tail = HALF && (second ? sec.wtail && kb == kblocks2 - 1 : ls.wtail && kb == kblocks - 1);
+            const uint64_t db = tail ? make_desc_kb<32>(a_addr + kAStage) : make_desc_kb<KB>(a_addr + kAStage);
             // with several offsets per stage the whole 64-channel block is always filled (unused slots with zeros)
             const int ksteps = (SLOTS > 1 && !second) ? 4 : min(KB / 16, ((second ? sec.cin2 : cin) - kb * KB) >> 4);
 #pragma unroll
@@ -1489,8 +1499,8 @@ bool conv_umma_supported(int cin, int cout, int dtype) {
 // Per-offset blocks, and for 16 or 32 input channels also the per-offset [cout][cin] images from which
 // stages that hold several offsets assemble their weight block.
 // Behind them, a second copy as 32-channel blocks (cout rows x 64 B, 64-byte swizzle) for widths that are an odd
-// multiple of 32 (the kernel variant with 32-channel K blocks) and for every single-offset weight (a second
-// operand is read in the K-block size of the layer it joins).
+// multiple of 32 (their last K block is half, see HALF) and for every single-offset weight (a second
+// operand of such a layer).
 static bool has_kb32_image(int kv, int cin) { return kv == 1 || (cin > 32 && cin % 64 == 32); }
 static size_t kb64_image_bytes(int kv, int cin, int cout) {
   const size_t blocks = static_cast<size_t>(kv) * ((cin + 63) / 64) * cout * 128;
@@ -1605,7 +1615,7 @@ static int conv_umma_mt(const __half* in, const __half* w, const umma::Lists& ls
   return PCE_OK;
 }
 
-template <int NS, int SUB, bool PUSH, int SLOTS, int KB = 64>
+template <int NS, int SUB, bool PUSH, int SLOTS, bool HALF = false>
 static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in, const __half* w, const umma::Lists& ls,
                         const umma::Second& sec, int n_out, int cin, int cout, __half* out, const umma::Epi& e, int tmem_cols,
                         int nacc) {
@@ -1626,13 +1636,12 @@ static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  cudaLaunchKernelEx(&cfg, umma::k_conv_umma<NS, SUB, PUSH, SLOTS, KB>, in, w, ls, sec, n_out, cin, cout, out, e, tmem_cols,
+  cudaLaunchKernelEx(&cfg, umma::k_conv_umma<NS, SUB, PUSH, SLOTS, HALF>, in, w, ls, sec, n_out, cin, cout, out, e, tmem_cols,
                      nacc);
 }
 
-// 1: layers whose width is an odd multiple of 32 channels (96, 160, 224) run with 32-channel K blocks, where every
-// ring stage is full (64-channel blocks pad half of every second stage); 0: 64-channel blocks everywhere.
-int umma_kb32_enabled = 1;
+// 1: the last K block of a width that is an odd multiple of 32 (96, 160, 224) stages half the weights; 0: it is padded.
+int umma_half_blocks = 1;
 
 // 1: maps with few tiles are split over several CTAs per tile, mid-size maps into equal shares of stages,
 // when the caller gives scratch (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
@@ -1664,7 +1673,7 @@ int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_co
   // only where they still have about an SM each.  Whole -> split, us (3x3x3, kernel only): 64->64 on 7.5 k rows 18.8 -> 9.6
   // (4 parts; 2: 12.2), on 25 k rows 18.9 -> 14.3 (2; 4 exceed the slots: 19.6); 128->128 on 2.9 k rows 30.9 -> 12.6 (4; 8:
   // 12.8), on 12 k rows 23.3 -> 13.7 (4); 256->256 on 7.5 k rows 60.6 -> 27.9 (4; 2: 39.6); 128->256 on 12 k rows 27 -> 22.5
-  // (2), on 23 k rows 38 -> 44 beyond the slots.  Widths that run in 32-channel blocks have half the work per stage and
+  // (2), on 23 k rows 38 -> 44 beyond the slots.  Widths with a half block have less work per stage and
   // gain up to a wave of tiles (96->96 on 37 k rows 37.4 -> 32.8, on 54 k rows 38.5 -> 36.5, two parts).  The rows of a
   // kernel of at most 8 offsets (down and up a level) have fewer of them than the estimate: twice the chain is asked for.
   const int each = kv <= 8 ? 8 : 4;
@@ -1745,12 +1754,12 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
       if (!e.push_slot[s]) e.push_base[s] = nullptr;
     }
   }
-  umma::Lists ls{nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0};
+  umma::Lists ls{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0};
   int slots = 1;
-  umma::Second sec{nullptr, nullptr, 0};
+  umma::Second sec{nullptr, nullptr, nullptr, 0};
   int sub = umma_force_sub == 1 || umma_force_sub == 2 ? umma_force_sub : 1;
   if (tiles) {
-    ls = umma::Lists{tiles->order, tiles->tile_ptr, tiles->stage_kp, tiles->stage_nbr, tiles->identity_stage ? 1 : 0, nullptr,
+    ls = umma::Lists{tiles->order, tiles->tile_ptr, tiles->stage_kp, tiles->stage_nbr, tiles->identity_stage ? 1 : 0, nullptr, nullptr,
                      (tiles->settled && umma_overlap_launches == 1) ? 1 : 0};
     slots = tiles->slots > 1 ? tiles->slots : 1;
     if (slots != 1) {
@@ -1767,21 +1776,24 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   if (ep && ep->extra_feats) {
     // the second operand rides on the identity stage of the tile lists
     if (!ls.identity || !ep->extra_packed_weights || ep->extra_c < 16 || ep->extra_c % 16) return PCE_ERR_UNSUPPORTED;
-    sec = umma::Second{static_cast<const __half*>(ep->extra_feats), static_cast<const __half*>(ep->extra_packed_weights),
+    sec = umma::Second{static_cast<const __half*>(ep->extra_feats), static_cast<const __half*>(ep->extra_packed_weights), nullptr,
                        ep->extra_c};
   }
   const size_t fixed = sizeof(umma::SharedCtl) + 1024 + 64 + 2 * sizeof(float) * cout;  // (+ staged scale / shift)
-  // 32-channel K blocks for widths that are an odd multiple of 32 (plain variant: one sub-tile, one offset per
-  // stage, no halo push); operands then come from the second image of the packed weights
-  const bool kb32 = umma_kb32_enabled && !kb64_slice && sub == 1 && slots == 1 && !(e.push_slot[0] || e.push_slot[1]) && cin > 32 &&
+  // the half block at the end of an odd multiple of 32 channels (one offset per stage); a slice of a packed buffer has no
+  // second image behind it
+  const bool half = umma_half_blocks && !kb64_slice && sub == 1 && slots == 1 && !(e.push_slot[0] || e.push_slot[1]) && cin > 32 &&
                     cin % 64 == 32 && !(tiles && umma_multi_tile);
-  const size_t stage = kb32 ? static_cast<size_t>(umma::kTileM) * 64 + static_cast<size_t>(cout) * 64
-                            : static_cast<size_t>(umma::kABytes) * sub + static_cast<size_t>(cout) * 128;
+  if (half) {
+    ls.wtail = reinterpret_cast<const __half*>(static_cast<const char*>(wpacked) + kb64_image_bytes(kv, cin, cout));
+    if (sec.in2 && sec.cin2 % 64 == 32)
+      sec.wtail = reinterpret_cast<const __half*>(reinterpret_cast<const char*>(sec.w2) + kb64_image_bytes(1, sec.cin2, cout));
+  }
+  const size_t stage = static_cast<size_t>(umma::kABytes) * sub + static_cast<size_t>(cout) * 128;
   static int sm_count[64] = {};
   // registers per thread by kernel variant (plain, push, 2 slots, 4 slots) and sub-tile count, in
   // allocation units of 8; read back from the compiled kernels at set-up
   static int regs_per_thread[4][2] = {{72, 72}, {80, 80}, {80, 80}, {96, 88}};
-  static int regs_kb32 = 72;
   int dev = 0;
   PCE_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return PCE_ERR_UNSUPPORTED;
@@ -1792,9 +1804,9 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));  \
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap)); \
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap))
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<4, 1, false, 1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<5, 1, false, 1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<6, 1, false, 1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
+    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<4, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
+    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<3, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
+    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<2, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
     PCE_SET_SMEM(4, 1);
     PCE_SET_SMEM(3, 1);
     PCE_SET_SMEM(2, 1);
@@ -1814,8 +1826,6 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
     PCE_REGS(3, 1, (umma::k_conv_umma<2, 1, false, 4>));
     PCE_REGS(3, 2, (umma::k_conv_umma<2, 2, false, 4>));
 #undef PCE_REGS
-    if (cudaFuncGetAttributes(&fa, umma::k_conv_umma<4, 1, false, 1, 32>) == cudaSuccess && fa.numRegs > 0)
-      regs_kb32 = (fa.numRegs + 7) / 8 * 8;
     int n = 0;
     PCE_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     sm_count[dev] = n > 0 ? n : 1;
@@ -1837,7 +1847,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   const bool push = e.push_slot[0] || e.push_slot[1];
   if (push && slots != 1) return PCE_ERR_UNSUPPORTED;  // the halo push has no several-offsets-per-stage variant
   const int variant = push ? 1 : (slots == 2 ? 2 : (slots == 4 ? 3 : 0));
-  const int by_regs = 65536 / (threads * (kb32 ? regs_kb32 : regs_per_thread[variant][sub - 1]));
+  const int by_regs = 65536 / (threads * regs_per_thread[variant][sub - 1]);
   auto tmem_for = [&](int sets) {
     int cols = 32;
     while (cols < sets * sub * cout) cols <<= 1;
@@ -1851,7 +1861,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
     return c > 4 ? 4 : c;
   };
   int ns = 2, nacc = 1, per_sm = 0;
-  for (int n = (kb32 ? 6 : 4); n >= (kb32 ? 4 : 2); --n) {  // (32-channel blocks: half-size stages, rings of 4 to 6)
+  for (int n = 4; n >= 2; --n) {
     for (int sets = 2; sets >= 1; --sets) {
       const int c = ctas_for(n, sets);
       const bool better = c * n > per_sm * ns || (c * n == per_sm * ns && c > per_sm);
@@ -1862,7 +1872,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
       }
     }
   }
-  if (umma_force_stages >= (kb32 ? 4 : 2) && umma_force_stages <= (kb32 ? 6 : 4)) ns = umma_force_stages;
+  if (umma_force_stages >= 2 && umma_force_stages <= 4) ns = umma_force_stages;
   if ((umma_force_nacc == 1 || umma_force_nacc == 2) && umma_force_nacc * sub * cout <= 512) nacc = umma_force_nacc;
   per_sm = ctas_for(ns, nacc);
   const int tmem_cols = tmem_for(nacc);
@@ -1894,20 +1904,11 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   const __half* in_h = static_cast<const __half*>(in);
   const __half* w_h = static_cast<const __half*>(wpacked);
   __half* out_h = static_cast<__half*>(out);
-  if (kb32) {
-    w_h = reinterpret_cast<const __half*>(static_cast<const char*>(wpacked) + kb64_image_bytes(kv, cin, cout));
-    if (sec.in2)
-      sec.w2 = reinterpret_cast<const __half*>(reinterpret_cast<const char*>(sec.w2) + kb64_image_bytes(1, sec.cin2, cout));
-    if (ns == 6)
-      launch_umma<6, 1, false, 1, 32>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc);
-    else if (ns == 5)
-      launch_umma<5, 1, false, 1, 32>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc);
-    else
-      launch_umma<4, 1, false, 1, 32>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc);
-  } else {
 #define PCE_GO(NS, SB)                                                                                              \
   do {                                                                                                              \
-    if (push)                                                                                                         \
+    if (SB == 1 && half)                                                                                              \
+      launch_umma<NS, 1, false, 1, true>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc); \
+    else if (push)                                                                                                         \
       launch_umma<NS, SB, true, 1>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc);  \
     else if (slots == 2)                                                                                              \
       launch_umma<NS, SB, false, 2>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc); \
@@ -1922,7 +1923,6 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
     if (ns == 4) PCE_GO(4, 2); else if (ns == 3) PCE_GO(3, 2); else PCE_GO(2, 2);
   }
 #undef PCE_GO
-  }
   PCE_LAUNCH_CHECK();
   if (streamk) {
     // the second kernel of a stream-K layer is set up on the SMs while the convolution's last CTAs drain
