@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "launch_math.h"
 
 namespace pce {
 namespace f32 {
@@ -110,7 +111,7 @@ struct Shape {
 };
 
 template <int BM, int BN, bool VEC>
-__global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f32(Args a, int parts) {
+__global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f32(Args a, int parts, int row_blocks) {
   constexpr int TN = Shape<BM, BN>::TN, TY = Shape<BM, BN>::TY;
   constexpr int TM = BM / TY;
   constexpr int TX = Shape<BM, BN>::TX, NT = Shape<BM, BN>::NT;
@@ -124,11 +125,12 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
   const uint32_t sb_addr = static_cast<uint32_t>(__cvta_generic_to_shared(sb));
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
-  const int part = blockIdx.x;
+  const F32Block place = f32_block(blockIdx.x, parts, row_blocks);
+  const int part = place.part;
   // the last rows of the order have the rare offsets, so the longest chains: they start first
-  const int row0 = static_cast<int>(gridDim.y - 1 - blockIdx.y) * BM;  // first slot of the processing order
+  const int row0 = (row_blocks - 1 - place.row_block) * BM;  // first slot of the processing order
   const int tile = row0 >> 7, in_tile = row0 & 127;
-  const int n0 = blockIdx.z * BN;
+  const int n0 = place.slice * BN;
   const int cin_p = (a.cin + 3) & ~3;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the tile's stages that at least one of this block's rows has (a block is a quarter of a tile)
@@ -362,8 +364,10 @@ static int launch(const Args& a, int parts, cudaStream_t st) {
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(parts, div_up(a.n_out, BM), div_up(a.cout, BN));
-  if (cfg.gridDim.y > 65535u) return PCE_ERR_UNSUPPORTED;
+  const int row_blocks = div_up(a.n_out, BM);
+  const long long blocks = f32_blocks(a.n_out, BM, a.cout, BN, parts);
+  if (blocks > 0x7FFFFFFFll) return PCE_ERR_UNSUPPORTED;  // (an output of 4 TB)
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -376,7 +380,7 @@ static int launch(const Args& a, int parts, cudaStream_t st) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  PCE_CUDA(cudaLaunchKernelEx(&cfg, k_conv_f32<BM, BN, VEC>, a, parts));
+  PCE_CUDA(cudaLaunchKernelEx(&cfg, k_conv_f32<BM, BN, VEC>, a, parts, row_blocks));
   PCE_LAUNCH_CHECK();
   return PCE_OK;
 }

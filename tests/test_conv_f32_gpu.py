@@ -43,3 +43,27 @@ def test_tiled_fp32_in_the_explicit_dataflow(n, cin, cout):
     km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
     out = PF.conv_forward_d1(feats.cuda(), w.cuda(), km)
     assert co.rel_l2(out.cpu(), co.conv_forward(feats, w, d2)) <= 1e-5
+
+
+def test_tiled_fp32_beyond_65535_row_blocks():
+    """More rows than 65535 blocks of 32 (lists) and of 128 (dense product), which the kernel of one thread group per
+    row always took.  Bound: two fp32 sums of at most 27 * 28 products in different orders."""
+    import pcengine_b200 as pce
+    from pcengine_b200 import functional as PF
+    n = 65535 * 32 + 33
+    lin = torch.randperm(256 * 256 * 64, device="cuda", generator=torch.Generator("cuda").manual_seed(0))[:n]
+    coords = torch.stack([0 * lin, lin // (256 * 64), lin // 64 % 256, lin % 64], 1).int().contiguous()
+    km = pce.KernelMap(coords, (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], [255, 255, 63], True)
+    x, w = torch.randn(n, 28, device="cuda"), torch.randn(27, 28, 28, device="cuda")
+    got = PF.conv_forward(x, w, km.csr())
+    want = PF.conv_forward(x, w, km.csr(), kernel_choice="simt")
+    for part in (slice(0, n // 2), slice(n // 2, n), slice(n - 40, n)):
+        assert float((got[part] - want[part]).norm() / want[part].norm()) <= 1e-5
+    del got, want
+    x = torch.randn(65535 * 128 + 129, 28, device="cuda")
+    got = PF.linear_forward(x, w[0].contiguous())
+    for part in (slice(0, 1 << 20), slice(len(x) - 140, len(x))):
+        want = x[part].double() @ w[0].double()
+        assert float((got[part] - want).norm() / want.norm()) <= 1e-5
+    whole = x @ w[0]  # (another fp32 order)
+    assert float((got - whole).norm() / whole.norm()) <= 1e-5
