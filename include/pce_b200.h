@@ -352,7 +352,7 @@ PCE_API int pce_build_tile_lists(const uint32_t* mask, const int32_t* rowptr, co
                                  size_t workspace_bytes, int32_t* tile_ptr, int32_t* stage_kp,
                                  int32_t* stage_nbr, int32_t stage_cap, void* stream);
 
-/* pce_csr_sort_rows and pce_build_tile_lists of up to four lists in ONE cooperative launch, for maps of at most 32
+/* pce_csr_sort_rows and pce_build_tile_lists of up to PCE_PLAN_MAX_USES lists in ONE cooperative launch, for maps of at most 32
  * offsets; same order and lists.  The neighbours come from nbr (row r's from starts[r] on, starts NULL: entry r) or
  * from a dense table[kp * n + row], which then also gives the mask.  counts[kv] (may be NULL): rows that have each
  * offset.  lists[v] names the arrays to fill (its `order` is ignored), stage_caps[v] their room in stages. */

@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(256) k_parents(const int4* __restrict__ coords
 // ---- row order and stages per tile ------------------------------------------------------------------------------
 
 // The row order (rows sorted by bitmask, its bits permuted so that the rarest offset is the most significant one; stable)
-// and tile_ptr of up to four (tile height, identity stage, offsets per stage) of ONE direction of a map with at most 32
+// and tile_ptr of up to kMaxVariants (tile height, identity stage, offsets per stage) of ONE direction of a map with at most 32
 // offsets; the stages themselves are then filled by k_tile_lists (kmap.cu) over the whole GPU.  Two kernels: maps of up
 // to 64 k rows are sorted by ONE cluster of eight blocks (keys in registers, digit counts and the scatter itself through
 // distributed shared memory: nothing waits for L2 or for a grid barrier), larger ones by a cooperative grid.  The

@@ -49,7 +49,10 @@ struct Query {
   int* map;        // [kv][n]
 };
 
-constexpr int kMaxVariants = 4;
+// Sets of lists per direction of a map: every use a plan can name may want its own (two tile heights x 1, 2 or 4 offsets
+// per stage are six today).
+constexpr int kMaxVariants = PCE_PLAN_MAX_USES;
+static_assert(kMaxVariants <= 16, "one warp of a block per set; the sums of a block's sets share a row of 32 words");
 
 struct Variant {  // one set of tile lists (as pce_tile_lists)
   int tile_rows, identity, slots;

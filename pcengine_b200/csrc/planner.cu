@@ -491,7 +491,6 @@ static int build_direction(pce_plan* p, PlanLane* l, pce_pass* ps, blk::Order o,
     bool seen = false;
     for (int v = 0; v < o.n_variants; ++v) seen = seen || (o.variant[v].tile_rows == rows && o.variant[v].slots == slots);
     if (seen) continue;
-    if (o.n_variants == blk::kMaxVariants) return PCE_ERR_UNSUPPORTED;
     const int n_tiles = div_up(o.n, rows);
     const size_t cap = static_cast<size_t>(n_tiles) * ((o.kv + slots - 1) / slots + (identity_stage ? 1 : 0));
     blk::Variant& V = o.variant[o.n_variants++];

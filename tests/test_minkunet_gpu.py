@@ -408,3 +408,32 @@ def test_planned_map_with_more_than_32_offsets_keeps_its_csr():
     torch.cuda.synchronize()
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     plan.close()
+
+
+@pytest.mark.parametrize("waves", [0, 6])
+def test_plan_with_five_list_shapes_on_one_map(waves):
+    """Widths on one level whose layers want lists of three, or on a map of six waves of 256-row tiles, which narrow layers
+    then take, of five different (tile height, offsets per stage): the plan (in block form through the strided layer behind
+    them) serves them all, as the lazy path builds them."""
+    import pcengine_b200 as pce
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = max(3000, waves * 256 * sms)
+    lin = torch.randperm(512 * 512, device="cuda", generator=torch.Generator("cuda").manual_seed(1))[:n]
+    coords = torch.stack([0 * lin, lin // 512, lin % 512, (lin // 512 + lin % 512) // 3], 1).int().contiguous()
+    widths = [(16, 32), (16, 64), (32, 32), (32, 64), (64, 64)]
+    plan = pce.MapPlan([(3, 1, False, a, b) for a, b in widths] + [(2, 2, False, 64, 64)])
+    x = pce.spTensor(torch.zeros(n, 16, device="cuda").half(), coords, None, [0, 0, 0], [511, 511, 341], init_tag=["D2"])
+    assert plan.begin(x)
+    key = next(iter(plan.index))
+    planned = x.planner.fetch(x, key, None).csr()
+    alone = pce.KernelMap(coords, (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], [511, 511, 341], True).csr()
+    assert len(planned._tiles) == (5 if waves else 3)
+    for (sort, rows, identity, slots), hit in planned._tiles.items():
+        alone.tiles(sort, rows, identity, slots)
+        want = alone._tiles[(sort, rows, identity, slots)]
+        stages = int(want[2][-1])
+        assert torch.equal(hit[1].tensor(), want[1]) and torch.equal(hit[2].tensor(), want[2])
+        assert torch.equal(hit[3].tensor()[: stages * slots], want[3][: stages * slots])
+        assert torch.equal(hit[4].tensor()[: stages * slots * rows], want[4][: stages * slots * rows])
+    del planned, x
+    plan.close()
