@@ -190,3 +190,35 @@ def test_slab_tensors_refuse_layers_that_would_need_rows_across_a_cut():
     with pytest.raises(NotImplementedError, match="kernel size == stride"):
         pce.conv3d(8, 8, 2, 2, padding=1)(x)
     assert x.slabs.level_of([2, 2, 2]) == 1
+
+
+def test_collation_runs_on_the_device_of_its_samples(monkeypatch):
+    """Samples on a GPU that is not the current one: the library call is made with that GPU current, and the current one
+    is as before afterwards (stand-ins for the tensors and the runtime: no GPU)."""
+    import contextlib
+    import types
+
+    from pcengine_b200 import _lib, utils
+    current, calls = [0], []
+
+    @contextlib.contextmanager
+    def device(d):
+        before, current[0] = current[0], d.index
+        yield
+        current[0] = before
+
+    class Sample:
+        is_cuda, dtype, device = True, torch.int32, torch.device("cuda", 1)
+        dim, size, is_contiguous, data_ptr = (lambda s: 2), (lambda s, d: (5, 3)[d]), (lambda s: True), (lambda s: 64)
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: types.SimpleNamespace(data_ptr=lambda: 256, device=k["device"]))
+    monkeypatch.setattr(_lib, "stream_ptr", lambda d: 1000 + d.index)
+    monkeypatch.setattr(_lib, "lib", types.SimpleNamespace(pce_collate_coords=lambda *a: calls.append((current[0], a[-1])) or 0))
+    out, cmax = utils._collate_cuda([Sample(), Sample()])
+    assert calls == [(1, 1001)] and current == [0] and out.device.index == 1 and cmax == [0, 0, 0]
+    calls.clear()
+    current[0] = 1
+    utils._collate_cuda([Sample()])
+    assert calls == [(1, 1001)] and current == [1]
