@@ -129,7 +129,11 @@ __global__ void __launch_bounds__(256) k_block_insert(const int4* __restrict__ c
     }
     if (L.table == nullptr) continue;
     if (__ballot_sync(kFull, active) == 0u) return;
-    if (l > 0 && *reinterpret_cast<volatile int*>(ctl + kCtlStatus) != PCE_OK) return;  // the chain has failed already
+    if (l > 0) {  // the chain may have failed already; other warps write the word meanwhile, so one lane reads it for all
+      int status = lane == 0 ? *reinterpret_cast<volatile int*>(ctl + kCtlStatus) : 0;
+      status = __shfl_sync(kFull, status, 0);
+      if (status != PCE_OK) return;
+    }
     const int ux = x + 32768, uy = y + 32768, uz = z + 32768;
     const unsigned long long key = active ? block_key(b, ux >> 2, uy >> 2, uz >> 2) : 0ull;
     const int bit = ((ux & 3) << 4) | ((uy & 3) << 2) | (uz & 3);

@@ -87,3 +87,27 @@ def test_gather_scatter_codes(n, stride):
     got = pce.KernelMap(torch.from_numpy(coords).cuda(), *args, d2["cmax_out"], stride == 1).d1()
     for name, t in zip(("imap", "icsr", "omap", "ocsr"), got):
         assert np.array_equal(t.cpu().numpy(), want[name])
+
+
+def test_chain_given_up_while_it_is_built():
+    """60 000 voxels with a coarse block each: the coarse tables fill up while other warps still insert, the chain is given
+    up and the levels are found one by one.  Planned and lazy passes agree bit for bit, pass after pass."""
+    import pcengine_b200 as pce
+    coords, cmin = _cloud("alone", 60000)
+    cd, x0 = torch.from_numpy(coords).cuda(), torch.randn(len(coords), 16, generator=torch.Generator().manual_seed(2)).half().cuda()
+    layers = [(3, 1), (2, 2), (3, 1), (2, 2), (3, 1)]
+    torch.manual_seed(3)
+    convs = [pce.conv3d(16, 16, k, s).cuda().half() for k, s in layers]
+    plan = pce.MapPlan([(k, s, False, 16, 16) for k, s in layers])
+    outs = []
+    for planned in (False, True, True):
+        x = pce.spTensor(x0, cd, None, cmin, cmax_of(coords), init_tag=["D2"] * 5)
+        assert plan.begin(x) if planned else True
+        with torch.no_grad():
+            for conv in convs:
+                x = conv(x)
+        outs.append((x.feats, x.coords))
+    for feats, out_coords in outs[1:]:
+        assert torch.equal(feats, outs[0][0]) and torch.equal(torch.as_tensor(out_coords), outs[0][1])
+    del x, outs
+    plan.close()
