@@ -17,6 +17,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "common.cuh"
+#include "launch_math.h"
 #include "coop_sort.cuh"
 #include "kmap_blocks.cuh"
 
@@ -514,26 +515,18 @@ __global__ void __launch_bounds__(coop::kThreads, 2) k_d1_codes(CodeArgs a) {
   coop::cg::grid_group grid = coop::cg::this_grid();
   const int tid = threadIdx.x, b = blockIdx.x, g = gridDim.x;
   const int kv = a.in.kv, n_in = a.in.n_rows, n_out = a.out.n_rows;
-  const int total = kv * n_in;
-  const int per = (total + g - 1) / g;
-  const int f0 = static_cast<int>(min(static_cast<long long>(total), static_cast<long long>(b) * per));
-  const int f1 = f0 + min(per, total - f0);
+  const Piece flags = piece_of(static_cast<unsigned>(kv) * n_in, b, g);  // (fewer than 2^31: the host checks)
   const int kinds = a.mirror ? 2 : 3;
-  int row0[2], row1[2];
-  for (int k = 0; k < 2; ++k) {
-    const int n = k == 0 ? n_in : n_out, rows = (n + g - 1) / g;
-    row0[k] = min(n, b * rows);
-    row1[k] = min(n, row0[k] + rows);
-  }
+  const Piece part[2] = {piece_of(n_in, b, g), piece_of(n_out, b, g)};
   {
     int mine = 0, sum;
-    for (int i = f0 + tid; i < f1; i += coop::kThreads) mine += a.in.table[i] >= 0 ? 1 : 0;
+    for (unsigned i = flags.first + tid; i < flags.end; i += coop::kThreads) mine += a.in.table[i] >= 0 ? 1 : 0;
     coop::block_exclusive(mine, warp_sum, sum);
     if (tid == 0) a.sums[b] = sum;
     for (int k = 0; k < kinds - 1; ++k) {
       const RowArgs& rows = k == 0 ? a.in : a.out;
       mine = 0;
-      for (int r = row0[k] + tid; r < row1[k]; r += coop::kThreads) {
+      for (unsigned r = part[k].first + tid; r < part[k].end; r += coop::kThreads) {
         int cnt = 0;
         for (int kp = 0; kp < kv; ++kp) cnt += row_entry(rows, kp, r) >= 0 ? 1 : 0;
         a.count[k][r] = cnt;
@@ -552,44 +545,45 @@ __global__ void __launch_bounds__(coop::kThreads, 2) k_d1_codes(CodeArgs a) {
     before[k] = sum;
   }
   constexpr int kItems = 4;
-  for (int i0 = f0; i0 < f1; i0 += coop::kThreads * kItems) {
-    const int at = i0 + tid * kItems;
+  for (unsigned i0 = flags.first; i0 < flags.end; i0 += coop::kThreads * kItems) {
+    const unsigned at = i0 + tid * kItems;
     int flag[kItems], mine = 0, sum;
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-      flag[q] = at + q < f1 && a.in.table[at + q] >= 0 ? 1 : 0;
+      flag[q] = at + q < flags.end && a.in.table[at + q] >= 0 ? 1 : 0;
       mine += flag[q];
     }
     int place = before[0] + coop::block_exclusive(mine, warp_sum, sum);
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-      if (at + q < f1) a.rank[at + q] = place;
+      if (at + q < flags.end) a.rank[at + q] = place;
       place += flag[q];
     }
     before[0] += sum;
   }
   for (int k = 0; k < kinds - 1; ++k) {
-    for (int r0 = row0[k]; r0 < row1[k]; r0 += coop::kThreads) {
-      const int r = r0 + tid;
+    const unsigned n = k == 0 ? n_in : n_out;
+    for (unsigned r0 = part[k].first; r0 < part[k].end; r0 += coop::kThreads) {
+      const unsigned r = r0 + tid;
       int sum;
-      const int place = before[k + 1] + coop::block_exclusive(r < row1[k] ? a.count[k][r] : 0, warp_sum, sum);
-      if (r < row1[k]) {
+      const int place = before[k + 1] + coop::block_exclusive(r < part[k].end ? a.count[k][r] : 0, warp_sum, sum);
+      if (r < part[k].end) {
         (k == 0 ? a.icsr : a.ocsr)[r] = place;
         if (k == 0 && a.mirror) a.ocsr[r] = place;
       }
       before[k + 1] += sum;
     }
-    const int n = k == 0 ? n_in : n_out;
-    if (row1[k] == n && row0[k] < n && tid == 0) {
+    if (part[k].end == n && part[k].first < n && tid == 0) {
       (k == 0 ? a.icsr : a.ocsr)[n] = before[k + 1];
       if (k == 0 && a.mirror) a.ocsr[n] = before[k + 1];
     }
   }
   grid.sync();
-  for (int r = b * coop::kThreads + tid; r < n_in + n_out; r += g * coop::kThreads) {
+  const long long both = static_cast<long long>(n_in) + n_out;
+  for (long long r = b * coop::kThreads + tid; r < both; r += g * coop::kThreads) {
     const bool to = r >= n_in;
     const RowArgs& rows = to ? a.out : a.in;
-    const int row = to ? r - n_in : r;
+    const int row = static_cast<int>(to ? r - n_in : r);
     int* codes = to ? a.omap : a.imap;
     int p = (to ? a.ocsr : a.icsr)[row];
 #pragma unroll 3

@@ -29,4 +29,16 @@ inline long long f32_blocks(int n_out, int rows_per_block, int c_out, int channe
   return row_blocks * slices * parts;
 }
 
+// Piece `part` of `parts` contiguous pieces of n entries.  Unsigned: n + parts and part * per stay below 2^32 for every
+// n < 2^31 and a grid's number of parts.
+struct Piece {
+  unsigned first, end;
+};
+
+PCE_HD Piece piece_of(unsigned n, unsigned part, unsigned parts) {
+  const unsigned per = (n + parts - 1) / parts;
+  const unsigned first = part * per < n ? part * per : n;
+  return Piece{first, per < n - first ? first + per : n};
+}
+
 }  // namespace pce

@@ -37,3 +37,21 @@ def test_blocks_of_the_tiled_fp32_kernel(tmp_path):
           NEED(row0 >= 0 && row0 < n && row0 + (bm - 1) >= 0);
         }
       }""")
+
+
+def test_pieces_of_a_cooperative_grid(tmp_path):
+    """Contiguous pieces cover every entry once, up to 2^31 - 1 entries, and a piece's walk in strides of a block's 2048
+    entries (512 threads, four each) does not wrap around behind the last one."""
+    _run(tmp_path, """
+      const unsigned sizes[] = {1, 2, 4095, 4096, 4097, 2147479552u, 2147483639u, 2147483646u, 2147483647u};
+      for (unsigned n : sizes) for (unsigned parts : {1u, 2u, 295u, 296u, 1024u}) {
+        unsigned covered = 0;
+        for (unsigned p = 0; p < parts; ++p) {
+          const Piece a = piece_of(n, p, parts);
+          NEED(a.first == covered && a.end >= a.first && a.end <= n);
+          covered = a.end;
+          const unsigned past = a.end + 2048u + 2048u;
+          NEED(past > a.end);
+        }
+        NEED(covered == n);
+      }""")
