@@ -517,6 +517,7 @@ static int build_map_blocks(pce_plan* p, PlanLane* l, pce_pass* ps, int i, const
   cudaStream_t st = l->stream;
   pce_planned_map& out = ps->maps[i];
   const int kv = sp.ks[0] * sp.ks[1] * sp.ks[2], n_in = in.n, n_out = outl.n;
+  if (static_cast<long long>(kv) * n_in >= (1ll << 31)) return PCE_ERR_UNSUPPORTED;  // neighbours are counted in 32 bits, as in the dense table
   for (int d = 0; d < 3; ++d) out.cmax_out[d] = outl.cmax[d];
   out.n_in = n_in;
   out.n_out = n_out;

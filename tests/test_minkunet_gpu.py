@@ -437,3 +437,18 @@ def test_plan_with_five_list_shapes_on_one_map(waves):
         assert torch.equal(hit[4].tensor()[: stages * slots * rows], want[4][: stages * slots * rows])
     del planned, x
     plan.close()
+
+
+def test_planned_map_beyond_32_bit_counts_is_refused():
+    """27 offsets x 79 536 432 voxels are 2^31 + 16 possible pairs: refused, as the dense form refuses them."""
+    import pcengine_b200 as pce
+    lin = torch.arange(2 ** 31 // 27 + 1, device="cuda")
+    coords = torch.stack([0 * lin, lin // 262144, lin // 512 % 512, lin % 512], 1).int().contiguous()
+    del lin
+    plan = pce.MapPlan([(3, 1, False, 16, 32), (2, 2, False, 32, 64)])
+    x = pce.spTensor(torch.empty(len(coords), 0, device="cuda"), coords, None, [0, 0, 0], [511, 511, 511], init_tag=["D2"])
+    assert plan.begin(x)
+    with pytest.raises(RuntimeError, match="unsupported"):
+        x.planner.fetch(x, next(iter(plan.index)), None)
+    del x
+    plan.close()
