@@ -356,13 +356,13 @@ struct CollateArgs {
 namespace pce {
 // (batch, x, y, z) rows of up to 64 samples, and the maximum of every coordinate.
 __global__ void __launch_bounds__(256) k_collate(const __grid_constant__ CollateArgs a, int4* __restrict__ out, int* __restrict__ cmax) {
-  const int rows = a.first[a.n_samples];
+  const unsigned rows = a.first[a.n_samples];
   int m[3] = {static_cast<int>(0x80000000), static_cast<int>(0x80000000), static_cast<int>(0x80000000)};
-  for (int i = blockIdx.x * 256 + threadIdx.x; i < rows; i += gridDim.x * 256) {
+  for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < rows; i += gridDim.x * 256) {  // (int would wrap near 2^31 rows)
     int lo = 0, hi = a.n_samples;  // last sample whose first row is not behind i
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (a.first[mid] <= i)
+      if (static_cast<unsigned>(a.first[mid]) <= i)
         lo = mid;
       else
         hi = mid;
