@@ -103,18 +103,19 @@ typedef struct pce_epilogue {
    * be a multiple of 8 elements and the pointers 16-byte aligned. */
   int32_t in_ld;
   int32_t out_ld;
-  /* Scratch for maps with few tiles (optional).  A 128-row tile is one sequential chain of
-   * (offset, K block) stages on one CTA; a map with fewer tiles than the GPU has CTA slots leaves
-   * SMs idle while those chains run, and one with a few times as many ends in a half-empty wave.
-   * With split_scratch of at least pce_conv_split_scratch_bytes(...) bytes (16-byte aligned) the
-   * tiles are split between CTAs -- a cluster of 2, 4 or 8 CTAs per tile on small maps, which add
-   * their fp32 sums through shared memory (any non-empty scratch will do), equal shares of the
-   * stages whatever tiles they fall in on mid-size ones, where the CTAs leave fp32 partial sums
-   * here and a second kernel adds them in a fixed order and applies the epilogue (deterministic;
-   * the fp32 sum is associated differently than in the one-CTA chain).  Without scratch the layer
-   * runs whole. */
+  /* Maps with few tiles (optional).  A 128-row tile is one sequential chain of (offset, K block)
+   * stages on one CTA; a map with fewer tiles than the GPU has CTA slots leaves SMs idle while
+   * those chains run, and one with a few times as many ends in a half-empty wave.  With `split`
+   * set, small maps run a cluster of 2, 4 or 8 CTAs per tile (pce_conv_split_parts), which add
+   * their fp32 sums through shared memory.  With split_scratch of at least
+   * pce_conv_split_scratch_wanted(...) bytes (16-byte aligned), mid-size maps are cut into equal
+   * shares of the stages whatever tiles they fall in: the CTAs leave fp32 partial sums here and a
+   * second kernel adds them in a fixed order and applies the epilogue.  Both are deterministic;
+   * the fp32 sum is associated differently than in the one-CTA chain.  A scratch, however small,
+   * implies `split`; with neither the layer runs whole. */
   void* split_scratch;
   size_t split_scratch_bytes;
+  int32_t split;
 } pce_epilogue;
 
 /* The kernel map re-laid for the tensor-core kernel (pce_build_tile_lists): output
@@ -151,7 +152,7 @@ typedef struct pce_tile_lists {
 
 PCE_API const char* pce_strerror(int status);
 /* 100 * major + minor of this header's struct layouts (101: pce_epilogue.in_ld / out_ld,
- * pce_tile_lists.settled); a binding checks it before it passes structs. */
+ * pce_tile_lists.settled; 104: pce_epilogue.split); a binding checks it before it passes structs. */
 PCE_API int pce_version(void);
 /* cudaError_t of the most recent failing CUDA call made by this library on the
  * calling thread (0 if none). */
@@ -381,7 +382,7 @@ PCE_API int pce_pack_weights(const void* weights, int32_t kv, int32_t c_in, int3
  * faster; tile lists of 512 rows always run on the former; what = 5: hash-table queries of the
  * map builder with four cooperating lanes per query (1) or one thread per query (0, default);
  * what = 6: sort the rows on the most significant `value` bits of their key only (0 = all, default);
- * what = 7: 0 never splits tiles between CTAs; 1 (default) as pce_conv_split_scratch_bytes says;
+ * what = 7: 0 never splits tiles between CTAs; 1 (default) as pce_epilogue.split and split_scratch say;
  *           2 only the split of small maps into parts, no shares of stages on mid-size maps.
  * what = 8: 0 stages the last K block of a width that is an odd multiple of 32 channels padded to 64
  *           (1, default: its weights as 32 channels, no padding; same results).
@@ -399,18 +400,19 @@ PCE_API int pce_device_status(int32_t* status_host, int32_t reset);
 PCE_API int pce_debug_timeout(int32_t* where4);
 
 /* Parts per tile (1, 2, 4 or 8) that pce_conv_fwd uses for a tensor-core layer of n_rows outputs
- * gathered from n_src input rows when pce_epilogue.split_scratch is given; 1 = the layer is not split
+ * gathered from n_src input rows when pce_epilogue.split is set; 1 = the layer is not split
  * into parts (large maps, layers with 16 or 32 input channels, short stage chains, up-sampling
  * layers: few pairs per output row). */
 PCE_API int32_t pce_conv_split_parts(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out, int32_t kv,
                                      int32_t sm_count);
 
-/* Bytes of pce_epilogue.split_scratch with which pce_conv_fwd splits a tensor-core layer of n_rows
- * outputs gathered from n_src input rows; 0 = the layer runs whole. */
+/* Bytes of pce_epilogue.split_scratch that are enough for any split of a tensor-core layer of n_rows
+ * outputs gathered from n_src input rows; 0 = the layer runs whole.  (Layers split into parts use
+ * none of it since version 104.) */
 PCE_API size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
-/* What the engine gives: 0 where such a split was measured slower than the whole layer, and a
- * token size where the parts need no scratch of their own. */
+/* What the engine gives: the partial sums of layers cut into shares of stages, 0 where that was
+ * measured slower than the whole layer or the layer is split into parts. */
 PCE_API size_t pce_conv_split_scratch_wanted(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
 
@@ -567,8 +569,8 @@ PCE_API int pce_pass_release(pce_pass* pass, void* stream);
  * layer of ref: script/spconv.py:297-304), with the fused epilogue of pce_epilogue.  Buffers are
  * [rows of coordinate level `level`] x width fp16 matrices placed in `arena` in order of first use
  * (256-byte aligned; PCE_ERR_WORKSPACE when it is too small; sum over buffers of rows x width x 2
- * bytes with rows <= the input's rows, plus 400 MB for the fp32 partial sums of layers on small maps
- * that are split over several CTAs per tile (pce_conv_split_parts), always fits); an operation reads / writes a column range of one
+ * bytes with rows <= the input's rows, plus 400 MB for the fp32 partial sums of layers on
+ * mid-size maps that are cut into shares of stages (pce_conv_split_scratch_wanted), always fits); an operation reads / writes a column range of one
  * (col, c_in / c_out wide, multiples of 8), so skip concatenations cost nothing.  Buffer -1 is the
  * network input (`input`, row pitch in_ld), -2 its output (`output`, out_ld).  Maps are fetched as
  * operations first need them (pce_pass_map), so the pass's map construction overlaps the kernels.

@@ -49,7 +49,7 @@ const char* pce_strerror(int status) {
   }
 }
 
-int pce_version(void) { return 103; }  // 103: pce_planned_csr.starts / row_nbr / counts, pce_planned_map.map may be NULL
+int pce_version(void) { return 104; }  // 104: pce_epilogue.split; 103: pce_planned_csr.starts / row_nbr / counts, pce_planned_map.map may be NULL
 
 int pce_last_cuda_error(void) { return g_last_cuda_error; }
 

@@ -1644,7 +1644,7 @@ static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in
 int umma_half_blocks = 1;
 
 // 1: maps with few tiles are split over several CTAs per tile, mid-size maps into equal shares of stages,
-// when the caller gives scratch (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
+// when the caller asks for it (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
 int umma_split_enabled = 1;
 
 // Parts per tile for a layer of n_rows outputs (8, 4, 2 or 1; see the rule below).  Layers with 16 or 32 input channels
@@ -1706,7 +1706,8 @@ int conv_streamk_grid(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
   return static_cast<int>(slots);
 }
 
-// Scratch (bytes of fp32 partial sums) that lets a layer be split, 0 when it runs whole.
+// Scratch (bytes) that is enough for any split of a layer, 0 when it runs whole.  Parts need none: their bound is what
+// callers of earlier versions sized by.
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   const int parts = conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count);
   if (parts > 1) return static_cast<size_t>(parts) * n_rows * cout * sizeof(float);
@@ -1718,7 +1719,7 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
 // their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
 // 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
-  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 16;  // (parts add up in shared memory)
+  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;  // (parts add up in shared memory)
   if (chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
   return conv_split_scratch_bytes(n_rows, n_src, cin, cout, kv, sm_count);
 }
@@ -1881,16 +1882,16 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   if (smem > 227 * 1024) return PCE_ERR_UNSUPPORTED;
   const int n_tiles = div_up(n_out, umma::kTileM * sub);
   int grid = n_tiles < sm_count[dev] * per_sm ? n_tiles : sm_count[dev] * per_sm;
-  // few tiles, long stage chains: several CTAs per tile, partial sums through the caller's scratch
+  // few tiles, long stage chains: several CTAs per tile, or shares of stages with partial sums in the caller's scratch
   int parts = 1;
   bool streamk = false;
-  if (tiles && sub == 1 && slots == 1 && !push && ep && ep->split_scratch &&
-      (reinterpret_cast<uintptr_t>(ep->split_scratch) & 15) == 0) {
+  const bool scratch = ep && ep->split_scratch && (reinterpret_cast<uintptr_t>(ep->split_scratch) & 15) == 0;
+  if (tiles && sub == 1 && slots == 1 && !push && ep && (ep->split || scratch)) {
     parts = conv_split_parts(n_out, n_in, cin, cout, kv, sm_count[dev]);
     if (parts > 1) {
       grid = n_tiles * parts;
       e.parts = parts;
-    } else {
+    } else if (scratch) {
       const int g = conv_streamk_grid(n_out, n_in, cin, cout, kv, sm_count[dev]);
       if (g > 0 && g <= sm_count[dev] * per_sm &&
           static_cast<size_t>(g) * 2 * umma::kTileM * cout * sizeof(float) <= ep->split_scratch_bytes) {

@@ -922,7 +922,7 @@ static int net_run_on(pce_pass* ps, const pce_net_buffer* buffers, int32_t n_buf
   std::vector<char*> base(n_buffers, nullptr);
   size_t used = 0;
   char* arena_c = static_cast<char*>(arena);
-  char* split = nullptr;  // scratch of split layers (fp32 partial sums)
+  char* split = nullptr;  // scratch of layers cut into shares of stages (fp32 partial sums)
   size_t split_bytes = 0;
   auto fetch = [&](int i) -> int {
     if (i < 0 || i >= n_specs) return PCE_ERR_INVALID;
@@ -1010,8 +1010,9 @@ static int net_run_on(pce_pass* ps, const pce_net_buffer* buffers, int32_t n_buf
       if (c.tile_rows == rows && (c.slots > 1 ? c.slots : 1) == slots && (c.identity_stage || op.extra_c == 0)) tl = &c;
     }
     if (!tl) return PCE_ERR_INVALID;  // the plan was declared without this layer's widths
-    // small and mid-size maps: tiles split between CTAs; the fp32 partial sums live behind the buffers
-    // (one region, reused by every split layer: the layers run in stream order)
+    // small and mid-size maps: tiles split between CTAs; the fp32 partial sums of shares of stages live behind the
+    // buffers (one region, reused by every such layer: the layers run in stream order)
+    ep.split = 1;
     const size_t want = conv_split_scratch_wanted(dst_rows, src_rows, op.c_in, op.c_out, op.kv, p->sm_count);
     if (want > 0) {
       const size_t need = pad256(want);

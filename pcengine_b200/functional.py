@@ -100,13 +100,14 @@ def supports_second_operand(dtype, c_in: int, c_out: int, c2: int) -> bool:
             and c2 >= 16)
 
 
-def _pack(ep: Optional[FusedEpilogue], c_out, n_out, dtype, in_ld: int = 0, out_ld: int = 0, split=None):
-    if ep is None and not in_ld and not out_ld and split is None:
+def _pack(ep: Optional[FusedEpilogue], c_out, n_out, dtype, in_ld: int = 0, out_ld: int = 0, split: bool = False,
+          scratch=None):
+    if ep is None and not in_ld and not out_ld and not split:
         return None
     e = ep.pack(c_out, n_out, dtype) if ep is not None else _lib.Epilogue()
-    e.in_ld, e.out_ld = in_ld, out_ld
-    if split is not None:
-        e.split_scratch, e.split_scratch_bytes = split.data_ptr(), split.numel() * split.element_size()
+    e.in_ld, e.out_ld, e.split = in_ld, out_ld, split
+    if scratch is not None:
+        e.split_scratch, e.split_scratch_bytes = scratch.data_ptr(), scratch.numel() * scratch.element_size()
     return C.byref(e)
 
 
@@ -115,9 +116,7 @@ SPLIT_TILES = True
 
 
 def _split_scratch(n_rows: int, n_src: int, c_in: int, c_out: int, kv: int, device):
-    """Scratch of a layer that the library will split between CTAs, or None."""
-    if not SPLIT_TILES:
-        return None
+    """Scratch of a layer that the library will cut into shares of stages, or None."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     sms = _SM_COUNT.get(idx)
     if sms is None:
@@ -303,7 +302,8 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
                    residual=epilogue is not None and epilogue.residual is not None,
                    start=torch.cuda.Event(enable_timing=True), end=torch.cuda.Event(enable_timing=True))
         rec["start"].record()
-    tiles = split = None
+    tiles = scratch = None
+    split = False
     stream = _lib.stream_ptr(feats.device)
     if packed is not None:
         # (the halo push lives in the one-accumulator kernel: 128-row tiles)
@@ -317,8 +317,9 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
             lists.settled = 1 if lists.stream == stream else 0
             lists.stream = stream
         tiles = C.byref(lists)
-        if rows == 128 and not pushes:
-            split = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
+        if SPLIT_TILES and rows == 128 and not pushes:
+            split = True
+            scratch = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
     elif (kernel_choice == "auto" and feats.dtype == torch.float32
           and (csr._fp32 is not None or csr.wants_tiles()
                or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
@@ -328,7 +329,7 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
     _lib.check(lib.pce_conv_fwd(feats.data_ptr(), feats.size(0), c_in, kernel.data_ptr(), _lib.ptr(packed), kv, c_out,
                                 csr.mask.data_ptr(), _lib.ptr(rowptr), _lib.ptr(nbr), tiles, csr.n_rows,
                                 out.data_ptr(), _lib.dtype_code(feats.dtype),
-                                _pack(epilogue, c_out, csr.n_rows, feats.dtype, in_ld, out_ld, split),
+                                _pack(epilogue, c_out, csr.n_rows, feats.dtype, in_ld, out_ld, split, scratch),
                                 _KERNEL[kernel_choice], stream), "pce_conv_fwd")
     if rec is not None:
         rec["end"].record()

@@ -1,4 +1,6 @@
 """Tiles shared by a cluster of CTAs at the edges of their rule, against the oracle (GPU)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -31,3 +33,29 @@ def test_parts_of_a_tile(n, cin, cout, parts):
     outs = [PF.conv_forward(x.cuda(), w.cuda(), km.csr(), ep) for _ in range(2)]
     assert torch.equal(*outs) and co.rel_l2(outs[0].float().cpu(), want) <= 1e-3
     assert PF.device_status() == 0
+
+
+def test_parts_need_no_scratch():
+    """The flag alone splits a small map: the engine allocates the output and nothing else, the sums are those that a call
+    with scratch gives, and another association than the whole chain's."""
+    import pcengine_b200 as pce
+    from pcengine_b200 import _lib
+    from pcengine_b200 import functional as PF
+    coords = surface_cloud(8, 66)[:3000]
+    n, sms = len(coords), torch.cuda.get_device_properties(0).multi_processor_count
+    assert _lib.lib.pce_conv_split_parts(n, n, 256, 256, 27, sms) > 1
+    assert _lib.lib.pce_conv_split_scratch_wanted(n, n, 256, 256, 27, sms) == 0
+    csr = pce.KernelMap(torch.from_numpy(np.ascontiguousarray(coords)).cuda(), (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True).csr()
+    g = torch.Generator().manual_seed(1)
+    x, w = torch.randn(n, 256, generator=g).half().cuda(), (torch.randn(27, 256, 256, generator=g) / 83).half().cuda()
+    first = PF.conv_forward(x, w, csr)
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    again = PF.conv_forward(x, w, csr)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before + 1
+    lists, packed, scratch = csr.tiles(True, 128, False, 1), PF.packed_weights(w), torch.empty(16, device="cuda")
+    out, e = torch.empty_like(first), _lib.Epilogue(split_scratch=scratch.data_ptr(), split_scratch_bytes=64)
+    _lib.check(_lib.lib.pce_conv_fwd(x.data_ptr(), n, 256, None, packed.data_ptr(), 27, 256, None, None, None, C.byref(lists), n,
+                                     out.data_ptr(), _lib.PCE_F16, C.byref(e), _lib.KERNEL_AUTO, _lib.stream_ptr(x.device)), "pce_conv_fwd")
+    PF.SPLIT_TILES = False  # (the test's fixture puts it back)
+    whole = PF.conv_forward(x, w, csr)
+    assert torch.equal(first, again) and torch.equal(first, out) and not torch.equal(first, whole)
