@@ -321,9 +321,12 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
             split = True
             scratch = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
     elif (kernel_choice == "auto" and feats.dtype == torch.float32
-          and (csr._fp32 is not None or csr.wants_tiles()
-               or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
-        tiles = C.byref(csr.lists_fp32())  # the tiled fp32 kernel (any widths, where a wider layer has left lists)
+          and (csr.parents or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
+        # The tiled fp32 kernel: by the layer's widths, and for every layer between voxels and their parents, whose
+        # rowptr would first need the dense table (2x2x2 layers of 4->16 to 16->32, map included, us, lists against
+        # rowptr: 20 k voxels 129-158 against 177-231, 200 k 169-182 against 210-234; on a kept map within 3 of each
+        # other at 20 k).  By the layer and the map alone: lists that another layer has left change no result.
+        tiles = C.byref(csr.lists_fp32())
     # the tensor-core kernel reads the tile lists only: a planned map's rowptr / nbr are not built for its sake
     rowptr, nbr = (csr._rowptr, csr._nbr) if tiles is not None else csr.row_lists()
     _lib.check(lib.pce_conv_fwd(feats.data_ptr(), feats.size(0), c_in, kernel.data_ptr(), _lib.ptr(packed), kv, c_out,

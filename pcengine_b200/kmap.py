@@ -35,6 +35,11 @@ def candidates_per_input(ks, stride) -> int:
     return n
 
 
+def leads_to_parents(ks, stride, pad, subm: bool) -> bool:
+    """Whether a layer's outputs are the parents of its inputs, through at most 32 offsets."""
+    return not subm and tuple(ks) == tuple(stride) and not any(pad) and ks[0] * ks[1] * ks[2] <= 32
+
+
 # Rows per tile of the tile lists (128 or 256) when the caller does not say.
 TILE_ROWS = 128
 
@@ -51,13 +56,14 @@ class NeighbourCSR:
       the row order, or with rowptr / nbr (``mask_ready`` False until then);
     * neither: a planned map whose tile lists were filled by the planner.
 
-    ``counts``: device int32 [kv], rows that have each offset."""
+    ``counts``: device int32 [kv], rows that have each offset.
+    ``parents``: a direction of a map between voxels and their parents (:func:`leads_to_parents`)."""
 
     __slots__ = ("_mask", "_rowptr", "_nbr", "n_rows", "n_src", "kv", "_order", "_tiles", "_fp32", "_fill", "_pairs", "_lists",
-                 "_table", "_counts", "_mask_ready")
+                 "_table", "_counts", "_mask_ready", "parents")
 
     def __init__(self, mask, rowptr, nbr, n_rows, n_src, kv=None, fill=None, pairs=None, lists=None, table=None, counts=None,
-                 mask_ready=True):
+                 mask_ready=True, parents=False):
         self._mask, self._rowptr, self._nbr, self.n_rows, self.n_src = mask, rowptr, nbr, n_rows, n_src
         self.kv = kv
         self._order = None
@@ -66,6 +72,7 @@ class NeighbourCSR:
         self._fill = fill
         self._pairs = pairs  # callable -> one-element device tensor, for a CSR without rowptr
         self._lists, self._table, self._counts, self._mask_ready = lists, table, counts, mask_ready
+        self.parents = parents
 
     def pair_count(self) -> torch.Tensor:
         """Number of (row, offset) pairs as a NEW one-element device tensor (no read-back, and nothing that
@@ -96,10 +103,6 @@ class NeighbourCSR:
         self._materialise()
         return self._nbr
 
-    def wants_tiles(self) -> bool:
-        """Whether tile lists are cheaper than rowptr / nbr here (a map between voxels and their parents)."""
-        return self._rowptr is None and (self._table is not None or (self._lists is not None and self._lists[0] is None))
-
     def row_lists(self):
         """(starts, nbr): every row's first neighbour and the neighbours, in whatever form is at hand."""
         if self._rowptr is None and self._lists is not None and self._lists[0] is not None:
@@ -115,8 +118,9 @@ class NeighbourCSR:
             starts, nbr = self._lists
             return NeighbourCSR(self.mask[:max(n_rows, 1)], None, None, n_rows, self.n_src, self.kv, lists=(starts[: max(n_rows, 1)], nbr),
                                 fill=lambda: (self.rowptr[: n_rows + 1], self.nbr),
-                                pairs=lambda: self.rowptr[n_rows: n_rows + 1].clone())
-        return NeighbourCSR(self.mask[:max(n_rows, 1)], self.rowptr[: n_rows + 1], self.nbr, n_rows, self.n_src, self.kv)
+                                pairs=lambda: self.rowptr[n_rows: n_rows + 1].clone(), parents=self.parents)
+        return NeighbourCSR(self.mask[:max(n_rows, 1)], self.rowptr[: n_rows + 1], self.nbr, n_rows, self.n_src, self.kv,
+                            parents=self.parents)
 
     def order(self):
         """Output rows sorted by indicator bitmask (int32 [n_rows], built once): the order in which
@@ -337,7 +341,7 @@ class KernelMap:
         """The map between the inputs and their parents (kernel size == stride, no padding): output coordinates and
         both directions at once.  False when the layer, or a very sparse cloud, needs the general form."""
         ks, dev, kv, n = self.ks, self.device, self.kv, self.n_in
-        if ks != self.stride or any(self.pad) or kv > 32 or n == 0:
+        if not leads_to_parents(ks, self.stride, self.pad, self.subm) or n == 0:
             return False
         ws = _lib.workspace(lib.pce_parents_workspace_bytes(n), dev)
         oc = torch.empty((n, 4), dtype=torch.int32, device=dev)
@@ -391,7 +395,8 @@ class KernelMap:
             return self._csr[key]
         mask, rowptr, nbr = self._dense.csr(key, self._sizes[0] if self._sizes is not None else None)
         n_rows, n_src = (self.n_in, self.n_out) if key else (self.n_out, self.n_in)
-        out = self._csr[key] = NeighbourCSR(mask, rowptr, nbr, n_rows, n_src, self.kv)
+        out = self._csr[key] = NeighbourCSR(mask, rowptr, nbr, n_rows, n_src, self.kv,
+                                            parents=leads_to_parents(self.ks, self.stride, self.pad, self.subm))
         return out
 
     def _csr_from_blocks(self) -> NeighbourCSR:
@@ -417,7 +422,7 @@ class KernelMap:
         if transposed:
             return NeighbourCSR(up_mask, None, None, self.n_in, self.n_out, self.kv, fill=lambda: dense.csr(True)[1:],
                                 pairs=pairs, lists=(None, up_nbr),
-                                counts=counts)
+                                counts=counts, parents=True)
         mask = torch.empty((max(self.n_out, 1), 1), dtype=torch.int32, device=self.device)
 
         def fill():
@@ -425,7 +430,7 @@ class KernelMap:
             mask.copy_(full)
             return rowptr, nbr
         return NeighbourCSR(mask, None, None, self.n_out, self.n_in, self.kv, fill=fill, pairs=pairs, table=child, counts=counts,
-                            mask_ready=False)
+                            mask_ready=False, parents=True)
 
     # -- reference forms -----------------------------------------------------
     def pairs(self):

@@ -22,7 +22,7 @@ import torch
 from . import _lib
 from . import functional as PF
 from ._lib import lib
-from .kmap import KernelMap, NeighbourCSR, _DenseTables, make_geom
+from .kmap import KernelMap, NeighbourCSR, _DenseTables, leads_to_parents, make_geom
 from .spconv import _ONES, _triple
 from .utils import conv_info_decoder, conv_info_encoder, output_stride_compute
 
@@ -158,6 +158,7 @@ class PlannedKernelMap(KernelMap):
         self._pairs = self._d1 = self._sizes = self._state = self._parents = None
         self._blocks = False
         self.dataflow = "D2"
+        parents = leads_to_parents(ks, self.stride, self.pad, self.subm)
         for transposed, has, c in ((False, out.has_fwd, out.fwd), (True, out.has_tr, out.tr)):
             if not has:
                 continue
@@ -174,6 +175,7 @@ class PlannedKernelMap(KernelMap):
                                    fill=_csr_filler(int(c.table), kv, int(c.n_rows), int(c.reverse_kp), int(c.identity_kp),
                                                     int(c.nbr_cap), device, keep),
                                    pairs=_pair_counter(d.knnz, int(c.n_rows) if c.identity_kp >= 0 else 0))
+            csr.parents = parents
             for i in range(c.n_lists):
                 t = c.lists[i]
                 slots = max(int(t.slots), 1)

@@ -67,3 +67,42 @@ def test_tiled_fp32_beyond_65535_row_blocks():
         assert float((got[part] - want).norm() / want.norm()) <= 1e-5
     whole = x @ w[0]  # (another fp32 order)
     assert float((got - whole).norm() / whole.norm()) <= 1e-5
+
+
+@pytest.mark.parametrize("ks,stride,transposed,cin,cout", [(3, 1, False, 4, 32), (3, 1, False, 32, 16), (3, 1, False, 64, 8),
+                                                           (5, 1, False, 16, 16), (2, 2, False, 32, 16), (2, 2, True, 24, 24),
+                                                           (3, 2, False, 32, 16)])
+def test_narrow_fp32_layers_do_not_depend_on_what_ran_before(ks, stride, transposed, cin, cout):
+    """Fewer than 768 weights per offset: the same bits on a fresh map, on one where a wide layer has left tile lists,
+    on one whose rowptr or dense table somebody asked for, and on a planned one with and without a wide layer."""
+    import pcengine_b200 as pce
+    from pcengine_b200 import functional as PF
+    coords = random_cloud(3, 24, 3000)
+    subm = stride == 1
+    cmax = [c if subm else (c - (ks - 1)) // stride for c in cmax_of(coords)]
+    cd = torch.from_numpy(coords).cuda()
+
+    def fresh():
+        return pce.KernelMap(cd, (ks,) * 3, (stride,) * 3, (0, 0, 0), [0, 0, 0], cmax, subm)
+    n_src = fresh().csr(transposed).n_src
+    g = torch.Generator().manual_seed(5)
+    x, w = torch.randn(n_src, cin, generator=g).cuda(), torch.randn(ks ** 3, cin, cout, generator=g).cuda()
+    first = PF.conv_forward(x, w, fresh().csr(transposed))
+
+    def after_wide(km):
+        PF.conv_forward(torch.zeros(n_src, 48, device="cuda"), torch.zeros(ks ** 3, 48, 48, device="cuda"), km.csr(transposed))
+    for before in (after_wide, lambda km: km.csr(transposed).rowptr, lambda km: km.map,
+                   lambda km: PF.conv_forward(x, w, km.csr(transposed), kernel_choice="simt")):
+        km = fresh()
+        before(km)
+        assert torch.equal(PF.conv_forward(x, w, km.csr(transposed)), first)
+    use, wide = (ks, stride, transposed, cin, cout), (ks, stride, transposed, 48, 48)
+    down = (2, 2, False, 4, 4) if subm or transposed else use  # (ahead of a transposed use; behind a submanifold one: block form)
+    for layers in ([use, down], [use, wide, down]) if subm else ([down, use], [down, use, down, wide]) if transposed else ([use],):
+        plan = pce.MapPlan(layers, dtype=torch.float32)
+        t = pce.spTensor(torch.zeros(len(coords), 4).cuda(), cd, None, [0, 0, 0], cmax_of(coords), init_tag=["D2"])
+        assert plan.begin(t)
+        csr = t.planner.fetch(t, next(iter(plan.index)), None).csr(transposed)
+        assert torch.equal(PF.conv_forward(x, w, csr), first)
+        del t, csr
+        plan.close()
