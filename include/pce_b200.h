@@ -379,9 +379,9 @@ PCE_API int pce_pack_weights(const void* weights, int32_t kv, int32_t c_in, int3
  * 2 = on, but tile lists are never read before that kernel has finished); what = 4: 1 runs
  * layers with one offset per stage on the kernel with several accumulators per CTA and decoupled
  * row / weight rings (k_conv_umma_mt), 0 (default) on the one-accumulator kernel, which measured
- * faster; tile lists of 512 rows always run on the former; what = 5: hash-table queries of the
- * map builder with four cooperating lanes per query (1) or one thread per query (0, default);
- * what = 6: sort the rows on the most significant `value` bits of their key only (0 = all, default);
+ * faster; tile lists of 512 rows always run on the former; what = 5: 1 makes pce_map_build_d2
+ * query odd submanifold maps in the hash table like all others, 0 (default) in the table of blocks; what = 6: no
+ * effect any more;
  * what = 7: 0 never splits tiles between CTAs; 1 (default) as pce_epilogue.split and split_scratch say;
  *           2 only the split of small maps into parts, no shares of stages on mid-size maps.
  * what = 8: 0 stages the last K block of a width that is an odd multiple of 32 channels padded to 64

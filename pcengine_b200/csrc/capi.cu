@@ -18,14 +18,13 @@ extern int umma_force_sub;
 extern int umma_force_nacc;
 extern int umma_overlap_launches;
 extern int umma_multi_tile;
-extern int kmap_query_lanes4;
+extern int kmap_hash_only;
 extern int umma_split_enabled;
 extern int umma_half_blocks;
 extern int plan_short_route;
 int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
-extern int kmap_sort_top_bits;
 int conv_umma(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out, int cin,
               int cout, void* out, const pce_epilogue* ep, cudaStream_t st);
 }  // namespace pce
@@ -95,13 +94,10 @@ int pce_tune(int32_t what, int32_t value) {
     return PCE_OK;
   }
   if (what == 5) {
-    kmap_query_lanes4 = value ? 1 : 0;
+    kmap_hash_only = value ? 1 : 0;
     return PCE_OK;
   }
-  if (what == 6) {
-    kmap_sort_top_bits = value > 0 ? value : 0;
-    return PCE_OK;
-  }
+  if (what == 6) return PCE_OK;  // (sorted on part of the key once; every bit is sorted on)
   if (what == 7) {
     umma_split_enabled = value < 0 ? 0 : value;
     return PCE_OK;

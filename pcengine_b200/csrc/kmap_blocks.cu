@@ -247,10 +247,6 @@ __global__ void __launch_bounds__(256) k_block_rows(const int4* __restrict__ coo
 
 constexpr int kQueryThreads = 128;
 
-struct Window {  // the blocks around one voxel and where its neighbourhood starts in them
-  int lx, ly, lz;
-};
-
 // Occupancies and places of the (up to) eight blocks that the neighbourhood [l, l + k) of a voxel touches, left in
 // shared memory as column `threadIdx.x` of [8][threads].  All first probes are in flight before the first is used.
 __device__ __forceinline__ void gather_blocks(const Block* __restrict__ table, unsigned tmask, bool live, int b, int lx, int ly, int lz,

@@ -223,9 +223,9 @@ def test_device_voxelisation_edge_cases():
         pce.sparse_quantize(torch.zeros((4, 3), dtype=torch.float64, device="cuda"), 0.1)
 
 
-def test_cooperative_query_builds_the_same_maps():
-    """Four lanes per query (64-byte probe rounds, ballots) and one thread per query give identical
-    kernel maps: submanifold (mirrored probes), strided with the transposed table, 5x5x5."""
+def test_hash_and_block_queries_build_the_same_maps():
+    """The table of blocks and the hash table give identical kernel maps: submanifold (mirrored probes), 5x5x5;
+    strided maps with the transposed table, which have the hash table alone."""
     import pcengine_b200 as pce
     from pcengine_b200 import _lib
     coords = surface_cloud(19, 80, batch=2)
@@ -236,8 +236,8 @@ def test_cooperative_query_builds_the_same_maps():
     for ks, stride, subm, cm in cases:
         maps = []
         try:
-            for lanes4 in (0, 1):
-                _lib.lib.pce_tune(5, lanes4)
+            for hash_only in (0, 1):
+                _lib.lib.pce_tune(5, hash_only)
                 km = pce.KernelMap(cd, ks, stride, (0, 0, 0), [0, 0, 0], cm, subm)
                 maps.append((km.map.clone(), None if km.map_out is None else km.map_out.clone(), km.knnz.clone(), km.kpos.clone()))
         finally:
