@@ -901,7 +901,7 @@ namespace blk {
 // At most 0.75 full when every voxel has a block to itself (scanned surfaces: 2 to 8 voxels per block).
 unsigned table_slots(long long n) {
   unsigned t = 1024;
-  while (3ll * t < 4ll * n) t <<= 1;
+  while (t < 1u << 31 && 3ll * t < 4ll * n) t <<= 1;  // (beyond 1.6 G voxels fuller than that: no map of that size is built)
   return t;
 }
 

@@ -30,6 +30,9 @@ def test_status_strings_and_size_queries_need_no_gpu():
     assert lib.pce_version() >= 100
     assert lib.pce_map_workspace_bytes(100000, 27, 100000) > 16 * 262144
     assert lib.pce_csr_from_pairs_workspace_bytes(1000, 100) > 0
+    for n in (0, 1, 2 ** 31 - 1):  # up to the last int32 row
+        for name in ("pce_subm_workspace_bytes", "pce_order_workspace_bytes", "pce_parents_workspace_bytes", "pce_quantize_workspace_bytes"):
+            assert getattr(lib, name)(n) > 4 * n, (name, n)
 
 
 def test_product_refuses_cpu_tensors():
