@@ -27,9 +27,9 @@ def pytest_collection_modifyitems(config, items):
             item.add_marker(skip)
 
 
-# Layers on small maps are split over several CTAs per tile (fp32 partial sums added by a second kernel),
-# which associates the fp32 sum differently from the one-CTA chain.  Tests that assert BIT-identity between
-# schedules (tile heights, row orders, slabs vs whole scene, the two kernels) run with the split off, which is
+# Layers on small maps are split over several CTAs per tile (fp32 sums added up through a cluster's shared memory), and
+# mid-size ones cut into shares of stages (added by a second kernel), which associates the fp32 sum differently from
+# the one-CTA chain.  Tests that assert BIT-identity between schedules (tile heights, row orders, slabs vs whole scene, the two kernels) run with the split off, which is
 # what they are about; parity tests against the oracle and the reference run the default, split, path, and
 # tests marked `split_tiles` exercise it explicitly.
 _SPLIT_ON_MODULES = {"test_baseline_configs_gpu", "test_ref_golden", "test_reference_python_gpu", "test_backend_dropin_gpu",

@@ -22,7 +22,7 @@ def test_tiled_fp32_convolution_equals_the_oracle(n, cin, cout):
     d2 = ko.build_d2(coords, (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
     km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
     csr = km.csr()
-    csr.lists_fp32()  # (with lists at hand a layer of any widths runs on the tiled kernel)
+    csr.lists_fp32()
     res, shift = torch.randn(n, cout), torch.randn(cout)
     ep = PF.FusedEpilogue(scale=None, shift=shift.cuda(), residual=res.cuda(), act="relu")
     out = PF.conv_forward(feats.cuda(), w.cuda(), csr, ep)

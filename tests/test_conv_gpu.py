@@ -647,8 +647,8 @@ def _split_layer_case(cin, cout, n_side, ks, stream_k):
 @pytest.mark.split_tiles
 @pytest.mark.parametrize("cin,cout,n_side,ks", [(256, 256, 20, 3), (128, 256, 30, 3), (96, 96, 48, 3), (128, 128, 26, 5), (256, 128, 24, 2)])
 def test_small_maps_split_over_several_ctas(cin, cout, n_side, ks):
-    """A map with few 128-row tiles runs with several CTAs per tile: every CTA takes a part of the tile's
-    stage list, the fp32 partial sums are added in order by a second kernel that also applies the epilogue
+    """A map with few 128-row tiles runs with a cluster of CTAs per tile: every CTA takes a part of the tile's
+    stage list, the fp32 sums are added in order through the cluster's shared memory and finished with the epilogue
     (scale, shift, residual or second operand, activation).  Same features as the oracle and as the unsplit
     kernel within fp16 rounding, bit-identical run to run."""
     _split_layer_case(cin, cout, n_side, ks, stream_k=False)
@@ -656,11 +656,22 @@ def test_small_maps_split_over_several_ctas(cin, cout, n_side, ks):
 
 @pytest.mark.split_tiles
 @pytest.mark.parametrize("cin,cout,n_side,ks", [(256, 256, 128, 3), (192, 96, 150, 3), (384, 256, 110, 3), (64, 64, 140, 3)])
-def test_mid_size_maps_cut_into_equal_shares_of_stages(cin, cout, n_side, ks):
+def test_mid_size_maps_cut_into_equal_shares_of_stages(cin, cout, n_side, ks, monkeypatch):
     """A map of half a wave to one wave of tiles with long stage chains is cut into equal shares of ring stages, one share per CTA slot,
     wherever the cuts fall inside the tiles; tiles that two or more CTAs worked on are summed in CTA order
-    and finished by a second kernel.  Same checks as for the split into parts."""
+    and finished by a second kernel.  Same checks as for the split into parts.  (The engine gives the scratch for
+    this to layers with chains of 48 stages and more; here every layer gets it that can be cut.)"""
+    from pcengine_b200 import _lib
+    from pcengine_b200 import functional as PF
+    given = []
+
+    def scratch(n_rows, n_src, c_in, c_out, kv, device):
+        sms = torch.cuda.get_device_properties(device).multi_processor_count
+        given.append(_lib.lib.pce_conv_split_scratch_bytes(n_rows, n_src, c_in, c_out, kv, sms))
+        return torch.empty(given[-1] // 4, device=device)
+    monkeypatch.setattr(PF, "_split_scratch", scratch)
     _split_layer_case(cin, cout, n_side, ks, stream_k=True)
+    assert given and min(given) > 0
 
 
 def test_push_rows_gathers_into_consecutive_rows():

@@ -326,9 +326,8 @@ def test_one_call_pass_equals_the_layer_by_layer_pass():
 
 def test_planner_routes_build_the_same_lists():
     """A planned map of at most 32 offsets whose layers all run on tile lists arrives without rowptr / nbr
-    (the lists were filled straight from the dense table, the row order came from knnz): its bitmask, row order
-    and tile lists are those of the route through the neighbour CSR (pce_tune(9, 0)), the logits are the same
-    bit for bit, and rowptr / nbr appear, equal to the other route's, when they are first asked for."""
+    (in block form: order and lists straight from the blocks' neighbours): its bitmask, row order and tile lists
+    are those of the route through the dense table and its CSR (pce_tune(9, 0)), the logits are the same bit for bit, and rowptr / nbr appear, equal to the other route's, when they are first asked for."""
     import pcengine_b200 as pce
     from pcengine_b200 import _lib
     coords = surface_cloud(46, 72, batch=2)
