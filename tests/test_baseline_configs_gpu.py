@@ -147,3 +147,20 @@ def test_full_width_network_on_one_lidar_scan():
         assert np.array_equal(as_np(km.kpos), d2["kpos"]) and np.array_equal(as_np(km.qkpos), d2["qkpos"])
         assert np.array_equal(as_np(km.out_coords), d2["out_coords"])
     assert co.rel_l2(y.feats.float().cpu(), want) <= 5e-3
+
+
+def test_single_layer_row_of_the_bench_times_kernels(monkeypatch):
+    """Every figure of the 20 k-voxel row comes from a call that launches kernels of the library: a map object alone, which
+    builds nothing until it is asked, is not one."""
+    import bench
+    from pcengine_b200._lib import lib
+    launches = []
+
+    def timed(fn, *args):
+        before = lib.pce_kernel_launches()
+        fn()
+        launches.append(lib.pce_kernel_launches() - before)
+        return 1e-3
+    monkeypatch.setattr(bench, "_timed", timed)
+    bench.config1_row(torch.device("cuda", 0), dict(hbm_gbs=1.0, tflops=1.0))
+    assert len(launches) == 3 and min(launches) > 0
