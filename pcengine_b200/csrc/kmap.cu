@@ -1306,6 +1306,7 @@ int pce_map_build_d1(const int32_t* map, const int32_t* map_out, int32_t kv, int
   if (!ar.ok) return PCE_ERR_WORKSPACE;
   void* args[] = {&a};
   PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_d1_codes), dim3(g), dim3(coop::kThreads), args, 0, st));
+  PCE_LAUNCH_CHECK();
   return PCE_OK;
 }
 
