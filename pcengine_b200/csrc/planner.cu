@@ -12,8 +12,8 @@
 // produces the same maps (same entry points as the lazy path, so bit-identical) ahead of time.
 //
 // Lanes: a map needs the coordinates of its level(s) and nothing else, so only the chain of
-// down-sampled coordinates is sequential.  Lane 0 runs that chain (each step reads one size back
-// and therefore synchronises lane 0's stream only); the map lanes take the maps in first-use
+// down-sampled coordinates is sequential.  Lane 0 runs that chain (in block form, run_chain, all levels at once with one
+// wait for their sizes; else each step reads one size back and synchronises lane 0's stream only); the map lanes take the maps in first-use
 // order, wait on the host until the levels they read exist, make their stream wait for the
 // level's event and queue hash / query / CSR / row order / tile lists.  One lane alone was
 // measured launch-bound: 400 launches in 3.3 ms for a 5-level network whose convolutions wait

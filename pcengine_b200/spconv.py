@@ -105,10 +105,10 @@ def _with_bias(epilogue: Optional[FusedEpilogue], bias) -> Optional[FusedEpilogu
 # Measured crossover of the two dataflows on B200 (submanifold 3x3x3, fp16, kernel-only, L2 flushed:
 # `bench.py --workload selector`, summarised in profiles/selector_sweep.md): channel widths 16..256 x
 # {indoor surfaces, LiDAR, fully dense block} x {about 25 k, 200 k rows}.  The fused output-stationary
-# dataflow (D2) is faster in 35 of the 36 cells (by 1.0-16x; the explicit one moves 2*(C_in + C_out)*pairs
-# extra elements through HBM).  The explicit dataflow (D1) wins where D2's per-tile weight staging
-# dominates: wide layers on small, very sparse maps (256 -> 256 on 25 k rows with 1.2 pairs per row:
-# 56 vs 82 us); at 96..128 channels on such maps the two tie (1.02-1.04).  Each entry: D1 when the
+# dataflow (D2) is faster by 1.4-19x in 35 of the 36 cells (the explicit one moves 2*(C_in + C_out)*pairs
+# extra elements through HBM).  The entry is the closest cell, wide layers on small, very sparse maps, where D2's
+# per-tile weight staging dominates (256 -> 256 on 25 k rows with 1.2 pairs per row): the explicit dataflow (D1) won it
+# when the table was made (56 us against 82) and is 1.2x behind on the present kernels (54 against 46).  Each entry: D1 when the
 # layer is fp16, both widths >= c_min, the map has at most rows_max output rows and at most ppr_max pairs
 # per row.
 _D1_WINS = (dict(half=True, c_min=256, rows_max=40000, ppr_max=2.0),)
