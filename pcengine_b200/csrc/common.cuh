@@ -36,6 +36,10 @@ inline int cuda_fail(cudaError_t e) {
     if (s__ != PCE_OK) return s__; \
   } while (0)
 
+// 16 pinned words of the calling thread, mapped, in which a call that waits for its work reads sizes back; given back when
+// the thread ends.  nullptr: no memory.
+int* thread_words();
+
 inline int div_up(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 
 // Multiprocessors of the current device (looked up once per device), 0 on failure.

@@ -849,13 +849,37 @@ __global__ void __launch_bounds__(512)
 
 // ---- host helpers ------------------------------------------------------------
 
+// What a thread keeps for its read-backs; freed when it ends (a service that takes a thread per request keeps nothing).
+struct ThreadState {
+  int* words = nullptr;
+  cudaEvent_t ev[64] = {};  // per device
+  ~ThreadState() {
+    if (words) cudaFreeHost(words);
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+  }
+};
+static thread_local ThreadState thread_state;
+
+int* thread_words() {
+  int*& w = thread_state.words;
+  if (!w) {
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&w), 64, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+      cuda_fail(e);
+      w = nullptr;
+    }
+  }
+  return w;
+}
+
 // Waits for everything queued on `st` without burning a core: polls an event, yielding the
 // processor between polls, for a short while (the usual case: a few microseconds of work ahead),
 // then sleeps on it.  cudaStreamSynchronize spins, and the size read-back of a strided layer can
 // wait for milliseconds behind other work; with one process per GPU and several planner threads
 // per process, spinning starves the threads that queue the kernels being waited for.
 int wait_for_stream(cudaStream_t st) {
-  static thread_local cudaEvent_t ev[64] = {};
+  cudaEvent_t* ev = thread_state.ev;
   int dev = 0;
   PCE_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) {
@@ -1061,9 +1085,8 @@ int pce_downsample_coords(const int32_t* in_coords, int32_t n_in, const pce_geom
   PCE_LAUNCH_CHECK();
   // read back through pinned memory: a copy to pageable memory would make the copy call itself wait
   // (spinning) for the stream, a pinned one returns at once and the wait below sleeps
-  static thread_local int* pinned = nullptr;
-  if (!pinned) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pinned), 64, cudaHostAllocDefault));
-  int* host = pinned;
+  int* host = thread_words();
+  if (!host) return PCE_ERR_CUDA;
   host[0] = host[1] = host[2] = 0;
   PCE_CUDA(cudaMemcpyAsync(host, ctr, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   PCE_TRY(wait_for_stream(st));
@@ -1231,8 +1254,8 @@ int pce_parents(const int32_t* in_coords, int32_t n_in, const pce_geom* g, void*
   if (!blk::parents(g) || n_in == 0) return PCE_ERR_UNSUPPORTED;
   if (!in_coords || !out_coords || !up_mask || !up_nbr || !child) return PCE_ERR_INVALID;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  static thread_local int* host = nullptr;  // mapped: the kernel writes the sizes itself
-  if (!host) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+  int* host = thread_words();  // (mapped: the kernel writes the sizes itself)
+  if (!host) return PCE_ERR_CUDA;
   int* host_dev = nullptr;
   PCE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&host_dev), host, 0));
   blk::Chain c;

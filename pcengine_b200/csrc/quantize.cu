@@ -289,8 +289,8 @@ static int voxelise(const float* points, int n, const float* voxel, int batch, v
     PCE_LAUNCH_CHECK();
     return PCE_OK;
   }
-  static thread_local int* host = nullptr;  // mapped: the kernel writes the two words itself
-  if (!host) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+  int* host = thread_words();  // (mapped: the kernel writes the two words itself)
+  if (!host) return PCE_ERR_CUDA;
   PCE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&out.host), host, 0));
   host[0] = PCE_ERR_CUDA;
   Arena ar(workspace, workspace_bytes);
@@ -415,8 +415,8 @@ extern "C" int pce_collate_coords(const int32_t* const* coords, const int32_t* r
     }
     done += total;
   }
-  static thread_local int* host = nullptr;
-  if (!host) PCE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), 64, cudaHostAllocPortable));
+  int* host = thread_words();
+  if (!host) return PCE_ERR_CUDA;
   PCE_CUDA(cudaMemcpyAsync(host, scratch, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   PCE_CUDA(cudaStreamSynchronize(st));
   for (int d = 0; d < 3; ++d) cmax_host[d] = host[d];
