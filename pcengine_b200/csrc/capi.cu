@@ -172,7 +172,7 @@ int pce_conv_fwd(const void* in_feats, int32_t n_in, int32_t c_in, const void* w
              (ep->out_ld > 0 && ep->out_ld != c_out)))
     return PCE_ERR_UNSUPPORTED;  // the second operand, the halo push and row pitches need the tensor-core kernel
   if (dtype == PCE_F32 && weights && tiles && tiles->tile_ptr && tiles->stage_kp && tiles->stage_nbr && tiles->tile_rows == 128 &&
-      tiles->slots <= 1 && n_in > 0 && kernel_choice != PCE_KERNEL_SIMT)
+      tiles->slots <= 1 && kernel_choice != PCE_KERNEL_SIMT)  // (no inputs: the lists are empty, every row is its epilogue)
     return conv_f32(in_feats, weights, tiles, n_out, c_in, c_out, kv, out_feats, ep, st);
   if (!weights || !mask || !rowptr || (n_in > 0 && !nbr)) return PCE_ERR_INVALID;
   return conv_simt(in_feats, weights, mask, rowptr, nbr, n_out, c_in, c_out, kv, out_feats, dtype, ep, false, st);

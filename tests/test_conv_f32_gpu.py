@@ -106,3 +106,20 @@ def test_narrow_fp32_layers_do_not_depend_on_what_ran_before(ks, stride, transpo
         assert torch.equal(PF.conv_forward(x, w, csr), first)
         del t, csr
         plan.close()
+
+
+@pytest.mark.parametrize("cin,cout", [(4, 8), (16, 16), (48, 32)])
+def test_fp32_layers_from_an_empty_level(cin, cout):
+    """A cloud in one plane has no coarser level (the bounds leave it no outputs): the layer back up has rows and no
+    inputs, and gives its bias."""
+    import pcengine_b200 as pce
+    coords = random_cloud(4, 12, 200)
+    coords[:, 3] = 0
+    coords = coords[sorted({tuple(c): i for i, c in enumerate(coords.tolist())}.values())]
+    x = pce.spTensor(torch.randn(len(coords), cin).cuda(), torch.from_numpy(coords).cuda(), None, [0, 0, 0], cmax_of(coords), init_tag=["D2"])
+    down, up = pce.conv3d(cin, cout, 2, 2).cuda(), pce.conv3d(cout, cin, 2, 2, bias=True, transposed=True).cuda()
+    with torch.no_grad():
+        y = down(x)
+        z = up(y)
+    assert y.feats.shape == (0, cout)
+    assert torch.equal(z.feats, up.bias.expand(len(coords), cin))
