@@ -114,7 +114,13 @@ def _pair_counter(knnz, identity_rows: int):
 
 
 class _PlannedDense(_DenseTables):
-    """The dense tables of a map that the planner made in block form, as the planner's other arrays look."""
+    """The dense tables of a planned map: the planner's arrays, or, for a map in block form, built on first use and made to
+    look like them."""
+
+    def __getattr__(self, name):
+        if name == "words":  # (where the planner has left the tables, whose parts are arrays of their own)
+            return torch.cat([getattr(self, part).tensor() for part in ("knnz", "kpos", "qkpos", "status")])
+        raise AttributeError(name)
 
     def build(self) -> "_DenseTables":
         if not self.built:

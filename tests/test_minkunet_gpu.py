@@ -451,3 +451,25 @@ def test_planned_map_beyond_32_bit_counts_is_refused():
         x.planner.fetch(x, next(iter(plan.index)), None)
     del x
     plan.close()
+
+
+@pytest.mark.parametrize("layers", [[(3, 1, False, 16, 16), (3, 2, False, 16, 32)], [(5, 1, False, 16, 16), (2, 2, False, 16, 32)],
+                                    [(3, 1, False, 16, 16), (2, 2, False, 16, 32)]])
+def test_planned_maps_answer_like_any_other(layers):
+    """Sizes, pair lists and the coded forms of planned maps, in general form (a 3x3x3 stride-2 layer in the plan, 125 offsets)
+    and in block form, are those of a map built alone."""
+    import pcengine_b200 as pce
+    coords = surface_cloud(48, 30)
+    cd, cm = torch.from_numpy(coords).cuda(), cmax_of(coords)
+    plan = pce.MapPlan(layers)
+    x = pce.spTensor(torch.zeros(len(coords), 16).half().cuda(), cd, None, [0, 0, 0], cm, init_tag=["D2"])
+    assert plan.begin(x)
+    for key, (ks, stride, _, _, _) in zip(plan.index, layers):
+        km = x.planner.fetch(x, key, None)
+        cmax = cm if stride == 1 else [(v - (ks - 1)) // stride for v in cm]
+        alone = pce.KernelMap(cd, (ks,) * 3, (stride,) * 3, (0, 0, 0), [0, 0, 0], cmax, stride == 1)
+        assert km.sizes() == alone.sizes() and km.sizes()[0] > 0
+        for a, b in zip(km.pairs() + km.d1(), alone.pairs() + alone.d1()):
+            assert torch.equal(a, b)
+    del km, x
+    plan.close()
