@@ -333,7 +333,9 @@ static int launch_simt(const void* in, const void* w, const uint32_t* mask, cons
   int g = 1;
   while (g < need && g < 32) g <<= 1;
   const int vec_in = sizeof(T) == 4 ? 4 : 8;
-  const bool vec = (cin % vec_in == 0) && (cout % 4 == 0);
+  // 16-byte pieces of the input rows, four weights at a time: of widths that allow it, from addresses that do
+  const bool vec = (cin % vec_in == 0) && (cout % 4 == 0) && reinterpret_cast<uintptr_t>(in) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(w) % (4 * sizeof(T)) == 0;
   const int rows_per_block = 256 / g;
   const int grid = div_up(n_out, rows_per_block);
   const T* in_t = static_cast<const T*>(in);

@@ -692,3 +692,31 @@ def test_push_rows_gathers_into_consecutive_rows():
     with pytest.raises(ValueError):
         _lib.check(_lib.lib.pce_push_rows(src.data_ptr(), 96, None, 8, 24, dst.data_ptr(), 128, st), "pce_push_rows")
     assert _lib.lib.pce_push_rows(src.data_ptr(), 96, None, 0, 64, dst.data_ptr(), 128, st) == 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float16, 1e-3)])
+@pytest.mark.parametrize("what", ["features", "weights"])
+def test_rows_and_weights_that_start_off_a_16_byte_boundary(dtype, tol, what):
+    """A view that begins one element into its storage (widths that would allow 16-byte loads) on the kernel of one thread
+    group per row, its dense form and the tiled fp32 kernel."""
+    import pcengine_b200 as pce
+    from pcengine_b200 import functional as PF
+    coords = random_cloud(7, 12, 300)
+    d2 = ko.build_d2(coords, (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
+    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
+
+    def off(t):
+        view = torch.cat([t.flatten()[:1], t.flatten()]).cuda()[1:].view(t.shape)
+        assert view.data_ptr() % 16 and view.is_contiguous()
+        return view
+    g = torch.Generator().manual_seed(8)
+    for cin, cout in ((16, 16), (32, 64)):
+        x = torch.randn(300, cin, generator=g).to(dtype)
+        w = (torch.randn(27, cin, cout, generator=g) / (27 * cin) ** 0.5).to(dtype)
+        xd, wd = (off(x), w.cuda()) if what == "features" else (x.cuda(), off(w))
+        for choice in ("simt",) if dtype == torch.float16 else ("simt", "auto"):
+            y = PF.conv_forward(xd, wd, km.csr(), kernel_choice=choice)
+            assert co.rel_l2(y.float().cpu(), co.conv_forward(x, w, d2)) <= tol
+        if dtype == torch.float32:
+            y = PF.linear_forward(xd, off(w[0]) if what == "weights" else wd[0].contiguous())
+            assert co.rel_l2(y.cpu(), x @ w[0]) <= tol
