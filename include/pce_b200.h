@@ -13,7 +13,8 @@
  *   - every function returns a pce status code and never throws.
  *
  * Coordinates are int32 rows (b, x, y, z), b in [0, 65534], x/y/z in
- * [-32768, 32767]; rows must be unique.  Geometry triples use the reference's
+ * [-32768, 32767]; rows must be unique and start on a 16-byte boundary
+ * (PCE_ERR_INVALID otherwise).  Geometry triples use the reference's
  * x, y, z order (script/utils.py:233-242).
  *
  * Paths cited as "ref:" are relative to the reference project's root.
@@ -81,7 +82,7 @@ typedef struct pce_geom {
 typedef struct pce_epilogue {
   const float* scale;   /* [c_out] */
   const float* shift;   /* [c_out] */
-  const void* residual; /* [n_out, c_out], same dtype as the features */
+  const void* residual; /* [n_out, c_out], same dtype as the features (tensor-core kernel: 16-byte aligned) */
   int32_t act;
   float slope;
   const void* extra_feats;          /* [n_out, extra_c] fp16 */

@@ -206,6 +206,12 @@ def stream_ptr(device=None) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+def whole_rows(coords: torch.Tensor) -> torch.Tensor:
+    """int32 [N,4] coordinates, contiguous and on a 16-byte boundary (the kernels read a row in one piece)."""
+    coords = coords.contiguous()
+    return coords if coords.data_ptr() % 16 == 0 else coords.clone()
+
+
 def dtype_code(dt: torch.dtype) -> int:
     if dt == torch.float32:
         return PCE_F32

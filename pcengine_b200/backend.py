@@ -53,7 +53,7 @@ def _build_d2(in_coords, k_size_code, k_vol, l_stride_code, padding_code, mins, 
     _lib.require_cuda(in_coords, "in_coords")
     if in_coords.dtype != torch.int32:
         raise ValueError("in_coords must be int32")
-    in_coords = in_coords if in_coords.is_contiguous() else in_coords.contiguous()
+    in_coords = _lib.whole_rows(in_coords)
     ks, stride, pad = _dec(k_size_code), _dec(l_stride_code), _dec(padding_code)
     if ks[0] * ks[1] * ks[2] != k_vol:
         raise ValueError("kernel volume does not match the kernel size code")

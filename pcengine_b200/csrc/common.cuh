@@ -76,6 +76,11 @@ struct Arena {
   size_t left() const { return cap - off; }
 };
 
+// Whether an address cannot be read and written in 16-byte pieces (coordinate rows, feature rows).
+inline bool off16(const void* a, const void* b = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) != 0;
+}
+
 inline size_t pad256(size_t b) { return (b + 255) & ~size_t(255); }
 
 // ---- packed coordinate key -------------------------------------------------

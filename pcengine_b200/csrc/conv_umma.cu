@@ -1750,6 +1750,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
                   ep->in_ld > 0 ? ep->in_ld : cin, ep->out_ld > 0 ? ep->out_ld : cout};
     // rows stay 16-byte aligned: the pitch is a multiple of 8 halves and covers the channels
     if (e.ld_in < cin || e.ld_out < cout || (e.ld_in & 7) || (e.ld_out & 7)) return PCE_ERR_INVALID;
+    if (off16(ep->residual) || off16(ep->extra_feats, ep->extra_packed_weights)) return PCE_ERR_INVALID;
     for (int s = 0; s < 2; ++s) {
       if (e.push_slot[s] && (!e.push_base[s] || (reinterpret_cast<uintptr_t>(e.push_base[s]) & 15))) return PCE_ERR_INVALID;
       if (!e.push_slot[s]) e.push_base[s] = nullptr;

@@ -1061,7 +1061,7 @@ int pce_downsample_coords(const int32_t* in_coords, int32_t n_in, const pce_geom
                           size_t workspace_bytes, int32_t* out_coords, int32_t out_cap, int32_t* n_out_host,
                           void* stream) {
   if (!g || !n_out_host || n_in < 0 || out_cap < 0) return PCE_ERR_INVALID;
-  if (n_in > 0 && (!in_coords || !out_coords)) return PCE_ERR_INVALID;
+  if ((n_in > 0 && (!in_coords || !out_coords)) || off16(in_coords, out_coords)) return PCE_ERR_INVALID;
   for (int i = 0; i < 3; ++i)
     if (g->ks[i] < 1 || g->stride[i] < 1) return PCE_ERR_INVALID;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1111,7 +1111,7 @@ int pce_map_build_d2(const int32_t* in_coords, int32_t n_in, const int32_t* out_
                      const pce_geom* g, void* workspace, size_t workspace_bytes, int32_t* map, int32_t* knnz,
                      int32_t* kpos, int32_t* qkpos, int32_t* map_out, int32_t* status, void* stream) {
   if (!g || !knnz || !kpos || !qkpos || n_in < 0 || n_out < 0) return PCE_ERR_INVALID;
-  if ((n_in > 0 && (!in_coords || !map)) || (n_out > 0 && !out_coords)) return PCE_ERR_INVALID;
+  if ((n_in > 0 && (!in_coords || !map)) || (n_out > 0 && !out_coords) || off16(in_coords, out_coords)) return PCE_ERR_INVALID;
   for (int i = 0; i < 3; ++i)
     if (g->ks[i] < 1 || g->stride[i] < 1) return PCE_ERR_INVALID;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1176,7 +1176,7 @@ int pce_map_build_d2_noalloc(const int32_t* in_coords, int32_t n_in, const int32
                              const pce_geom* g, int32_t* map, int32_t* knnz, int32_t* kpos, int32_t* qkpos,
                              int32_t* map_out, int32_t* status, void* stream) {
   if (!g || !knnz || !kpos || !qkpos || n_in < 0 || n_out < 0) return PCE_ERR_INVALID;
-  if ((n_in > 0 && (!in_coords || !map)) || (n_out > 0 && !out_coords)) return PCE_ERR_INVALID;
+  if ((n_in > 0 && (!in_coords || !map)) || (n_out > 0 && !out_coords) || off16(in_coords, out_coords)) return PCE_ERR_INVALID;
   for (int i = 0; i < 3; ++i)
     if (g->ks[i] < 1 || g->stride[i] < 1) return PCE_ERR_INVALID;
   if (n_out > kNoAllocMaxRows) return PCE_ERR_CAPACITY;  // the built-in table holds 131072 output rows
@@ -1210,7 +1210,7 @@ size_t pce_subm_workspace_bytes(int32_t n) { return blk::subm_workspace_bytes(n)
 
 int pce_subm_neighbours(const int32_t* coords, int32_t n, const pce_geom* g, void* workspace, size_t workspace_bytes,
                         uint32_t* mask, int32_t* starts, int32_t* nbr, int32_t* state, void* stream) {
-  if (!g || n < 0 || !state || (n > 0 && (!coords || !mask || !starts || !nbr))) return PCE_ERR_INVALID;
+  if (!g || n < 0 || !state || (n > 0 && (!coords || !mask || !starts || !nbr)) || off16(coords)) return PCE_ERR_INVALID;
   if (!blk::covers(g)) return PCE_ERR_UNSUPPORTED;
   if (static_cast<long long>(g->ks[0]) * g->ks[1] * g->ks[2] * n >= (1ll << 31)) return PCE_ERR_UNSUPPORTED;
   return blk::subm_neighbours(coords, n, g, workspace, workspace_bytes, mask, starts, nbr, state, static_cast<cudaStream_t>(stream));
@@ -1252,7 +1252,7 @@ int pce_parents(const int32_t* in_coords, int32_t n_in, const pce_geom* g, void*
     if (g->ks[d] < 1 || g->stride[d] < 1) return PCE_ERR_INVALID;
   *n_out_host = 0;
   if (!blk::parents(g) || n_in == 0) return PCE_ERR_UNSUPPORTED;
-  if (!in_coords || !out_coords || !up_mask || !up_nbr || !child) return PCE_ERR_INVALID;
+  if (!in_coords || !out_coords || !up_mask || !up_nbr || !child || off16(in_coords, out_coords)) return PCE_ERR_INVALID;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int* host = thread_words();  // (mapped: the kernel writes the sizes itself)
   if (!host) return PCE_ERR_CUDA;

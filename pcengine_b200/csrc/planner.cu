@@ -776,7 +776,7 @@ void pce_plan_destroy(pce_plan* p) {
 
 int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t* cmin, const int32_t* cmax, void* stream,
                    pce_pass** out) {
-  if (!p || !coords || n < 1 || !cmin || !cmax || !out) return PCE_ERR_INVALID;
+  if (!p || !coords || n < 1 || !cmin || !cmax || !out || off16(coords)) return PCE_ERR_INVALID;
   int dev = -1;
   PCE_CUDA(cudaGetDevice(&dev));
   if (dev != p->device) return PCE_ERR_INVALID;

@@ -237,6 +237,7 @@ static int launch_voxelise(const float* points, int n, const float* v, int batch
 
 static int quantize_by_sort(const float* points, int n, const float* voxel, int batch, void* workspace, size_t workspace_bytes,
                             int32_t* out_coords, int32_t* out_index, int32_t* out_inverse, int* n_unique, cudaStream_t st) {
+  if (off16(out_coords)) return PCE_ERR_INVALID;
   Arena ar(workspace, workspace_bytes);
   unsigned long long* keys = ar.take<unsigned long long>(n);
   unsigned long long* skeys = ar.take<unsigned long long>(n);
@@ -391,7 +392,8 @@ __global__ void __launch_bounds__(256) k_collate(const __grid_constant__ Collate
 
 extern "C" int pce_collate_coords(const int32_t* const* coords, const int32_t* rows, int32_t n_samples, int32_t width,
                                   int32_t* out_coords, int32_t* scratch, int32_t* cmax_host, void* stream) {
-  if (!coords || !rows || n_samples < 1 || width < 3 || !out_coords || !scratch || !cmax_host) return PCE_ERR_INVALID;
+  if (!coords || !rows || n_samples < 1 || width < 3 || !out_coords || !scratch || !cmax_host || off16(out_coords))
+    return PCE_ERR_INVALID;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   PCE_CUDA(cudaMemsetAsync(scratch, 0x80, 3 * sizeof(int), st));  // 0x80808080: below every packable coordinate
   size_t done = 0;

@@ -290,7 +290,7 @@ class KernelMap:
         _lib.require_cuda(in_coords, "coords")
         if in_coords.dtype != torch.int32 or in_coords.dim() != 2 or in_coords.size(1) != 4:
             raise ValueError("coords must be an int32 [N,4] tensor of (b,x,y,z)")
-        in_coords = in_coords.contiguous()
+        in_coords = _lib.whole_rows(in_coords)
         dev = in_coords.device
         self.device = dev
         self.ks, self.stride, self.pad = tuple(ks), tuple(stride), tuple(pad)

@@ -338,12 +338,12 @@ class MapPlan:
         carries a CUDA event in ``x.coords_ready``, just that event, which lets the maps of the
         next pass be built while the current pass still computes.  Returns False (and leaves ``x``
         on the lazy path) when the tensor does not fit the plan (other stride, maps already
-        present, an override of the tile policy in force, an empty tensor) or when eight earlier
+        present, an override of the tile policy in force, an empty tensor, coordinates off a 16-byte boundary) or when eight earlier
         passes of this plan are still referenced (their maps kept alive by the caller)."""
         coords = x.coords
         if (not self.handle or not coords.is_cuda or coords.size(0) == 0 or x.stride != self.in_stride or x.kmaps
                 or PF.TILE_ROWS is not None or not PF.SORT_ROWS or coords.dtype != torch.int32
-                or not coords.is_contiguous()):
+                or not coords.is_contiguous() or coords.data_ptr() % 16):
             return False
         dev = coords.device
         h = self._handle_for(dev)

@@ -246,3 +246,39 @@ def test_hash_and_block_queries_build_the_same_maps():
             assert (a is None and b is None) or torch.equal(a, b)
         d2 = ko.build_d2(coords, ks, stride, (0, 0, 0), [0, 0, 0], cmax, subm)
         assert np.array_equal(maps[1][0].cpu().numpy(), d2["map"].reshape(-1))
+
+
+def test_coordinates_that_start_off_a_16_byte_boundary():
+    """Rows that begin one word into their storage: the map object takes them (a copy), a plan leaves them to it, the
+    library's own entry points refuse them; a residual that is read in 16-byte pieces is refused too."""
+    import ctypes as C
+
+    import pcengine_b200 as pce
+    from pcengine_b200 import _lib
+    from pcengine_b200 import functional as PF
+    from pcengine_b200.kmap import make_geom
+    coords = surface_cloud(20, 24)
+    cd, cm = torch.from_numpy(coords).cuda(), cmax_of(coords)
+    off = torch.cat([cd.flatten()[:1], cd.flatten()])[1:].view(-1, 4)
+    assert off.data_ptr() % 16 and off.is_contiguous() and torch.equal(off, cd)
+    for ks, st in ((3, 1), (2, 2), (3, 2)):
+        cmax = cm if st == 1 else [(v - (ks - 1)) // st for v in cm]
+        a, b = (pce.KernelMap(c, (ks,) * 3, (st,) * 3, (0, 0, 0), [0, 0, 0], cmax, st == 1) for c in (cd, off))
+        assert torch.equal(a.map, b.map) and torch.equal(a.csr().mask, b.csr().mask)
+    plan = pce.MapPlan([(3, 1, False, 16, 16)])
+    assert not plan.begin(pce.spTensor(torch.zeros(len(coords), 16).half().cuda(), off, None, [0, 0, 0], cm, init_tag=["D2"]))
+    plan.close()
+    g = make_geom((3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cm, True)
+    n, ws = len(coords), torch.empty(1 << 24, dtype=torch.uint8, device="cuda")
+    ints = [torch.empty(27 * n, dtype=torch.int32, device="cuda") for _ in range(5)]
+    status = _lib.lib.pce_subm_neighbours(off.data_ptr(), n, C.byref(g), ws.data_ptr(), ws.numel(), ints[0].data_ptr(), ints[1].data_ptr(),
+                                          ints[2].data_ptr(), ints[3].data_ptr(), _lib.stream_ptr(off.device))
+    assert status == _lib.PCE_ERR_INVALID
+    status = _lib.lib.pce_map_build_d2(off.data_ptr(), n, off.data_ptr(), n, C.byref(g), ws.data_ptr(), ws.numel(), *[t.data_ptr() for t in ints[:4]],
+                                       None, ints[4].data_ptr(), _lib.stream_ptr(off.device))
+    assert status == _lib.PCE_ERR_INVALID
+    x, w = torch.zeros(n, 64).half().cuda(), torch.zeros(27, 64, 64).half().cuda()
+    res = torch.zeros(n * 64 + 1, dtype=torch.float16, device="cuda")[1:].view(n, 64)
+    km = pce.KernelMap(cd, (3,) * 3, (1,) * 3, (0, 0, 0), [0, 0, 0], cm, True)
+    with pytest.raises(ValueError):
+        PF.conv_forward(x, w, km.csr(), PF.FusedEpilogue(residual=res))
