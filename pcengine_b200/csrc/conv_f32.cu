@@ -111,7 +111,7 @@ struct Shape {
 };
 
 template <int BM, int BN, bool VEC>
-__global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f32(Args a, int parts, int row_blocks) {
+__global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f32(Args a, int log2_parts) {
   constexpr int TN = Shape<BM, BN>::TN, TY = Shape<BM, BN>::TY;
   constexpr int TM = BM / TY;
   constexpr int TX = Shape<BM, BN>::TX, NT = Shape<BM, BN>::NT;
@@ -125,12 +125,15 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
   const uint32_t sb_addr = static_cast<uint32_t>(__cvta_generic_to_shared(sb));
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
-  const F32Block place = f32_block(blockIdx.x, parts, row_blocks);
+  const int parts = 1 << log2_parts;
+  const F32Block place =
+      f32_block(blockIdx.x, blockIdx.y, blockIdx.z, F32Grid{gridDim.x, gridDim.y, gridDim.z}, log2_parts, BM, BN);
+  if (place.channel0 >= a.cout) return;  // (the same for all blocks of a cluster)
   const int part = place.part;
   // the last rows of the order have the rare offsets, so the longest chains: they start first
-  const int row0 = (row_blocks - 1 - place.row_block) * BM;  // first slot of the processing order
+  const int row0 = place.row0;  // first slot of the processing order
   const int tile = row0 >> 7, in_tile = row0 & 127;
-  const int n0 = place.slice * BN;
+  const int n0 = static_cast<int>(place.channel0);
   const int cin_p = (a.cin + 3) & ~3;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the tile's stages that at least one of this block's rows has (a block is a quarter of a tile)
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
     nst = s_count;
   }
   const int chunks = (nst * cin_p + BK - 1) / BK;
-  const int c0 = static_cast<int>(static_cast<long long>(chunks) * part / parts);
-  const int c1 = static_cast<int>(static_cast<long long>(chunks) * (part + 1) / parts);
+  const int c0 = static_cast<int>(static_cast<long long>(chunks) * part >> log2_parts);
+  const int c1 = static_cast<int>(static_cast<long long>(chunks) * (part + 1) >> log2_parts);
 
   // ---- what this thread brings ----
   const int grp = tid & 3;            // 4-channel group inside a chunk
@@ -364,10 +367,8 @@ static int launch(const Args& a, int parts, cudaStream_t st) {
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  const int row_blocks = div_up(a.n_out, BM);
-  const long long blocks = f32_blocks(a.n_out, BM, a.cout, BN, parts);
-  if (blocks > 0x7FFFFFFFll) return PCE_ERR_UNSUPPORTED;  // (an output of 4 TB)
-  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  const F32Grid grid = f32_grid(a.n_out, BM, a.cout, BN, parts);
+  cfg.gridDim = dim3(grid.x, grid.y, grid.z);
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -380,7 +381,7 @@ static int launch(const Args& a, int parts, cudaStream_t st) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  PCE_CUDA(cudaLaunchKernelEx(&cfg, k_conv_f32<BM, BN, VEC>, a, parts, row_blocks));
+  PCE_CUDA(cudaLaunchKernelEx(&cfg, k_conv_f32<BM, BN, VEC>, a, parts == 8 ? 3 : (parts == 4 ? 2 : 0)));
   PCE_LAUNCH_CHECK();
   return PCE_OK;
 }

@@ -10,23 +10,28 @@
 
 namespace pce {
 
-// The tiled fp32 kernel takes all its blocks from gridDim.x: the parts of a cluster next to each other, then the row
-// blocks, then the slices of the output channels.  (gridDim.y and z end at 65535, which is 2 M rows of 32.)
-struct F32Block {
-  int part, row_block, slice;
+// The tiled fp32 kernel: the parts of a cluster (a power of two) next to each other and then the row blocks along x, which
+// reaches 2^31 - 1 (y and z end at 65535: 2 M rows of 32), the slices of the output channels along y and z.
+struct F32Grid {
+  unsigned x, y, z;
 };
 
-PCE_HD F32Block f32_block(unsigned block, int parts, int row_blocks) {
-  const unsigned rest = block / static_cast<unsigned>(parts);
-  const unsigned slice = rest / static_cast<unsigned>(row_blocks);
-  return F32Block{static_cast<int>(block - rest * static_cast<unsigned>(parts)),
-                  static_cast<int>(rest - slice * static_cast<unsigned>(row_blocks)), static_cast<int>(slice)};
+inline F32Grid f32_grid(int n_out, int rows_per_block, int c_out, int channels_per_block, int parts) {
+  const unsigned row_blocks = static_cast<unsigned>((static_cast<long long>(n_out) + rows_per_block - 1) / rows_per_block);
+  const unsigned slices = static_cast<unsigned>((static_cast<long long>(c_out) + channels_per_block - 1) / channels_per_block);
+  const unsigned z = (slices + 65534u) / 65535u;
+  return F32Grid{row_blocks * static_cast<unsigned>(parts), (slices + z - 1) / z, z};
 }
 
-inline long long f32_blocks(int n_out, int rows_per_block, int c_out, int channels_per_block, int parts) {
-  const long long row_blocks = (static_cast<long long>(n_out) + rows_per_block - 1) / rows_per_block;
-  const long long slices = (static_cast<long long>(c_out) + channels_per_block - 1) / channels_per_block;
-  return row_blocks * slices * parts;
+struct F32Block {
+  int part, row0;      // first row: the last rows come first
+  long long channel0;  // may lie behind the last channel
+};
+
+PCE_HD F32Block f32_block(unsigned x, unsigned y, unsigned z, F32Grid g, int log2_parts, int rows_per_block, int channels_per_block) {
+  return F32Block{static_cast<int>(x & ((1u << log2_parts) - 1u)),
+                  static_cast<int>(((g.x - 1u - x) >> log2_parts) * static_cast<unsigned>(rows_per_block)),
+                  (static_cast<long long>(z) * g.y + y) * channels_per_block};
 }
 
 // Piece `part` of `parts` contiguous pieces of n entries.  Unsigned: n + parts and part * per stay below 2^32 for every

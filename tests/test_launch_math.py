@@ -18,24 +18,27 @@ def _run(tmp_path, body):
 
 
 def test_blocks_of_the_tiled_fp32_kernel(tmp_path):
-    """Row blocks beyond 65535 (the end of gridDim.y) and up to the last int32 row: every block has one place, in the
-    order parts, row blocks, slices, and the rows it names stay within int32."""
+    """Row blocks beyond 65535 (the end of gridDim.y and z) and up to the last int32 row, channel slices beyond 65535: the
+    blocks' rows and channels cover the output once, the last rows first, parts of a cluster next to each other."""
     _run(tmp_path, """
       const int rows[] = {1, 32, 33, 2097120, 2097121, 8388480, 8388481, 2147483647};
-      for (int n : rows) for (int bm : {32, 128}) for (int parts : {1, 4, 8}) for (int slices : {1, 3}) {
-        if (parts > 1 && n > 100000000) continue;  // (clusters are for small maps)
-        const long long blocks = f32_blocks(n, bm, slices * 48, 48, parts);
-        const int row_blocks = static_cast<int>((static_cast<long long>(n) + bm - 1) / bm);
-        NEED(blocks == static_cast<long long>(row_blocks) * slices * parts && blocks <= 2147483647ll);
-        const long long probes[] = {0, 1, parts, 65535ll * parts, 65536ll * parts, 1ll * row_blocks * parts - 1, 1ll * row_blocks * parts, blocks - 1};
-        for (long long b : probes) {
-          if (b >= blocks) continue;
-          const F32Block p = f32_block(static_cast<unsigned>(b), parts, row_blocks);
-          NEED(p.part >= 0 && p.part < parts && p.row_block >= 0 && p.row_block < row_blocks && p.slice >= 0 && p.slice < slices);
-          NEED((static_cast<long long>(p.slice) * row_blocks + p.row_block) * parts + p.part == b);
-          const int row0 = (row_blocks - 1 - p.row_block) * bm;
-          NEED(row0 >= 0 && row0 < n && row0 + (bm - 1) >= 0);
+      const int widths[] = {1, 48, 49, 65535 * 48, 65535 * 48 + 1, 2147483647};
+      for (int n : rows) for (int bm : {32, 128}) for (int lg : {0, 2, 3}) for (int c : widths) {
+        if (lg > 0 && n > 100000000) continue;  // (clusters are for small maps)
+        const F32Grid g = f32_grid(n, bm, c, 48, 1 << lg);
+        const unsigned row_blocks = static_cast<unsigned>((static_cast<long long>(n) + bm - 1) / bm);
+        NEED(g.x == row_blocks << lg && g.x <= 2147483647u && g.y >= 1 && g.y <= 65535u && g.z >= 1 && g.z <= 65535u);
+        NEED(static_cast<long long>(g.y) * g.z * 48 >= c && (static_cast<long long>(g.y) * g.z - g.z) * 48 < c);
+        const unsigned xs[] = {0u, 1u, (1u << lg) - 1u, 1u << lg, 65535u << lg, g.x - 1u};
+        for (unsigned x : xs) {
+          if (x >= g.x) continue;
+          const F32Block p = f32_block(x, 0, 0, g, lg, bm, 48);
+          NEED(p.part == static_cast<int>(x % (1u << lg)));
+          NEED(p.row0 == static_cast<int>((row_blocks - 1 - x / (1u << lg)) * static_cast<unsigned>(bm)) && p.row0 < n && p.row0 + (bm - 1) >= 0);
         }
+        const F32Block last = f32_block(0, g.y - 1, g.z - 1, g, lg, bm, 48), next = f32_block(0, 0, g.z - 1, g, lg, bm, 48);
+        NEED(last.channel0 == (static_cast<long long>(g.y) * g.z - 1) * 48);
+        if (g.z > 1) NEED(next.channel0 == f32_block(0, g.y - 1, g.z - 2, g, lg, bm, 48).channel0 + 48);
       }""")
 
 
