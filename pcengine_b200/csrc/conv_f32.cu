@@ -68,6 +68,7 @@ __device__ __forceinline__ f2 both(float a) {
   return r;
 }
 __device__ __forceinline__ void fma2(f2& d, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void fma_zero(f2& d, f2 a) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(0ull)); }  // d += a x 0
 __device__ __forceinline__ float2 unpack(f2 v) {
   float2 r;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
@@ -81,6 +82,35 @@ __device__ __forceinline__ float finish(const Args& a, float v, int row, int c) 
   if (a.act == PCE_ACT_RELU) v = v > 0.f ? v : 0.f;
   if (a.act == PCE_ACT_LEAKY) v = v > 0.f ? v : v * a.slope;
   return v;
+}
+
+// Four outputs of one row over the neighbours the row has, stored in place of sums that came out infinite or NaN.  In the
+// tile a row takes the offsets it lacks as rows of zeros, and 0 x inf is NaN; its own neighbours decide.
+__device__ __noinline__ void redo_four(Args a, const int* stage, const int* kp, int nst, int row_in_tile, int row, int c0) {
+  for (int c = c0; c < min(c0 + 4, a.cout); ++c) {
+    float acc = 0.f;
+    for (int i = 0; i < nst; ++i) {
+      const int nid = __ldg(a.stage_nbr + static_cast<size_t>(stage[i]) * 128 + row_in_tile);
+      if (nid < 0) continue;
+      const float* x = a.in + static_cast<size_t>(nid) * a.cin;
+      const float* w = a.w + static_cast<size_t>(kp[i]) * a.cin * a.cout + c;
+      for (int k = 0; k < a.cin; ++k) acc = fmaf(__ldg(x + k), __ldg(w + static_cast<size_t>(k) * a.cout), acc);
+    }
+    a.out[static_cast<size_t>(row) * a.cout + c] = finish(a, acc, row, c);
+  }
+}
+// The same for a thread's tile: rows `ty_rows` apart, groups of four channels `half` apart.
+__device__ __noinline__ void redo_tile(Args a, const int* stage, const int* kp, int nst, int slot0, int rows, int ty_rows, int c0,
+                                       int groups, int half) {
+  for (int i = 0; i < rows; ++i) {
+    const int slot = slot0 + i * ty_rows;
+    if (slot >= a.n_out) continue;
+    for (int j = 0; j < groups; ++j)
+      redo_four(a, stage, kp, nst, slot & 127, a.order ? __ldg(a.order + slot) : slot, c0 + j * half);
+  }
+}
+__device__ __forceinline__ bool all_finite(const float (&v)[4]) {  // (0 x inf and 0 x NaN are NaN)
+  return fmaf(v[0], 0.f, fmaf(v[1], 0.f, fmaf(v[2], 0.f, v[3] * 0.f))) == 0.f;
 }
 
 // Where a thread's piece of the K dimension stands: stage and channel of its first element.
@@ -292,6 +322,13 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (parts == 1) {
+    f2 probe = 0ull;  // stays zero while all sums are finite
+    if (kLists) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) fma_zero(probe, acc[i][j]);
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       const int slot = row0 + ty + i * TY;
@@ -314,6 +351,8 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
         }
       }
     }
+    if (kLists && !(unpack(probe).x == 0.f && unpack(probe).y == 0.f))
+      redo_tile(a, s_stage, s_kp, nst, row0 + ty, TM, TY, n0 + tx * 4, TN / 4, BN / 2);
     return;
   }
   // K cut over the blocks of a cluster: every block leaves its sums in its own shared memory, then finishes
@@ -348,6 +387,7 @@ __global__ void __launch_bounds__(Shape<BM, BN>::NT, BM == 32 ? 4 : 2) k_conv_f3
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (c + u < a.cout) o[u] = finish(a, v[u], row, c + u);
+    if (kLists && !all_finite(v)) redo_four(a, s_stage, s_kp, nst, in_tile + r, row, c);
   }
   cluster.sync();  // no block leaves while another reads its sums
 }

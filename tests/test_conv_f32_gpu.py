@@ -123,3 +123,26 @@ def test_fp32_layers_from_an_empty_level(cin, cout):
         z = up(y)
     assert y.feats.shape == (0, cout)
     assert torch.equal(z.feats, up.bias.expand(len(coords), cin))
+
+
+@pytest.mark.parametrize("cin,cout,n", [(28, 28, 60), (28, 28, 400), (32, 32, 400), (64, 130, 400), (33, 24, 300)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_infinities_and_nans_stay_with_the_rows_that_meet_them(cin, cout, n, bad):
+    """One weight, then one feature, that is not finite: exactly the outputs whose row has that offset (or that neighbour)
+    are touched, as on the kernel of one thread group per row, in whole chains and in chains cut over a cluster."""
+    import pcengine_b200 as pce
+    from pcengine_b200 import functional as PF
+    coords = random_cloud(n, 5 if n < 100 else 12, n)
+    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3, 3, 3), (1, 1, 1), (0, 0, 0), [0, 0, 0], cmax_of(coords), True)
+    g = torch.Generator().manual_seed(n + cin)
+    x, w = torch.randn(n, cin, generator=g), torch.randn(27, cin, cout, generator=g)
+    for t in (w.clone().index_put_((torch.tensor(3), torch.tensor(2), torch.tensor(1)), torch.tensor(bad)), w):
+        y = x.clone()
+        if t is w:
+            y[17, 3] = bad
+        got = PF.conv_forward(y.cuda(), t.cuda(), km.csr()).cpu()
+        want = PF.conv_forward(y.cuda(), t.cuda(), km.csr(), kernel_choice="simt").cpu()
+        ok = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), ok) and 0 < int((~ok).sum()) < ok.numel()
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        assert float((got[ok] - want[ok]).norm() / want[ok].norm()) <= 1e-5
