@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional
 
 import torch
@@ -227,6 +228,11 @@ def _pad_for_tensor_cores(feats, kernel, epilogue, kernel_choice):
     return feats, kernel, epilogue, True
 
 
+@functools.lru_cache(maxsize=1024)
+def _fp32_takes_lists(c_in: int, c_out: int, kv: int) -> bool:
+    return bool(lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))
+
+
 _SM_COUNT = {}
 _TILE_ROWS_MEMO = {}
 
@@ -321,7 +327,7 @@ def conv_forward(feats: torch.Tensor, kernel: torch.Tensor, csr: NeighbourCSR, e
             split = True
             scratch = _split_scratch(csr.n_rows, feats.size(0), c_in, c_out, kv, feats.device)
     elif (kernel_choice == "auto" and feats.dtype == torch.float32
-          and (csr.parents or lib.pce_conv_takes_lists(c_in, c_out, kv, _lib.PCE_F32))):
+          and (csr.parents or _fp32_takes_lists(c_in, c_out, kv))):
         # The tiled fp32 kernel: by the layer's widths, and for every layer between voxels and their parents, whose
         # rowptr would first need the dense table (2x2x2 layers of 4->16 to 16->32, map included, us, lists against
         # rowptr: 20 k voxels 129-158 against 177-231, 200 k 169-182 against 210-234; on a kept map within 3 of each
