@@ -101,10 +101,13 @@ def supports_second_operand(dtype, c_in: int, c_out: int, c2: int) -> bool:
             and c2 >= 16)
 
 
+_SPLIT_ONLY = C.byref(_lib.Epilogue(split=1))  # (the library reads it)
+
+
 def _pack(ep: Optional[FusedEpilogue], c_out, n_out, dtype, in_ld: int = 0, out_ld: int = 0, split: bool = False,
           scratch=None):
-    if ep is None and not in_ld and not out_ld and not split:
-        return None
+    if ep is None and not in_ld and not out_ld and scratch is None:
+        return _SPLIT_ONLY if split else None
     e = ep.pack(c_out, n_out, dtype) if ep is not None else _lib.Epilogue()
     e.in_ld, e.out_ld, e.split = in_ld, out_ld, split
     if scratch is not None:
