@@ -332,7 +332,7 @@ PCE_API int32_t pce_conv_takes_lists(int32_t c_in, int32_t c_out, int32_t kv, in
 
 /* Processing order for the tensor-core kernel: output rows sorted (stable radix sort) by
  * their indicator bitmask with the bits permuted by rarity, the rarest offset most
- * significant (kv > 64: by their five rarest offsets, then bitmask by bitmask), so rows with the same neighbourhood pattern land in the same tile, rows
+ * significant (kv > 64: by their four rarest offsets, then bitmask by bitmask), so rows with the same neighbourhood pattern land in the same tile, rows
  * with a rare offset land next to each other, and a tile skips every offset none of its
  * rows has.  Purely a scheduling aid with no reference counterpart.  order[n_rows]
  * receives the permutation; kv <= 128; workspace >= 64*n_rows + 16 MiB bytes. */

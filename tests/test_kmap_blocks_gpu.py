@@ -111,3 +111,37 @@ def test_chain_given_up_while_it_is_built():
         assert torch.equal(feats, outs[0][0]) and torch.equal(torch.as_tensor(out_coords), outs[0][1])
     del x, outs
     plan.close()
+
+
+def _mix64(k):
+    with np.errstate(over="ignore"):
+        k = k ^ (k >> np.uint64(33))
+        k = k * np.uint64(0xff51afd7ed558ccd)
+        k = k ^ (k >> np.uint64(33))
+        k = k * np.uint64(0xc4ceb9fe1a85ec53)
+        return k ^ (k >> np.uint64(33))
+
+
+@pytest.mark.parametrize("rows,kv", [(1, 65), (257, 75), (5000, 125), (4096, 128)])
+def test_row_order_beyond_64_offsets(rows, kv):
+    """The stable sort by (rank of the set of the four rarest offsets, hash of the bitmask): empty rows, rows with fewer
+    than four offsets, rows with all of them."""
+    from math import comb
+    from pcengine_b200.kmap import NeighbourCSR
+    rng = np.random.default_rng(rows)
+    bits = rng.random((rows, kv)) < rng.choice([0.0, 0.01, 0.05, 0.5, 1.0], (rows, 1))
+    words = (kv + 31) // 32
+    mask = np.packbits(np.pad(bits, ((0, 0), (0, 32 * words - kv))), axis=1, bitorder="little").view(np.uint32)
+    csr = NeighbourCSR(torch.from_numpy(mask.view(np.int32)).cuda(), None, None, rows, rows, kv)
+    order = csr.order().cpu().numpy()
+    place = kv - 1 - np.argsort(np.argsort(bits.sum(0), kind="stable"), kind="stable")
+    permuted = np.zeros((rows, 128), bool)
+    permuted[:, place] = bits
+    halves = np.packbits(permuted, axis=1, bitorder="little").view(np.uint64)
+    hashes = _mix64(halves[:, 0] ^ _mix64(halves[:, 1])) >> np.uint64(32)
+    sets = np.zeros(rows, np.uint64)
+    for r in range(rows):
+        for q, p in enumerate(np.nonzero(permuted[r])[0][::-1][:4]):
+            sets[r] += np.uint64(sum(comb(int(p), i) for i in range(5 - q)))
+    key = sets * np.uint64(389) + (hashes * np.uint64(389) >> np.uint64(32))
+    assert key.max() < 1 << 32 and np.array_equal(order, np.argsort(key, kind="stable"))
