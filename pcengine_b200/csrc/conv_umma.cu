@@ -40,6 +40,8 @@
 //
 // Replaces fetch_on_demand_gemm_fp16_tc4_async and the cuBLAS centre GEMM of the
 // reference (ref: backend/spconv.cuh:1567-1730, backend/spconv.cu:273-298,338).
+#include <cuda.h>
+
 #include "common.cuh"
 
 namespace pce {
@@ -139,6 +141,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait: false when the abort flag is up or the deadline passed.
 template <class Ctl>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, Ctl* ctl, int where = 9, int item = 0) {
@@ -208,6 +221,16 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uin
       : "memory");
 }
 
+// The same with the descriptors' halves apart.
+__device__ __forceinline__ void tc_mma_f16_lohi(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // K-major, 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart, descriptor version 1.
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
   const uint32_t lo = ((smem_addr >> 4) & 0x3FFFu) | (1u << 16);
@@ -232,6 +255,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, "
+      "%18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t pack_half2(uint32_t lo, uint32_t hi) {
+  const __half2 h = __floats2half2_rn(__uint_as_float(lo), __uint_as_float(hi));
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -314,8 +352,9 @@ __global__ void k_pack_weight_slots(const __half* __restrict__ w, int kv, int ci
 // Work of tiles [0, t): `unit` per stage, and one per tile for its fixed cost (the epilogue).  A listed offset of up to 64
 // channels costs about what the tile itself does, a wider one twice that (64->64 on 1.5 M rows 118 us with 1:1, 123 with
 // 2:1; 128->128 on 200 k rows 53 with 1:1, 51 with 2:1).
-__device__ __forceinline__ long long cost_before(const int* tile_ptr, int t, int unit) {
-  return static_cast<long long>(unit) * (tile_ptr ? static_cast<long long>(__ldg(tile_ptr + t)) : static_cast<long long>(t)) + t;
+__device__ __forceinline__ long long cost_before(const int* tile_ptr, int t, int unit, int fixed = 1) {
+  return static_cast<long long>(unit) * (tile_ptr ? static_cast<long long>(__ldg(tile_ptr + t)) : static_cast<long long>(t)) +
+         static_cast<long long>(fixed) * t;
 }
 
 // The tile that begins nearest to the point where the work reaches `target`: a share then misses its due by at most half
@@ -323,12 +362,12 @@ __device__ __forceinline__ long long cost_before(const int* tile_ptr, int t, int
 // stages where a share holds about 15.)  cost_before is strictly increasing.  Found by a whole warp: 32 probes per round, so a list of n tiles takes log32(n) dependent loads instead of the
 // log2(n) of a binary search (about 20 L2 round trips per CTA for both ends of its range, a fixed
 // 15 us that was a tenth of the large layers and a third of the small ones).
-__device__ __forceinline__ int warp_tile_at_cost(const int* tile_ptr, int n_tiles, long long target, int unit, int lane) {
+__device__ __forceinline__ int warp_tile_at_cost(const int* tile_ptr, int n_tiles, long long target, int unit, int lane, int fixed = 1) {
   int lo = 0, hi = n_tiles;  // the answer lies in [lo, hi]
   while (lo < hi) {
     const int step = (hi - lo + 31) / 32;
     const int p = min(lo + (lane + 1) * step - 1, hi - 1);
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, cost_before(tile_ptr, p, unit) >= target);
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, cost_before(tile_ptr, p, unit, fixed) >= target);
     if (m == 0) {  // no tile in [lo, hi) reaches the target
       lo = hi;
       break;
@@ -338,7 +377,7 @@ __device__ __forceinline__ int warp_tile_at_cost(const int* tile_ptr, int n_tile
     lo = f == 0 ? lo : min(lo + f * step - 1, hi - 1) + 1;
     hi = hit;
   }
-  if (lo > 0 && target - cost_before(tile_ptr, lo - 1, unit) < cost_before(tile_ptr, lo, unit) - target) --lo;
+  if (lo > 0 && target - cost_before(tile_ptr, lo - 1, unit, fixed) < cost_before(tile_ptr, lo, unit, fixed) - target) --lo;
   return lo;
 }
 
@@ -1421,6 +1460,510 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 2 + 4 * EPIW), SUB == 1 ? 2 : 
   }
 }
 
+// =====================================================================================================
+// k_conv_deep: the same layer with ONE CTA per SM, its rows gathered by the TMA engine.
+//
+// What bounds k_conv_umma on layers of one offset per stage is instruction latency: a producer warp needs 1000 to 1400 cycles
+// for a stage (index shuffles, eight row copies, barrier), the MMA warp 400 to 700 for its four products, and a copy
+// that only fills in zeros takes three times as long as one that moves data.  Here
+//   * rows come by tile::gather4, four rows per operation.  One operation costs the issuing warp 80 cycles, which made
+//     it look slow from one warp (2576 cycles for a stage's 128 rows); sixteen warps that issue half a stage each keep
+//     the L2 port busy (240 cycles a stage, 68 of 64 to 72 bytes per clock and SM) and do nothing else.  The data arrives
+//     through the async proxy: nobody has to order it before the products.
+//   * groups of four rows that all lack the offset are not copied: the warp stores zeros, once for as long as the same
+//     group of the slot stays without rows (an out-of-range row costs the TMA engine 40 cycles);
+//   * the MMA warp's ring is unrolled: with a slot's descriptors and barriers known up to their base a stage takes 230 to 300
+//     cycles to issue, from a running slot number 400 to 700;
+//   * the SM's shared memory is one ring of 4 to 9 stages, and two teams of epilogue warps take the tiles in turn with two
+//     or four accumulators between them: no product waits for a tile's stores;
+//   * a third as many CTAs have shares three times as long, against which the heaviest tiles (27 offsets, where the mean is
+//     2 to 5) weigh less.
+// Lists, shares of tiles, second operand, split tiles and bounded waits are k_conv_umma's.  Widths are multiples of
+// 32 input channels (the last 32 of an odd multiple are a half block, as there).
+constexpr int kDeepMaxRing = 9;
+constexpr int kDeepMaxAcc = 4;
+constexpr int kDeepTeams = 2;
+constexpr int kDeepMmaWarp = 4 * kDeepTeams;   // epilogue warps first: warp & 3 is a warp's quarter of tensor memory
+constexpr int kDeepProducers = kDeepMmaWarp + 1;
+constexpr int kDeepBounds = 512;               // tile bounds of a CTA kept in shared memory
+// producer warps per slot: each fills its part of the slot's rows
+constexpr int deep_parts(int ring) { return ring == 4 ? 4 : 2; }
+constexpr int deep_threads(int ring) { return 32 * (kDeepProducers + ring * deep_parts(ring)); }
+
+struct DeepMaps {
+  CUtensorMap in;     // [n_in][cin], boxes of one row x 64 channels
+  CUtensorMap in32;   // boxes of 32 channels (the half block)
+  CUtensorMap sec;    // the second operand's
+  CUtensorMap sec32;
+};
+
+struct DeepCtl {
+  unsigned long long full[kDeepMaxRing];
+  unsigned long long empty[kDeepMaxRing];
+  unsigned long long accfull[kDeepMaxAcc];
+  unsigned long long accempty[kDeepMaxAcc];
+  uint32_t tmem_base;
+  int range[2];
+  volatile int abort_flag;
+  int bounds[kDeepBounds];
+};
+
+// Rows r.x .. r.w (negative: zeros) of the map's box at column x, one after the other from dst on.
+__device__ __forceinline__ void gather4(uint32_t dst, const CUtensorMap* map, int x, const int4& r, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w), "r"(bar)
+      : "memory");
+}
+
+template <bool HALF, int RING>
+__global__ void __launch_bounds__(deep_threads(RING), 1)
+    k_conv_deep(const __grid_constant__ DeepMaps maps, const __half* __restrict__ wpacked, const Lists ls, const Second sec, int n_out,
+                int cin, int cout, __half* __restrict__ out, const Epi ep, int tmem_cols, int nacc) {
+  constexpr int PARTS = deep_parts(RING), kPartRows = kTileM / PARTS, kQuads = kPartRows / 4;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
+  uint8_t* tiles = smem_raw + pad;  // 1024-byte aligned
+  const uint32_t tiles_addr = raw_addr + pad;
+  constexpr int KB = 64;
+  const int b_bytes = cout * 128;
+  const int stage_bytes = kABytes + b_bytes;
+  DeepCtl* ctl = reinterpret_cast<DeepCtl*>(tiles + RING * stage_bytes);
+  float* affine = reinterpret_cast<float*>(ctl + 1);
+  static_assert(sizeof(DeepCtl) % 16 == 0, "the staged scale/shift are read as float4");
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  const int kblocks = (cin + KB - 1) / KB;
+  const int kblocks2 = sec.in2 ? (sec.cin2 + KB - 1) / KB : 0;
+  const int n_tiles = (n_out + kTileM - 1) / kTileM;
+  if (tid == 0) {
+    for (int s = 0; s < RING; ++s) {
+      mbar_init(smem_u32(&ctl->full[s]), PARTS);
+      mbar_init(smem_u32(&ctl->empty[s]), 1);
+    }
+    for (int s = 0; s < nacc; ++s) {
+      mbar_init(smem_u32(&ctl->accfull[s]), 1);
+      mbar_init(smem_u32(&ctl->accempty[s]), 128);
+    }
+    ctl->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp < kDeepMmaWarp && (ep.scale || ep.shift)) {
+    for (int c = tid; c < cout; c += 32 * kDeepMmaWarp) {
+      affine[c] = ep.scale ? __ldg(ep.scale + c) : 1.f;
+      affine[cout + c] = ep.shift ? __ldg(ep.shift + c) : 0.f;
+    }
+  }
+  if (warp == kDeepMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)),
+                 "r"(static_cast<uint32_t>(tmem_cols))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (!ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");  // (as in k_conv_umma)
+  const int parts = ep.parts > 1 ? ep.parts : 1;
+  if (parts > 1) {
+    if (tid == 0) {
+      ctl->range[0] = static_cast<int>(blockIdx.x) / parts;
+      ctl->range[1] = static_cast<int>(blockIdx.x) / parts + 1;
+    }
+  } else if (warp < 2) {
+    // a tile's stores cost about two ring stages: 64->64 on 200 k rows 20.7 us so, 22.9 with one, 28.3 with a quarter; 5x5x5 on
+    // 300 k rows 110, 129, 140; 96->96 on 240 k rows 36 so, 44 with four
+    const int unit = kblocks, fixed = 2;
+    const long long total = cost_before(ls.tile_ptr, n_tiles, unit, fixed);
+    const unsigned b = blockIdx.x + warp;
+    const int t = b >= gridDim.x ? n_tiles : warp_tile_at_cost(ls.tile_ptr, n_tiles, total * b / gridDim.x, unit, lane, fixed);
+    if (lane == 0) ctl->range[warp] = t;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  const int t0 = ctl->range[0], t1 = ctl->range[1];
+  for (int i = tid; i <= t1 - t0 && i < kDeepBounds; i += deep_threads(RING)) ctl->bounds[i] = first_stage(ls.tile_ptr, t0 + i);
+  __syncthreads();
+  auto bound = [&](int t) { return t - t0 < kDeepBounds ? ctl->bounds[t - t0] : first_stage(ls.tile_ptr, t); };
+  struct Work {
+    int first;        // first stage of the lists (of this CTA's part)
+    int main, ident;  // ring stages of the listed offsets; with the identity stage
+  };
+  auto work_of = [&](int t) {
+    const int b0 = bound(t), b1 = bound(t + 1);
+    int sa = b0, sb = b1;
+    if (parts > 1) {
+      const int n = sb - sa, part = static_cast<int>(blockIdx.x) % parts;
+      const int a = sa + static_cast<int>(static_cast<long long>(n) * part / parts);
+      sb = sa + static_cast<int>(static_cast<long long>(n) * (part + 1) / parts);
+      sa = a;
+    }
+    Work w;
+    w.first = sa;
+    w.ident = (ls.identity && sb > sa && sb == b1) ? 1 : 0;
+    w.main = (sb - sa - w.ident) * kblocks;
+    return w;
+  };
+
+  bool part_any = false;
+  if (warp >= kDeepProducers) {
+    // =========================== producers: warp p fills part p % PARTS of slot p / PARTS, use after use ===========================
+    const int slot = (warp - kDeepProducers) / PARTS, part = (warp - kDeepProducers) % PARTS;
+    const uint32_t a_part = tiles_addr + slot * stage_bytes + part * kPartRows * 128;  // (half blocks: rows of 64 bytes)
+    const uint32_t full = smem_u32(&ctl->full[slot]), empty = smem_u32(&ctl->empty[slot]);
+    const unsigned inv = ((1u << 20) + kblocks - 1) / kblocks;  // stage / kblocks of a tile's at most 128 x kblocks stages
+    int t = t0, before = 0, j = slot;  // `before`: ring stages in front of tile t; j: the slot's next stage
+    Work w = {0, 0, 0};
+    int in_tile = 0;
+    if (t < t1) {
+      w = work_of(t);
+      in_tile = w.main + (w.ident ? kblocks2 : 0);
+    }
+    int4 rows = make_int4(-1, -1, -1, -1);
+    int kb = 0, kp = 0;
+    bool second = false;
+    auto fetch = [&]() -> bool {  // the slot's next stage: its rows (asked for) and what they are multiplied with
+      while (t < t1 && j >= before + in_tile) {
+        before += in_tile;
+        if (++t < t1) {
+          w = work_of(t);
+          in_tile = w.main + (w.ident ? kblocks2 : 0);
+        }
+      }
+      if (t >= t1) return false;
+      const int i = j - before;
+      second = i >= w.main;
+      const int o = static_cast<int>((static_cast<unsigned>(second ? w.main : i) * inv) >> 20);
+      kb = second ? i - w.main : i - o * kblocks;
+      const int g = w.first + o;
+      if (lane < kQuads) {
+        if (ls.tile_ptr) {
+          rows = __ldg(reinterpret_cast<const int4*>(ls.stage_nbr + static_cast<size_t>(g) * kTileM + part * kPartRows) + lane);
+        } else {
+          const int r = g * kTileM + part * kPartRows + 4 * lane;
+          rows = make_int4(r < n_out ? r : -1, r + 1 < n_out ? r + 1 : -1, r + 2 < n_out ? r + 2 : -1, r + 3 < n_out ? r + 3 : -1);
+        }
+      }
+      if (part == 0 && ls.tile_ptr && !second) kp = __ldg(ls.stage_kp + g) & 255;  // (bits 8..: sub-tile presence)
+      j += RING;
+      return true;
+    };
+    bool ok = true, was_half = false;
+    uint32_t use = 0, zeroed = 0;  // zeroed: groups of the part that hold zeros
+    bool more = fetch();
+    if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
+    while (more) {
+      // (the copies below read rows, kb, kp and second; the next stage is fetched behind them)
+      const int nkb = second ? kblocks2 : kblocks;
+      const bool half = HALF && kb == nkb - 1 && (second ? sec.wtail : ls.wtail) != nullptr;
+      const int quad_bytes = half ? 256 : 512;
+      const uint32_t a_addr = half ? tiles_addr + slot * stage_bytes + part * kPartRows * 64 : a_part;
+      const bool any = lane < kQuads && (rows.x & rows.y & rows.z & rows.w) >= 0;  // (a row that is there has no sign bit)
+      const uint32_t gathered = __ballot_sync(0xFFFFFFFFu, any);
+      if (use > 0) ok = mbar_wait(empty, (use - 1) & 1, ctl);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      if (!ok) break;
+      constexpr uint32_t kAll = kQuads == 32 ? 0xFFFFFFFFu : (1u << kQuads) - 1u;
+      const uint32_t blank = kAll & ~gathered;
+      if (half != was_half) zeroed = 0;  // (another layout)
+      was_half = half;
+      const uint32_t fill = blank & ~zeroed;
+      if (fill) {
+        for (uint32_t m = fill; m; m &= m - 1u) {
+          const uint32_t at = a_addr + (__ffs(m) - 1) * quad_bytes + lane * 16;
+          if (lane * 16 < quad_bytes) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(0) : "memory");
+        }
+        fence_proxy_async();  // plain stores, read by the tensor core
+        __syncwarp();
+      }
+      zeroed = blank;
+      if (elect_one()) {
+        const uint32_t row_bytes = static_cast<uint32_t>(__popc(gathered) * quad_bytes);
+        if (part == 0) {
+          const uint32_t w_bytes = half ? static_cast<uint32_t>(cout) * 64u : static_cast<uint32_t>(b_bytes);
+          mbar_arrive_expect_tx(full, row_bytes + w_bytes);
+          const __half* wtail = second ? sec.wtail : ls.wtail;
+          const __half* wsrc = second ? sec.w2 + static_cast<size_t>(kb) * cout * KB
+                                      : wpacked + (static_cast<size_t>(kb) + static_cast<size_t>(kp) * kblocks) * cout * KB;
+          if (half) wsrc = wtail + (static_cast<size_t>(second ? 0 : kp) * (2 * nkb - 1) + 2 * kb) * cout * 32;
+          bulk_copy_g2s(tiles_addr + slot * stage_bytes + kABytes, wsrc, w_bytes, full);
+        } else {
+          mbar_arrive_expect_tx(full, row_bytes);
+        }
+      }
+      __syncwarp();
+      if (any) gather4(a_addr + lane * quad_bytes, second ? (half ? &maps.sec32 : &maps.sec) : (half ? &maps.in32 : &maps.in), kb * KB, rows, full);
+      ++use;
+      more = fetch();
+    }
+    if (!ok && use > 0 && lane == 0) {
+      // aborting: give the slot's copies a bounded chance to land before the CTA leaves
+      for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(full, (use - 1) & 1); ++spin) {
+      }
+    }
+  } else if (warp == kDeepMmaWarp) {
+    // =========================== MMA issuer: one thread ===========================
+    if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (elect_one()) {
+      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(cout >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
+      const uint32_t lo0 = (tiles_addr >> 4) | (1u << 16), step = static_cast<uint32_t>(stage_bytes) >> 4;
+      constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29), kHi32 = (512u >> 4) | (1u << 14) | (4u << 29);  // (make_desc_kb)
+      const int last1 = ((cin - 1) & 63) / 16 + 1, last2 = ((sec.cin2 - 1) & 63) / 16 + 1;  // K steps of the last K block
+      const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
+      uint32_t par = 0, lo = lo0, at = 0;  // at: 8 x the slot
+      bool ok = true;
+      for (int t = t0; t < t1 && ok; ++t) {
+        const Work work = work_of(t);
+        const int round = (t - t0) >> (nacc == 4 ? 2 : 1), buf = (t - t0) & (nacc - 1);
+        const uint32_t acc = tmem_base + static_cast<uint32_t>(buf * cout);
+        if (round > 0) ok = mbar_wait(smem_u32(&ctl->accempty[buf]), (round - 1) & 1, ctl);
+        uint32_t accumulate = 0;
+        auto blocks = [&](int n, int nkb, int last, bool half_end) {  // n stages, nkb to an offset
+          int kb = nkb;
+          for (; n > 0 && ok; --n) {
+            ok = mbar_wait(full0 + at, par, ctl);
+            if (!ok) break;
+            tc_fence_after();
+            if (--kb > 0 || (last == 4 && !half_end)) {
+              tc_mma_f16_lohi(acc, lo, kHi, lo + (kABytes >> 4), kHi, idesc, accumulate);
+              tc_mma_f16_lohi(acc, lo + 2, kHi, lo + (kABytes >> 4) + 2, kHi, idesc, 1u);
+              tc_mma_f16_lohi(acc, lo + 4, kHi, lo + (kABytes >> 4) + 4, kHi, idesc, 1u);
+              tc_mma_f16_lohi(acc, lo + 6, kHi, lo + (kABytes >> 4) + 6, kHi, idesc, 1u);
+            } else if (half_end) {
+              tc_mma_f16_lohi(acc, lo, kHi32, lo + (kABytes >> 4), kHi32, idesc, accumulate);
+              tc_mma_f16_lohi(acc, lo + 2, kHi32, lo + (kABytes >> 4) + 2, kHi32, idesc, 1u);
+            } else {
+              for (int k = 0; k < last; ++k)
+                tc_mma_f16_lohi(acc, lo + 2 * k, kHi, lo + (kABytes >> 4) + 2 * k, kHi, idesc, k > 0 ? 1u : accumulate);
+            }
+            tc_commit(empty0 + at);
+            accumulate = 1;
+            if (kb == 0) kb = nkb;
+            at += 8;
+            lo += step;
+            if (at == 8 * RING) {
+              at = 0;
+              lo = lo0;
+              par ^= 1;
+            }
+          }
+        };
+        if (!ok) break;
+        tc_fence_after();
+        blocks(work.main, kblocks, last1, HALF && ls.wtail);
+        if (work.ident && kblocks2) blocks(kblocks2, kblocks2, last2, HALF && sec.wtail);
+        if (!ok) break;
+        if (work.main > 0 || (work.ident && kblocks2))
+          tc_commit(smem_u32(&ctl->accfull[buf]));  // arrives when every MMA of the tile has finished
+        else
+          mbar_arrive(smem_u32(&ctl->accfull[buf]));  // no MMA was issued: the epilogue writes zeros
+      }
+    }
+    __syncwarp();
+    tc_fence_before();
+  } else {
+    // =========================== epilogue ===========================
+    const int team = warp >> 2;
+    const int lane_quarter = warp & 3;
+    const int slot_in_tile = lane_quarter * 32 + lane;
+    const bool wide_out = (ep.ld_out & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+    const bool wide_res = (reinterpret_cast<uintptr_t>(ep.residual) & 31) == 0;
+    const bool scaled = ep.scale || ep.shift;
+    const bool plain = wide_out && !scaled && !ep.residual && ep.act == PCE_ACT_NONE;
+    auto row_of = [&](int t) {
+      const int slot = t * kTileM + slot_in_tile;
+      return t < t1 && slot < n_out ? (ls.order ? __ldg(ls.order + slot) : slot) : n_out;
+    };
+    int my_row = row_of(t0 + team);
+    if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int t = t0 + team; t < t1; t += kDeepTeams) {
+      const int it = t - t0;
+      const Work work = work_of(t);
+      const int buf = it & (nacc - 1), round = it / nacc;
+      const bool store_row = my_row < n_out;
+      const bool any = work.main + (work.ident ? kblocks2 : 0) > 0;
+      __half* orow = out + static_cast<size_t>(store_row ? my_row : 0) * ep.ld_out;
+      const __half* rrow = (ep.residual && store_row) ? ep.residual + static_cast<size_t>(my_row) * cout : nullptr;
+      my_row = row_of(t + kDeepTeams);  // (a tile ahead)
+      if (rrow) {
+        // the rows are known before the accumulator is: pull the residual rows into L2 while waiting
+        const char* rp = reinterpret_cast<const char*>(rrow);
+        for (int off = 0; off < cout * 2; off += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + off));
+      }
+      bool ok = mbar_wait(smem_u32(&ctl->accfull[buf]), round & 1, ctl);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      if (t == t1 - 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      if (parts > 1) {  // (one tile per CTA; its sums stay in tensor memory until the cluster adds them up below)
+        part_any = any;
+        break;
+      }
+      const uint32_t taddr = tmem_base + static_cast<uint32_t>(buf * cout) + (static_cast<uint32_t>(lane_quarter * 32) << 16);
+      if (plain && any) {
+        // nothing but the conversion: kept apart, since the code of all the other cases, stepped over or predicated off, took
+        // longer to fetch than this takes to run
+        int c0 = 0;
+#pragma unroll 1
+        for (; c0 + 32 <= cout; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld32(taddr + c0, r);
+          tmem_ld_wait();
+          uint4 o[4];
+          uint32_t* po = reinterpret_cast<uint32_t*>(o);
+#pragma unroll
+          for (int q = 0; q < 16; ++q) po[q] = pack_half2(r[2 * q], r[2 * q + 1]);
+          if (store_row) {
+            store32(orow + c0, o[0], o[1]);
+            store32(orow + c0 + 16, o[2], o[3]);
+          }
+        }
+        if (c0 < cout) {
+          uint32_t r[16];
+          tmem_ld16(taddr + c0, r);
+          tmem_ld_wait();
+          uint4 o[2];
+          uint32_t* po = reinterpret_cast<uint32_t*>(o);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) po[q] = pack_half2(r[2 * q], r[2 * q + 1]);
+          if (store_row) store32(orow + c0, o[0], o[1]);
+        }
+      } else
+#pragma unroll 1
+      for (int c0 = 0; c0 < cout; c0 += 16) {
+        uint4 ra, rb;
+        if (rrow) {  // issued ahead of the tensor-memory load, consumed after it
+          if (wide_res) {
+            load32(rrow + c0, ra, rb);
+          } else {
+            ra = *reinterpret_cast<const uint4*>(rrow + c0);
+            rb = *reinterpret_cast<const uint4*>(rrow + c0 + 8);
+          }
+        }
+        uint32_t r[16];
+        if (any) {  // warp-uniform: the tensor-memory load is warp-collective
+          tmem_ld16(taddr + c0, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) r[q] = 0u;
+        }
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
+        if (scaled) {
+#pragma unroll
+          for (int q = 0; q < 16; q += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(affine + c0 + q);
+            const float4 t4 = *reinterpret_cast<const float4*>(affine + cout + c0 + q);
+            v[q] = fmaf(v[q], s4.x, t4.x);
+            v[q + 1] = fmaf(v[q + 1], s4.y, t4.y);
+            v[q + 2] = fmaf(v[q + 2], s4.z, t4.z);
+            v[q + 3] = fmaf(v[q + 3], s4.w, t4.w);
+          }
+        }
+        if (rrow) {
+          const __half2* ha = reinterpret_cast<const __half2*>(&ra);
+          const __half2* hb = reinterpret_cast<const __half2*>(&rb);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 fa = __half22float2(ha[q]);
+            const float2 fb = __half22float2(hb[q]);
+            v[2 * q] += fa.x;
+            v[2 * q + 1] += fa.y;
+            v[8 + 2 * q] += fb.x;
+            v[8 + 2 * q + 1] += fb.y;
+          }
+        }
+        if (ep.act == PCE_ACT_RELU) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) v[q] = v[q] > 0.f ? v[q] : 0.f;
+        } else if (ep.act == PCE_ACT_LEAKY) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) v[q] = v[q] > 0.f ? v[q] : v[q] * ep.slope;
+        }
+        uint4 oa, ob;
+        __half2* pa = reinterpret_cast<__half2*>(&oa);
+        __half2* pb = reinterpret_cast<__half2*>(&ob);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          pa[q] = __floats2half2_rn(v[2 * q], v[2 * q + 1]);
+          pb[q] = __floats2half2_rn(v[8 + 2 * q], v[8 + 2 * q + 1]);
+        }
+        if (store_row) {
+          if (wide_out) {
+            store32(orow + c0, oa, ob);
+          } else {
+            *reinterpret_cast<uint4*>(orow + c0) = oa;
+            *reinterpret_cast<uint4*>(orow + c0 + 8) = ob;
+          }
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(smem_u32(&ctl->accempty[buf]));  // 128 arrivals hand the accumulator back
+    }
+    tc_fence_before();
+  }
+  if (parts > 1) {
+    // the parts' sums, added up through the cluster's shared memory as in k_conv_umma
+    const int part = static_cast<int>(blockIdx.x) % parts;
+    const int fit = (RING * stage_bytes / (kTileM * 4)) & ~15;
+    const int rows_each = kTileM / parts;
+    const bool scaled = ep.scale || ep.shift;
+    for (int base = 0; base < cout; base += fit) {
+      const int cols = min(fit, cout - base);
+      __syncthreads();
+      if (warp < 4) {
+        const int r = warp * 32 + lane;
+        const uint32_t taddr = tmem_base + static_cast<uint32_t>(base) + (static_cast<uint32_t>(warp * 32) << 16);
+        for (int c0 = 0; c0 < cols; c0 += 16) {
+          uint32_t v[16];
+          if (part_any) {
+            tmem_ld16(taddr + c0, v);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = 0u;
+          }
+          uint4* dst = reinterpret_cast<uint4*>(tiles) + (c0 / 4) * kTileM + r;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) dst[q * kTileM] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+      }
+      tc_fence_before();
+      cluster_sync();
+      for (int i = tid; i < rows_each * (cols / 8); i += deep_threads(RING)) {
+        const int r = part * rows_each + i % rows_each, c0 = i / rows_each * 8;
+        const int slot = t0 * kTileM + r;
+        if (slot >= n_out) continue;
+        const int row = ls.order ? __ldg(ls.order + slot) : slot;
+        const uint32_t src = tiles_addr + static_cast<uint32_t>((c0 / 4) * kTileM + r) * 16u;
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int p = 0; p < parts; ++p) {
+          const float4 x = cluster_ld4(src, p), y = cluster_ld4(src + kTileM * 16u, p);
+          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+          v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+        }
+        const int c = base + c0;
+        if (scaled) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = fmaf(v[q], affine[c + q], affine[cout + c + q]);
+        }
+        finish8(v, row, c, cout, out, ep);
+      }
+      cluster_sync();  // (the other parts have read this CTA's sums)
+    }
+  }
+  __syncthreads();
+  if (warp == kDeepMmaWarp) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                 "r"(static_cast<uint32_t>(tmem_cols))
+                 : "memory");
+  }
+}
+
 // Second kernel of a stream-K layer: for every tile that was cut between CTAs, adds the pieces in CTA order
 // (fp32) and applies the epilogue; tiles that one CTA finished are left alone.  Block (x, t) handles 256 of the
 // tile's (row, 8 output channels) items: its first warp works out which CTAs hold pieces of tile t (consecutive
@@ -1715,13 +2258,68 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
   return grid > 0 ? static_cast<size_t>(grid) * 2 * umma::kTileM * cout * sizeof(float) : 0;
 }
 
+// Input widths of k_conv_deep: whole K blocks, or a half block at the end (below 64 channels several offsets share a stage,
+// or the block is mostly padding).
+static bool deep_widths(int cin) { return cin >= 64 && cin % 32 == 0; }
+
 // The same where a split was measured faster; the framework's own callers ask this one.  Equal shares of stages repay
 // their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
 // 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
+  if (deep_widths((cin + 15) / 16 * 16)) return 0;  // (k_conv_deep: shares three times as long leave little to balance)
   if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;  // (parts add up in shared memory)
   if (chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
   return conv_split_scratch_bytes(n_rows, n_src, cin, cout, kv, sm_count);
+}
+
+// cuTensorMapEncodeTiled, looked up once (the library does not link the driver's).
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiled encode_tiled() {
+  static EncodeTiled fn = nullptr;
+  EncodeTiled f = __atomic_load_n(&fn, __ATOMIC_RELAXED);
+  if (!f) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess)
+      return nullptr;
+    f = reinterpret_cast<EncodeTiled>(p);
+    __atomic_store_n(&fn, f, __ATOMIC_RELAXED);
+  }
+  return f;
+}
+
+// Rows of `width` fp16 values, `pitch` apart, as boxes of one row x `box` channels (64: 128-byte swizzle, 32: 64-byte).
+static bool row_map(CUtensorMap* map, const void* base, long long rows, int width, int pitch, int box) {
+  const EncodeTiled encode = encode_tiled();
+  if (!encode || rows < 1) return false;
+  const cuuint64_t dim[2] = {static_cast<cuuint64_t>(width), static_cast<cuuint64_t>(rows)}, stride[1] = {static_cast<cuuint64_t>(pitch) * 2};
+  const cuuint32_t boxes[2] = {static_cast<cuuint32_t>(box), 1}, step[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dim, stride, boxes, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+typedef void (*DeepKernel)(const umma::DeepMaps, const __half*, const umma::Lists, const umma::Second, int, int, int, __half*, const umma::Epi, int, int);
+static DeepKernel deep_kernel(bool half, int ring) {
+  static const DeepKernel table[2][6] = {
+      {umma::k_conv_deep<false, 4>, umma::k_conv_deep<false, 5>, umma::k_conv_deep<false, 6>, umma::k_conv_deep<false, 7>,
+       umma::k_conv_deep<false, 8>, umma::k_conv_deep<false, 9>},
+      {umma::k_conv_deep<true, 4>, umma::k_conv_deep<true, 5>, umma::k_conv_deep<true, 6>, umma::k_conv_deep<true, 7>,
+       umma::k_conv_deep<true, 8>, umma::k_conv_deep<true, 9>}};
+  return table[half ? 1 : 0][ring - 4];
+}
+
+// Parts per tile of k_conv_deep (4, 2 or 1): as long as every part has an SM to itself and a chain worth cutting.  Kernel
+// only, us, one / two / four parts: 256->256 on 24 tiles 39.3 / 27.6 / 20.4, on 60 tiles 38.2 / 27.5 / 34.4, on 94 tiles
+// 31.2 / 34.1; 128->128 on 24 tiles 16.9 / 14.2 / 11.9, on 60 tiles 16.9 / 14.5 / 21.1; 64->64 on 24 tiles 10.3 / 10.2 / 9.2, on
+// 60 tiles 10.4 / 10.4 / 16.8.  (Eight parts leave each a few stages: 256->256 on 24 tiles 30.5.)
+static int deep_split(int n_tiles, int n_out, int n_src, int cin, int kv, int sm_count) {
+  if (!umma_split_enabled) return 1;
+  const int chain = chain_estimate(n_out, n_src, cin, kv);
+  if (4ll * n_tiles <= sm_count && chain >= 16) return 4;
+  if (2ll * n_tiles <= sm_count && chain >= 32) return 2;
+  return 1;
 }
 
 // tiles == nullptr: the dense rows x matrix product (every row fetches itself, one offset).
@@ -1738,6 +2336,48 @@ int conv_umma(const void* in, int n_in, const void* wpacked, int kv, const pce_t
 int conv_umma_kb64(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out, int cin,
                    int cout, void* out, const pce_epilogue* ep, cudaStream_t st) {
   return conv_umma_impl(in, n_in, wpacked, kv, tiles, n_out, cin, cout, out, ep, st, true);
+}
+
+// `split`: the caller allows several CTAs per tile.
+static int conv_deep(const umma::DeepMaps& maps, const __half* w, const umma::Lists& ls, const umma::Second& sec, int n_in, int n_out, int cin,
+                     int cout, int kv, __half* out, umma::Epi e, bool half, bool split, int dev, int sm_count, cudaStream_t st) {
+  static bool attr_set[64] = {};
+  if (!attr_set[dev]) {
+    for (int r = 4; r <= umma::kDeepMaxRing; ++r)
+      for (int v = 0; v < 2; ++v)
+        PCE_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(deep_kernel(v != 0, r)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      227 * 1024));
+    attr_set[dev] = true;
+  }
+  const size_t stage = static_cast<size_t>(umma::kABytes) + static_cast<size_t>(cout) * 128;
+  const size_t rest = sizeof(umma::DeepCtl) + 1024 + 64 + 2 * sizeof(float) * cout;
+  const int ring = std::min<int>(umma::kDeepMaxRing, static_cast<int>((227 * 1024 - rest) / stage));
+  const int nacc = cout <= 128 ? 4 : 2;
+  int cols = 32;
+  while (cols < nacc * cout) cols <<= 1;
+  const int n_tiles = div_up(n_out, umma::kTileM);
+  const int parts = split ? deep_split(n_tiles, n_out, n_in, cin, kv, sm_count) : 1;
+  e.parts = parts;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(parts > 1 ? n_tiles * parts : std::min(n_tiles, sm_count));
+  cfg.blockDim = dim3(umma::deep_threads(ring));
+  cfg.dynamicSmemBytes = ring * stage + rest;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (umma_overlap_launches) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (parts > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(parts);
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  PCE_CUDA(cudaLaunchKernelEx(&cfg, deep_kernel(half, ring), maps, w, ls, sec, n_out, cin, cout, out, e, cols, nacc));
+  PCE_LAUNCH_CHECK();
+  return PCE_OK;
 }
 
 static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv, const pce_tile_lists* tiles, int n_out,
@@ -1838,6 +2478,18 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
       return conv_umma_mt(static_cast<const __half*>(in), static_cast<const __half*>(wpacked), ls, sec, n_out, cin, cout,
                           static_cast<__half*>(out), e, sub, sm_count[dev], st);
     if (sub > 2) return PCE_ERR_UNSUPPORTED;  // 512-row super-tiles exist for k_conv_umma_mt only
+  }
+  // One CTA per SM wherever its producers can take the layer (k_conv_deep); the tuning hooks below are k_conv_umma's.
+  if (slots == 1 && sub == 1 && !(e.push_slot[0] || e.push_slot[1]) && deep_widths(cin) && (cin % 64 == 0 || half) && !off16(in) &&
+      !off16(ls.stage_nbr) && !umma_force_stages && !umma_force_nacc && umma_split_enabled != 3) {
+    umma::DeepMaps maps;
+    bool mapped = row_map(&maps.in, in, n_in, cin, e.ld_in, 64) && (!half || row_map(&maps.in32, in, n_in, cin, e.ld_in, 32));
+    if (sec.in2)
+      mapped = mapped && row_map(&maps.sec, sec.in2, n_out, sec.cin2, sec.cin2, 64) &&
+               (!sec.wtail || row_map(&maps.sec32, sec.in2, n_out, sec.cin2, sec.cin2, 32));
+    if (mapped)
+      return conv_deep(maps, static_cast<const __half*>(wpacked), ls, sec, n_in, n_out, cin, cout, kv, static_cast<__half*>(out), e,
+                       half, tiles && ep && (ep->split || ep->split_scratch), dev, sm_count[dev], st);
   }
   // Configuration = (ring depth, accumulator sets).  What the kernel needs most is row gathers in
   // flight, i.e. stages resident per SM = resident CTAs x ring depth; the CTAs per SM are bounded by
