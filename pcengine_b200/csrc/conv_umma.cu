@@ -1485,7 +1485,7 @@ constexpr int kDeepMaxAcc = 4;
 constexpr int kDeepTeams = 2;
 constexpr int kDeepMmaWarp = 4 * kDeepTeams;   // epilogue warps first: warp & 3 is a warp's quarter of tensor memory
 constexpr int kDeepProducers = kDeepMmaWarp + 1;
-constexpr int kDeepBounds = 512;               // tile bounds of a CTA kept in shared memory
+constexpr int kDeepBounds = 184;               // tile bounds of a CTA kept in shared memory (more cost 96 and 128 channels a stage)
 // producer warps per slot: each fills its part of the slot's rows
 constexpr int deep_parts(int ring) { return ring == 4 ? 4 : 2; }
 constexpr int deep_threads(int ring) { return 32 * (kDeepProducers + ring * deep_parts(ring)); }
@@ -1771,6 +1771,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
     const bool wide_res = (reinterpret_cast<uintptr_t>(ep.residual) & 31) == 0;
     const bool scaled = ep.scale || ep.shift;
     const bool plain = wide_out && !scaled && !ep.residual && ep.act == PCE_ACT_NONE;
+    const bool folded = wide_out && scaled && !ep.residual && ep.act == PCE_ACT_RELU;
     auto row_of = [&](int t) {
       const int slot = t * kTileM + slot_in_tile;
       return t < t1 && slot < n_out ? (ls.order ? __ldg(ls.order + slot) : slot) : n_out;
@@ -1827,6 +1828,27 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
           uint32_t* po = reinterpret_cast<uint32_t*>(o);
 #pragma unroll
           for (int q = 0; q < 8; ++q) po[q] = pack_half2(r[2 * q], r[2 * q + 1]);
+          if (store_row) store32(orow + c0, o[0], o[1]);
+        }
+      } else if (folded && any) {
+        // a folded BatchNorm and ReLU: what most layers of a network have
+#pragma unroll 1
+        for (int c0 = 0; c0 < cout; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(taddr + c0, r);
+          tmem_ld_wait();
+          uint4 o[2];
+          uint32_t* po = reinterpret_cast<uint32_t*>(o);
+#pragma unroll
+          for (int q = 0; q < 16; q += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(affine + c0 + q);
+            const float4 t4 = *reinterpret_cast<const float4*>(affine + cout + c0 + q);
+            // (a NaN becomes zero, as in the general form)
+            const float a = fmaxf(fmaf(__uint_as_float(r[q]), s4.x, t4.x), 0.f), b = fmaxf(fmaf(__uint_as_float(r[q + 1]), s4.y, t4.y), 0.f);
+            const float c = fmaxf(fmaf(__uint_as_float(r[q + 2]), s4.z, t4.z), 0.f), d = fmaxf(fmaf(__uint_as_float(r[q + 3]), s4.w, t4.w), 0.f);
+            po[q / 2] = pack_half2(__float_as_uint(a), __float_as_uint(b));
+            po[q / 2 + 1] = pack_half2(__float_as_uint(c), __float_as_uint(d));
+          }
           if (store_row) store32(orow + c0, o[0], o[1]);
         }
       } else
