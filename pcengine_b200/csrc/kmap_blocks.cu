@@ -583,8 +583,7 @@ constexpr int kClusterRowsAlone = 24576;  // with the GPU to itself, more blocks
 constexpr int kClusterBins = 1 << kOrderBits;
 
 struct ClusterShared {
-  unsigned key[kClusterThreads * kClusterItems];
-  int val[kClusterThreads * kClusterItems];
+  uint2 entry[kClusterThreads * kClusterItems];  // (key, row)
   unsigned short count[kClusterWarps][kClusterBins];  // (a block has at most 8192 rows)
   int total[kClusterBins];                             // read by the other blocks
   int base[kClusterBins];
@@ -713,8 +712,8 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
         const int d = static_cast<int>((key[j] >> shift) & (kClusterBins - 1));
         const int at = sh.base[d] + sh.count[warp][d] + rank[j];
         const int to = at / chunk, in = at - to * chunk;
-        cluster.map_shared_rank(sh.key, to)[in] = key[j];
-        cluster.map_shared_rank(sh.val, to)[in] = val[j];
+        // one store for both: remote stores to scattered words are what a pass takes (32 lanes, 32 words, one at a time)
+        cluster.map_shared_rank(sh.entry, to)[in] = make_uint2(key[j], static_cast<unsigned>(val[j]));
       }
     }
     cluster.sync();
@@ -722,8 +721,9 @@ __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kCluste
     for (int j = 0; j < kClusterItems; ++j) {
       const int i = local0 + 32 * j;
       if (j < items && row0 + i < n) {
-        key[j] = sh.key[i];
-        val[j] = sh.val[i];
+        const uint2 e = sh.entry[i];
+        key[j] = e.x;
+        val[j] = static_cast<int>(e.y);
       }
     }
   }
