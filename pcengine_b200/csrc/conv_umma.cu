@@ -94,6 +94,8 @@ struct Lists {
   const __half* wtail;   // the weights' 32-channel image, for the last K block of a width that is an odd multiple of 32
   const __half* wslots;  // SLOTS > 1: weights as [kv][cout][cin] (one 16-byte chunk row per output channel)
   int settled;           // the lists were complete before the previous kernel of the stream was launched
+  int entries;           // k_conv_deep: offsets per listed stage (1 or 2), each a ring stage of its own there
+  int tall;              // k_conv_deep: the lists' tiles are 256 rows, two of the kernel's
 };
 
 // Second operand: out[row] += in2[row] @ w2, joined to the accumulation at the identity stage.
@@ -1537,7 +1539,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
   const int lane = tid & 31;
   const int kblocks = (cin + KB - 1) / KB;
   const int kblocks2 = sec.in2 ? (sec.cin2 + KB - 1) / KB : 0;
-  const int n_tiles = (n_out + kTileM - 1) / kTileM;
+  const int tall = ls.tall, n_tiles = (n_out + (kTileM << tall) - 1) >> (7 + tall);  // the lists' tiles
   if (tid == 0) {
     for (int s = 0; s < RING; ++s) {
       mbar_init(smem_u32(&ctl->full[s]), PARTS);
@@ -1582,16 +1584,18 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  const int t0 = ctl->range[0], t1 = ctl->range[1];
-  for (int i = tid; i <= t1 - t0 && i < kDeepBounds; i += deep_threads(RING)) ctl->bounds[i] = first_stage(ls.tile_ptr, t0 + i);
+  const int first_tile = ctl->range[0], last_tile = ctl->range[1];
+  for (int i = tid; i <= last_tile - first_tile && i < kDeepBounds; i += deep_threads(RING))
+    ctl->bounds[i] = first_stage(ls.tile_ptr, first_tile + i);
   __syncthreads();
-  auto bound = [&](int t) { return t - t0 < kDeepBounds ? ctl->bounds[t - t0] : first_stage(ls.tile_ptr, t); };
+  const int t0 = first_tile << tall, t1 = min(last_tile << tall, (n_out + kTileM - 1) / kTileM);  // in tiles of 128 rows
+  auto bound = [&](int t) { return t - first_tile < kDeepBounds ? ctl->bounds[t - first_tile] : first_stage(ls.tile_ptr, t); };
   struct Work {
-    int first;        // first stage of the lists (of this CTA's part)
+    int first;        // first entry of the lists (of this CTA's part)
     int main, ident;  // ring stages of the listed offsets; with the identity stage
   };
   auto work_of = [&](int t) {
-    const int b0 = bound(t), b1 = bound(t + 1);
+    const int b0 = bound(t >> tall), b1 = bound((t >> tall) + 1);
     int sa = b0, sb = b1;
     if (parts > 1) {
       const int n = sb - sa, part = static_cast<int>(blockIdx.x) % parts;
@@ -1600,9 +1604,9 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       sa = a;
     }
     Work w;
-    w.first = sa;
+    w.first = sa * ls.entries;
     w.ident = (ls.identity && sb > sa && sb == b1) ? 1 : 0;
-    w.main = (sb - sa - w.ident) * kblocks;
+    w.main = (sb - sa - w.ident) * ls.entries * kblocks;
     return w;
   };
 
@@ -1639,13 +1643,16 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       const int g = w.first + o;
       if (lane < kQuads) {
         if (ls.tile_ptr) {
-          rows = __ldg(reinterpret_cast<const int4*>(ls.stage_nbr + static_cast<size_t>(g) * kTileM + part * kPartRows) + lane);
+          rows = __ldg(reinterpret_cast<const int4*>(ls.stage_nbr + (static_cast<size_t>(g) << (7 + tall)) + ((t & tall) * kTileM + part * kPartRows)) + lane);
         } else {
           const int r = g * kTileM + part * kPartRows + 4 * lane;
           rows = make_int4(r < n_out ? r : -1, r + 1 < n_out ? r + 1 : -1, r + 2 < n_out ? r + 2 : -1, r + 3 < n_out ? r + 3 : -1);
         }
       }
-      if (part == 0 && ls.tile_ptr && !second) kp = __ldg(ls.stage_kp + g) & 255;  // (bits 8..: sub-tile presence)
+      if (part == 0 && ls.tile_ptr && !second) {
+        kp = __ldg(ls.stage_kp + g);
+        kp = kp < 0 ? 0 : kp & 255;  // (negative: an entry without an offset, no rows; bits 8..: sub-tile presence)
+      }
       j += RING;
       return true;
     };
@@ -2066,7 +2073,7 @@ bool conv_umma_supported(int cin, int cout, int dtype) {
 // Behind them, a second copy as 32-channel blocks (cout rows x 64 B, 64-byte swizzle) for widths that are an odd
 // multiple of 32 (their last K block is half, see HALF) and for every single-offset weight (a second
 // operand of such a layer).
-static bool has_kb32_image(int kv, int cin) { return kv == 1 || (cin > 32 && cin % 64 == 32); }
+static bool has_kb32_image(int kv, int cin) { return kv == 1 || cin % 64 == 32; }
 static size_t kb64_image_bytes(int kv, int cin, int cout) {
   const size_t blocks = static_cast<size_t>(kv) * ((cin + 63) / 64) * cout * 128;
   return blocks + ((cin == 16 || cin == 32) ? static_cast<size_t>(kv) * cout * cin * 2 : 0);
@@ -2280,9 +2287,8 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
   return grid > 0 ? static_cast<size_t>(grid) * 2 * umma::kTileM * cout * sizeof(float) : 0;
 }
 
-// Input widths of k_conv_deep: whole K blocks, or a half block at the end (below 64 channels several offsets share a stage,
-// or the block is mostly padding).
-static bool deep_widths(int cin) { return cin >= 64 && cin % 32 == 0; }
+// Input widths of k_conv_deep: whole K blocks, or a half block at the end (32 channels: one half block).
+static bool deep_widths(int cin) { return cin >= 32 && cin % 32 == 0; }
 
 // The same where a split was measured faster; the framework's own callers ask this one.  Equal shares of stages repay
 // their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
@@ -2363,25 +2369,23 @@ int conv_umma_kb64(const void* in, int n_in, const void* wpacked, int kv, const 
 // `split`: the caller allows several CTAs per tile.
 static int conv_deep(const umma::DeepMaps& maps, const __half* w, const umma::Lists& ls, const umma::Second& sec, int n_in, int n_out, int cin,
                      int cout, int kv, __half* out, umma::Epi e, bool half, bool split, int dev, int sm_count, cudaStream_t st) {
-  static bool attr_set[64] = {};
-  if (!attr_set[dev]) {
-    for (int r = 4; r <= umma::kDeepMaxRing; ++r)
-      for (int v = 0; v < 2; ++v)
-        PCE_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(deep_kernel(v != 0, r)), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      227 * 1024));
-    attr_set[dev] = true;
-  }
   const size_t stage = static_cast<size_t>(umma::kABytes) + static_cast<size_t>(cout) * 128;
   const size_t rest = sizeof(umma::DeepCtl) + 1024 + 64 + 2 * sizeof(float) * cout;
   const int ring = std::min<int>(umma::kDeepMaxRing, static_cast<int>((227 * 1024 - rest) / stage));
+  static bool attr_set[64][2][umma::kDeepMaxRing + 1] = {};  // (a variant is loaded when it is first wanted)
+  if (!attr_set[dev][half][ring]) {
+    PCE_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(deep_kernel(half, ring)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  227 * 1024));
+    attr_set[dev][half][ring] = true;
+  }
   const int nacc = cout <= 128 ? 4 : 2;
   int cols = 32;
   while (cols < nacc * cout) cols <<= 1;
   const int n_tiles = div_up(n_out, umma::kTileM);
-  const int parts = split ? deep_split(n_tiles, n_out, n_in, cin, kv, sm_count) : 1;
+  const int parts = split && !ls.tall ? deep_split(n_tiles, n_out, n_in, cin, kv, sm_count) : 1;
   e.parts = parts;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(parts > 1 ? n_tiles * parts : std::min(n_tiles, sm_count));
+  cfg.gridDim = dim3(parts > 1 ? n_tiles * parts : std::min((n_tiles + ls.tall) >> ls.tall, sm_count));
   cfg.blockDim = dim3(umma::deep_threads(ring));
   cfg.dynamicSmemBytes = ring * stage + rest;
   cfg.stream = st;
@@ -2418,13 +2422,13 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
       if (!e.push_slot[s]) e.push_base[s] = nullptr;
     }
   }
-  umma::Lists ls{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0};
+  umma::Lists ls{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0, 1, 0};
   int slots = 1;
   umma::Second sec{nullptr, nullptr, nullptr, 0};
   int sub = umma_force_sub == 1 || umma_force_sub == 2 ? umma_force_sub : 1;
   if (tiles) {
     ls = umma::Lists{tiles->order, tiles->tile_ptr, tiles->stage_kp, tiles->stage_nbr, tiles->identity_stage ? 1 : 0, nullptr, nullptr,
-                     (tiles->settled && umma_overlap_launches == 1) ? 1 : 0};
+                     (tiles->settled && umma_overlap_launches == 1) ? 1 : 0, 1, 0};
     slots = tiles->slots > 1 ? tiles->slots : 1;
     if (slots != 1) {
       // several offsets per stage: the lists must match the layer's width, and the packed weights carry
@@ -2502,16 +2506,31 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
     if (sub > 2) return PCE_ERR_UNSUPPORTED;  // 512-row super-tiles exist for k_conv_umma_mt only
   }
   // One CTA per SM wherever its producers can take the layer (k_conv_deep); the tuning hooks below are k_conv_umma's.
-  if (slots == 1 && sub == 1 && !(e.push_slot[0] || e.push_slot[1]) && deep_widths(cin) && (cin % 64 == 0 || half) && !off16(in) &&
+  const bool pairs = slots == 2;  // 32 input channels: a half block per offset there, two offsets to a stage below
+  const bool deep_half = umma_half_blocks && !kb64_slice && cin % 64 == 32;
+  // Two narrow offsets to a stage are half the stages, which counts once a map has more than about five tiles per SM and the
+  // outputs are narrow too.  Kernel only, us, k_conv_umma / k_conv_deep: 32->32 on 60 k rows 12.7 / 11.3, on 120 k 15.7 / 17.1,
+  // on 480 k 31.5 / 46.8; 32->64 on 60 k 14.9 / 11.7, on 120 k 19.1 / 17.5, on 480 k 49.4 / 46.9.
+  const bool packed = pairs && cout <= 32 && div_up(n_out, umma::kTileM) > 5 * sm_count[dev];
+  if (!packed && (slots == 1 ? sub == 1 : pairs) && !(e.push_slot[0] || e.push_slot[1]) && deep_widths(cin) && (cin % 64 == 0 || deep_half) && !off16(in) &&
       !off16(ls.stage_nbr) && !umma_force_stages && !umma_force_nacc && umma_split_enabled != 3) {
+    umma::Lists dl = ls;
+    umma::Second ds = sec;
+    dl.entries = pairs ? 2 : 1;
+    dl.tall = sub == 2 ? 1 : 0;
+    if (deep_half) {
+      dl.wtail = reinterpret_cast<const __half*>(static_cast<const char*>(wpacked) + kb64_image_bytes(kv, cin, cout));
+      if (ds.in2 && ds.cin2 % 64 == 32)
+        ds.wtail = reinterpret_cast<const __half*>(reinterpret_cast<const char*>(ds.w2) + kb64_image_bytes(1, ds.cin2, cout));
+    }
     umma::DeepMaps maps;
-    bool mapped = row_map(&maps.in, in, n_in, cin, e.ld_in, 64) && (!half || row_map(&maps.in32, in, n_in, cin, e.ld_in, 32));
-    if (sec.in2)
-      mapped = mapped && row_map(&maps.sec, sec.in2, n_out, sec.cin2, sec.cin2, 64) &&
-               (!sec.wtail || row_map(&maps.sec32, sec.in2, n_out, sec.cin2, sec.cin2, 32));
+    bool mapped = row_map(&maps.in, in, n_in, cin, e.ld_in, 64) && (!deep_half || row_map(&maps.in32, in, n_in, cin, e.ld_in, 32));
+    if (ds.in2)
+      mapped = mapped && row_map(&maps.sec, ds.in2, n_out, ds.cin2, ds.cin2, 64) &&
+               (!ds.wtail || row_map(&maps.sec32, ds.in2, n_out, ds.cin2, ds.cin2, 32));
     if (mapped)
-      return conv_deep(maps, static_cast<const __half*>(wpacked), ls, sec, n_in, n_out, cin, cout, kv, static_cast<__half*>(out), e,
-                       half, tiles && ep && (ep->split || ep->split_scratch), dev, sm_count[dev], st);
+      return conv_deep(maps, static_cast<const __half*>(wpacked), dl, ds, n_in, n_out, cin, cout, kv, static_cast<__half*>(out), e,
+                       deep_half, tiles && ep && (ep->split || ep->split_scratch), dev, sm_count[dev], st);
   }
   // Configuration = (ring depth, accumulator sets).  What the kernel needs most is row gathers in
   // flight, i.e. stages resident per SM = resident CTAs x ring depth; the CTAs per SM are bounded by

@@ -34,6 +34,7 @@ def _both(f):
 @pytest.mark.parametrize("kind,n,cin,cout,ks", [
     ("sheet", 1, 64, 16, 3), ("sheet", 3, 64, 64, 3), ("sheet", 127, 96, 96, 3), ("sheet", 128, 128, 128, 3), ("sheet", 129, 64, 160, 3),
     ("block", 1331, 160, 224, 3), ("block", 1331, 256, 256, 3), ("random", 5000, 64, 112, 3), ("random", 5000, 128, 192, 5),
+    ("sheet", 129, 32, 32, 3), ("block", 1331, 32, 96, 3), ("sheet", 94720, 32, 32, 3), ("sheet", 94721, 32, 32, 3), ("random", 5000, 32, 64, 5),
     ("sheet", 20001, 96, 64, 3), ("sheet", 40000, 64, 256, 3), ("random", 30000, 64, 64, 5)])
 def test_layers(kind, n, cin, cout, ks):
     from pcengine_b200 import functional as PF
@@ -62,7 +63,7 @@ def test_layers(kind, n, cin, cout, ks):
     assert PF.device_status() == 0
 
 
-@pytest.mark.parametrize("n,cin,cin2,cout", [(129, 64, 32, 64), (3000, 96, 96, 96), (3000, 128, 96, 128), (3000, 96, 64, 256), (3000, 64, 160, 64)])
+@pytest.mark.parametrize("n,cin,cin2,cout", [(129, 64, 32, 64), (3000, 32, 32, 32), (3000, 32, 64, 64), (3000, 96, 96, 96), (3000, 128, 96, 128), (3000, 96, 64, 256), (3000, 64, 160, 64)])
 def test_second_operand(n, cin, cin2, cout):
     """Widths of the second operand that are whole K blocks, end in a half block and end in padding."""
     from pcengine_b200 import functional as PF
@@ -77,7 +78,7 @@ def test_second_operand(n, cin, cin2, cout):
     assert co.rel_l2(got.float().cpu(), want) <= 5e-4 and torch.equal(got, other)
 
 
-@pytest.mark.parametrize("n,cin,cout", [(1, 64, 64), (130, 96, 32), (1000, 128, 256), (20000, 256, 48)])
+@pytest.mark.parametrize("n,cin,cout", [(1, 64, 64), (130, 96, 32), (129, 32, 32), (1000, 128, 256), (20000, 256, 48)])
 def test_dense_product_and_column_ranges(n, cin, cout):
     """1x1x1 layers, and a layer that reads and writes column ranges of wider matrices."""
     from pcengine_b200 import functional as PF
