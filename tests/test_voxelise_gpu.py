@@ -36,3 +36,28 @@ def test_device_collation_equals_the_host_path(k, width):
     a, b = batch("cuda"), batch("cpu")
     assert torch.equal(a.coords.cpu(), b.coords) and torch.equal(a.feats.cpu(), b.feats)
     assert a.coords_max == b.coords_max and a.batchsize == k
+
+
+@pytest.mark.parametrize("n,kind", [(4097, "one voxel"), (9000, "two voxels"), (70000, "wide"), (100000, "sorted"), (100000, "lines")])
+def test_voxelisation_by_buckets(n, kind):
+    """Clouds that miss the buckets (a voxel of more points than a bucket holds, key and index beyond a word) and clouds in
+    orders that a sample at equal distances could misjudge."""
+    import pcengine_b200 as pce
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(-40, 40, (n, 3))
+    if kind == "one voxel":
+        pts = rng.uniform(0.01, 0.11, (n, 3))
+    elif kind == "two voxels":
+        pts = rng.uniform(0.01, 0.11, (n, 3)) + 0.125 * (np.arange(n) % 2)[:, None]
+    elif kind == "wide":
+        pts *= 90
+    elif kind == "sorted":
+        pts = pts[np.lexsort(pts.T[::-1])]
+    elif kind == "lines":  # every 98th point, the distance of the samples, lies on one line
+        pts[n // 2048::n // 1024, :2] = 0.5
+    pts = pts.astype(np.float32)
+    voxel = float(np.float32(0.125))
+    want = pce.sparse_quantize(pts, voxel, return_index=True, return_inverse=True)
+    got = pce.sparse_quantize(torch.from_numpy(pts).cuda(), voxel, return_index=True, return_inverse=True)
+    for a, b in zip(got, want):
+        assert np.array_equal(a.cpu().numpy(), b)
