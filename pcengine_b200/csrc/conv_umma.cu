@@ -1485,6 +1485,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 2 + 4 * EPIW), SUB == 1 ? 2 : 
 constexpr int kDeepMaxRing = 9;
 constexpr int kDeepMaxAcc = 4;
 constexpr int kDeepTeams = 2;
+constexpr int kDeepWide = 128;  // output channels from which a tile's columns are shared by the teams
 constexpr int kDeepMmaWarp = 4 * kDeepTeams;   // epilogue warps first: warp & 3 is a warp's quarter of tensor memory
 constexpr int kDeepProducers = kDeepMmaWarp + 1;
 constexpr int kDeepBounds = 184;               // tile bounds of a CTA kept in shared memory (more cost 96 and 128 channels a stage)
@@ -1534,6 +1535,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
   DeepCtl* ctl = reinterpret_cast<DeepCtl*>(tiles + RING * stage_bytes);
   float* affine = reinterpret_cast<float*>(ctl + 1);
   static_assert(sizeof(DeepCtl) % 16 == 0, "the staged scale/shift are read as float4");
+  const bool wide = cout >= kDeepWide;  // both teams take half of every tile's columns
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -1547,7 +1549,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
     }
     for (int s = 0; s < nacc; ++s) {
       mbar_init(smem_u32(&ctl->accfull[s]), 1);
-      mbar_init(smem_u32(&ctl->accempty[s]), 128);
+      mbar_init(smem_u32(&ctl->accempty[s]), wide ? 256 : 128);
     }
     ctl->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1571,6 +1573,8 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       ctl->range[0] = static_cast<int>(blockIdx.x) / parts;
       ctl->range[1] = static_cast<int>(blockIdx.x) / parts + 1;
     }
+  } else if (static_cast<int>(gridDim.x) == n_tiles) {  // a tile each
+    if (tid < 2) ctl->range[tid] = static_cast<int>(blockIdx.x) + tid;
   } else if (warp < 2) {
     // a tile's stores cost about two ring stages: 64->64 on 200 k rows 20.7 us so, 22.9 with one, 28.3 with a quarter; 5x5x5 on
     // 300 k rows 110, 129, 140; 96->96 on 240 k rows 36 so, 44 with four
@@ -1783,9 +1787,14 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       const int slot = t * kTileM + slot_in_tile;
       return t < t1 && slot < n_out ? (ls.order ? __ldg(ls.order + slot) : slot) : n_out;
     };
-    int my_row = row_of(t0 + team);
+    // Two teams: a tile each in turn, or (wide outputs, and a CTA with one tile) half the columns each of every tile, which ends
+    // the last tile sooner: 256 columns of a tile take one team about 8000 cycles.
+    const bool halves = wide || t1 - t0 == 1;
+    const int c_mid = halves ? (cout / 2 + 15) & ~15 : 0, c_from = team ? c_mid : 0, c_to = halves && !team ? c_mid : cout;
+    const int t_step = halves ? 1 : kDeepTeams, t_first = halves ? t0 : t0 + team;
+    int my_row = row_of(t_first);
     if (ls.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int t = t0 + team; t < t1; t += kDeepTeams) {
+    for (int t = t_first; t < t1; t += t_step) {
       const int it = t - t0;
       const Work work = work_of(t);
       const int buf = it & (nacc - 1), round = it / nacc;
@@ -1793,7 +1802,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       const bool any = work.main + (work.ident ? kblocks2 : 0) > 0;
       __half* orow = out + static_cast<size_t>(store_row ? my_row : 0) * ep.ld_out;
       const __half* rrow = (ep.residual && store_row) ? ep.residual + static_cast<size_t>(my_row) * cout : nullptr;
-      my_row = row_of(t + kDeepTeams);  // (a tile ahead)
+      my_row = row_of(t + t_step);  // (a tile ahead)
       if (rrow) {
         // the rows are known before the accumulator is: pull the residual rows into L2 while waiting
         const char* rp = reinterpret_cast<const char*>(rrow);
@@ -1812,9 +1821,9 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       if (plain && any) {
         // nothing but the conversion: kept apart, since the code of all the other cases, stepped over or predicated off, took
         // longer to fetch than this takes to run
-        int c0 = 0;
+        int c0 = c_from;
 #pragma unroll 1
-        for (; c0 + 32 <= cout; c0 += 32) {
+        for (; c0 + 32 <= c_to; c0 += 32) {
           uint32_t r[32];
           tmem_ld32(taddr + c0, r);
           tmem_ld_wait();
@@ -1827,7 +1836,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
             store32(orow + c0 + 16, o[2], o[3]);
           }
         }
-        if (c0 < cout) {
+        if (c0 < c_to) {
           uint32_t r[16];
           tmem_ld16(taddr + c0, r);
           tmem_ld_wait();
@@ -1840,7 +1849,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
       } else if (folded && any) {
         // a folded BatchNorm and ReLU: what most layers of a network have
 #pragma unroll 1
-        for (int c0 = 0; c0 < cout; c0 += 16) {
+        for (int c0 = c_from; c0 < c_to; c0 += 16) {
           uint32_t r[16];
           tmem_ld16(taddr + c0, r);
           tmem_ld_wait();
@@ -1860,7 +1869,7 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
         }
       } else
 #pragma unroll 1
-      for (int c0 = 0; c0 < cout; c0 += 16) {
+      for (int c0 = c_from; c0 < c_to; c0 += 16) {
         uint4 ra, rb;
         if (rrow) {  // issued ahead of the tensor-memory load, consumed after it
           if (wide_res) {
