@@ -44,14 +44,16 @@ constexpr int kCode = 1186111;
 // One warp per input row: copy the row to every buffer slot its CSR entries name
 // (ref: backend/spconv.cuh:48-81 gather_all_input_major_csr_*); 16-byte pieces when the row
 // length allows.
+// `group` lanes (a power of two, at most 32) take a row: as many as it has 16-byte pieces, so that narrow rows do not leave
+// the rest of a warp idle.
 template <typename T>
-__global__ void k_d1_gather(const T* __restrict__ in, int n_in, int cin, const int* __restrict__ qkpos,
-                            const int* __restrict__ icsr, const int* __restrict__ imap, T* __restrict__ buf) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= n_in) return;
-  const int a = __ldg(icsr + warp), b = __ldg(icsr + warp + 1);
-  const T* src = in + static_cast<size_t>(warp) * cin;
+__global__ void __launch_bounds__(256) k_d1_gather(const T* __restrict__ in, int n_in, int cin, const int* __restrict__ qkpos,
+                                                   const int* __restrict__ icsr, const int* __restrict__ imap, T* __restrict__ buf, int group) {
+  const int row = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / group);
+  const int lane = threadIdx.x & (group - 1);
+  if (row >= n_in) return;
+  const int a = __ldg(icsr + row), b = __ldg(icsr + row + 1);
+  const T* src = in + static_cast<size_t>(row) * cin;
   const int row_bytes = cin * static_cast<int>(sizeof(T));
   const bool vec = (row_bytes % 16 == 0) && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(buf)) % 16 == 0);
   for (int e = a; e < b; ++e) {
@@ -61,9 +63,9 @@ __global__ void k_d1_gather(const T* __restrict__ in, int n_in, int cin, const i
     if (vec) {
       const uint4* s4 = reinterpret_cast<const uint4*>(src);
       uint4* d4 = reinterpret_cast<uint4*>(dst);
-      for (int c = lane; c < row_bytes / 16; c += 32) d4[c] = __ldg(s4 + c);
+      for (int c = lane; c < row_bytes / 16; c += group) d4[c] = __ldg(s4 + c);
     } else {
-      for (int c = lane; c < cin; c += 32) dst[c] = src[c];
+      for (int c = lane; c < cin; c += group) dst[c] = src[c];
     }
   }
 }
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// One warp per output row, lanes over 16-byte pieces of the row: fp32 sums over the row's buffer rows
+// `group` lanes (a power of two, at most 32) per output row, each a 16-byte piece of the row: fp32 sums over the row's buffer rows
 // (kp ascending, as the CSR lists them), plus the centre product -- read from `centre` when the
 // tensor-core kernel computed it as a dense product beforehand, else formed here from W[centre] --
 // then the epilogue and one 16-byte store per piece
@@ -137,17 +139,17 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_d1_scatter(const T* __restrict__ bout, const int* __restrict__ qkpos, const int* __restrict__ ocsr,
                  const int* __restrict__ omap, int n_out, int cout, const T* __restrict__ in, const T* __restrict__ wmid,
-                 const T* centre, int cin, T* out, EpiDev ep) {
+                 const T* centre, int cin, T* out, EpiDev ep, int group) {
   constexpr int kVec = 16 / static_cast<int>(sizeof(T));  // elements per 16-byte piece
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const int row = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / group);
+  const int lane = threadIdx.x & (group - 1);
   if (row >= n_out) return;
   const int a = __ldg(ocsr + row), b = __ldg(ocsr + row + 1);
   const bool vec = (cout % kVec == 0) &&
                    ((reinterpret_cast<uintptr_t>(bout) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(centre) |
                      reinterpret_cast<uintptr_t>(ep.residual)) % 16 == 0);
   const int pieces = vec ? cout / kVec : (cout + kVec - 1) / kVec;
-  for (int p0 = 0; p0 < pieces; p0 += 32) {
+  for (int p0 = 0; p0 < pieces; p0 += group) {
     const int p = p0 + lane;
     const int c0 = p * kVec;
     float acc[kVec];
@@ -211,6 +213,15 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Lanes per row of the gather and the scatter: one per 16-byte piece, at most a warp.  128 fp16 channels on 40 k rows, 16 lanes
+// against 32: gather 9.6 -> 6.1 us, scatter 20.2 -> 13.1.
+static int lanes_for(int channels, size_t bytes) {
+  const int pieces = static_cast<int>((channels * bytes + 15) / 16);
+  int lanes = 1;
+  while (lanes < pieces && lanes < 32) lanes *= 2;
+  return lanes;
+}
+
 template <typename T>
 static int run_d1(const void* in, int n_in, int cin, const void* w, const void* wpacked, int kv, int cout,
                   const int* qkpos, int qsum, const int* imap, const int* icsr, const int* omap, const int* ocsr,
@@ -221,8 +232,8 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
   const T* in_t = static_cast<const T*>(in);
   const T* w_t = static_cast<const T*>(w);
   if (n_in > 0 && qsum > 0) {
-    k_d1_gather<T><<<div_up(static_cast<long long>(n_in) * 32, 256), 256, 0, st>>>(in_t, n_in, cin, qkpos, icsr, imap,
-                                                                                    bin);
+    const int group = lanes_for(cin, sizeof(T));
+    k_d1_gather<T><<<div_up(static_cast<long long>(n_in) * group, 256), 256, 0, st>>>(in_t, n_in, cin, qkpos, icsr, imap, bin, group);
     PCE_LAUNCH_CHECK();
     // The per-offset GEMM: the tile-list kernels (tensor cores when packed weights are given, the tiled fp32 one)
     // when the scratch for the lists fits behind the two halves of the buffer, else one thread group per row.
@@ -280,8 +291,9 @@ static int run_d1(const void* in, int n_in, int cin, const void* w, const void* 
         wmid = w_t + static_cast<size_t>(centre_kp) * cin * cout;
       }
     }
-    k_d1_scatter<T><<<div_up(static_cast<long long>(n_out) * 32, 256), 256, 0, st>>>(
-        qsum > 0 ? bout : nullptr, qkpos, ocsr, omap, n_out, cout, in_t, wmid, centre, cin, static_cast<T*>(out), ep);
+    const int group = lanes_for(cout, sizeof(T));
+    k_d1_scatter<T><<<div_up(static_cast<long long>(n_out) * group, 256), 256, 0, st>>>(
+        qsum > 0 ? bout : nullptr, qkpos, ocsr, omap, n_out, cout, in_t, wmid, centre, cin, static_cast<T*>(out), ep, group);
     PCE_LAUNCH_CHECK();
   }
   return PCE_OK;
