@@ -145,3 +145,30 @@ def test_row_order_beyond_64_offsets(rows, kv):
             sets[r] += np.uint64(sum(comb(int(p), i) for i in range(5 - q)))
     key = sets * np.uint64(389) + (hashes * np.uint64(389) >> np.uint64(32))
     assert key.max() < 1 << 32 and np.array_equal(order, np.argsort(key, kind="stable"))
+
+
+@pytest.mark.parametrize("n", [255, 257, 400000])
+def test_table_in_one_launch(n):
+    """Presence and neighbours of a cloud of fewer voxels than a block's threads, and of more than a resident grid's, against
+    sorted keys."""
+    import pcengine_b200 as pce
+    g = torch.Generator("cuda").manual_seed(n)
+    side = 1 << 10
+    lin = torch.randperm(side * side, generator=g, device="cuda")[:n]
+    x, y = lin // side, lin % side
+    coords = torch.stack([lin % 3, x, y, (x + 2 * y) // 16], 1).int().contiguous()
+    km = pce.KernelMap(coords, (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, coords[:, 1:].amax(0).tolist(), True)
+    csr = km.csr()
+    starts, nbr = csr.row_lists()
+    key = lambda c: ((c[:, 0].long() * 2048 + c[:, 1] + 1) * 2048 + c[:, 2] + 1) * 2048 + c[:, 3] + 1
+    keys, rows = torch.sort(key(coords))
+    at = torch.zeros(n, dtype=torch.long, device="cuda")
+    mask = csr.mask[:, 0].long()
+    for kp in range(27):
+        d = torch.tensor([0, kp // 9 - 1, kp // 3 % 3 - 1, kp % 3 - 1], device="cuda")
+        want = key(coords + d)
+        i = torch.searchsorted(keys, want).clamp_(max=n - 1)
+        found = keys[i] == want
+        assert torch.equal((mask >> kp & 1).bool(), found)
+        assert torch.equal(nbr[(starts.long() + at)[found]].long(), rows[i[found]])
+        at += found
