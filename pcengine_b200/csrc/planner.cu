@@ -150,7 +150,11 @@ struct LevelState {
   int ready = 0;             // host side: n is known, ev is recorded (guarded by plan->m)
 };
 
-constexpr int kMapLanes = 4;  // one-scan pass 890 us with two, 862 with three, 855 with four; eight scans 2300, 2271, 2257
+// Map lanes of passes that run in one call: one scan 890 us with two, 862 with three, 855 with four; eight scans 2300, 2271,
+// 2257.  Where a network runs layer by layer its launches and the lanes' wait for one another in the driver, and two are
+// enough (fp32 network of half width, rooms of 8 k / 16 k / 30 k voxels: 1893 / 1932 / 2013 us with two, 1952 / 1993 / 2029 with
+// four).
+constexpr int kMapLanes = 4, kMapLanesByLayer = 2;
 constexpr int kLanes = 1 + kMapLanes;
 
 }  // namespace pce
@@ -208,6 +212,7 @@ struct pce_plan {
   std::condition_variable cv;
   std::deque<pce_pass*> idle;  // released passes (arena + events), oldest first
   int n_passes = 0;            // pass objects created so far
+  bool one_call = false;       // pce_net_run has run one of them
   bool stop = false;
 };
 
@@ -655,6 +660,16 @@ static int build_map(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
 static int run_map_lane(pce_plan* p, PlanLane* l, pce_pass* ps) {
   PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->start, 0));
   if (ps->has_released) PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->released, 0));
+  if (p->chain && plan_short_route) {
+    // Which maps a lane gets differs from pass to pass: room for the largest (no level has more rows than the input) at once,
+    // or a later pass stops to free and to allocate.
+    void* ws = nullptr;
+    PCE_TRY(scratch_for(l, blk::order_workspace_bytes(ps->levels[0].n), &ws));
+  }
+  if (l - p->lanes > kMapLanesByLayer) {
+    std::lock_guard<std::mutex> lk(p->m);
+    if (!p->one_call) return PCE_OK;
+  }
   for (;;) {
     int i;
     {
@@ -1037,6 +1052,10 @@ int pce_net_run(pce_pass* ps, const pce_net_buffer* buffers, int32_t n_buffers, 
   if (dtype != PCE_F16) return PCE_ERR_UNSUPPORTED;
   // (A stream of the highest priority for the pass, forked from and joined to the caller's, was measured:
   // 3.93 -> 3.98 ms per 8-scan step beside the next pass's map construction, no change on 1 or 2 scans.)
+  {
+    std::lock_guard<std::mutex> lk(ps->plan->m);
+    ps->plan->one_call = true;
+  }
   return net_run_on(ps, buffers, n_buffers, ops, n_ops, input, in_ld, output, out_ld, arena, arena_bytes, dtype,
                     static_cast<cudaStream_t>(stream));
 }
