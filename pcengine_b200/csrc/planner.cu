@@ -195,6 +195,8 @@ struct PlanLane {
   cudaStream_t stream = nullptr;
   void* scratch = nullptr;
   size_t scratch_cap = 0;
+  void* order_ws = nullptr;     // of the pass at hand, block form
+  size_t order_bytes = 0;
   std::deque<pce_pass*> queue;  // guarded by plan->m
   std::thread thread;
 };
@@ -506,9 +508,8 @@ static int build_direction(pce_plan* p, PlanLane* l, pce_pass* ps, blk::Order o,
   if (o.n_variants == 0 || o.n == 0) return PCE_OK;
   o.order = ps->take_n<int32_t>(o.n);
   if (!o.order) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
-  void* ws = nullptr;
-  PCE_TRY(scratch_for(l, blk::order_workspace_bytes(o.n), &ws));
-  PCE_TRY(blk::order_lists(o, ws, l->scratch_cap, false, l->stream));
+  if (!l->order_ws) return PCE_ERR_INVALID;  // (only passes in block form come here)
+  PCE_TRY(blk::order_lists(o, l->order_ws, l->order_bytes, false, l->stream));
   for (int v = 0; v < o.n_variants; ++v) {
     const blk::Variant& V = o.variant[v];
     out->lists[out->n_lists++] = pce_tile_lists{o.order, V.tile_ptr, V.stage_kp, V.stage_nbr, V.tile_rows, identity_stage, V.slots, 1};
@@ -660,15 +661,18 @@ static int build_map(pce_plan* p, PlanLane* l, pce_pass* ps, int i) {
 static int run_map_lane(pce_plan* p, PlanLane* l, pce_pass* ps) {
   PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->start, 0));
   if (ps->has_released) PCE_CUDA(cudaStreamWaitEvent(l->stream, ps->released, 0));
-  if (p->chain && plan_short_route) {
-    // Which maps a lane gets differs from pass to pass: room for the largest (no level has more rows than the input) at once,
-    // or a later pass stops to free and to allocate.
-    void* ws = nullptr;
-    PCE_TRY(scratch_for(l, blk::order_workspace_bytes(ps->levels[0].n), &ws));
-  }
   if (l - p->lanes > kMapLanesByLayer) {
     std::lock_guard<std::mutex> lk(p->m);
     if (!p->one_call) return PCE_OK;
+  }
+  l->order_ws = nullptr;
+  if (p->chain && plan_short_route) {
+    // The row orders' scratch comes with the pass, for the largest of its maps (no level has more rows than the input): a
+    // lane gets other maps in every pass, and scratch of its own would grow, with a stop to free and to allocate, until it
+    // has had them all.
+    l->order_bytes = blk::order_workspace_bytes(ps->levels[0].n);
+    l->order_ws = ps->take(l->order_bytes);
+    if (!l->order_ws) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
   }
   for (;;) {
     int i;
