@@ -1,5 +1,8 @@
 // Fused gather-matmul-scatter on the 5th-generation tensor cores (tcgen05 + tensor
-// memory), fp16 in / fp32 accumulate, output stationary, persistent and warp-specialised.
+// memory), fp16 in / fp32 accumulate, output stationary, persistent and warp-specialised.  Two
+// kernels share lists, shares and options: k_conv_deep (one CTA per SM, rows by TMA gathers) takes
+// the layers whose input width is a multiple of 32, k_conv_umma, described first, all others, halo
+// pushes and narrow layers on large maps; the rule stands in conv_umma_impl.
 //
 // The kernel reads the map as TILE LISTS (built once per kernel map by pce_build_tile_lists):
 // output rows are taken in sorted order (pce_csr_sort_rows) in tiles of 128 or 256; for every
@@ -20,10 +23,8 @@
 //              (cp.async.bulk, the TMA engine).  Stage indices are read four stages ahead
 //              (coalesced reads) into registers that are never moved, so the loads stay in
 //              flight until the stage that uses them.
-//              Measured on B200 (random 128-byte rows, L2 resident): cp.async sustains more
-//              than 100 GB/s per SM, while TMA tile::gather4 and per-row bulk copies cost
-//              about 43 ns per operation per issuing warp (11 GB/s per SM per warp), so the
-//              row gather stays on cp.async and only the dense weight block uses TMA.
+//              (tile::gather4 costs its warp 43 ns an operation: too slow from a few warps, and
+//              what k_conv_deep below spreads over sixteen.)
 //   one MMA warp: one lane issues tcgen05.mma (M=128, N=C_out, K=16; one per sub-tile on the
 //              same weight descriptor) and commits to mbarriers.
 //   4 epilogue warps: tcgen05.ld the finished accumulator, apply
@@ -1470,16 +1471,22 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 2 + 4 * EPIW), SUB == 1 ? 2 : 
 // that only fills in zeros takes three times as long as one that moves data.  Here
 //   * rows come by tile::gather4, four rows per operation.  One operation costs the issuing warp 80 cycles, which made
 //     it look slow from one warp (2576 cycles for a stage's 128 rows); sixteen warps that issue half a stage each keep
-//     the L2 port busy (240 cycles a stage, 68 of 64 to 72 bytes per clock and SM) and do nothing else.  The data arrives
+//     the L2 port busy (240 cycles a stage, 68 of about 71 bytes per clock and SM) and do nothing else.  The data arrives
 //     through the async proxy: nobody has to order it before the products.
 //   * groups of four rows that all lack the offset are not copied: the warp stores zeros, once for as long as the same
 //     group of the slot stays without rows (an out-of-range row costs the TMA engine 40 cycles);
-//   * the MMA warp's ring is unrolled: with a slot's descriptors and barriers known up to their base a stage takes 230 to 300
-//     cycles to issue, from a running slot number 400 to 700;
+//   * one thread issues the products in a short loop over running descriptors.  Unrolled over the ring, with every slot's
+//     descriptors and barriers known up to their base, a stage is cheaper by itself (230 to 300 cycles against 400 to 700),
+//     but that code, like an epilogue that carries every option through every tile, does not fit the instruction caches
+//     beside the other roles': layers took up to twice as long;
 //   * the SM's shared memory is one ring of 4 to 9 stages, and two teams of epilogue warps take the tiles in turn with two
 //     or four accumulators between them: no product waits for a tile's stores;
 //   * a third as many CTAs have shares three times as long, against which the heaviest tiles (27 offsets, where the mean is
 //     2 to 5) weigh less.
+// Kernel only, us, k_conv_umma / this: 64->64 on 200 k rows of a room 29.9 / 22.3, 96->96 on 240 k rows of four scans 45.9 / 38.3,
+// 256->256 on 1.5 M rows 544 / 502, 64->64 5x5x5 on 1.5 M rows 408 / 278.  What bounds it now: with 256 channels the round trip of a
+// ring of four 48 KB stages (41 bytes per clock and SM from L2, tensor pipe half busy); with few, the heaviest CTA's chain of
+// stages and the set-up of a layer (about 4 us to the first product).
 // Lists, shares of tiles, second operand, split tiles and bounded waits are k_conv_umma's.  Widths are multiples of
 // 32 input channels (the last 32 of an odd multiple are a half block, as there).
 constexpr int kDeepMaxRing = 9;
