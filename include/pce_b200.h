@@ -107,11 +107,13 @@ typedef struct pce_epilogue {
   /* Maps with few tiles (optional).  A 128-row tile is one sequential chain of (offset, K block)
    * stages on one CTA; a map with fewer tiles than the GPU has CTA slots leaves SMs idle while
    * those chains run, and one with a few times as many ends in a half-empty wave.  With `split`
-   * set, small maps run a cluster of 2, 4 or 8 CTAs per tile (pce_conv_split_parts), which add
-   * their fp32 sums through shared memory.  With split_scratch of at least
-   * pce_conv_split_scratch_wanted(...) bytes (16-byte aligned), mid-size maps are cut into equal
-   * shares of the stages whatever tiles they fall in: the CTAs leave fp32 partial sums here and a
-   * second kernel adds them in a fixed order and applies the epilogue.  Both are deterministic;
+   * set, small maps run a cluster of 2 or 4 CTAs per tile (8 too where c_in is no multiple of 32;
+   * pce_conv_split_parts), which add their fp32 sums through shared memory.  With split_scratch of
+   * at least pce_conv_split_scratch_wanted(...) bytes (16-byte aligned), mid-size maps of layers
+   * whose c_in is no multiple of 32 are cut into equal shares of the stages whatever tiles they
+   * fall in: the CTAs leave fp32 partial sums here and a second kernel adds them in a fixed order
+   * and applies the epilogue.  (The others have one CTA per SM and are not cut into shares: they
+   * leave the scratch alone.)  Both are deterministic;
    * the fp32 sum is associated differently than in the one-CTA chain.  A scratch, however small,
    * implies `split`; with neither the layer runs whole. */
   void* split_scratch;
@@ -403,19 +405,20 @@ PCE_API int pce_device_status(int32_t* status_host, int32_t reset);
 PCE_API int pce_debug_timeout(int32_t* where4);
 
 /* Parts per tile (1, 2, 4 or 8) that pce_conv_fwd uses for a tensor-core layer of n_rows outputs
- * gathered from n_src input rows when pce_epilogue.split is set; 1 = the layer is not split
- * into parts (large maps, layers with 16 or 32 input channels, short stage chains, up-sampling
- * layers: few pairs per output row). */
+ * gathered from n_src input rows through 128-row tile lists when pce_epilogue.split is set and none
+ * of its matrices is pushed to a neighbour or lies off a 16-byte boundary; 1 = the layer is not
+ * split into parts (large maps, short stage chains, up-sampling layers: few pairs per output row).
+ * Layers whose c_in is a multiple of 32 have 4 parts at most. */
 PCE_API int32_t pce_conv_split_parts(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out, int32_t kv,
                                      int32_t sm_count);
 
 /* Bytes of pce_epilogue.split_scratch that are enough for any split of a tensor-core layer of n_rows
- * outputs gathered from n_src input rows; 0 = the layer runs whole.  (Layers split into parts use
+ * outputs gathered from n_src input rows; 0 = the layer uses none.  (Layers split into parts use
  * none of it since version 104.) */
 PCE_API size_t pce_conv_split_scratch_bytes(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
 /* What the engine gives: the partial sums of layers cut into shares of stages, 0 where that was
- * measured slower than the whole layer or the layer is split into parts. */
+ * measured slower than the whole layer, the layer is split into parts or c_in is a multiple of 32. */
 PCE_API size_t pce_conv_split_scratch_wanted(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out,
                                             int32_t kv, int32_t sm_count);
 

@@ -2235,8 +2235,6 @@ int umma_half_blocks = 1;
 // when the caller asks for it (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
 int umma_split_enabled = 1;
 
-// Parts per tile for a layer of n_rows outputs (8, 4, 2 or 1; see the rule below).  Layers with 16 or 32 input channels
-// (shallow levels) are never split.
 // Estimated ring stages per tile: min(kv, 16) offsets x K blocks, fewer where the map has fewer source rows than
 // output rows (a transposed 2x2x2 layer has ONE pair per output row: its tiles list up to 8 offsets, each nearly
 // empty, and splitting them only adds the partial sums; measured 16 -> 30 us on 159 tiles of 128 -> 128).
@@ -2249,7 +2247,23 @@ static int chain_estimate(int n_rows, int n_src, int cin, int kv) {
   return static_cast<int>(offsets) * ((cin + 63) / 64);
 }
 
-int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
+// Input widths of k_conv_deep: whole K blocks, or a half block at the end (32 channels: one half block).
+static bool deep_widths(int cin) { return cin >= 32 && cin % 32 == 0; }
+
+// Parts per tile of k_conv_deep (4, 2 or 1): as long as every part has an SM to itself and a chain worth cutting.  Kernel
+// only, us, one / two / four parts: 256->256 on 24 tiles 39.3 / 27.6 / 20.4, on 60 tiles 38.2 / 27.5 / 34.4, on 94 tiles
+// 31.2 / 34.1; 128->128 on 24 tiles 16.9 / 14.2 / 11.9, on 60 tiles 16.9 / 14.5 / 21.1; 64->64 on 24 tiles 10.3 / 10.2 / 9.2, on
+// 60 tiles 10.4 / 10.4 / 16.8.  (Eight parts leave each a few stages: 256->256 on 24 tiles 30.5.)
+static int deep_split(int n_tiles, int n_out, int n_src, int cin, int kv, int sm_count) {
+  if (!umma_split_enabled) return 1;
+  const int chain = chain_estimate(n_out, n_src, cin, kv);
+  if (4ll * n_tiles <= sm_count && chain >= 16) return 4;
+  if (2ll * n_tiles <= sm_count && chain >= 32) return 2;
+  return 1;
+}
+
+// Parts per tile of k_conv_umma (8, 4, 2 or 1).  Layers with 16 input channels (shallow levels) are never split.
+static int umma_split(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   if (!umma_split_enabled || n_rows < 1) return 1;
   const int cin_p = (cin + 15) / 16 * 16;
   if (cin_p == 16 || cin_p == 32) return 1;
@@ -2272,7 +2286,14 @@ int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_co
   return 1;
 }
 
-// Maps of half a wave to one wave of tiles (tiles / CTA slots in (0.5, 1]) that conv_split_parts leaves
+// Parts per tile that conv_umma runs a layer with when its caller allows parts.
+int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
+  if (n_rows < 1) return 1;
+  if (deep_widths(cin)) return deep_split(div_up(n_rows, umma::kTileM), n_rows, n_src, cin, kv, sm_count > 0 ? sm_count : 148);
+  return umma_split(n_rows, n_src, cin, cout, kv, sm_count);
+}
+
+// Maps of half a wave to one wave of tiles (tiles / CTA slots in (0.5, 1]) that umma_split leaves
 // whole: CTAs take equal shares of the STAGES instead of whole tiles (stream-K), wherever the cuts fall, so
 // every CTA slot works for the same time instead of some running a whole chain while others idle.  A tile
 // that two or more CTAs worked on costs fp32 partial sums (written, then read by k_sum_cut_tiles), which is
@@ -2285,7 +2306,7 @@ int conv_streamk_grid(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
   if (!umma_split_enabled || umma_split_enabled == 2 || n_rows < 1) return 0;
   const int cin_p = (cin + 15) / 16 * 16;
   if (cin_p == 16 || cin_p == 32) return 0;
-  if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;
+  if (umma_split(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;
   const int chain = chain_estimate(n_rows, n_src, cin, kv);
   const long long n_tiles = (static_cast<long long>(n_rows) + umma::kTileM - 1) / umma::kTileM;
   const long long slots = static_cast<long long>(sm_count > 0 ? sm_count : 148) * (cout <= 128 ? 3 : 2);
@@ -2299,18 +2320,15 @@ int conv_streamk_grid(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   const int parts = conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count);
   if (parts > 1) return static_cast<size_t>(parts) * n_rows * cout * sizeof(float);
+  if (deep_widths(cin)) return 0;  // (k_conv_deep: shares three times as long leave little to balance)
   const int grid = conv_streamk_grid(n_rows, n_src, cin, cout, kv, sm_count);
   return grid > 0 ? static_cast<size_t>(grid) * 2 * umma::kTileM * cout * sizeof(float) : 0;
 }
-
-// Input widths of k_conv_deep: whole K blocks, or a half block at the end (32 channels: one half block).
-static bool deep_widths(int cin) { return cin >= 32 && cin % 32 == 0; }
 
 // The same where a split was measured faster; the framework's own callers ask this one.  Equal shares of stages repay
 // their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
 // 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
-  if (deep_widths((cin + 15) / 16 * 16)) return 0;  // (k_conv_deep: shares three times as long leave little to balance)
   if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;  // (parts add up in shared memory)
   if (chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
   return conv_split_scratch_bytes(n_rows, n_src, cin, cout, kv, sm_count);
@@ -2352,18 +2370,6 @@ static DeepKernel deep_kernel(bool half, int ring) {
       {umma::k_conv_deep<true, 4>, umma::k_conv_deep<true, 5>, umma::k_conv_deep<true, 6>, umma::k_conv_deep<true, 7>,
        umma::k_conv_deep<true, 8>, umma::k_conv_deep<true, 9>}};
   return table[half ? 1 : 0][ring - 4];
-}
-
-// Parts per tile of k_conv_deep (4, 2 or 1): as long as every part has an SM to itself and a chain worth cutting.  Kernel
-// only, us, one / two / four parts: 256->256 on 24 tiles 39.3 / 27.6 / 20.4, on 60 tiles 38.2 / 27.5 / 34.4, on 94 tiles
-// 31.2 / 34.1; 128->128 on 24 tiles 16.9 / 14.2 / 11.9, on 60 tiles 16.9 / 14.5 / 21.1; 64->64 on 24 tiles 10.3 / 10.2 / 9.2, on
-// 60 tiles 10.4 / 10.4 / 16.8.  (Eight parts leave each a few stages: 256->256 on 24 tiles 30.5.)
-static int deep_split(int n_tiles, int n_out, int n_src, int cin, int kv, int sm_count) {
-  if (!umma_split_enabled) return 1;
-  const int chain = chain_estimate(n_out, n_src, cin, kv);
-  if (4ll * n_tiles <= sm_count && chain >= 16) return 4;
-  if (2ll * n_tiles <= sm_count && chain >= 32) return 2;
-  return 1;
 }
 
 // tiles == nullptr: the dense rows x matrix product (every row fetches itself, one offset).
@@ -2597,7 +2603,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   bool streamk = false;
   const bool scratch = ep && ep->split_scratch && (reinterpret_cast<uintptr_t>(ep->split_scratch) & 15) == 0;
   if (tiles && sub == 1 && slots == 1 && !push && ep && (ep->split || scratch)) {
-    parts = conv_split_parts(n_out, n_in, cin, cout, kv, sm_count[dev]);
+    parts = umma_split(n_out, n_in, cin, cout, kv, sm_count[dev]);
     if (parts > 1) {
       grid = n_tiles * parts;
       e.parts = parts;

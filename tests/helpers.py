@@ -1,4 +1,8 @@
-"""Shared builders for the test-suite: seeded voxel clouds and oracle wrappers."""
+"""Shared builders for the test-suite: seeded voxel clouds, oracle wrappers and a list of launches."""
+import json
+import os
+import tempfile
+
 import numpy as np
 
 
@@ -28,3 +32,20 @@ def surface_cloud(seed, d, batch=1):
 
 def cmax_of(coords):
     return coords[:, 1:].max(0).tolist() if len(coords) else [0, 0, 0]
+
+
+def launches(f):
+    """[(kernel name, blocks along x), ...] of what f() launches, in the order of their start."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    f()  # (allocations, packed weights, kernel attributes)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as d:
+        prof.export_chrome_trace(os.path.join(d, "trace.json"))
+        with open(os.path.join(d, "trace.json")) as fh:
+            events = json.load(fh)["traceEvents"]
+    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    return [(e["name"], e["args"]["grid"][0]) for e in kernels]

@@ -35,6 +35,21 @@ def test_status_strings_and_size_queries_need_no_gpu():
             assert getattr(lib, name)(n) > 4 * n, (name, n)
 
 
+def test_split_queries_say_what_is_launched():
+    """Layers whose input width is a multiple of 32 run one CTA per SM: four parts a tile at most, no shares of stages.  The
+    others keep up to eight parts, and the scratch of shares on mid-size maps."""
+    from pcengine_b200._lib import lib
+    for cin in (32, 64, 96, 160, 256, 512):
+        for rows in (1, 127, 3072, 9500, 14208, 28416, 56832, 2 ** 31 - 1):
+            parts = lib.pce_conv_split_parts(rows, rows, cin, 256, 27, 148)
+            assert parts in (1, 2, 4) and (parts == 1 or parts * -(-rows // 128) <= 148), (cin, rows, parts)
+            assert lib.pce_conv_split_scratch_wanted(rows, rows, cin, 256, 27, 148) == 0
+            assert lib.pce_conv_split_scratch_bytes(rows, rows, cin, 256, 27, 148) == (parts * rows * 256 * 4 if parts > 1 else 0)
+    assert lib.pce_conv_split_parts(3072, 3072, 208, 256, 27, 148) == 8
+    assert lib.pce_conv_split_scratch_wanted(26000, 26000, 240, 256, 27, 148) > 0
+    assert lib.pce_conv_split_parts(3072, 3072, 16, 64, 27, 148) == 1
+
+
 def test_product_refuses_cpu_tensors():
     import pytest
     import torch

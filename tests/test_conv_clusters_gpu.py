@@ -7,14 +7,21 @@ import torch
 
 from oracle import conv_oracle as co
 from oracle import kmap_oracle as ko
-from tests.helpers import cmax_of, surface_cloud
+from tests.helpers import cmax_of, launches, surface_cloud
 
 pytestmark = [pytest.mark.gpu, pytest.mark.split_tiles]
 
 
-@pytest.mark.parametrize("n,cin,cout,parts", [(1, 64, 64, 4), (127, 96, 96, 8), (129, 128, 160, 8), (3072, 256, 256, 8), (3073, 256, 256, 4),
-                                              (9400, 64, 256, 4), (9500, 64, 256, 2), (14208, 128, 128, 4), (14209, 128, 128, 2),
-                                              (28416, 64, 64, 2), (28417, 64, 64, 1), (56832, 96, 96, 2), (56833, 96, 96, 1)])
+# one CTA per SM (widths that are multiples of 32): 37 | 38 tiles of the 148 SMs hold four parts each, 74 | 75 two
+_DEEP = [(1, 64, 64, 4), (127, 96, 96, 4), (129, 128, 160, 4), (3072, 256, 256, 4), (3073, 256, 256, 4), (4736, 64, 64, 4), (4737, 64, 64, 1),
+         (4736, 96, 32, 4), (4737, 96, 32, 2), (9400, 64, 256, 1), (9472, 192, 48, 2), (9473, 192, 48, 1), (9500, 64, 256, 1),
+         (14208, 128, 128, 1), (28416, 64, 64, 1), (56832, 96, 96, 1)]
+# two or three (the others): 24 | 25 tiles eight parts, 444 (296 beyond 128 output channels) CTA slots four and two
+_UMMA = [(1, 48, 64, 4), (127, 80, 96, 8), (129, 112, 160, 8), (3072, 208, 256, 8), (3073, 208, 256, 4), (9472, 80, 256, 4), (9473, 80, 256, 2),
+         (14208, 144, 128, 4), (14209, 144, 128, 2), (28416, 80, 64, 2), (28417, 80, 64, 1)]
+
+
+@pytest.mark.parametrize("n,cin,cout,parts", _DEEP + _UMMA)
 def test_parts_of_a_tile(n, cin, cout, parts):
     import pcengine_b200 as pce
     from pcengine_b200 import _lib
@@ -32,6 +39,11 @@ def test_parts_of_a_tile(n, cin, cout, parts):
     ep = PF.FusedEpilogue(shift=shift.cuda(), residual=res.cuda(), act="relu")
     outs = [PF.conv_forward(x.cuda(), w.cuda(), km.csr(), ep) for _ in range(2)]
     assert torch.equal(*outs) and co.rel_l2(outs[0].float().cpu(), want) <= 1e-3
+    if sms == 148:  # what the library says is what it launches
+        xd, wd, tiles = x.cuda(), w.cuda(), -(-n // 128)
+        (name, blocks), = launches(lambda: PF.conv_forward(xd, wd, km.csr(), ep))
+        assert ("k_conv_deep" if cin % 32 == 0 else "k_conv_umma") in name
+        assert blocks == parts * tiles if parts > 1 else blocks <= tiles
     assert PF.device_status() == 0
 
 

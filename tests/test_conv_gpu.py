@@ -6,7 +6,7 @@ import torch
 
 from oracle import conv_oracle as co
 from oracle import kmap_oracle as ko
-from tests.helpers import cmax_of, random_cloud, surface_cloud
+from tests.helpers import cmax_of, launches, random_cloud, surface_cloud
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.float32: 1e-5, torch.float16: 1e-3}
@@ -615,6 +615,7 @@ def _split_layer_case(cin, cout, n_side, ks, stream_k):
     scratch = _lib.lib.pce_conv_split_scratch_bytes(csr.n_rows, n, cin, cout, ks ** 3, sms)
     if stream_k:
         assert parts == 1 and scratch > 0, "the case is meant to be cut into shares of stages"
+        assert _lib.lib.pce_conv_split_scratch_bytes(csr.n_rows, n, (cin + 31) // 32 * 32, cout, ks ** 3, sms) == 0
     else:
         assert parts > 1 and scratch == parts * csr.n_rows * cout * 4, "the case is meant to be split into parts"
     g = torch.Generator().manual_seed(cin + cout + n_side)
@@ -641,11 +642,14 @@ def _split_layer_case(cin, cout, n_side, ks, stream_k):
         finally:
             PF.SPLIT_TILES = True
         assert co.rel_l2(a.float().cpu(), whole.float().cpu()) <= 5e-4  # same products, another fp32 association
+    names = [name for name, _ in launches(lambda: PF.conv_forward(x.cuda(), w.cuda(), csr, eps[1]))]
+    assert any("k_sum_cut_tiles" in name for name in names) == stream_k
     assert PF.device_status() == 0
 
 
 @pytest.mark.split_tiles
-@pytest.mark.parametrize("cin,cout,n_side,ks", [(256, 256, 20, 3), (128, 256, 30, 3), (96, 96, 48, 3), (128, 128, 26, 5), (256, 128, 24, 2)])
+@pytest.mark.parametrize("cin,cout,n_side,ks", [(256, 256, 20, 3), (128, 256, 30, 3), (96, 96, 48, 3), (128, 128, 26, 5), (256, 128, 24, 2),
+                                                (240, 256, 20, 3), (48, 96, 48, 3), (80, 128, 26, 5), (240, 128, 24, 2)])
 def test_small_maps_split_over_several_ctas(cin, cout, n_side, ks):
     """A map with few 128-row tiles runs with a cluster of CTAs per tile: every CTA takes a part of the tile's
     stage list, the fp32 sums are added in order through the cluster's shared memory and finished with the epilogue
@@ -655,12 +659,13 @@ def test_small_maps_split_over_several_ctas(cin, cout, n_side, ks):
 
 
 @pytest.mark.split_tiles
-@pytest.mark.parametrize("cin,cout,n_side,ks", [(256, 256, 128, 3), (192, 96, 150, 3), (384, 256, 110, 3), (64, 64, 140, 3)])
+@pytest.mark.parametrize("cin,cout,n_side,ks", [(240, 256, 128, 3), (176, 96, 150, 3), (400, 256, 110, 3), (48, 64, 140, 3)])
 def test_mid_size_maps_cut_into_equal_shares_of_stages(cin, cout, n_side, ks, monkeypatch):
     """A map of half a wave to one wave of tiles with long stage chains is cut into equal shares of ring stages, one share per CTA slot,
     wherever the cuts fall inside the tiles; tiles that two or more CTAs worked on are summed in CTA order
     and finished by a second kernel.  Same checks as for the split into parts.  (The engine gives the scratch for
-    this to layers with chains of 48 stages and more; here every layer gets it that can be cut.)"""
+    this to layers with chains of 48 stages and more; here every layer gets it that can be cut.  Input widths that are
+    multiples of 32 never are: they run one CTA per SM.)"""
     from pcengine_b200 import _lib
     from pcengine_b200 import functional as PF
     given = []
