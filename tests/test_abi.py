@@ -50,6 +50,20 @@ def test_split_queries_say_what_is_launched():
     assert lib.pce_conv_split_parts(3072, 3072, 16, 64, 27, 148) == 1
 
 
+def test_parts_of_long_and_of_short_chains():
+    """Layers of 125 offsets are cut beyond one SM per part, and layers up a level, one pair per row, are not cut at all."""
+    from pcengine_b200._lib import lib
+
+    def parts(rows, src, cin, cout, kv):
+        return lib.pce_conv_split_parts(rows, src, cin, cout, kv, 148)
+    assert parts(11000, 11000, 256, 32, 125) == 4 and parts(10476, 10476, 96, 128, 125) == 2
+    assert parts(12766, 12766, 96, 96, 125) == 2 and parts(16000, 16000, 256, 64, 125) == 1
+    assert parts(5000, 5000, 64, 16, 125) == 2 and parts(10778, 10778, 64, 16, 125) == 1
+    assert parts(4376, 4265, 160, 16, 8) == 1 and parts(4376, 4265, 256, 256, 8) == 1 and parts(3428, 2600, 192, 192, 8) == 1
+    assert parts(7080, 9668, 192, 48, 8) == 2 and parts(4167, 5412, 128, 48, 8) == 1 and parts(4167, 5412, 192, 192, 8) == 1
+    assert parts(4500, 4500, 128, 128, 27) == 2 and parts(4096, 4096, 128, 128, 27) == 4  # (clusters of four: 33 fit 148 SMs)
+
+
 def test_product_refuses_cpu_tensors():
     import pytest
     import torch

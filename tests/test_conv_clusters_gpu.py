@@ -12,28 +12,31 @@ from tests.helpers import cmax_of, launches, surface_cloud
 pytestmark = [pytest.mark.gpu, pytest.mark.split_tiles]
 
 
-# one CTA per SM (widths that are multiples of 32): 37 | 38 tiles of the 148 SMs hold four parts each, 74 | 75 two
-_DEEP = [(1, 64, 64, 4), (127, 96, 96, 4), (129, 128, 160, 4), (3072, 256, 256, 4), (3073, 256, 256, 4), (4736, 64, 64, 4), (4737, 64, 64, 1),
-         (4736, 96, 32, 4), (4737, 96, 32, 2), (9400, 64, 256, 1), (9472, 192, 48, 2), (9473, 192, 48, 1), (9500, 64, 256, 1),
-         (14208, 128, 128, 1), (28416, 64, 64, 1), (56832, 96, 96, 1)]
+# one CTA per SM (widths that are multiples of 32): 32 | 33 tiles have four parts each, 74 | 75 two; with 125 offsets 88 | 89 four
+# from three K blocks on and 111 | 112 two from two on
+_DEEP = [(1, 64, 64, 3, 4), (127, 96, 96, 3, 4), (129, 128, 160, 3, 4), (3072, 256, 256, 3, 4), (4096, 64, 64, 3, 4), (4097, 64, 64, 3, 1),
+         (4096, 96, 32, 3, 4), (4097, 96, 32, 3, 2), (9400, 64, 256, 3, 1), (9472, 192, 48, 3, 2), (9473, 192, 48, 3, 1), (9500, 64, 256, 3, 1),
+         (14208, 128, 128, 3, 1), (28416, 64, 64, 3, 1), (56832, 96, 96, 3, 1),
+         (4096, 64, 32, 5, 4), (4097, 32, 64, 5, 2), (9472, 64, 256, 5, 2), (9473, 64, 32, 5, 1), (9473, 160, 32, 5, 4), (11264, 192, 64, 5, 4),
+         (11265, 160, 48, 5, 2), (14208, 96, 128, 5, 2), (14209, 96, 16, 5, 1)]
 # two or three (the others): 24 | 25 tiles eight parts, 444 (296 beyond 128 output channels) CTA slots four and two
-_UMMA = [(1, 48, 64, 4), (127, 80, 96, 8), (129, 112, 160, 8), (3072, 208, 256, 8), (3073, 208, 256, 4), (9472, 80, 256, 4), (9473, 80, 256, 2),
-         (14208, 144, 128, 4), (14209, 144, 128, 2), (28416, 80, 64, 2), (28417, 80, 64, 1)]
+_UMMA = [(1, 48, 64, 3, 4), (127, 80, 96, 3, 8), (129, 112, 160, 3, 8), (3072, 208, 256, 3, 8), (3073, 208, 256, 3, 4), (9472, 80, 256, 3, 4),
+         (9473, 80, 256, 3, 2), (14208, 144, 128, 3, 4), (14209, 144, 128, 3, 2), (28416, 80, 64, 3, 2), (28417, 80, 64, 3, 1)]
 
 
-@pytest.mark.parametrize("n,cin,cout,parts", _DEEP + _UMMA)
-def test_parts_of_a_tile(n, cin, cout, parts):
+@pytest.mark.parametrize("n,cin,cout,ks,parts", _DEEP + _UMMA)
+def test_parts_of_a_tile(n, cin, cout, ks, parts):
     import pcengine_b200 as pce
     from pcengine_b200 import _lib
     from pcengine_b200 import functional as PF
     coords = np.ascontiguousarray(surface_cloud(8, int(n ** 0.5 * 1.2) + 2)[:n])
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     if sms == 148:
-        assert _lib.lib.pce_conv_split_parts(n, n, cin, cout, 27, sms) == parts
-    d2 = ko.build_d2(coords, (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
-    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (3,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
+        assert _lib.lib.pce_conv_split_parts(n, n, cin, cout, ks ** 3, sms) == parts
+    d2 = ko.build_d2(coords, (ks,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
+    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (ks,) * 3, (1,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), True)
     g = torch.Generator().manual_seed(n + cin)
-    x, w = torch.randn(n, cin, generator=g).half(), (torch.randn(27, cin, cout, generator=g) / (27 * cin) ** 0.5).half()
+    x, w = torch.randn(n, cin, generator=g).half(), (torch.randn(ks ** 3, cin, cout, generator=g) / (ks ** 3 * cin) ** 0.5).half()
     shift, res = torch.randn(cout, generator=g), torch.randn(n, cout, generator=g).half()
     want = torch.relu(co.conv_forward(x, w, d2) + shift + res.float())
     ep = PF.FusedEpilogue(shift=shift.cuda(), residual=res.cuda(), act="relu")
