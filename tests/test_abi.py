@@ -56,8 +56,8 @@ def test_parts_of_long_and_of_short_chains():
 
     def parts(rows, src, cin, cout, kv):
         return lib.pce_conv_split_parts(rows, src, cin, cout, kv, 148)
-    assert parts(11000, 11000, 256, 32, 125) == 4 and parts(10476, 10476, 96, 128, 125) == 2
-    assert parts(12766, 12766, 96, 96, 125) == 2 and parts(16000, 16000, 256, 64, 125) == 1
+    assert parts(11000, 11000, 256, 32, 125) == 2 and parts(10476, 10476, 96, 128, 125) == 2
+    assert parts(12544, 12544, 96, 96, 125) == 2 and parts(12545, 12545, 256, 64, 125) == 1
     assert parts(5000, 5000, 64, 16, 125) == 2 and parts(10778, 10778, 64, 16, 125) == 1
     assert parts(4376, 4265, 160, 16, 8) == 1 and parts(4376, 4265, 256, 256, 8) == 1 and parts(3428, 2600, 192, 192, 8) == 1
     assert parts(7080, 9668, 192, 48, 8) == 2 and parts(4167, 5412, 128, 48, 8) == 1 and parts(4167, 5412, 192, 192, 8) == 1
