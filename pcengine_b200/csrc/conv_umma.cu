@@ -2254,10 +2254,11 @@ static bool deep_widths(int cin) { return cin >= 32 && cin % 32 == 0; }
 // only, us, one / two / four parts: 256->256 on 24 tiles 39.3 / 27.6 / 20.4, on 60 tiles 38.2 / 27.5 / 34.4, on 94 tiles
 // 31.2 / 34.1; 128->128 on 24 tiles 16.9 / 14.2 / 11.9, on 60 tiles 16.9 / 14.5 / 21.1; 64->64 on 24 tiles 10.3 / 10.2 / 9.2, on
 // 60 tiles 10.4 / 10.4 / 16.8.  (Eight parts leave each a few stages: 256->256 on 24 tiles 30.5.)
-// * Clusters of four find their SMs inside one GPC: 33 of them fit 148 SMs, not 37 (64->48 on 35 tiles 8.6 / - / 12.8).
-// * At most 8 offsets (down and up a level): a row has few of them, one going up, so a part is a few stages; parts going down only,
-//   from three K blocks on (160->16 on 17 tiles - / 7.4 / 6.8, 192->48 on 56 8.4 / 7.7 / 14.8; 128->32 on 17 5.8 / 5.8 / 6.2), two of them for
-//   narrow outputs or four K blocks (256->64 on 46 tiles 8.4 / 8.2; 192->192 on 33 8.2 / 9.8).
+// * Clusters of four find their SMs inside one GPC: 33 of them fit 148 SMs, not 37 (64->48 on 35 tiles 8.6 / - / 12.8; 5x5x5 64->160 on 33 tiles
+//   - / 18.0 / 15.1).
+// * At most 8 offsets (down and up a level): a row has few of them, one going up, so a part is a few stages.  None going up; two
+//   going down need four K blocks, or three and narrow outputs (192->48 on 56 tiles 8.4 / 7.7 / 14.8, 256->64 on 46 8.4 / 8.2; 192->192 on 33
+//   8.2 / 9.8).
 // * More than 32 offsets: tiles at the end of the order have 125 where most have 20 to 50, and the layer lasts as long as
 //   the longest chain, so cutting pays beyond an SM per part.  One K block (64->32): 67 tiles 17.7 / 11.7 / 18.7, 100 tiles 18.6 /
 //   19.3.  More: 37 tiles 192->192 56 / 32.6 / 29.9, rooms of 82 tiles 96->128 49.5 / 36.7 / 34.3 and 256->48 68.4 / 44.2 / 36.2, a uniform
@@ -2269,13 +2270,9 @@ static int deep_split(int n_tiles, int n_out, int n_src, int cin, int cout, int 
   const int chain = chain_estimate(n_out, n_src, cin, kv), kblocks = (cin + 63) / 64;
   const long long t = n_tiles;
   const bool two = 2 * t <= sm_count;
-  const bool four = 9 * t <= 2 * sm_count;
-  if (kv <= 8) {
-    if (n_src <= n_out || chain < 24) return 1;
-    return four ? 4 : (two && (chain >= 32 || cout <= 64) ? 2 : 1);
-  }
-  if (chain < 16) return 1;
-  if (four) return 4;
+  if (chain < 16 || (kv <= 8 && n_src <= n_out)) return 1;
+  if (40 * t <= 9 * sm_count) return 4;
+  if (kv <= 8) return two && (chain >= 32 || (chain >= 24 && cout <= 64)) ? 2 : 1;
   if (kv <= 32) return two && chain >= 32 ? 2 : 1;
   if (kblocks == 1) return two ? 2 : 1;
   return 4 * t <= sm_count ? 4 : (3 * t <= 2 * sm_count ? 2 : 1);

@@ -60,8 +60,8 @@ def test_parts_of_long_and_of_short_chains():
     assert parts(12544, 12544, 96, 96, 125) == 2 and parts(12545, 12545, 256, 64, 125) == 1
     assert parts(5000, 5000, 64, 16, 125) == 2 and parts(10778, 10778, 64, 16, 125) == 1
     assert parts(4376, 4265, 160, 16, 8) == 1 and parts(4376, 4265, 256, 256, 8) == 1 and parts(3428, 2600, 192, 192, 8) == 1
-    assert parts(7080, 9668, 192, 48, 8) == 2 and parts(4167, 5412, 128, 48, 8) == 1 and parts(4167, 5412, 192, 192, 8) == 1
-    assert parts(4500, 4500, 128, 128, 27) == 2 and parts(4096, 4096, 128, 128, 27) == 4  # (clusters of four: 33 fit 148 SMs)
+    assert parts(7080, 9668, 192, 48, 8) == 2 and parts(4400, 5412, 128, 48, 8) == 1 and parts(4400, 5412, 192, 192, 8) == 1
+    assert parts(4500, 4500, 128, 128, 27) == 2 and parts(4224, 4224, 128, 128, 27) == 4  # (clusters of four: 33 fit 148 SMs)
 
 
 def test_product_refuses_cpu_tensors():

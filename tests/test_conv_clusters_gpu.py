@@ -12,12 +12,12 @@ from tests.helpers import cmax_of, launches, surface_cloud
 pytestmark = [pytest.mark.gpu, pytest.mark.split_tiles]
 
 
-# one CTA per SM (widths that are multiples of 32): 32 | 33 tiles have four parts each, 74 | 75 two; with 125 offsets 37 | 38 four and
+# one CTA per SM (widths that are multiples of 32): 33 | 34 tiles have four parts each, 74 | 75 two; with 125 offsets 37 | 38 four and
 # 98 | 99 two from two K blocks on
-_DEEP = [(1, 64, 64, 3, 4), (127, 96, 96, 3, 4), (129, 128, 160, 3, 4), (3072, 256, 256, 3, 4), (4096, 64, 64, 3, 4), (4097, 64, 64, 3, 1),
-         (4096, 96, 32, 3, 4), (4097, 96, 32, 3, 2), (9400, 64, 256, 3, 1), (9472, 192, 48, 3, 2), (9473, 192, 48, 3, 1), (9500, 64, 256, 3, 1),
+_DEEP = [(1, 64, 64, 3, 4), (127, 96, 96, 3, 4), (129, 128, 160, 3, 4), (3072, 256, 256, 3, 4), (4224, 64, 64, 3, 4), (4225, 64, 64, 3, 1),
+         (4224, 96, 32, 3, 4), (4225, 96, 32, 3, 2), (9400, 64, 256, 3, 1), (9472, 192, 48, 3, 2), (9473, 192, 48, 3, 1), (9500, 64, 256, 3, 1),
          (14208, 128, 128, 3, 1), (28416, 64, 64, 3, 1), (56832, 96, 96, 3, 1),
-         (4096, 64, 32, 5, 4), (4097, 32, 64, 5, 2), (4736, 96, 48, 5, 4), (4737, 96, 48, 5, 2), (9472, 64, 256, 5, 2), (9473, 64, 32, 5, 1),
+         (4224, 64, 32, 5, 4), (4225, 32, 64, 5, 2), (4736, 96, 48, 5, 4), (4737, 96, 48, 5, 2), (9472, 64, 256, 5, 2), (9473, 64, 32, 5, 1),
          (9473, 160, 32, 5, 2), (12544, 96, 128, 5, 2), (12545, 96, 16, 5, 1)]
 # two or three (the others): 24 | 25 tiles eight parts, 444 (296 beyond 128 output channels) CTA slots four and two
 _UMMA = [(1, 48, 64, 3, 4), (127, 80, 96, 3, 8), (129, 112, 160, 3, 8), (3072, 208, 256, 3, 8), (3073, 208, 256, 3, 4), (9472, 80, 256, 3, 4),
