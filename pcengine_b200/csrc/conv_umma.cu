@@ -2250,6 +2250,26 @@ static int chain_estimate(int n_rows, int n_src, int cin, int kv) {
 // Input widths of k_conv_deep: whole K blocks, or a half block at the end (32 channels: one half block).
 static bool deep_widths(int cin) { return cin >= 32 && cin % 32 == 0; }
 
+// Layers of 32 input channels that k_conv_umma runs faster: it takes two offsets to a stage, which is half the
+// stages, and up to four CTAs per SM, where a layer's set-up weighs.  Kernel only, us, k_conv_umma / k_conv_deep:
+// * down and up a level (at most 8 offsets): 32->16 and 32->32 4.1 / 5.2 on 94 tiles, 5.6 / 7.0 on 326, 32->48 4.4 / 5.3 on 108, 42.7 / 46.7
+//   on 5659 (on the way up 16.3 / 17.7 on 2415, 42.0 / 39.3 on 5434), 32->96 4.4 / 5.1 on 35 but 7.0 / 6.4 on 500; with one to three tiles per SM
+//   also 32->64 (7.5 / 8.0 on 225) and on the way up 32->128 (6.2 / 7.4 on 199, 7.2 / 8.0 on 326).  (64->128 up: rooms 7.6 / 9.0 on 440, scans
+//   9.0 / 8.4 on 426.)
+// * other strided kernels that leave fewer rows: 32->32 6.8 / 8.8 on 279 tiles, 32->48 16.6 / 21.1 on 1781, but 7.7 / 7.2 on 104; 32->64
+//   22.0 / 23.9 on 1820, but 20.9 / 18.8 on 233.
+// * all others from five tiles per SM on: 32->32 15.7 / 17.1 on 938, 31.5 / 46.8 on 3750, but 32->48 16.5 / 14.5 on 798 (45.8 / 48.8 on 4322),
+//   5x5x5 51.0 / 42.7 on 1489, 32->64 19.1 / 17.5 on 938.  Below that it depends on the cloud: 3x3x3 32->16 16.5 / 21.3 on 439 tiles of a
+//   uniform one, 12.7 / 10.4 on 436 of a room.
+static bool umma_faster(int n_out, int n_in, int cin, int cout, int kv, int sm_count) {
+  const long long t = div_up(n_out, umma::kTileM), sms = sm_count;
+  const bool mid = t > sms && t <= 3 * sms, many = t > 5 * sms;
+  if (cin != 32) return false;
+  if (kv <= 8) return cout <= 32 || (cout <= 48 && (n_in > n_out || t <= 16 * sms)) || (mid && cout <= (n_in < n_out ? 192 : 64));
+  if (n_in > n_out) return (cout <= 48 && t > sms) || (cout <= 64 && many);
+  return many && cout <= 32;
+}
+
 // Parts per tile of k_conv_deep (4, 2 or 1): as long as every part has an SM to itself and a chain worth cutting.  Kernel
 // only, us, one / two / four parts: 256->256 on 24 tiles 39.3 / 27.6 / 20.4, on 60 tiles 38.2 / 27.5 / 34.4, on 94 tiles
 // 31.2 / 34.1; 128->128 on 24 tiles 16.9 / 14.2 / 11.9, on 60 tiles 16.9 / 14.5 / 21.1; 64->64 on 24 tiles 10.3 / 10.2 / 9.2, on
@@ -2305,7 +2325,8 @@ static int umma_split(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
 // Parts per tile that conv_umma runs a layer with when its caller allows parts.
 int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   if (n_rows < 1) return 1;
-  if (deep_widths(cin)) return deep_split(div_up(n_rows, umma::kTileM), n_rows, n_src, cin, cout, kv, sm_count > 0 ? sm_count : 148);
+  if (deep_widths(cin) && !umma_faster(n_rows, n_src, cin, cout, kv, sm_count > 0 ? sm_count : 148))
+    return deep_split(div_up(n_rows, umma::kTileM), n_rows, n_src, cin, cout, kv, sm_count > 0 ? sm_count : 148);
   return umma_split(n_rows, n_src, cin, cout, kv, sm_count);
 }
 
@@ -2546,10 +2567,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   // One CTA per SM wherever its producers can take the layer (k_conv_deep); the tuning hooks below are k_conv_umma's.
   const bool pairs = slots == 2;  // 32 input channels: a half block per offset there, two offsets to a stage below
   const bool deep_half = umma_half_blocks && !kb64_slice && cin % 64 == 32;
-  // Two narrow offsets to a stage are half the stages, which counts once a map has more than about five tiles per SM and the
-  // outputs are narrow too.  Kernel only, us, k_conv_umma / k_conv_deep: 32->32 on 60 k rows 12.7 / 11.3, on 120 k 15.7 / 17.1,
-  // on 480 k 31.5 / 46.8; 32->64 on 60 k 14.9 / 11.7, on 120 k 19.1 / 17.5, on 480 k 49.4 / 46.9.
-  const bool packed = pairs && cout <= 32 && div_up(n_out, umma::kTileM) > 5 * sm_count[dev];
+  const bool packed = pairs && umma_faster(n_out, n_in, cin, cout, kv, sm_count[dev]);
   if (!packed && (slots == 1 ? sub == 1 : pairs) && !(e.push_slot[0] || e.push_slot[1]) && deep_widths(cin) && (cin % 64 == 0 || deep_half) && !off16(in) &&
       !off16(ls.stage_nbr) && !umma_force_stages && !umma_force_nacc && umma_split_enabled != 3) {
     umma::Lists dl = ls;

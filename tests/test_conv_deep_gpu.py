@@ -6,7 +6,7 @@ import torch
 
 from oracle import conv_oracle as co
 from oracle import kmap_oracle as ko
-from tests.helpers import cmax_of, random_cloud, surface_cloud
+from tests.helpers import cmax_of, launches, random_cloud, surface_cloud
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +110,27 @@ def test_values_of_absent_rows_do_not_leak():
     assert torch.equal(torch.isfinite(got), torch.isfinite(want))
     ok = torch.isfinite(want).all(1)
     assert co.rel_l2(got[ok], want[ok]) <= 5e-4
+
+
+# the limits of the rule for 32 input channels: one, three and five tiles per SM, widths, and layers between two levels
+@pytest.mark.parametrize("way,n,cout,kernel", [
+    ("up", 129, 48, "umma"), ("up", 129, 64, "deep"), ("up", 20000, 64, "umma"), ("up", 20000, 192, "umma"), ("up", 20000, 208, "deep"),
+    ("down", 20000, 48, "umma"), ("down", 20000, 64, "deep"), ("down", 40000, 64, "umma"),
+    ("same", 30000, 16, "deep"), ("same", 94720, 32, "deep"), ("same", 94721, 32, "umma"), ("same", 94721, 48, "deep")])
+def test_narrow_layers_run_on_the_faster_kernel(way, n, cout, kernel):
+    import pcengine_b200 as pce
+    from pcengine_b200 import functional as PF
+    coords = np.ascontiguousarray(surface_cloud(9, int(n ** 0.5 * 1.2) + 2)[:n])
+    ks, st, same = (3, 1, True) if way == "same" else (2, 2, False)
+    d2 = ko.build_d2(coords, (ks,) * 3, (st,) * 3, (0,) * 3, [0] * 3, cmax_of(coords), same)
+    km = pce.KernelMap(torch.from_numpy(coords).cuda(), (ks,) * 3, (st,) * 3, (0,) * 3, [0] * 3, d2["cmax_out"], same)
+    csr = km.csr(transposed=way == "up")
+    g = torch.Generator().manual_seed(n + cout)
+    x, w = torch.randn(csr.n_src, 32, generator=g).half(), (torch.randn(ks ** 3, 32, cout, generator=g) / (ks ** 3 * 32) ** 0.5).half()
+    xd, wd = x.cuda(), w.cuda()
+    got = PF.conv_forward(xd, wd, csr)
+    assert co.rel_l2(got.float().cpu(), co.conv_forward(x, w, d2, transposed=way == "up")) <= 5e-4
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        (name, _), = launches(lambda: PF.conv_forward(xd, wd, csr))
+        assert "k_conv_" + kernel in name
+    assert PF.device_status() == 0
