@@ -150,7 +150,7 @@ struct LevelState {
   int ready = 0;             // host side: n is known, ev is recorded (guarded by plan->m)
 };
 
-// Map lanes of passes that run in one call: one scan 890 us with two, 862 with three, 855 with four; eight scans 2300, 2271,
+// Map lanes of passes that run in one call (as the pass used before did): one scan 890 us with two, 862 with three, 855 with four; eight scans 2300, 2271,
 // 2257.  Where a network runs layer by layer its launches and the lanes' wait for one another in the driver, and two are
 // enough (fp32 network of half width, rooms of 8 k / 16 k / 30 k voxels: 1893 / 1932 / 2013 us with two, 1952 / 1993 / 2029 with
 // four).
@@ -180,6 +180,7 @@ struct pce_pass {
   int lanes_done = 0;
   int error = PCE_OK;
   bool finished = false;
+  bool one_call = false;                   // pce_net_run has run it
 
   void* take(size_t bytes) {
     std::lock_guard<std::mutex> lk(arena_m);
@@ -214,7 +215,7 @@ struct pce_plan {
   std::condition_variable cv;
   std::deque<pce_pass*> idle;  // released passes (arena + events), oldest first
   int n_passes = 0;            // pass objects created so far
-  bool one_call = false;       // pce_net_run has run one of them
+  bool one_call = false;       // the pass last used ran in one call (pce_net_run)
   bool stop = false;
 };
 
@@ -865,6 +866,7 @@ int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t*
   ps->lanes_done = 0;
   ps->error = PCE_OK;
   ps->finished = false;
+  ps->one_call = false;
   // everything queued on `stream` so far (the coordinates' producer) precedes the planner's
   // first kernel
   cudaError_t e = cudaEventRecord(ps->start, static_cast<cudaStream_t>(stream));
@@ -885,6 +887,10 @@ int pce_plan_begin(pce_plan* p, const int32_t* coords, int32_t n, const int32_t*
 int pce_pass_map(pce_pass* ps, int32_t index, void* stream, pce_planned_map* out) {
   if (!ps || !out || index < 0 || index >= static_cast<int32_t>(ps->maps.size())) return PCE_ERR_INVALID;
   pce_plan* p = ps->plan;
+  {
+    std::lock_guard<std::mutex> lk(p->m);
+    p->one_call = ps->one_call;
+  }
   // the lane is usually microseconds away: a short poll before the sleep, whose wake-up alone takes 20 to 50 us
   for (const auto t0 = std::chrono::steady_clock::now(); std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(100);) {
     {
@@ -1058,7 +1064,7 @@ int pce_net_run(pce_pass* ps, const pce_net_buffer* buffers, int32_t n_buffers, 
   // 3.93 -> 3.98 ms per 8-scan step beside the next pass's map construction, no change on 1 or 2 scans.)
   {
     std::lock_guard<std::mutex> lk(ps->plan->m);
-    ps->plan->one_call = true;
+    ps->plan->one_call = ps->one_call = true;
   }
   return net_run_on(ps, buffers, n_buffers, ops, n_ops, input, in_ld, output, out_ld, arena, arena_bytes, dtype,
                     static_cast<cudaStream_t>(stream));

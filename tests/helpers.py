@@ -34,11 +34,10 @@ def cmax_of(coords):
     return coords[:, 1:].max(0).tolist() if len(coords) else [0, 0, 0]
 
 
-def launches(f):
-    """[(kernel name, blocks along x), ...] of what f() launches, in the order of their start."""
+def traced(f):
+    """The kernels that f() launches, as the profiler's events in the order of their start."""
     import torch
     from torch.profiler import ProfilerActivity, profile
-    f()  # (allocations, packed weights, kernel attributes)
     torch.cuda.synchronize()
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         f()
@@ -47,5 +46,10 @@ def launches(f):
         prof.export_chrome_trace(os.path.join(d, "trace.json"))
         with open(os.path.join(d, "trace.json")) as fh:
             events = json.load(fh)["traceEvents"]
-    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
-    return [(e["name"], e["args"]["grid"][0]) for e in kernels]
+    return sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+
+
+def launches(f):
+    """[(kernel name, blocks along x), ...] of a repeated f()."""
+    f()  # (allocations, packed weights, kernel attributes)
+    return [(e["name"], e["args"]["grid"][0]) for e in traced(f)]

@@ -5,7 +5,7 @@ import torch
 
 from oracle import conv_oracle as co
 from oracle import minkunet_oracle as mo
-from tests.helpers import cmax_of, surface_cloud
+from tests.helpers import cmax_of, surface_cloud, traced
 
 pytestmark = pytest.mark.gpu
 
@@ -322,6 +322,38 @@ def test_one_call_pass_equals_the_layer_by_layer_pass():
         assert torch.equal(got2.feats, want2.feats) and not torch.equal(got2.feats, want.feats)
     from pcengine_b200 import functional as PF
     assert PF.device_status() == 0
+
+
+def test_map_lanes_follow_the_way_the_pass_before_ran():
+    """A plan whose passes ran in one call and then run layer by layer goes back to two map lanes: kernels on the caller's
+    stream, on the coordinates' and on two more.  A pass that is planned and dropped, and maps looked at after a one-call
+    pass, change nothing."""
+    import pcengine_b200 as pce
+    coords = surface_cloud(61, 90, batch=2)
+    model = pce.MinkUNet(4, 19, cr=0.5)
+    pce.randomize_batchnorm(model, 5)
+    model = model.half().eval().cuda()
+    feats = torch.randn(len(coords), 4).half().cuda()
+
+    def tensor():
+        return pce.spTensor(feats, torch.from_numpy(coords).cuda(), None, [0, 0, 0], cmax_of(coords), batchsize=2,
+                            init_tag=pce.MinkUNet.tags())
+
+    def streams():
+        return len({e["args"]["stream"] for e in traced(lambda: model(tensor()))})
+    with torch.no_grad():
+        for _ in range(4):
+            model(tensor())
+        x = tensor()
+        assert model.plan(x) and len(model(tensor()).kmaps) == 9
+        del x
+        assert max(streams() for _ in range(3)) > 4
+        model.one_call = False
+        model(tensor())
+        assert max(streams() for _ in range(3)) <= 4
+        model.one_call = True
+        model(tensor())
+        assert max(streams() for _ in range(3)) > 4
 
 
 def test_planner_routes_build_the_same_lists():
