@@ -509,7 +509,14 @@ static int build_direction(pce_plan* p, PlanLane* l, pce_pass* ps, blk::Order o,
   if (o.n_variants == 0 || o.n == 0) return PCE_OK;
   o.order = ps->take_n<int32_t>(o.n);
   if (!o.order) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
-  if (!l->order_ws) return PCE_ERR_INVALID;  // (only passes in block form come here)
+  // The row orders' scratch comes out of the pass's arena, when a lane's first map wants it or a larger one comes: a lane gets
+  // other maps in every pass, and scratch of its own would grow, with a stop to free and to allocate, until it has had them all.
+  const size_t need = blk::order_workspace_bytes(o.n);
+  if (l->order_bytes < need) {
+    l->order_ws = ps->take(need);
+    if (!l->order_ws) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
+    l->order_bytes = need;
+  }
   PCE_TRY(blk::order_lists(o, l->order_ws, l->order_bytes, false, l->stream));
   for (int v = 0; v < o.n_variants; ++v) {
     const blk::Variant& V = o.variant[v];
@@ -667,14 +674,7 @@ static int run_map_lane(pce_plan* p, PlanLane* l, pce_pass* ps) {
     if (!p->one_call) return PCE_OK;
   }
   l->order_ws = nullptr;
-  if (p->chain && plan_short_route) {
-    // The row orders' scratch comes with the pass, for the largest of its maps (no level has more rows than the input): a
-    // lane gets other maps in every pass, and scratch of its own would grow, with a stop to free and to allocate, until it
-    // has had them all.
-    l->order_bytes = blk::order_workspace_bytes(ps->levels[0].n);
-    l->order_ws = ps->take(l->order_bytes);
-    if (!l->order_ws) return ps->arena.error ? ps->arena.error : PCE_ERR_CUDA;
-  }
+  l->order_bytes = 0;
   for (;;) {
     int i;
     {
