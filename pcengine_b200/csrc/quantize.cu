@@ -205,15 +205,18 @@ __global__ void __launch_bounds__(coop::kThreads)
 
 // The same by one bucket per block (sample_sort.cuh): three grid barriers instead of ten for the keys of a scan (29 bits, four
 // radix passes).  What bounds it: the latency of two sorts in shared memory (of the sample, of the bucket) and the barriers.
-// 90 k points of a scan: 49.6 -> 32.9 us.  Returns to the host for the radix sort when a bucket overflows or key and index do not
-// fit a word.  `bounds` is [grid][8], `counters` [grid] (zeroed here), `counts` [grid], `region` [grid][kCap].
+// 90 k points of a scan: 49.6 -> 32.9 us.  Points that share one voxel (returns at the
+// sensor) may fill several buckets: 90 k points, a third in one voxel, 119 -> 77 us a call against buckets that end with a key.
+// Returns to the host for the radix sort when a bucket overflows or key and index do not
+// fit a word.  `bounds` is [grid][8], `counters` [grid] (zeroed here), `counts` [grid], `last` [grid] (a bucket's
+// voxels and its last key), `region` [grid][kCap].
 constexpr int kBucketItems = 2;  // points per thread: chunks of kTarget points
 static_assert(kBucketItems * samp::kThreads == samp::kTarget, "a block reads as many points as a bucket holds on average");
 constexpr int kTryRadix = -1000;
 
 __global__ void __launch_bounds__(samp::kThreads)
     k_voxelise_buckets(const float* __restrict__ pts, int n, double vx, double vy, double vz, int batch, int* bounds, int* counters,
-                       int* counts, unsigned long long* region, VoxelOut out) {
+                       int* counts, unsigned long long* last, unsigned long long* region, VoxelOut out) {
   using namespace samp;
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(samp::kThreads)
     const word_t key = (((static_cast<word_t>(v[0] - mx) << by) | static_cast<word_t>(v[1] - my)) << bz) | static_cast<word_t>(v[2] - mz);
     return key << index_bits | static_cast<word_t>(i);
   };
-  splitters(sh, g, n, index_bits, [&](int i) {
+  splitters(sh, g, n, [&](int i) {
     int v[3];
     cell(i, v);
     return pack(v, i);
@@ -313,8 +316,10 @@ __global__ void __launch_bounds__(samp::kThreads)
     }
   }
   sort_bucket(sh, mine, region + static_cast<size_t>(me) * kCap);
-  // heads of equal keys, rounds of kThreads words: voxels in front of the word's
-  auto head_at = [&](int i) { return i < mine && (i == 0 || sh.words[i] >> index_bits != sh.words[i - 1] >> index_bits); };
+  // heads of equal keys, rounds of kThreads words: voxels in front of the word's.  The first word counts as a head until
+  // the bucket in front is known to end with another voxel.
+  bool opens = true;
+  auto head_at = [&](int i) { return i < mine && (i == 0 ? opens : sh.words[i] >> index_bits != sh.words[i - 1] >> index_bits); };
   int heads = 0;
   for (int i = tid; i < ((mine + 31) & ~31); i += kThreads) heads += __popc(__ballot_sync(0xFFFFFFFFu, head_at(i)));  // (per warp)
   if (lane == 0) s_warp[warp] = heads;
@@ -323,20 +328,43 @@ __global__ void __launch_bounds__(samp::kThreads)
     int total = 0;
     for (int v = 0; v < kWarps; ++v) total += s_warp[v];
     counts[me] = total;
+    last[me] = sh.words[max(mine, 1) - 1] >> index_bits;
   }
   grid.sync();
-  int before = 0, all = 0;
-  for (int b = lane; b < g; b += 32) {
-    const int v = __ldcg(counts + b);
-    all += v;
-    before += b < me ? v : 0;
+  // voxels in front of this bucket, and whether its first word belongs to the last of them
+  if (warp == 0) {
+    int before = 0, all = 0, joined = 0;
+    word_t end[kMaxBuckets / 32];
+    int count[kMaxBuckets / 32];
+#pragma unroll
+    for (int r = 0; r < kMaxBuckets / 32; ++r) {
+      const int b = 32 * r + lane;
+      end[r] = b > 0 && b < g ? __ldcg(last + b - 1) : kLast;
+      count[r] = b < g ? __ldcg(counts + b) : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < kMaxBuckets / 32; ++r) {
+      const int b = 32 * r + lane;
+      const bool joins = end[r] != kLast && end[r] == sh.split[b] >> index_bits;  // (a bucket's first word is its splitter)
+      all += count[r] - (joins ? 1 : 0);
+      before += b < me ? count[r] - (joins ? 1 : 0) : 0;
+      joined |= joins && b == me ? 1 : 0;
+    }
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    all = __reduce_add_sync(0xFFFFFFFFu, all);
+    joined = __any_sync(0xFFFFFFFFu, joined);
+    if (lane == 0) {
+      s_b[0] = before;
+      s_b[1] = joined;
+      if (me == 0) {
+        out.host[0] = PCE_OK;
+        out.host[1] = all;
+      }
+    }
   }
-  before = __reduce_add_sync(0xFFFFFFFFu, before);
-  all = __reduce_add_sync(0xFFFFFFFFu, all);
-  if (me == 0 && tid == 0) {
-    out.host[0] = PCE_OK;
-    out.host[1] = all;
-  }
+  __syncthreads();
+  int before = s_b[0];
+  opens = !s_b[1];
   const word_t index_mask = (1ull << index_bits) - 1ull;
   for (int i0 = 0; i0 < mine; i0 += kThreads) {
     const int i = i0 + tid;
@@ -381,11 +409,12 @@ static int launch_buckets(const float* points, int n, const float* v, int batch,
   int* bounds = ar.take<int>(static_cast<size_t>(g) * 8);
   int* counters = ar.take<int>(g);
   int* counts = ar.take<int>(g);
+  unsigned long long* last = ar.take<unsigned long long>(g);
   unsigned long long* region = ar.take<unsigned long long>(static_cast<size_t>(g) * samp::kCap);
   if (!ar.ok) return PCE_ERR_WORKSPACE;
   double vx = v[0], vy = v[1], vz = v[2];
   VoxelOut o = out;
-  void* args[] = {&points, &n, &vx, &vy, &vz, &batch, &bounds, &counters, &counts, &region, &o};
+  void* args[] = {&points, &n, &vx, &vy, &vz, &batch, &bounds, &counters, &counts, &last, &region, &o};
   PCE_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_voxelise_buckets), dim3(g), dim3(samp::kThreads), args, sizeof(samp::Shared), st));
   PCE_LAUNCH_CHECK();
   return PCE_OK;

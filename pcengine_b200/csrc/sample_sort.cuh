@@ -6,8 +6,10 @@
 // so that no two are equal and a stable order is simply the order of the words.  Every block sorts the same words, taken at
 // equal distances, which gives splitters for one bucket per block; entries go into the buckets' fixed regions of
 // 4 x target words (a position per block and bucket from one atomic), and every block sorts its bucket.  Splitters are
-// cut at the key, so that equal keys share a bucket.  A bucket that overflows (a key that is repeated very often, or a
-// sample that misses the distribution) is seen by every block behind the barrier: the caller then sorts by radix.
+// whole words, so that a key that is repeated very often spreads over as many buckets as its entries need: the caller joins
+// equal keys across the border of two buckets.  (A splitter is itself an entry, the smallest of its bucket: none is empty.)
+// A bucket that overflows (a sample that misses the distribution) is seen by every block behind the barrier: the caller
+// then sorts by radix.
 // (For the row orders, 27-bit keys, the radix sort's three passes are as fast from 120 k entries on: 52 and 48 us for 240 k.)
 #pragma once
 
@@ -28,7 +30,7 @@ constexpr word_t kLast = ~0ull;           // behind every word
 
 struct Shared {
   word_t words[kCap];        // the sample, then the bucket
-  word_t split[kMaxBuckets];  // first key of every bucket (the first unused)
+  word_t split[kMaxBuckets];  // first word of every bucket (of the first: unused)
   int count[kMaxBuckets];
   int start[kMaxBuckets];
 };
@@ -91,14 +93,14 @@ __device__ __forceinline__ void sort_words(word_t* w, int m) {
   __syncthreads();
 }
 
-// Splitters of the buckets; word(i) gives entry i of n, whose index fills the low `index_bits`.
+// Splitters of the buckets; word(i) gives entry i of n (at least kSamples where there are two buckets or more).
 template <typename Word>
-__device__ __forceinline__ void splitters(Shared& sh, int buckets, int n, int index_bits, Word word) {
+__device__ __forceinline__ void splitters(Shared& sh, int buckets, int n, Word word) {
   if (buckets > 1) {
     for (int s = threadIdx.x; s < kSamples; s += kThreads)
       sh.words[s] = word(static_cast<int>((static_cast<long long>(s) * n + n / 2) / kSamples));
     sort_words(sh.words, kSamples);
-    for (int b = threadIdx.x; b < buckets; b += kThreads) sh.split[b] = sh.words[b * kSamples / buckets] >> index_bits << index_bits;
+    for (int b = threadIdx.x; b < buckets; b += kThreads) sh.split[b] = sh.words[b * kSamples / buckets];
   }
   __syncthreads();
 }

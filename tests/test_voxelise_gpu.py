@@ -5,6 +5,8 @@ import numpy as np
 import pytest
 import torch
 
+from tests.helpers import traced
+
 pytestmark = pytest.mark.gpu
 
 
@@ -38,10 +40,11 @@ def test_device_collation_equals_the_host_path(k, width):
     assert a.coords_max == b.coords_max and a.batchsize == k
 
 
-@pytest.mark.parametrize("n,kind", [(4097, "one voxel"), (9000, "two voxels"), (70000, "wide"), (100000, "sorted"), (100000, "lines")])
+@pytest.mark.parametrize("n,kind", [(4097, "one voxel"), (9000, "two voxels"), (70000, "wide"), (100000, "sorted"), (100000, "lines"),
+                                    (151552, "one voxel"), (90000, "a third in one voxel"), (100000, "hundred voxels"), (100000, "misjudged")])
 def test_voxelisation_by_buckets(n, kind):
-    """Clouds that miss the buckets (a voxel of more points than a bucket holds, key and index beyond a word) and clouds in
-    orders that a sample at equal distances could misjudge."""
+    """Voxels of more points than a bucket holds, clouds that miss the buckets (key and index beyond a word, points that no
+    sample stands for) and clouds in orders that a sample at equal distances could misjudge."""
     import pcengine_b200 as pce
     rng = np.random.default_rng(n)
     pts = rng.uniform(-40, 40, (n, 3))
@@ -55,9 +58,19 @@ def test_voxelisation_by_buckets(n, kind):
         pts = pts[np.lexsort(pts.T[::-1])]
     elif kind == "lines":  # every 98th point, the distance of the samples, lies on one line
         pts[n // 2048::n // 1024, :2] = 0.5
+    elif kind == "a third in one voxel":  # (in places all over the cloud)
+        pts[rng.permutation(n)[:n // 3]] = 0.06
+    elif kind == "hundred voxels":
+        pts = rng.uniform(0.01, 0.11, (n, 3)) + 0.125 * rng.integers(0, 100, n)[:, None]
+    elif kind == "misjudged":  # every point that the samples are taken from lies in front of all others
+        pts[:, 0] = 20 + pts[:, 0] / 4
+        pts[(np.arange(1024) * n + n // 2) // 1024, 0] = -30
     pts = pts.astype(np.float32)
     voxel = float(np.float32(0.125))
     want = pce.sparse_quantize(pts, voxel, return_index=True, return_inverse=True)
     got = pce.sparse_quantize(torch.from_numpy(pts).cuda(), voxel, return_index=True, return_inverse=True)
     for a, b in zip(got, want):
         assert np.array_equal(a.cpu().numpy(), b)
+    names = [e["name"] for e in traced(lambda: pce.sparse_quantize(torch.from_numpy(pts).cuda(), voxel))]
+    assert any("k_voxelise_buckets" in name for name in names)
+    assert any("k_voxelise<" in name for name in names) == (kind in ("wide", "misjudged"))
