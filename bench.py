@@ -471,8 +471,8 @@ def indoor_rows(dev, pk, iters: int = 5, warmup: int = 2, both: bool = True):
 def selector_rows(dev, iters: int = 5, warmup: int = 2):
     """``--workload selector``: both dataflows on clouds that span the selector's inputs -- channel width
     (16..256), sparsity (indoor surfaces ~2.7 pairs per row, LiDAR ~3.4, a fully dense block 27) and map
-    size (about 25 k and 200 k rows) -- submanifold 3x3x3, fp16, kernel-only, L2 flushed.  The table
-    ``pcengine_b200.spconv._D1_WINS`` is what this sweep says."""
+    size (about 25 k and 200 k rows) -- submanifold 3x3x3, fp16, kernel-only, L2 flushed.  The fused
+    dataflow wins them all; ``pcengine_b200.spconv._D1_WINS`` holds the wider layers where it does not."""
     import pcengine_b200 as pce
     from pcengine_b200 import functional as PF
     synth = _synth()

@@ -103,15 +103,15 @@ def _with_bias(epilogue: Optional[FusedEpilogue], bias) -> Optional[FusedEpilogu
 
 
 # Measured crossover of the two dataflows on B200 (submanifold 3x3x3, fp16, kernel-only, L2 flushed:
-# `bench.py --workload selector`, summarised in profiles/selector_sweep.md): channel widths 16..256 x
-# {indoor surfaces, LiDAR, fully dense block} x {about 25 k, 200 k rows}.  The fused output-stationary
-# dataflow (D2) is faster by 1.4-19x in 35 of the 36 cells (the explicit one moves 2*(C_in + C_out)*pairs
-# extra elements through HBM).  The entry is the closest cell, wide layers on small, very sparse maps, where D2's
-# per-tile weight staging dominates (256 -> 256 on 25 k rows with 1.2 pairs per row): the explicit dataflow (D1) won it
-# when the table was made (56 us against 82) and is 1.2x behind on the present kernels (54 against 46).  Each entry: D1 when the
-# layer is fp16, both widths >= c_min, the map has at most rows_max output rows and at most ppr_max pairs
-# per row.
-_D1_WINS = (dict(half=True, c_min=256, rows_max=40000, ppr_max=2.0),)
+# `bench.py --workload selector`, summarised with the sweep of wider inputs in profiles/selector_sweep.md): the fused
+# output-stationary dataflow (D2) is faster in every cell of channel widths 16..256 x {indoor surfaces, LiDAR, fully
+# dense block} x {about 25 k, 200 k rows}, by 1.3-7x (the explicit one, D1, moves 2*(C_in + C_out)*pairs extra elements
+# through HBM), and in every cell beyond 256 output channels.  The entry is where it loses: long inputs of small, sparse
+# maps, whose every tile streams the weights of all its offsets (D2 / D1, us: 512->256 66 / 48 on 14 k rows with 1.3 pairs a
+# row, 79 / 79 on 30 k with 2.0, 768->256 111 / 93 there; but 39 / 42 on 8 k rows, 82 / 99 on 40 k with 2.0, 512->192 62 / 71 on
+# 30 k with 1.6, 384->256 57 / 62 on 30 k).  Each entry: D1 when the layer is fp16, its widths and the map's output rows
+# lie in the ranges (both ends included) and the map has at most ppr_max pairs per row.
+_D1_WINS = (dict(half=True, c_in=(512, 1 << 30), c_out=(256, 256), rows=(10000, 30000), ppr_max=2.0),)
 
 
 def _choose_dataflow(tag: str, in_channel: int, out_channel: int, pairs_per_row=None, n_rows: Optional[int] = None,
@@ -123,9 +123,9 @@ def _choose_dataflow(tag: str, in_channel: int, out_channel: int, pairs_per_row=
     if tag != "auto":
         return tag
     for e in _D1_WINS:
-        if (dtype == torch.float16) != e["half"] or min(in_channel, out_channel) < e["c_min"]:
+        if (dtype == torch.float16) != e["half"] or n_rows is None or pairs_per_row is None:
             continue
-        if n_rows is None or n_rows > e["rows_max"] or pairs_per_row is None:
+        if not all(lo <= v <= hi for v, (lo, hi) in ((in_channel, e["c_in"]), (out_channel, e["c_out"]), (n_rows, e["rows"]))):
             continue
         ppr = pairs_per_row() if callable(pairs_per_row) else pairs_per_row
         if ppr <= e["ppr_max"]:

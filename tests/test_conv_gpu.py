@@ -579,18 +579,18 @@ def test_weights_rewritten_through_data_need_invalidate_packed():
 
 
 def test_auto_tag_selects_the_measured_dataflow():
-    """Tag 'auto': a wide fp16 layer on a small, very sparse map runs the explicit dataflow (the one
-    cell of the sweep where it is faster), a dense neighbourhood or a narrow layer the fused one; both
+    """Tag 'auto': an fp16 layer of very wide inputs on a small, sparse map runs the explicit dataflow (the
+    cells of the sweeps where it is faster), a dense neighbourhood or a narrower layer the fused one; both
     give the oracle's features."""
     import pcengine_b200 as pce
     rng = np.random.default_rng(77)
-    lin = rng.choice(80 ** 3, 6000, replace=False)   # ~1% occupancy: hardly any neighbours
-    sparse = np.stack([np.zeros_like(lin), lin // 6400, (lin // 80) % 80, lin % 80], 1).astype(np.int32)
-    dense = surface_cloud(78, 40)
+    lin = rng.choice(110 ** 3, 11000, replace=False)   # ~1% occupancy: hardly any neighbours
+    sparse = np.stack([np.zeros_like(lin), lin // 12100, (lin // 110) % 110, lin % 110], 1).astype(np.int32)
+    dense = surface_cloud(78, 125)[:11000]
     torch.manual_seed(6)
-    for coords, c, want_flow in ((sparse, 256, "D1"), (dense, 256, "D2"), (sparse, 64, "D2")):
+    for coords, c, c_out, want_flow in ((sparse, 512, 256, "D1"), (dense, 512, 256, "D2"), (sparse, 256, 256, "D2"), (sparse, 64, 64, "D2")):
         feats = torch.randn(len(coords), c).half()
-        conv = pce.conv3d(c, c, 3).cuda().half()
+        conv = pce.conv3d(c, c_out, 3).cuda().half()
         x = _tensor(pce, coords, feats, tags=("auto",))
         y = conv(x)
         km = x.kmaps[(conv.kernel_size_code, x.stride, conv.stride_code)]
