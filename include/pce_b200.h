@@ -383,14 +383,12 @@ PCE_API int pce_pack_weights(const void* weights, int32_t kv, int32_t c_in, int3
  * layers with one offset per stage on the kernel with several accumulators per CTA and decoupled
  * row / weight rings (k_conv_umma_mt), 0 (default) on the one-accumulator kernel, which measured
  * faster; tile lists of 512 rows always run on the former; what = 5: 1 makes pce_map_build_d2
- * query odd submanifold maps in the hash table like all others, 0 (default) in the table of blocks; what = 6: no
- * effect any more;
+ * query odd submanifold maps in the hash table like all others, 0 (default) in the table of blocks; what = 6 and
+ * 8: no effect any more;
  * what = 7: 0 never splits tiles between CTAs; 1 (default) as pce_epilogue.split and split_scratch say;
  *           2 only the split of small maps into parts, no shares of stages on mid-size maps.  (Layers of whole or
- *           half 64-channel blocks run with one CTA per SM and are never cut into shares.)  what = 0 and 2, and 7 with
- *           3, keep such layers on the kernel with two or three CTAs per SM.
- * what = 8: 0 stages the last K block of a width that is an odd multiple of 32 channels padded to 64
- *           (1, default: its weights as 32 channels, no padding; same results).
+ *           half 64-channel blocks run with one CTA per SM and are never cut into shares.)  what = 0 and 2
+ *           keep such layers on the kernel with two to four CTAs per SM.
  * what = 9: 0 makes the planner build the neighbour CSR of every map and the tile lists from it; 1 (default)
  *           lets it skip the CSR where only tile lists are used (pce_planned_csr.rowptr == NULL). */
 PCE_API int pce_tune(int32_t what, int32_t value);

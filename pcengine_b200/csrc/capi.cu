@@ -20,7 +20,6 @@ extern int umma_overlap_launches;
 extern int umma_multi_tile;
 extern int kmap_hash_only;
 extern int umma_split_enabled;
-extern int umma_half_blocks;
 extern int plan_short_route;
 int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
 size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv, int sm_count);
@@ -97,13 +96,9 @@ int pce_tune(int32_t what, int32_t value) {
     kmap_hash_only = value ? 1 : 0;
     return PCE_OK;
   }
-  if (what == 6) return PCE_OK;  // (sorted on part of the key once; every bit is sorted on)
+  if (what == 6 || what == 8) return PCE_OK;  // (sorted on part of the key, padded the half blocks once)
   if (what == 7) {
-    umma_split_enabled = value < 0 ? 0 : value;
-    return PCE_OK;
-  }
-  if (what == 8) {
-    umma_half_blocks = value ? 1 : 0;
+    umma_split_enabled = value < 0 ? 0 : (value > 2 ? 1 : value);
     return PCE_OK;
   }
   if (what == 9) {

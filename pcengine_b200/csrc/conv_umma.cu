@@ -144,17 +144,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Whether the phase has completed, without waiting.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // Bounded wait: false when the abort flag is up or the deadline passed.
 template <class Ctl>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, Ctl* ctl, int where = 9, int item = 0) {
@@ -240,16 +229,6 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
   const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
   return (static_cast<uint64_t>(hi) << 32) | lo;
 }
-// The same for operand tiles of KB channels per row: KB = 64 as above; KB = 32 rows of 64 B, 64-byte swizzle
-// (16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)), 8-row groups 512 B apart.
-template <int KB>
-__device__ __forceinline__ uint64_t make_desc_kb(uint32_t smem_addr) {
-  if constexpr (KB == 64) return make_desc(smem_addr);
-  const uint32_t lo = ((smem_addr >> 4) & 0x3FFFu) | (1u << 16);
-  const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
@@ -451,12 +430,8 @@ __device__ __forceinline__ void finish8(float (&v)[8], int row, int c0, int cout
 // of the 64-channel K block, so SLOTS offsets of a tile share one ring stage: every row gathers one
 // neighbour per slot into its part of the 128-byte row, and the producers assemble the stage's weight
 // block from the per-offset images with cp.async (covered by the same barrier as the rows).
-// K blocks are 64 channels.  HALF: the last one of a width that is an odd multiple of 32 is half: its rows are gathered into the
-// first half of the 128-byte operand rows and its weights come from the second image of the packed weights, 32 channels
-// (64 bytes, 64-byte swizzle) per output channel, so that no padding is staged.  Against three 32-channel stages for 96
-// channels it is two stages per offset: 96->96 on 240 k rows 45.8 -> 43.1 us, on 37 k rows 34.6 -> 32.4.  A variant of its
-// own, since the choice between two images per stage costs every width (64->64 on 200 k rows 30.4 -> 32.1 us).
-template <int kStages, int SUB, bool PUSH, int SLOTS, bool HALF = false>
+// K blocks are 64 channels, the last one padded in the weights.
+template <int kStages, int SUB, bool PUSH, int SLOTS>
 __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
     k_conv_umma(const __half* __restrict__ in, const __half* __restrict__ wpacked, Lists ls, Second sec, int n_out, int cin,
                 int cout, __half* __restrict__ out, Epi ep, int tmem_cols, int nacc) {
@@ -641,14 +616,10 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
         const uint32_t a_addr = tiles_addr + s * stage_bytes;
         if (warp == 0 && elect_one()) {
           const uint32_t bbar = smem_u32(&ctl->bfull[s]);
-          const __half* wtail = second ? sec.wtail : ls.wtail;
-          const bool tail = HALF && wtail && kb == nkb - 1;
-          const uint32_t bytes = tail ? static_cast<uint32_t>(cout) * 64u : static_cast<uint32_t>(b_bytes);
-          mbar_arrive_expect_tx(bbar, bytes);
+          mbar_arrive_expect_tx(bbar, static_cast<uint32_t>(b_bytes));
           const __half* wsrc = second ? sec.w2 + static_cast<size_t>(kb) * cout * KB
                                       : wpacked + (static_cast<size_t>(kb) + static_cast<size_t>(kp) * kblocks) * cout * KB;
-          if (tail) wsrc = wtail + (static_cast<size_t>(second ? 0 : kp) * (2 * nkb - 1) + 2 * kb) * cout * 32;
-          bulk_copy_g2s(a_addr + kAStage, wsrc, bytes, bbar);
+          bulk_copy_g2s(a_addr + kAStage, wsrc, static_cast<uint32_t>(b_bytes), bbar);
         }
         if (chunk < min(kCpr, (width - kb * KB) >> 3)) {
           const char* src_kb = src_base + kb * (KB * 2);
@@ -815,8 +786,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
             fence_proxy_async();  // the gathered rows were written through the generic proxy
             tc_fence_after();
             const uint32_t a_addr = tiles_addr + s * stage_bytes;
-            const bool tail = HALF && (second ? sec.wtail && kb == kblocks2 - 1 : ls.wtail && kb == kblocks - 1);
-            const uint64_t db = tail ? make_desc_kb<32>(a_addr + kAStage) : make_desc_kb<KB>(a_addr + kAStage);
+            const uint64_t db = make_desc(a_addr + kAStage);
             // with several offsets per stage the whole 64-channel block is always filled (unused slots with zeros)
             const int ksteps = (SLOTS > 1 && !second) ? 4 : min(KB / 16, ((second ? sec.cin2 : cin) - kb * KB) >> 4);
 #pragma unroll
@@ -824,7 +794,7 @@ __global__ void __launch_bounds__(32 * (4 * SUB + 5), SUB == 1 ? 3 : 2)
               if (k < ksteps) {
 #pragma unroll
                 for (int sub = 0; sub < SUB; ++sub) {  // the same weight block feeds every sub-tile
-                  const uint64_t da = make_desc_kb<KB>(a_addr + sub * (kTileM * kRowBytes));
+                  const uint64_t da = make_desc(a_addr + sub * (kTileM * kRowBytes));
                   tc_mma_f16(tmem_acc + static_cast<uint32_t>(sub * cout), da + static_cast<uint64_t>(k * 2),
                              db + static_cast<uint64_t>(k * 2), idesc, k > 0 ? 1u : accumulate);
                 }
@@ -1726,7 +1696,8 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
     if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(cout >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
       const uint32_t lo0 = (tiles_addr >> 4) | (1u << 16), step = static_cast<uint32_t>(stage_bytes) >> 4;
-      constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29), kHi32 = (512u >> 4) | (1u << 14) | (4u << 29);  // (make_desc_kb)
+      constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29), kHi32 = (512u >> 4) | (1u << 14) | (4u << 29);
+      // (kHi: make_desc; kHi32: half blocks, rows of 64 B, 64-byte swizzle, 8-row groups 512 B apart)
       const int last1 = ((cin - 1) & 63) / 16 + 1, last2 = ((sec.cin2 - 1) & 63) / 16 + 1;  // K steps of the last K block
       const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
       uint32_t par = 0, lo = lo0, at = 0;  // at: 8 x the slot
@@ -1953,52 +1924,49 @@ __global__ void __launch_bounds__(deep_threads(RING), 1)
   if (parts > 1) {
     // the parts' sums, added up through the cluster's shared memory as in k_conv_umma
     const int part = static_cast<int>(blockIdx.x) % parts;
-    const int fit = (RING * stage_bytes / (kTileM * 4)) & ~15;
+    // (the ring holds them all: four stages' weight blocks alone are 512 bytes a column)
+    static_assert(RING >= 4, "room for 128 rows of fp32 sums");
     const int rows_each = kTileM / parts;
     const bool scaled = ep.scale || ep.shift;
-    for (int base = 0; base < cout; base += fit) {
-      const int cols = min(fit, cout - base);
-      __syncthreads();
-      if (warp < 4) {
-        const int r = warp * 32 + lane;
-        const uint32_t taddr = tmem_base + static_cast<uint32_t>(base) + (static_cast<uint32_t>(warp * 32) << 16);
-        for (int c0 = 0; c0 < cols; c0 += 16) {
-          uint32_t v[16];
-          if (part_any) {
-            tmem_ld16(taddr + c0, v);
-            tmem_ld_wait();
-          } else {
+    __syncthreads();
+    if (warp < 4) {
+      const int r = warp * 32 + lane;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+      for (int c0 = 0; c0 < cout; c0 += 16) {
+        uint32_t v[16];
+        if (part_any) {
+          tmem_ld16(taddr + c0, v);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = 0u;
-          }
-          uint4* dst = reinterpret_cast<uint4*>(tiles) + (c0 / 4) * kTileM + r;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) dst[q * kTileM] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          for (int q = 0; q < 16; ++q) v[q] = 0u;
         }
+        uint4* dst = reinterpret_cast<uint4*>(tiles) + (c0 / 4) * kTileM + r;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q * kTileM] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
-      tc_fence_before();
-      cluster_sync();
-      for (int i = tid; i < rows_each * (cols / 8); i += deep_threads(RING)) {
-        const int r = part * rows_each + i % rows_each, c0 = i / rows_each * 8;
-        const int slot = t0 * kTileM + r;
-        if (slot >= n_out) continue;
-        const int row = ls.order ? __ldg(ls.order + slot) : slot;
-        const uint32_t src = tiles_addr + static_cast<uint32_t>((c0 / 4) * kTileM + r) * 16u;
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int p = 0; p < parts; ++p) {
-          const float4 x = cluster_ld4(src, p), y = cluster_ld4(src + kTileM * 16u, p);
-          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-          v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
-        }
-        const int c = base + c0;
-        if (scaled) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v[q] = fmaf(v[q], affine[c + q], affine[cout + c + q]);
-        }
-        finish8(v, row, c, cout, out, ep);
-      }
-      cluster_sync();  // (the other parts have read this CTA's sums)
     }
+    tc_fence_before();
+    cluster_sync();
+    for (int i = tid; i < rows_each * (cout / 8); i += deep_threads(RING)) {
+      const int r = part * rows_each + i % rows_each, c0 = i / rows_each * 8;
+      const int slot = t0 * kTileM + r;
+      if (slot >= n_out) continue;
+      const int row = ls.order ? __ldg(ls.order + slot) : slot;
+      const uint32_t src = tiles_addr + static_cast<uint32_t>((c0 / 4) * kTileM + r) * 16u;
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int p = 0; p < parts; ++p) {
+        const float4 x = cluster_ld4(src, p), y = cluster_ld4(src + kTileM * 16u, p);
+        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+        v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+      }
+      if (scaled) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = fmaf(v[q], affine[c0 + q], affine[cout + c0 + q]);
+      }
+      finish8(v, row, c0, cout, out, ep);
+    }
+    cluster_sync();  // (the other parts have read this CTA's sums)
   }
   __syncthreads();
   if (warp == kDeepMmaWarp) {
@@ -2203,7 +2171,7 @@ static int conv_umma_mt(const __half* in, const __half* w, const umma::Lists& ls
   return PCE_OK;
 }
 
-template <int NS, int SUB, bool PUSH, int SLOTS, bool HALF = false>
+template <int NS, int SUB, bool PUSH, int SLOTS>
 static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in, const __half* w, const umma::Lists& ls,
                         const umma::Second& sec, int n_out, int cin, int cout, __half* out, const umma::Epi& e, int tmem_cols,
                         int nacc) {
@@ -2224,12 +2192,9 @@ static void launch_umma(int grid, size_t smem, cudaStream_t st, const __half* in
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  cudaLaunchKernelEx(&cfg, umma::k_conv_umma<NS, SUB, PUSH, SLOTS, HALF>, in, w, ls, sec, n_out, cin, cout, out, e, tmem_cols,
+  cudaLaunchKernelEx(&cfg, umma::k_conv_umma<NS, SUB, PUSH, SLOTS>, in, w, ls, sec, n_out, cin, cout, out, e, tmem_cols,
                      nacc);
 }
-
-// 1: the last K block of a width that is an odd multiple of 32 (96, 160, 224) stages half the weights; 0: it is padded.
-int umma_half_blocks = 1;
 
 // 1: maps with few tiles are split over several CTAs per tile, mid-size maps into equal shares of stages,
 // when the caller asks for it (see conv_split_parts, conv_streamk_grid); 2: only the former; 0: never.
@@ -2308,17 +2273,15 @@ static int umma_split(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
   const long long sms = sm_count > 0 ? sm_count : 148;
   const long long slots = sms * (cout <= 128 ? 3 : 2);
   // Parts pay while their CTAs are resident at once and each keeps a few stages of a chain that costs 0.6 us a stage; eight
-  // only where they still have about an SM each.  Whole -> split, us (3x3x3, kernel only): 64->64 on 7.5 k rows 18.8 -> 9.6
-  // (4 parts; 2: 12.2), on 25 k rows 18.9 -> 14.3 (2; 4 exceed the slots: 19.6); 128->128 on 2.9 k rows 30.9 -> 12.6 (4; 8:
-  // 12.8), on 12 k rows 23.3 -> 13.7 (4); 256->256 on 7.5 k rows 60.6 -> 27.9 (4; 2: 39.6); 128->256 on 12 k rows 27 -> 22.5
-  // (2), on 23 k rows 38 -> 44 beyond the slots.  Widths with a half block have less work per stage and
-  // gain up to a wave of tiles (96->96 on 37 k rows 37.4 -> 32.8, on 54 k rows 38.5 -> 36.5, two parts).  The rows of a
-  // kernel of at most 8 offsets (down and up a level) have fewer of them than the estimate: twice the chain is asked for.
+  // only where they still have about an SM each.  Whole -> split, us (3x3x3 on rooms, kernel only): 48->64 on 7.5 k rows 16.3 -> 8.5
+  // (4 parts), on 25 k 17.6 -> 13.3 (2); 144->128 on 2.9 k rows 31.0 -> 11.8 (8), on 12 k 29.8 -> 16.0 (4), on 25 k 36.5 -> 25.0 (2);
+  // 240->256 on 2.9 k rows 45.3 -> 19.8 (8), on 7.5 k 49.8 -> 23.1 (4), on 12 k 43.9 -> 31.1 (2); beyond the slots 128->256 on 23 k rows 38 -> 44.
+  // The rows of a kernel of at most 8 offsets (down and up a level) have fewer of them than the estimate: twice the chain is
+  // asked for.
   const int each = kv <= 8 ? 8 : 4;
-  const bool half_blocks = cin_p % 64 == 32;
   if (3 * n_tiles * 8 <= 4 * sms && chain >= each * 8) return 8;
   if (n_tiles * 4 <= slots && chain >= each * 4) return 4;
-  if (n_tiles * 2 <= (half_blocks ? 2 * slots : slots) && chain >= each * 2) return 2;
+  if (n_tiles * 2 <= slots && chain >= each * 2) return 2;
   return 1;
 }
 
@@ -2334,10 +2297,9 @@ int conv_split_parts(int n_rows, int n_src, int cin, int cout, int kv, int sm_co
 // whole: CTAs take equal shares of the STAGES instead of whole tiles (stream-K), wherever the cuts fall, so
 // every CTA slot works for the same time instead of some running a whole chain while others idle.  A tile
 // that two or more CTAs worked on costs fp32 partial sums (written, then read by k_sum_cut_tiles), which is
-// why it pays only for long chains on less than one wave.  Measured on B200 (LiDAR scans, kernel-only, us,
-// whole -> shares): 256->256 on 189 tiles 111 -> 82, on 273 tiles 111 -> 97, 384->256 on 273 tiles 156 -> 114;
-// but 256->256 on 489 tiles (1.65 waves) 119 -> 136, 128->128 on 273 tiles 59 -> 58, and the 2x2x2
-// strided / transposed layers (chains of 8 offsets at most) 35-49 -> 56-65: those run whole.
+// why it pays only for long chains on less than one wave.  Whole -> shares, us (kernel only, both kernels): 240->256 on 196 tiles
+// of a scan 60.8 -> 50.6, on 235 of a room 56.1 -> 41.8; but 256->256 on 489 tiles (1.65 waves) 119 -> 136, 128->128 on 273 tiles 59 -> 58, and the
+// 2x2x2 strided / transposed layers (chains of 8 offsets at most) 35-49 -> 56-65: those run whole.
 // Returns the grid (= the CTA slots) or 0.
 int conv_streamk_grid(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   if (!umma_split_enabled || umma_split_enabled == 2 || n_rows < 1) return 0;
@@ -2347,7 +2309,6 @@ int conv_streamk_grid(int n_rows, int n_src, int cin, int cout, int kv, int sm_c
   const int chain = chain_estimate(n_rows, n_src, cin, kv);
   const long long n_tiles = (static_cast<long long>(n_rows) + umma::kTileM - 1) / umma::kTileM;
   const long long slots = static_cast<long long>(sm_count > 0 ? sm_count : 148) * (cout <= 128 ? 3 : 2);
-  if (umma_split_enabled == 3) return (chain >= 8 && 2 * n_tiles > slots && n_tiles <= 4 * slots) ? static_cast<int>(slots) : 0;
   if (kv <= 8 || chain < 16 || 2 * n_tiles <= slots || n_tiles > slots) return 0;
   return static_cast<int>(slots);
 }
@@ -2363,8 +2324,8 @@ size_t conv_split_scratch_bytes(int n_rows, int n_src, int cin, int cout, int kv
 }
 
 // The same where a split was measured faster; the framework's own callers ask this one.  Equal shares of stages repay
-// their partial sums from chains of three K blocks on (lidar and indoor maps of 180 to 420 tiles, whole -> shares, us:
-// 192->128 48 -> 43, 256->128 60 -> 47, 256->256 72 -> 66; but 64->64 22 -> 27, 128->128 34 -> 41, 128->256 40 -> 57).
+// their partial sums from chains of three K blocks on (whole -> shares, us: 144->128 on 235 tiles 37.9 -> 29.3, 176->192 on 196 39.8 -> 37.2,
+// 240->256 53.6 -> 39.5; but 64->64 22 -> 27, 128->256 40 -> 57).
 size_t conv_split_scratch_wanted(int n_rows, int n_src, int cin, int cout, int kv, int sm_count) {
   if (conv_split_parts(n_rows, n_src, cin, cout, kv, sm_count) > 1) return 0;  // (parts add up in shared memory)
   if (chain_estimate(n_rows, n_src, cin, kv) < 48) return 0;
@@ -2507,15 +2468,6 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
                        ep->extra_c};
   }
   const size_t fixed = sizeof(umma::SharedCtl) + 1024 + 64 + 2 * sizeof(float) * cout;  // (+ staged scale / shift)
-  // the half block at the end of an odd multiple of 32 channels (one offset per stage); a slice of a packed buffer has no
-  // second image behind it
-  const bool half = umma_half_blocks && !kb64_slice && sub == 1 && slots == 1 && !(e.push_slot[0] || e.push_slot[1]) && cin > 32 &&
-                    cin % 64 == 32 && !(tiles && umma_multi_tile);
-  if (half) {
-    ls.wtail = reinterpret_cast<const __half*>(static_cast<const char*>(wpacked) + kb64_image_bytes(kv, cin, cout));
-    if (sec.in2 && sec.cin2 % 64 == 32)
-      sec.wtail = reinterpret_cast<const __half*>(reinterpret_cast<const char*>(sec.w2) + kb64_image_bytes(1, sec.cin2, cout));
-  }
   const size_t stage = static_cast<size_t>(umma::kABytes) * sub + static_cast<size_t>(cout) * 128;
   static int sm_count[64] = {};
   // registers per thread by kernel variant (plain, push, 2 slots, 4 slots) and sub-tile count, in
@@ -2531,9 +2483,6 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));  \
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap)); \
   PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<NS, SB, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap))
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<4, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<3, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-    PCE_CUDA(cudaFuncSetAttribute(umma::k_conv_umma<2, 1, false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
     PCE_SET_SMEM(4, 1);
     PCE_SET_SMEM(3, 1);
     PCE_SET_SMEM(2, 1);
@@ -2566,10 +2515,10 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   }
   // One CTA per SM wherever its producers can take the layer (k_conv_deep); the tuning hooks below are k_conv_umma's.
   const bool pairs = slots == 2;  // 32 input channels: a half block per offset there, two offsets to a stage below
-  const bool deep_half = umma_half_blocks && !kb64_slice && cin % 64 == 32;
+  const bool deep_half = !kb64_slice && cin % 64 == 32;  // (a slice of a packed buffer has no second image behind it)
   const bool packed = pairs && umma_faster(n_out, n_in, cin, cout, kv, sm_count[dev]);
   if (!packed && (slots == 1 ? sub == 1 : pairs) && !(e.push_slot[0] || e.push_slot[1]) && deep_widths(cin) && (cin % 64 == 0 || deep_half) && !off16(in) &&
-      !off16(ls.stage_nbr) && !umma_force_stages && !umma_force_nacc && umma_split_enabled != 3) {
+      !off16(ls.stage_nbr) && !umma_force_stages && !umma_force_nacc) {
     umma::Lists dl = ls;
     umma::Second ds = sec;
     dl.entries = pairs ? 2 : 1;
@@ -2657,9 +2606,7 @@ static int conv_umma_impl(const void* in, int n_in, const void* wpacked, int kv,
   __half* out_h = static_cast<__half*>(out);
 #define PCE_GO(NS, SB)                                                                                              \
   do {                                                                                                              \
-    if (SB == 1 && half)                                                                                              \
-      launch_umma<NS, 1, false, 1, true>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc); \
-    else if (push)                                                                                                         \
+    if (push)                                                                                                         \
       launch_umma<NS, SB, true, 1>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc);  \
     else if (slots == 2)                                                                                              \
       launch_umma<NS, SB, false, 2>(grid, smem, st, in_h, w_h, ls, sec, n_out, cin, cout, out_h, e, tmem_cols, nacc); \
