@@ -403,9 +403,9 @@ PCE_API int pce_device_status(int32_t* status_host, int32_t reset);
 PCE_API int pce_debug_timeout(int32_t* where4);
 
 /* Parts per tile (1, 2, 4 or 8) that pce_conv_fwd uses for a tensor-core layer of n_rows outputs
- * gathered from n_src input rows through 128-row tile lists when pce_epilogue.split is set and none
- * of its matrices is pushed to a neighbour or lies off a 16-byte boundary; 1 = the layer is not
- * split into parts (large maps, short stage chains, up-sampling layers: few pairs per output row).
+ * gathered from n_src input rows through 128-row tile lists (from 16-byte boundaries) when
+ * pce_epilogue.split is set and no rows are pushed to a neighbour; 1 = the layer is not split into
+ * parts (large maps, short stage chains, up-sampling layers: few pairs per output row).
  * Layers whose c_in is a multiple of 32 have 4 parts at most. */
 PCE_API int32_t pce_conv_split_parts(int32_t n_rows, int32_t n_src, int32_t c_in, int32_t c_out, int32_t kv,
                                      int32_t sm_count);
